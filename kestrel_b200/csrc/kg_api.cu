@@ -544,7 +544,8 @@ int kg_relatedness(kg_ctx* c, int64_t num_samples, uint64_t iterations, double m
         st = kg::prepare_cohort(c->cohort, c->cohort.raw.as<uint8_t>(), c->cohort.n_samples,
                                 c->cohort.n_sites, c->cohort.n_sites, true,
                                 c->af_set ? c->af.data() : nullptr, std::isnan(maf) ? -1.0 : maf,
-                                c->stream, err, false, iterations);
+                                c->stream, err, false, iterations,
+                                c->precision == KG_PREC_FP32C && c->cohort.n_multi == 0);   // multi-allelic sites need the lists
         if (!st)
             st = kg::prepare_ml_multi(c->cohort, c->multi_af, std::isnan(maf) ? -1.0 : maf, iterations, c->stream,
                                       err);
@@ -613,7 +614,8 @@ int kg_relatedness_gt(kg_ctx* c, int64_t num_samples, uint64_t iterations, kg_ou
         cudaEventRecord(ev0, c->stream);
         st = kg::prepare_cohort(c->cohort, c->cohort.raw.as<uint8_t>(), c->cohort.n_samples,
                                 c->cohort.n_sites, c->cohort.n_sites, true,
-                                c->af_set ? c->af.data() : nullptr, -1.0, c->stream, err, true);
+                                c->af_set ? c->af.data() : nullptr, -1.0, c->stream, err, true, 100,
+                                c->precision == KG_PREC_FP32C);
         if (!st) st = kg::prepare_multi(c->cohort, c->multi_af, ns, c->stream, err);
         if (st) {
             cudaEventDestroy(ev0);
@@ -806,12 +808,14 @@ int kg_relatedness_batch(kg_ctx* c, kg_cohort* cohorts, int n_cohorts, uint64_t 
             std::string e1;
             int s1 = kg::prepare_cohort(*co, k.codes, k.n_samples, k.n_sites, k.row_stride, false,
                                         k.allele_frequencies, std::isnan(maf) ? -1.0 : maf, c->stream, e1, false,
-                                        iterations);
+                                        iterations, c->precision == KG_PREC_FP32C);
             k.status = s1;
             if (s1) {
                 if (err.empty()) err = e1;
                 continue;
             }
+            if (cudaError_t e = cudaStreamSynchronize(c->stream); e != cudaSuccess)
+                return set_err(c, KG_ECUDA, std::string("prepare: ") + cudaGetErrorString(e));
             co->raw.release();  // packed planes are all the pair kernel needs
             kg::PairJob jb;
             jb.panel = co.get();
@@ -981,6 +985,8 @@ int kg_panel_load(kg_ctx* c, const uint8_t* codes, int64_t n_samples, int64_t n_
         st = kg::prepare_cohort(c->panel, codes, n_samples, n_sites, row_stride, false, af,
                                 std::isnan(maf) ? -1.0 : maf, c->stream, err);
         if (st) return set_err(c, st, err);
+        if (cudaError_t e = cudaStreamSynchronize(c->stream); e != cudaSuccess)   // the workers use other streams
+            return set_err(c, KG_ECUDA, std::string("prepare: ") + cudaGetErrorString(e));
         c->panel.raw.release();
         c->panel_ready = true;
         c->panel_gen++;

@@ -8,6 +8,7 @@
 //   per-pair driver, start points        src/coefficients.rs:77-136
 #include "kg_engine.h"
 #include "kg_allele.cuh"
+#include "kg_node.h"
 
 #include <algorithm>
 #include <cmath>
@@ -69,6 +70,7 @@ size_t Cohort::device_bytes() const {
            site_of.bytes + planes.bytes + cls_q.bytes + cls_part.bytes + mg.bytes + malleles.bytes + maf.bytes +
            mfreq.bytes + mkeep.bytes + mcount.bytes + mpart.bytes + cmulti.bytes + mgT.bytes + ml_keep.bytes +
            ml_nrows.bytes + ml_kidx.bytes + ml_rbase.bytes + ml_remap.bytes + ml_redf.bytes + ml_count.bytes +
+           nd_bins.bytes + nd_t.bytes + nd_place.bytes + nd_dig.bytes + nd_planes.bytes +
            ml_site.bytes + ml_orig.bytes + ml_kremap.bytes + ml_rows.bytes + ml_rows32.bytes + ml_gr.bytes + ml_obs.bytes;
 }
 
@@ -202,7 +204,7 @@ __global__ void compact_kernel(const uint8_t* __restrict__ keep, const int32_t* 
                                const int32_t* __restrict__ bsum, const double* __restrict__ pf,
                                const double* __restrict__ qf, int64_t n, int32_t* __restrict__ site_of,
                                float* __restrict__ p32, double* __restrict__ p64,
-                               double* __restrict__ q64) {
+                               double* __restrict__ q64, unsigned long long* __restrict__ t_min) {
     int64_t v = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (v >= n || !keep[v]) return;
     int64_t k = (int64_t)kidx[v] + bsum[v / SCAN_BLOCK];
@@ -210,6 +212,11 @@ __global__ void compact_kernel(const uint8_t* __restrict__ keep, const int32_t* 
     p64[freq_index(k)] = pf[v];
     q64[k] = qf[v];
     p32[freq_index(k)] = (float)pf[v];
+    // the smallest min(p, 1 - p), as 1 + its bits (0: some p is not within 0..1)
+    if (t_min == nullptr) return;
+    const double t = fmin(pf[v], 1.0 - pf[v]);
+    const unsigned long long key = pf[v] >= 0.0 && pf[v] <= 1.0 ? (unsigned long long)__double_as_longlong(t) + 1ull : 0ull;
+    if (key < *reinterpret_cast<volatile unsigned long long*>(t_min)) atomicMin(t_min, key);
 }
 
 __global__ void pad_kernel(const int32_t* __restrict__ nkept, int64_t cap, float* __restrict__ p32,
@@ -492,7 +499,7 @@ static int grid_for(int64_t n, int threads) { return (int)std::max<int64_t>(1, c
 
 int prepare_cohort(Cohort& c, const uint8_t* codes, int64_t n_samples, int64_t n_sites,
                    int64_t row_stride, bool codes_on_device, const double* af, double maf,
-                   cudaStream_t st, std::string& err, bool cls, uint64_t iterations) {
+                   cudaStream_t st, std::string& err, bool cls, uint64_t iterations, bool nodes) {
     if (n_samples <= 0 || n_sites <= 0 || row_stride < n_sites) {
         err = "n_samples and n_sites must be positive and row_stride >= n_sites";
         return KG_EINVAL;
@@ -504,6 +511,7 @@ int prepare_cohort(Cohort& c, const uint8_t* codes, int64_t n_samples, int64_t n
     c.n_samples = n_samples;
     c.n_sites = n_sites;
     c.n_kept = -1;
+    c.nd_n = 0;
     c.cls = cls;
     c.n_seg_max = ceil_div(n_sites, SEG_SITES);
     c.plane_stride = c.n_seg_max * SEG_WORDS;
@@ -536,7 +544,6 @@ int prepare_cohort(Cohort& c, const uint8_t* codes, int64_t n_samples, int64_t n
     KG_CUDA_TRY((cudaError_t)c.p64.reserve(sizeof(double) * cap));
     KG_CUDA_TRY((cudaError_t)c.q64.reserve(sizeof(double) * cap));
     KG_CUDA_TRY((cudaError_t)c.site_of.reserve(sizeof(int32_t) * n_sites));
-    KG_CUDA_TRY((cudaError_t)c.planes.reserve(sizeof(uint2) * n_samples * c.plane_stride));
     const double* daf = nullptr;
     if (af) {
         KG_CUDA_TRY((cudaError_t)c.af.reserve(sizeof(double) * 2 * n_sites));
@@ -545,7 +552,8 @@ int prepare_cohort(Cohort& c, const uint8_t* codes, int64_t n_samples, int64_t n
         daf = c.af.as<double>();
     }
     if (!(maf >= 0.0)) maf = 1.0 / (2.0 * (double)n_samples);
-    KG_CUDA_TRY(cudaMemsetAsync(c.nkept.p, 0, sizeof(int32_t) * 4, st));
+    KG_CUDA_TRY(cudaMemsetAsync(c.nkept.p, 0, sizeof(int32_t) * 2, st));
+    KG_CUDA_TRY(cudaMemsetAsync(c.nkept.as<int32_t>() + 2, 0xFF, sizeof(int32_t) * 2, st));
     count_kernel<<<grid_for(n_sites, 256), 256, 0, st>>>(draw, n_samples, n_sites, stride,
                                                           c.rc.as<int32_t>(), c.oc.as<int32_t>(),
                                                           c.hc.as<int32_t>(), c.nkept.as<int32_t>());
@@ -560,16 +568,9 @@ int prepare_cohort(Cohort& c, const uint8_t* codes, int64_t n_samples, int64_t n
     compact_kernel<<<grid_for(n_sites, 256), 256, 0, st>>>(
         c.keep.as<uint8_t>(), c.kidx.as<int32_t>(), c.bsum.as<int32_t>(), c.pfull.as<double>(),
         c.qfull.as<double>(), n_sites, c.site_of.as<int32_t>(), c.p32.as<float>(),
-        c.p64.as<double>(), c.q64.as<double>());
+        c.p64.as<double>(), c.q64.as<double>(), reinterpret_cast<unsigned long long*>(c.nkept.as<int32_t>() + 2));
     pad_kernel<<<grid_for(cap, 256), 256, 0, st>>>(c.nkept.as<int32_t>(), cap, c.p32.as<float>(),
                                                     c.p64.as<double>(), c.q64.as<double>());
-    {
-        int64_t work = n_samples * c.plane_stride;
-        int blocks = (int)std::min<int64_t>(ceil_div(work, 8), 148 * 32);
-        pack_kernel<<<blocks, 256, 0, st>>>(draw, n_samples, stride, c.site_of.as<int32_t>(),
-                                            c.nkept.as<int32_t>(), nullptr, c.planes.as<uint2>(),
-                                            c.plane_stride);
-    }
     if (cls) {
         KG_CUDA_TRY((cudaError_t)c.cls_part.reserve(sizeof(double) * GRAM_BLOCKS * 45));
         KG_CUDA_TRY((cudaError_t)c.cls_q.reserve(sizeof(double) * 81));
@@ -591,6 +592,23 @@ int prepare_cohort(Cohort& c, const uint8_t* codes, int64_t n_samples, int64_t n
         err = cls ? "no site with a call for every sample" : "no segregating site left after allele-frequency filtering";
         return KG_ENOSITES;
     }
+    if (nodes) {
+        unsigned long long key;
+        std::memcpy(&key, h + 2, sizeof(key));
+        double t_min = -1.0;
+        if (key > 0) {
+            key -= 1;
+            std::memcpy(&t_min, &key, sizeof(t_min));
+        }
+        const int bins = node_bins(cls, c.n_kept, n_samples, t_min);
+        if (bins > 0) return prepare_nodes(c, draw, stride, bins, t_min, st, err);
+    }
+    KG_CUDA_TRY((cudaError_t)c.planes.reserve(sizeof(uint2) * n_samples * c.plane_stride));
+    const int64_t work = n_samples * c.plane_stride;
+    const int blocks = (int)std::min<int64_t>(ceil_div(work, 8), 148 * 32);
+    pack_kernel<<<blocks, 256, 0, st>>>(draw, n_samples, stride, c.site_of.as<int32_t>(), c.nkept.as<int32_t>(),
+                                        nullptr, c.planes.as<uint2>(), c.plane_stride);
+    KG_CUDA_TRY(cudaGetLastError());
     return KG_OK;
 }
 
@@ -835,10 +853,44 @@ CohortDev make_cohort_dev(const PairJob& jb, uint64_t iterations) {
 
 int64_t list_capacity(const Cohort& panel) { return align4(panel.n_kept) + 32; }
 
+// The counts and times of two runs of one call.
+static void add_stats(kg_run_stats& a, const kg_run_stats& b) {
+    a.gh_passes += b.gh_passes;
+    a.obj_passes += b.obj_passes;
+    a.fp64_passes += b.fp64_passes;
+    a.fp64_pairs += b.fp64_pairs;
+    a.pair_sites += b.pair_sites;
+    a.work_units += b.work_units;
+    a.launches += b.launches;
+    a.flops_fp32 += b.flops_fp32;
+    a.flops_fp64 += b.flops_fp64;
+    for (int k = 0; k < 5; k++) a.shape_sites[k] += b.shape_sites[k];
+    a.nonconverged += b.nonconverged;
+    a.waves += b.waves;
+    a.slots = std::max(a.slots, b.slots);
+    a.admit_ms += b.admit_ms;
+    a.pass_ms += b.pass_ms;
+    a.solve_ms += b.solve_ms;
+    a.pair_kernel_ms += b.pair_kernel_ms;
+}
+
 int run_pairs(const std::vector<PairJob>& jobs, const RunConfig& cfg, Workspace& ws,
               cudaStream_t st, kg_run_stats& stats, std::string& err) {
     std::memset(&stats, 0, sizeof(stats));
     if (jobs.empty()) return KG_OK;
+    // pairs on frequency nodes and pairs on site lists run one after the other
+    std::vector<PairJob> on_nodes, on_lists;
+    for (const PairJob& jb : jobs) (jb.panel->nd_n > 0 ? on_nodes : on_lists).push_back(jb);
+    if (!on_nodes.empty()) {
+        const int r = run_nodes(on_nodes, cfg, ws, st, stats, err);
+        if (on_lists.empty() || (r != KG_OK && r != KG_ENOSITES)) return r;
+        kg_run_stats more;
+        std::string err2;
+        const int r2 = run_pairs(on_lists, cfg, ws, st, more, err2);
+        add_stats(stats, more);
+        if (r2 != KG_OK) err = err2;
+        return r2 != KG_OK ? r2 : r;
+    }
     int dev = 0;
     KG_CUDA_TRY(cudaGetDevice(&dev));
     if (ws.sm_count == 0) KG_CUDA_TRY(cudaDeviceGetAttribute(&ws.sm_count, cudaDevAttrMultiProcessorCount, dev));

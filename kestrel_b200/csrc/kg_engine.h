@@ -104,6 +104,14 @@ struct Cohort {
     DevBuf ml_rows32;          // float [rows][12]: the same rows in FP32, zero-padded to three float4
     DevBuf ml_gr;              // uint8 [n_samples][ml_stride]: reduced genotype, ML_ZERO_ROW or ML_MISSING
     DevBuf ml_obs;             // uint32 [n_samples][ml_stride / 32]: called at the kept site
+    // pairs on frequency nodes (kg_node.cu): nd_n bins (0: this cohort's pairs run on site lists)
+    int nd_n = 0;
+    int64_t nd_mp = 0;         // placed sites, bins padded
+    DevBuf nd_bins;            // int cursors, NodeBin per bin
+    DevBuf nd_t;               // double node frequencies
+    DevBuf nd_place;           // uint32 raw site per place, bit 31: genotypes exchanged
+    DevBuf nd_dig;             // int8 digits of the basis values
+    DevBuf nd_planes;          // uint2 [n_samples][nd_mp / 32]
     size_t device_bytes() const;
 };
 
@@ -111,10 +119,13 @@ struct Cohort {
 // codes_on_device; af may be NULL.  maf < 0 selects 1/(2 n_samples);
 // iterations caps the allele-frequency fit (the estimator's own cap).  With cls
 // the sites are those every sample calls, frequencies are counts over all
-// samples (or af), nothing is filtered by frequency, and Q is computed.
+// samples (or af), nothing is filtered by frequency, and Q is computed.  With
+// nodes the cohort is laid out for pairs on frequency nodes where that pays
+// (node_bins), else for site lists.
 int prepare_cohort(Cohort& c, const uint8_t* codes, int64_t n_samples, int64_t n_sites,
                    int64_t row_stride, bool codes_on_device, const double* af, double maf,
-                   cudaStream_t st, std::string& err, bool cls = false, uint64_t iterations = 100);
+                   cudaStream_t st, std::string& err, bool cls = false, uint64_t iterations = 100,
+                   bool nodes = false);
 
 // After prepare_cohort(..., cls = true): adds the cohort's tri- and
 // tetra-allelic sites (c.mg, c.malleles, c.maf uploaded, c.n_multi set) to the
@@ -205,6 +216,7 @@ struct RunConfig {
 // Reusable device workspace of the pair engine (per-slot lists and partial
 // sums, slot states, pass lists, queue, counters, cohort table).
 class WaveEngine;
+struct NodeEngine;
 
 struct Workspace {
     DevBuf scratch, queue, counters, table;
@@ -212,7 +224,9 @@ struct Workspace {
     DevBuf ml_partial;   // per slot and unit, the sums of the ML path's tri-/tetra-allelic sites
     DevBuf qp;           // per slot the QP's inputs and solution, and the wave's list of QP slots
     PinBuf host;   // per-wave counters read back by the host loop
+    DevBuf node_counts, node_table;   // kg_node.cu: counters; cohort, node and chunk tables
     int sm_count = 0;
+    std::shared_ptr<NodeEngine> nodes;
     // run_pairs' engine, kept between calls: a call of the same shape only
     // resets its state and reuses its instantiated graphs (declared last, so
     // it goes before the buffers its graphs point into)

@@ -38,7 +38,7 @@ __global__ void freq_kernel(const int32_t*, const int32_t*, const int32_t*, cons
 __global__ void scan_block_kernel(const uint8_t*, int64_t, int32_t*, int32_t*);
 __global__ void scan_sums_kernel(int32_t*, int64_t, int32_t*);
 __global__ void compact_kernel(const uint8_t*, const int32_t*, const int32_t*, const double*,
-                               const double*, int64_t, int32_t*, float*, double*, double*);
+                               const double*, int64_t, int32_t*, float*, double*, double*, unsigned long long*);
 __global__ void pad_kernel(const int32_t*, int64_t, float*, double*, double*);
 __global__ void pack_kernel(const uint8_t*, int64_t, int64_t, const int32_t*, const int32_t*,
                             const uint8_t*, uint2*, int64_t);
@@ -180,7 +180,7 @@ extern "C" int kg_relatedness_noalloc(const uint8_t* d_codes, int64_t n_samples,
                                          n_samples);
     kg::scan_block_kernel<<<(int)nb, 1024, 0, s>>>(keep, n_sites, kidx, bsum);
     kg::scan_sums_kernel<<<1, 1024, 0, s>>>(bsum, nb, nkept);
-    kg::compact_kernel<<<g256, 256, 0, s>>>(keep, kidx, bsum, pfull, qfull, n_sites, site_of, p32, p64, q64);
+    kg::compact_kernel<<<g256, 256, 0, s>>>(keep, kidx, bsum, pfull, qfull, n_sites, site_of, p32, p64, q64, nullptr);
     kg::pad_kernel<<<(int)((cap + 255) / 256), 256, 0, s>>>(nkept, cap, p32, p64, q64);
     kg::pack_kernel<<<256, 256, 0, s>>>(d_codes, n_samples, row_stride, site_of, nkept, nullptr, planes,
                                         plane_stride);

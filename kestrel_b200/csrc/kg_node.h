@@ -1,0 +1,55 @@
+// kg_node.h — pairs estimated from frequency nodes instead of site lists
+// (host-side interface of kg_node.cu).
+//
+// Every sum an SQP pass forms over a pair's sites (src/jacquard/objective.rs:
+// 9-20, grad_hess.rs:13-41) is, within one genotype-pair shape, a sum of a
+// smooth function phi of the site's allele frequency t.  phi is one of log d, r
+// t^k, r^2 t^k with d = eps + L.Delta, Delta on the simplex, whose
+// singularities keep a distance from t that grows with min(t, 1 - t).  So the
+// cohort's sites go into narrow frequency bins, in each bin phi is replaced by its
+// interpolant through a few Chebyshev nodes, and
+//   sum over the pair's sites of phi(t_s) = sum over nodes of W_node phi(t_node),
+//   W_node = sum over those sites of l_node(t_s)  (l: the Lagrange basis).
+// The weights W do not depend on Delta: they are formed once per pair, and every
+// pass then evaluates 9 x (nodes per bin) x (bins) points instead of all sites.
+// W of all pairs is a matrix product of genotype indicators with indicators
+// times l, which kg_node.cu runs on the tensor cores in exact integers.
+#pragma once
+
+#include <cuda_runtime.h>
+
+#include <cstdint>
+#include <string>
+#include <vector>
+
+#include "kg_engine.h"
+
+namespace kg {
+
+// Nodes per bin, signed 8-bit digits of l's fixed-point value (2^-30), and the
+// largest ratio of a bin's ends.  The interpolation error of the gradient
+// terms is then below 1.3e-9 of a term anywhere on the simplex (1e-11 over a
+// pair's sum), under the 6e-8 of a FP32 site term.  The FP64 form keeps its site
+// lists: with 12 nodes and 5 digits it ran 2.4 times as fast and 1e-13
+// accurate, but within 1e-9 of the list form's rows only where no pair's last
+// line search hangs on an ulp of the objective.
+constexpr int NODE_J = 8, NODE_L = 4;
+constexpr double NODE_RATIO = 1.189207115002721;   // 2^(1/4)
+constexpr int NODE_MAX_BINS = 64;
+constexpr int NODE_UNITS = 9;        // genotype pairs (gx, gy)
+constexpr int NODE_STAGE = 128;      // sites per tile of the product; a bin's sites are padded to it
+
+// Whether a prepared cohort's pairs run on nodes, given its kept sites and
+// their smallest min(p, 1 - p), and the bins that takes (0: it does not).
+int node_bins(bool cls, int64_t n_kept, int64_t n_samples, double t_min);
+
+// After the kept sites are compacted: bins, node points, digits and the
+// samples' planes in bin order (c.nd_*).  codes: device byte codes.
+int prepare_nodes(Cohort& c, const uint8_t* codes, int64_t stride, int bins, double t_min, cudaStream_t st,
+                  std::string& err);
+
+// All jobs (triangles over node-prepared cohorts) of one call.
+int run_nodes(const std::vector<PairJob>& jobs, const RunConfig& cfg, Workspace& ws, cudaStream_t st,
+              kg_run_stats& stats, std::string& err);
+
+}  // namespace kg

@@ -1,0 +1,95 @@
+"""Pairs on frequency nodes (kg_node.cu) against the oracle, at the sizes where
+the tiles can go wrong: one sample, sample counts around the 128-row tile, site
+counts around the padded bins, a narrow and a wide range of frequencies, a
+chunk boundary inside a row, a pair without a common site.
+
+The objective's bar: the interpolation error of log d is below 2e-11 of a
+site's term (FP32C's eight nodes a bin) and the fixed-point weights add less than
+2^-30, averaged over the pair's sites, on an objective of order 1, and the two
+sides stop within a KKT residual of 1e-8 of the same optimum, where the
+objective differs by its square: 1e-9 relative holds with a margin.  Delta and
+kinship keep the shared bar."""
+import numpy as np
+import pytest
+
+import kestrel_b200 as kb
+from kestrel_b200 import synth
+
+from .parity import compare
+
+pytestmark = pytest.mark.gpu
+
+OBJ = 1e-9
+
+
+def cohort(n, m, seed, missing=0.02):
+    return synth.make_cohort(n, m, seed, missing=missing).codes
+
+
+def check(est, codes, ref, **kw):
+    est.load(codes, kw.pop("af", None))
+    rows = est.relatedness(**kw)
+    st = est.run_stats()
+    assert st["fp64_passes"] == st["gh_passes"] > 0, "the cohort should run on nodes"
+    print(compare(rows, ref))
+    assert (np.abs(rows["obj"] - ref["obj"]) / np.abs(ref["obj"])).max() <= OBJ
+    return rows
+
+
+@pytest.mark.parametrize("n,m", [(1, 16_000), (2, 15_500), (31, 16_385), (129, 16_001)])
+def test_sizes(oracle, n, m):
+    codes = cohort(n, m, 700 + n)
+    with kb.Estimator() as est:
+        check(est, codes, oracle.relatedness(codes))
+
+
+@pytest.mark.parametrize("spread", ["half", "wide", "edges"])
+def test_frequencies(oracle, spread):
+    n, m = 12, 40_000
+    rng = np.random.default_rng(5)
+    p = {"half": np.full(m, 0.5),
+         "wide": np.exp(rng.uniform(np.log(2e-4), np.log(0.5), m)),
+         "edges": 0.5 * 2.0 ** (-0.25 * rng.integers(0, 14, m))}[spread]   # on the bins' ends
+    p = np.where(rng.random(m) < 0.5, p, 1.0 - p)
+    codes = synth.apply_missing(rng, synth.hwe_genotypes(rng, p, n), 0.05)
+    af = np.stack([p, 1.0 - p], 1)
+    with kb.Estimator() as est:
+        check(est, codes, oracle.relatedness(codes, af=af), af=af)
+
+
+def test_chunks_leave_the_rows_unchanged(oracle):
+    codes = cohort(140, 20_000, 9)
+    with kb.Estimator() as est:
+        whole = check(est, codes, oracle.relatedness(codes, num_samples=133), num_samples=133)
+        est.set_launch(1000)       # chunks that end inside a sample's pairs
+        parts = check(est, codes, whole, num_samples=133)
+        assert est.run_stats()["slots"] == 1000
+        est.set_launch(0)
+        batch = est.relatedness_batch([(codes, None, 133), (cohort(20, 3000, 10), None, None), (codes, None, 7)])
+    assert np.array_equal(whole.view(np.uint8), parts.view(np.uint8))
+    assert np.array_equal(whole.view(np.uint8), batch[0].view(np.uint8))
+    compare(batch[1], oracle.relatedness(cohort(20, 3000, 10)))
+
+
+def test_pair_without_a_common_site(oracle):
+    codes = cohort(5, 24_000, 11)
+    codes[1, :12_000] = 3
+    codes[3, 12_000:] = 3
+    with kb.Estimator() as est:
+        est.load(codes)
+        rows = est.relatedness(allow_nosites=True)
+        st = est.run_stats()
+    assert st["fp64_passes"] == st["gh_passes"] > 0
+    lone = (rows["x"] == 1) & (rows["y"] == 3)
+    assert np.isnan(rows["obj"][lone]).all() and np.isnan(rows["jacquard"][lone]).all()
+    assert np.isfinite(rows["obj"][~lone]).all()
+
+
+@pytest.mark.parametrize("n,m", [(1, 200), (3, 129), (130, 4097)])
+def test_cls_sizes(oracle, n, m):
+    codes = synth.make_cohort(n, m, 800 + n, missing=0.0).codes
+    ref = oracle.cls_relatedness(codes)
+    with kb.Estimator() as est:
+        est.load(codes)
+        rows = est.relatedness_gt()
+    compare(rows, ref)
