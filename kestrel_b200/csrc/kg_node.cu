@@ -831,7 +831,7 @@ struct NodeEngine {
         const WaveArgs& A = args[par];
         node_pass_kernel<<<pass_blocks, 128, 0, st>>>(A);
         wave_solve_kernel<<<solve_blocks, 128, WAVE_WPB * WARP_SMEM, st>>>(A);
-        wave_qp_kernel<<<qp_blocks, 128, 0, st>>>(A);
+        wave_qp_kernel<<<qp_blocks, QP_THREADS, 0, st>>>(A);
         wave_step_kernel<<<step_blocks, 128, 0, st>>>(A);
     }
 };
@@ -933,7 +933,7 @@ int run_nodes(const std::vector<PairJob>& jobs, const RunConfig& cfg, Workspace&
         E.pass_blocks = ws.sm_count * std::max(1, occ);
         KG_NODE_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, wave_solve_kernel, 128, WAVE_WPB * WARP_SMEM));
         E.solve_blocks = ws.sm_count * std::max(1, occ);
-        KG_NODE_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, wave_qp_kernel, 128, 0));
+        KG_NODE_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, wave_qp_kernel, QP_THREADS, 0));
         E.qp_blocks = ws.sm_count * std::max(1, occ);
         KG_NODE_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, wave_step_kernel, 128, 0));
         E.step_blocks = ws.sm_count * std::max(1, occ);

@@ -7,168 +7,181 @@
 //
 // It computes what the row-parallel form (qp_simplex_rows in kg_rowsolve.cuh)
 // computes, operation for operation and in the same order (the same FMAs,
-// divisions and sequential sums), so both give the same bits; with a thread
-// per slot a warp serves 32 pairs' QPs instead of two.  Q is read where it
-// lies (the slot's QP buffer, through L1); L and the vectors are fixed-size
-// arrays indexed by loop counters that unroll, so they stay in registers or
-// the thread's local memory.
+// quotients and sequential sums), so both give the same bits; with a thread
+// per slot a warp serves 32 pairs' QPs instead of two.
+//
+// The lanes' free sets differ, so the code has no branch on them: a fixed
+// variable's rows and columns are zeros and its pivot 1, which adds exact
+// zeros to every sum (branches on the free set ran each of its cases one after
+// the other: 4,300 instructions an iteration, this form about 1,300).  A
+// quotient by one divisor used several times (a pivot, the sum of y) is q = c r
+// with r = 1 / d, corrected by the remainder: with r correctly rounded that is
+// the correctly rounded quotient (Markstein, IBM J. Res. Dev. 34, 1990), in
+// three instructions instead of a division.
 #pragma once
 
 #include "kg_solver.cuh"
 
 namespace kg {
 
-// GMW81-modified LDL^T of the free block (mask F, nf free) of the 9 x 9 Q,
-// which it reads inside that block only; L unit lower triangular with
-// identity rows and columns for the fixed variables, d their diagonal 1.
-__device__ __forceinline__ void ldl_gmw_thread(const double (*Q)[9], unsigned F, int nf, double (&L)[9][9],
-                                               double (&d)[9]) {
+__host__ __device__ __forceinline__ int popc9(unsigned v) {
+    int n = 0;
+#pragma unroll
+    for (int i = 0; i < 9; i++) n += (v >> i) & 1u;
+    return n;
+}
+
+// c / d, given r = 1 / d correctly rounded.
+__host__ __device__ __forceinline__ double quot(double c, double d, double r) {
+    const double q = c * r;
+    return fma(fma(-q, d, c), r, q);
+}
+
+// Entry (i, j), i <= j, of the stored upper triangle of Q.
+__host__ __device__ constexpr int upper_at(int i, int j) { return i * 9 - i * (i - 1) / 2 + (j - i); }
+constexpr int QP_Q = 45;   // upper triangle of Q, then c
+constexpr int QP_IN = 54;
+
+// GMW81-modified LDL^T of the free block (mask F, nf free): L strictly lower
+// (row i at i (i - 1) / 2), d the pivots, rd their reciprocals; fixed variables
+// have zero rows and columns and pivot 1.  Q(i, j) reads the upper triangle.
+template <class QF>
+__host__ __device__ __forceinline__ void ldl_gmw_thread(const QF& Q, unsigned F, int nf, double (&L)[36],
+                                                        double (&d)[9], double (&rd)[9]) {
     double gamma = 0.0, xi = 0.0;
 #pragma unroll
     for (int r = 0; r < 9; r++) {
-        if (!((F >> r) & 1u)) continue;
-        double diag = fabs(Q[r][r]);
-        if (!(diag >= 0.0)) diag = 0.0;
-        gamma = fmax(gamma, diag);
-        double off = 0.0;
+        const bool rf = (F >> r) & 1u;
+        gamma = fmax(gamma, rf ? fabs(Q(r, r)) : 0.0);
 #pragma unroll
-        for (int j = r + 1; j < 9; j++)
-            if ((F >> j) & 1u) off = fmax(off, fabs(Q[r][j]));
-        if (!(off >= 0.0)) off = 0.0;
-        xi = fmax(xi, off);
+        for (int j = r + 1; j < 9; j++) xi = fmax(xi, rf && ((F >> j) & 1u) ? fabs(Q(r, j)) : 0.0);
     }
     const double eps = 2.220446049250313e-16;
     const double delta = eps * fmax(1.0, gamma + xi);
     const double t = sqrt((double)nf * (double)nf - 1.0);
     const double ratio = (nf <= 1) ? 0.0 : xi / t;
     const double beta2 = fmax(fmax(gamma, ratio), eps);
-#pragma unroll
-    for (int i = 0; i < 9; i++) {
-        d[i] = 0.0;
-#pragma unroll
-        for (int j = 0; j < 9; j++) L[i][j] = 0.0;
-    }
+    const double rbeta2 = 1.0 / beta2;
 #pragma unroll
     for (int j = 0; j < 9; j++) {
-        if (!((F >> j) & 1u)) {
-            d[j] = 1.0;
-            L[j][j] = 1.0;
-            continue;
-        }
+        const bool jf = (F >> j) & 1u;
         double p[9];
         double sjj = 0.0;
 #pragma unroll
         for (int s = 0; s < j; s++) {
-            p[s] = d[s] * L[j][s];
-            sjj = fma(p[s], L[j][s], sjj);
+            const double ljs = L[j * (j - 1) / 2 + s];
+            p[s] = d[s] * ljs;
+            sjj = fma(p[s], ljs, sjj);
         }
-        const double cjj = Q[j][j] - sjj;
-        double c[9];
+        const double cjj = Q(j, j) - sjj;
         double theta = 0.0;
 #pragma unroll
         for (int i = j + 1; i < 9; i++) {
-            if (!((F >> i) & 1u)) continue;
             double sij = 0.0;
 #pragma unroll
-            for (int s = 0; s < j; s++) sij = fma(p[s], L[i][s], sij);
-            c[i] = Q[i][j] - sij;
-            double a = fabs(c[i]);
-            if (!(a >= 0.0)) a = 0.0;
-            theta = fmax(theta, a);
+            for (int s = 0; s < j; s++) sij = fma(p[s], L[i * (i - 1) / 2 + s], sij);
+            const double cij = jf && ((F >> i) & 1u) ? Q(j, i) - sij : 0.0;
+            L[i * (i - 1) / 2 + j] = cij;
+            theta = fmax(theta, fabs(cij));
         }
-        const double dj = fmax(fmax(fabs(cjj), theta * theta / beta2), delta);
+        const double dj = fmax(fmax(fabs(cjj), quot(theta * theta, beta2, rbeta2)), delta);
+        d[j] = jf ? dj : 1.0;
+        rd[j] = 1.0 / d[j];
 #pragma unroll
-        for (int i = j + 1; i < 9; i++)
-            if ((F >> i) & 1u) L[i][j] = c[i] / dj;
-        L[j][j] = 1.0;
-        d[j] = dj;
+        for (int i = j + 1; i < 9; i++) {
+            double& l = L[i * (i - 1) / 2 + j];
+            l = quot(l, d[j], rd[j]);
+        }
     }
 }
 
-// L D L^T z = b for two right-hand sides, in the order of ldl_solve2_rows.
-__device__ __forceinline__ void ldl_solve2_thread(const double (&L)[9][9], const double (&d)[9], double (&b0)[9],
-                                                  double (&b1)[9]) {
-    double f0[9], f1[9];
+// L D L^T z = b for two right-hand sides (zero at fixed variables), in the
+// order of ldl_solve2_rows.
+__host__ __device__ __forceinline__ void ldl_solve2_thread(const double (&L)[36], const double (&d)[9],
+                                                           const double (&rd)[9], double (&b0)[9], double (&b1)[9]) {
 #pragma unroll
     for (int i = 0; i < 9; i++) {
         double s0 = 0.0, s1 = 0.0;
 #pragma unroll
         for (int j = 0; j < i; j++) {
-            s0 = fma(f0[j], L[i][j], s0);
-            s1 = fma(f1[j], L[i][j], s1);
+            s0 = fma(b0[j], L[i * (i - 1) / 2 + j], s0);
+            s1 = fma(b1[j], L[i * (i - 1) / 2 + j], s1);
         }
-        f0[i] = b0[i] - s0;
-        f1[i] = b1[i] - s1;
+        b0[i] = b0[i] - s0;
+        b1[i] = b1[i] - s1;
     }
 #pragma unroll
     for (int i = 0; i < 9; i++) {
-        f0[i] = f0[i] / d[i];
-        f1[i] = f1[i] / d[i];
+        b0[i] = quot(b0[i], d[i], rd[i]);
+        b1[i] = quot(b1[i], d[i], rd[i]);
     }
 #pragma unroll
     for (int i = 8; i >= 0; i--) {
         double t0 = 0.0, t1 = 0.0;
 #pragma unroll
         for (int j = i + 1; j < 9; j++) {
-            t0 = fma(b0[j], L[j][i], t0);
-            t1 = fma(b1[j], L[j][i], t1);
+            t0 = fma(b0[j], L[j * (j - 1) / 2 + i], t0);
+            t1 = fma(b1[j], L[j * (j - 1) / 2 + i], t1);
         }
-        b0[i] = f0[i] - t0;
-        b1[i] = f1[i] - t1;
+        b0[i] = b0[i] - t0;
+        b1[i] = b1[i] - t1;
     }
 }
 
-// The QP from y0 (y0 and y may alias).  Returns the iteration count.
-__device__ inline int qp_simplex_thread(const double (*Q)[9], const double (&c)[9], const double* y0,
-                                        const Tune& tu, double* y) {
+// The QP from y (in) to y (out); in(k): the upper triangle of Q (row-major,
+// k < 45), then c.  Returns the iteration count.
+template <class In>
+__host__ __device__ __forceinline__ int qp_simplex_thread(const In& in, const Tune& tu, double (&y)[9]) {
+    auto Q = [&](int i, int j) { return in(i <= j ? upper_at(i, j) : upper_at(j, i)); };
     unsigned work = 0;
 #pragma unroll
-    for (int i = 0; i < 9; i++) {
-        y[i] = y0[i];
+    for (int i = 0; i < 9; i++)
         if (y[i] == 0.0) work |= 1u << i;
-    }
     for (int it = 0; it < tu.qp_max_iter; it++) {
-        normalise9(y);
-        const unsigned F = (~work) & 0x1FFu;
-        const int nf = __popc(F);
-        if (nf == 0) return it;
-        // the free block's gradient c_f + Q_f y_f and the ones vector (the
-        // factorisation below reads Q inside the free block only)
-        double gf[9], on[9];
-#pragma unroll
-        for (int r = 0; r < 9; r++) {
-            const bool rf = (F >> r) & 1u;
+        {
             double s = 0.0;
 #pragma unroll
-            for (int j = 0; j < 9; j++)
-                if (rf && ((F >> j) & 1u)) s = fma(Q[r][j], y[j], s);
-            gf[r] = rf ? c[r] + s : 0.0;
+            for (int i = 0; i < 9; i++) s += y[i];
+            const double rs = 1.0 / s;
+#pragma unroll
+            for (int i = 0; i < 9; i++) y[i] = quot(y[i], s, rs);
+        }
+        const unsigned F = (~work) & 0x1FFu;
+        const int nf = popc9(F);
+        if (nf == 0) return it;
+        // the gradient c + Q y (fixed variables' y are 0) and, on the free
+        // block, the ones vector
+        double gq[9], gf[9], on[9];
+#pragma unroll
+        for (int r = 0; r < 9; r++) {
+            double s = 0.0;
+#pragma unroll
+            for (int j = 0; j < 9; j++) s = fma(Q(r, j), y[j], s);
+            gq[r] = in(QP_Q + r) + s;
+            const bool rf = (F >> r) & 1u;
+            gf[r] = rf ? gq[r] : 0.0;
             on[r] = rf ? 1.0 : 0.0;
         }
-        double L[9][9], d[9];
-        ldl_gmw_thread(Q, F, nf, L, d);
-        ldl_solve2_thread(L, d, gf, on);
+        {
+            double L[36], d[9], rd[9];
+            ldl_gmw_thread(Q, F, nf, L, d, rd);
+            ldl_solve2_thread(L, d, rd, gf, on);
+        }
         double sg = 0.0, so = 0.0;
 #pragma unroll
-        for (int i = 0; i < 9; i++)
-            if ((F >> i) & 1u) { sg += gf[i]; so += on[i]; }
+        for (int i = 0; i < 9; i++) { sg += gf[i]; so += on[i]; }
         const double lambda = sg / so;
-        double g2[9];
         double m = 0.0;
         bool m_nan = false;
 #pragma unroll
         for (int i = 0; i < 9; i++) {
-            g2[i] = lambda * on[i] - gf[i];
-            const double a = fabs(g2[i]);
-            if (isnan(a)) m_nan = true;
-            else m = fmax(m, a);
+            gf[i] = lambda * on[i] - gf[i];
+            const double a = fabs(gf[i]);
+            m_nan = m_nan || isnan(a);
+            m = fmax(m, a);
         }
         if (!m_nan && m <= tu.qp_zero_search_tol) {
             if (nf == 9) return it;
-            // the full gradient c + Q y
-            double gq[9];
-#pragma unroll
-            for (int r = 0; r < 9; r++) gq[r] = c[r] + dot_fma(9, Q[r], y);
             int best = -1;
             double gb = 0.0;
 #pragma unroll
@@ -177,26 +190,21 @@ __device__ inline int qp_simplex_thread(const double (*Q)[9], const double (&c)[
             if (gb - lambda >= -tu.qp_conv_tol) return it;
             work &= ~(1u << best);
         } else {
-            double pv[9];
-#pragma unroll
-            for (int i = 0; i < 9; i++) pv[i] = ((work >> i) & 1u) ? 0.0 : g2[i];
             double alpha = 1.0;
             int block = -1;
 #pragma unroll
             for (int i = 0; i < 9; i++) {
-                if (pv[i] < 0.0) {
-                    const double a = -y[i] / pv[i];
-                    if (a < alpha) { alpha = a; block = i; }
-                }
+                const double pv = ((work >> i) & 1u) ? 0.0 : gf[i];
+                gf[i] = pv;
+                const double a = -y[i] / (pv < 0.0 ? pv : -1.0);
+                if (pv < 0.0 && a < alpha) { alpha = a; block = i; }
             }
 #pragma unroll
-            for (int i = 0; i < 9; i++) y[i] = fmax(y[i] + alpha * pv[i], 0.0);
-            if (block >= 0) {
-                work |= 1u << block;
-#pragma unroll
-                for (int i = 0; i < 9; i++)
-                    if (i == block) y[i] = 0.0;
+            for (int i = 0; i < 9; i++) {
+                y[i] = fmax(y[i] + alpha * gf[i], 0.0);
+                if (i == block) y[i] = 0.0;
             }
+            if (block >= 0) work |= 1u << block;
         }
     }
     return tu.qp_max_iter;

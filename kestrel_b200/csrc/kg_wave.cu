@@ -1319,13 +1319,21 @@ __device__ __forceinline__ void solve_slot(const WaveArgs& A, int i, int lane, c
     // inputs go to the slot's QP buffer and the slot to this wave's QP list:
     // wave_qp_kernel solves them a thread per slot, wave_step_kernel takes the
     // step from the solution.
-    double* Qb = A.qp_buf + (int64_t)s * QP_VALS;
-    if (lane < 9) {
-#pragma unroll
-        for (int k = 0; k < 9; k++) Qb[lane * 9 + k] = Hr[k];
-        Qb[81 + lane] = pick9(g, lane) - dot_fma(9, Hr, x);
+    int at = 0;
+    if (lane == 0) {
+        at = atomicAdd(&A.wc_cur->n_qp, 1);
+        A.qp_list[at] = s;
     }
-    if (lane == 0) A.qp_list[atomicAdd(&A.wc_cur->n_qp, 1)] = s;
+    at = __shfl_sync(grp.mask, at, 0, 16);
+    if (lane < 9) {
+        double* Qb = A.qp_buf + at;
+        const int64_t st = A.n_slots;
+#pragma unroll
+        for (int k = 0; k < 9; k++)
+            if (k >= lane) Qb[(lane * 9 - lane * (lane - 1) / 2 + (k - lane)) * st] = Hr[k];
+        Qb[(QP_Q + lane) * st] = pick9(g, lane) - dot_fma(9, Hr, x);
+        Qb[(QP_IN + lane) * st] = pick9(x, lane);
+    }
 }
 
 // Two slots per warp, one per half-warp (the row-parallel solver needs nine
@@ -1349,26 +1357,27 @@ extern "C" __global__ void __launch_bounds__(128, 4) wave_solve_kernel(WaveArgs 
 }
 
 // The QP of every slot in this wave's QP list, a thread per slot (kg_qp1.cuh,
-// the same arithmetic as the row-parallel form); the solution replaces c's
-// neighbour in the slot's QP buffer.  Three blocks per SM (168 registers, a
-// few spilled) beat two without spills: the kernel is bound by its FP64
-// dependency chains, so warps count more than registers.
-extern "C" __global__ void __launch_bounds__(128, 3) wave_qp_kernel(WaveArgs A) {
+// the same arithmetic as the row-parallel form).  The list's QPs lie
+// value-major in memory, so a warp's loads are whole sectors; Q and c stay in
+// shared memory (432 bytes a thread, no bank conflicts), L and the vectors in
+// registers.
+extern "C" __global__ void __launch_bounds__(QP_THREADS) wave_qp_kernel(WaveArgs A) {
+    __shared__ double in[QP_IN * QP_THREADS];
     if (A.clk->stop) return;   // a device loop past its last wave
     const PhaseEnd pe{&A.clk->end[2], (threadIdx.x & 31) == 0};   // timed as part of the solve phase
     const int n = A.wc_cur->n_qp;
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        const int s = A.qp_list[i];
-        double* Qb = A.qp_buf + (int64_t)s * QP_VALS;
-        double c[9], x[9], y[9];
+    const int64_t st = A.n_slots;
+    double* my = in + threadIdx.x;
+    for (int i = blockIdx.x * QP_THREADS + threadIdx.x; i < n; i += gridDim.x * QP_THREADS) {
+        double* Qb = A.qp_buf + i;
 #pragma unroll
-        for (int r = 0; r < 9; r++) {
-            c[r] = Qb[81 + r];
-            x[r] = A.slots[s].xc[r];
-        }
-        qp_simplex_thread(reinterpret_cast<const double (*)[9]>(Qb), c, x, A.tune, y);
+        for (int v = 0; v < QP_IN; v++) my[v * QP_THREADS] = Qb[v * st];
+        double y[9];
 #pragma unroll
-        for (int k = 0; k < 9; k++) Qb[90 + k] = y[k];
+        for (int k = 0; k < 9; k++) y[k] = Qb[(QP_IN + k) * st];
+        qp_simplex_thread([my](int v) { return my[v * QP_THREADS]; }, A.tune, y);
+#pragma unroll
+        for (int k = 0; k < 9; k++) Qb[(QP_IN + k) * st] = y[k];
     }
 }
 
@@ -1384,13 +1393,13 @@ extern "C" __global__ void __launch_bounds__(128) wave_step_kernel(WaveArgs A) {
     for (int i = (blockIdx.x * WAVE_WPB + wib) * 2 + half; i < n; i += gridDim.x * WAVE_WPB * 2) {
         const int s = A.qp_list[i];
         SlotState& S = A.slots[s];
-        const double* Qb = A.qp_buf + (int64_t)s * QP_VALS;
+        const double* Qb = A.qp_buf + i;
         double x[9], g[9], p[9];
 #pragma unroll
         for (int k = 0; k < 9; k++) {
             x[k] = S.xc[k];
             g[k] = S.g[k];
-            p[k] = Qb[90 + k] - x[k];
+            p[k] = Qb[(QP_IN + k) * (int64_t)A.n_slots] - x[k];
         }
         const double gp = dot_fma(9, g, p);
         double xn[9];
@@ -1650,7 +1659,7 @@ int WaveEngine::open(Workspace& ws, cudaStream_t st, const RunConfig& cfg, int64
     }
     E.admit_blocks = ws.sm_count * aocc;
     E.solve_blocks = (int)((n_slots + 2 * WAVE_WPB - 1) / (2 * WAVE_WPB));   // two slots per warp
-    E.qp_blocks = (int)((n_slots + 127) / 128);                               // a thread per slot
+    E.qp_blocks = (int)((n_slots + QP_THREADS - 1) / QP_THREADS);             // a thread per slot
     E.multi_blocks = 0;
     if (cfg.ml_units > 0) {
         int mocc = 0;
@@ -1731,7 +1740,7 @@ int WaveEngine::open(Workspace& ws, cudaStream_t st, const RunConfig& cfg, int64
         }
         if (ce == cudaSuccess) {
             wave_solve_kernel<<<E.solve_blocks, 128, wsm, st>>>(Aw);
-            wave_qp_kernel<<<E.qp_blocks, 128, 0, st>>>(Aw);
+            wave_qp_kernel<<<E.qp_blocks, QP_THREADS, 0, st>>>(Aw);
             wave_step_kernel<<<E.solve_blocks, 128, 0, st>>>(Aw);
             ce = cudaEventRecordWithFlags(E.ev[par][3], st, cudaEventRecordExternal);
         }
@@ -1848,7 +1857,7 @@ int WaveEngine::run_until_idle(unsigned long long max_waves, std::string& err) {
             wave_pass_kernel<<<E.pass_blocks, 128, WAVE_WPB * PASS_WARP_SMEM, st>>>(Aw);
             if (E.multi_blocks) wave_multi_kernel<<<E.multi_blocks, MULTI_WARPS * 32, MULTI_SMEM, st>>>(Aw);
             wave_solve_kernel<<<E.solve_blocks, 128, WAVE_WPB * WARP_SMEM, st>>>(Aw);
-            wave_qp_kernel<<<E.qp_blocks, 128, 0, st>>>(Aw);
+            wave_qp_kernel<<<E.qp_blocks, QP_THREADS, 0, st>>>(Aw);
             wave_step_kernel<<<E.solve_blocks, 128, 0, st>>>(Aw);
             wave_end_kernel<<<1, 32, 0, st>>>(Aw, k, h, max_waves);
         }

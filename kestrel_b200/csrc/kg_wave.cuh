@@ -134,7 +134,7 @@ struct WaveArgs {
     double* ml_partial;            // per slot: ml_units * ML_VALS sums of its tri-/tetra-allelic sites
     int ml_units;                  // their work units per slot (0: no cohort has such sites)
     int ml_chunk;                  // kept sites per such unit (a multiple of 32, at most ML_CHUNK)
-    double* qp_buf;                // per slot QP_VALS: Q (9 x 9 row-major), c, the solution y
+    double* qp_buf;                // value v of the wave's QP i at [v * n_slots + i]: Q's upper triangle, c, y (in: x)
     int* qp_list;                  // the slots of this wave's QPs (wc_cur->n_qp of them)
     int unit_elems;                // list entries per pass work unit
     // pairs on frequency nodes (kg_node.cu) instead of site lists: no admit
@@ -167,8 +167,9 @@ constexpr int WAVE_WPB = 4;   // warps per block of the wave kernels
 // objective term.
 constexpr int ML_CHUNK = 8192;
 constexpr int ML_VALS = 56;
-// a slot's QP: Q at 0, c at 81, the solution at 90
-constexpr int QP_VALS = 100;
+// a QP's values in qp_buf: 45 of Q, 9 of c, 9 of y
+constexpr int QP_VALS = 63;
+constexpr int QP_THREADS = 32;   // one warp a block: few QPs spread over the SMs
 
 __device__ __forceinline__ int shape_ng(int s) { return s == 0 ? 4 : s == 3 ? 4 : s == 4 ? 2 : 3; }
 __device__ __forceinline__ int shape_nh(int s) { return s == 0 ? 7 : s == 3 ? 9 : s == 4 ? 3 : 5; }
