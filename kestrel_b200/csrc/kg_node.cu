@@ -26,6 +26,7 @@
 #include <math_constants.h>
 
 #include <algorithm>
+#include <climits>
 #include <cmath>
 #include <cstdlib>
 #include <cstring>
@@ -34,6 +35,7 @@
 #include "kg_engine.h"
 #include "kg_node.h"
 #include "kg_pair.cuh"
+#include "kg_qp1.cuh"
 #include "kg_tmem.cuh"
 #include "kg_wave.cuh"
 
@@ -49,9 +51,6 @@ namespace kg {
     } while (0)
 
 // ------------------------------------------------------------ preparation
-
-// A node's table entry at frequency t: t, 1 - t, t (1 - t), t^2 .. t^6.
-constexpr int NODE_VALS = 8;
 
 // A double bin: its first site (a multiple of NODE_STAGE), its stages.
 struct NodeBin {
@@ -128,22 +127,11 @@ __global__ void node_layout_kernel(NodeGrid G, int* __restrict__ hist, NodeBin* 
             at += st * NODE_STAGE;
         }
     }
-    for (int e = threadIdx.x; e < 2 * G.bins * J; e += blockDim.x) {
-        const bool mirror = e >= G.bins * J;
-        const int i = mirror ? e - G.bins * J : e, k = i / J, j = i - k * J;
+    for (int e = threadIdx.x; e < G.bins * J; e += blockDim.x) {
+        const int k = e / J, j = e - k * J;
         double lo, hi;
         bin_interval(G, k, lo, hi);
-        const double tl = 0.5 * (lo + hi) - 0.5 * (hi - lo) * cospi((2 * j + 1) / (2.0 * J));
-        const double x = mirror ? 1.0 - tl : tl, y = mirror ? tl : 1.0 - tl, x2 = x * x;
-        double* o = t + (int64_t)e * NODE_VALS;
-        o[0] = x;
-        o[1] = y;
-        o[2] = x * y;
-        o[3] = x2;
-        o[4] = x2 * x;
-        o[5] = x2 * x2;
-        o[6] = x2 * x2 * x;
-        o[7] = x2 * x2 * x2;
+        t[e] = 0.5 * (lo + hi) - 0.5 * (hi - lo) * cospi((2 * j + 1) / (2.0 * J));
     }
 }
 
@@ -234,7 +222,7 @@ int prepare_nodes(Cohort& c, const uint8_t* codes, int64_t stride, int bins, dou
     G.n_kept = c.n_kept;
     const size_t head = sizeof(int) * NODE_MAX_BINS + sizeof(NodeBin) * NODE_MAX_BINS;
     KG_NODE_TRY((cudaError_t)c.nd_bins.reserve(head));
-    KG_NODE_TRY((cudaError_t)c.nd_t.reserve(sizeof(double) * 2 * NODE_VALS * bins * NODE_J));
+    KG_NODE_TRY((cudaError_t)c.nd_t.reserve(sizeof(double) * bins * NODE_J));
     KG_NODE_TRY((cudaError_t)c.nd_place.reserve(sizeof(uint32_t) * mp));
     KG_NODE_TRY((cudaError_t)c.nd_dig.reserve((size_t)32 * mp));
     KG_NODE_TRY((cudaError_t)c.nd_planes.reserve(sizeof(uint2) * (mp / 32) * c.n_samples));
@@ -290,7 +278,7 @@ struct NodeProduct {
     int32_t bins;
     int64_t idx0, idx1;        // the pairs (x <= y) of this chunk: y (y + 1) / 2 + x
     int64_t slot0;             // slot of pair idx0 within w's columns
-    int64_t y0, first_unit, n_yx;   // first y; its first (y, x block) in the count from y = 0; how many
+    int64_t first_unit, n_yx;  // the first (y, x block) in the count from y = 0, how many
     double* w;
     int64_t stride;
     unsigned long long* stalled;
@@ -517,7 +505,7 @@ __global__ void __launch_bounds__(NW_THREADS, 1) node_weights_kernel(NodeProduct
     if (warp == 12) tmem_free<512>(tm);
 }
 
-// ------------------------------------------------------- first state, passes
+// --------------------------------------------------------- a chunk's slots
 
 // A run of one job's pairs (y-major: y (y + 1) / 2 + x) in consecutive slots.
 struct NodeSeg {
@@ -525,15 +513,132 @@ struct NodeSeg {
     int32_t slot0, n, job, pad;
 };
 
+// A job's nodes: W of slot s at w[(u nk + i) stride + s], u a genotype pair, i a node.
+struct NodeDev {
+    const double* w;
+    int64_t stride;
+    const double* t;      // the nodes' frequencies (at most 1/2)
+    double scale;         // what a unit of the (integer) weights stands for
+    int32_t nk;           // nodes per genotype pair: bins x NODE_J
+    int32_t pad;
+};
+
+// log d by table (node_log).
+constexpr int LOG_CELLS = 128, LOG_EXPS = 64;
+struct LogTable {
+    double2 cell[LOG_CELLS];   // {c, -log c}
+    double exp2[LOG_EXPS];     // (e - 40) log 2
+};
+
+// A slot's SQP state (src/sqp.rs:49-93) between its passes, value-major:
+// value v of slot s at [v * stride + s].
+enum : int {
+    NS_XC = 0,        // accepted point
+    NS_XT = 9,        // point of the pending pass
+    NS_P = 18,        // search direction
+    NS_F = 27,        // objective at xc
+    NS_GP = 28,       // g . p
+    NS_ALPHA = 29,
+    NS_N = 30,        // the pair's sites
+    NS_COEF = 31,     // PassCoef at xt (16)
+    NS_STEP = 47,     // PassCoef of xt - xc (16): difference passes
+    NS_VALS = 63
+};
+constexpr int NS_COEFS = (int)(sizeof(PassCoef) / sizeof(double));
+static_assert(NS_COEFS == 16, "PassCoef: a 4, b1 3, b2 3, c 4, d 2");
+
+// The waves' control words.
+struct NodeCtl {
+    int n[2];              // pending passes of the even and the odd waves
+    unsigned int ticket;   // blocks of the advance kernel that are done
+    int n_seg;             // runs of the chunk
+    unsigned long long max_waves;
+};
+
+struct NodeArgs {
+    const CohortDev* cohorts;
+    const NodeDev* nodes;      // per job
+    const NodeSeg* seg;        // the chunk's runs (ctl->n_seg)
+    int64_t stride;            // slots
+    double* state;             // NS_VALS
+    double* partial;           // UNIT_VALS x NODE_UNITS, value-major
+    int4* count;               // {iterations, backtracks, passes, job * 4 + kind} per slot
+    int* sites;                // NODE_UNITS per slot, value-major: the pair's sites by genotype pair
+    int* list_cur;             // slots with a pending pass
+    int* list_next;
+    int par;                   // 0: even waves
+    NodeCtl* ctl;
+    WaveClock* clk;
+    RunCounters* counters;
+    const LogTable* log_table;
+    Tune tune;
+};
+
+// Kinds of a pending pass: the pair's first, direct objective, objective change.
+enum : int { NP_FIRST = 0, NP_DIRECT = 1, NP_DIFF = 2 };
+
+__device__ __forceinline__ NodeSeg seg_of(const NodeSeg* seg, int n_seg, int s) {
+    int lo = 0, hi = n_seg - 1;
+    while (lo < hi) {
+        const int mid = (lo + hi + 1) >> 1;
+        if (seg[mid].slot0 <= s) lo = mid;
+        else hi = mid - 1;
+    }
+    return seg[lo];
+}
+
+__host__ __device__ inline void pair_of(int64_t idx, int64_t& x, int64_t& y) {
+    y = (int64_t)((sqrt(8.0 * (double)idx + 1.0) - 1.0) * 0.5);
+    while (y > 0 && y * (y + 1) / 2 > idx) y--;
+    while ((y + 1) * (y + 2) / 2 <= idx) y++;
+    x = idx - y * (y + 1) / 2;
+}
+
+__device__ __forceinline__ void node_write_row(const CohortDev& co, int64_t x, int64_t y, const double* d, double obj,
+                                               uint64_t iters, double cond) {
+    kg_output* o = co.out + (x * co.n_x - x * (x - 1) / 2 + (y - x));
+    o->x = (uint64_t)x;
+    o->y = (uint64_t)y;
+#pragma unroll
+    for (int i = 0; i < 9; i++) o->jacquard[i] = d[i];
+    o->obj = obj;
+    o->iters = iters;
+    o->cond = cond;
+}
+
+__device__ __forceinline__ void store_coef(double* v, int64_t stride, const double* x) {
+    PassCoef k;
+    make_coef(x, k);
+    const double* c = reinterpret_cast<const double*>(&k);
+#pragma unroll
+    for (int i = 0; i < NS_COEFS; i++) v[i * stride] = c[i];
+}
+
+// The step xt - xc of a difference pass, less its part along xc: both points
+// add up to 1 only to an ulp, and the objective would change by that ulp (its
+// slope along x itself is -1) where the step's own change is smaller still.
+__device__ __forceinline__ void store_step(double* v, int64_t stride, const double* xt, const double* xc) {
+    double d[9], s = 0.0;
+#pragma unroll
+    for (int i = 0; i < 9; i++) {
+        d[i] = xt[i] - xc[i];
+        s += d[i];
+    }
+#pragma unroll
+    for (int i = 0; i < 9; i++) d[i] = fma(-s, xc[i], d[i]);
+    store_coef(v, stride, d);
+}
+
 // Thread per slot: the pair's state before its first pass; thread 0 readies
-// the wave counters and the clock.
-__global__ void node_init_kernel(WaveArgs A, const NodeSeg* __restrict__ seg, int n_seg, int n,
-                                 unsigned long long max_waves) {
+// the control words and the clock.
+__global__ void node_init_kernel(NodeArgs A, int n_seg, int n, unsigned long long max_waves) {
     const int s = blockIdx.x * blockDim.x + threadIdx.x;
     if (s == 0) {
-        *A.wc_cur = WaveCounts{};
-        *A.wc_next = WaveCounts{};
-        A.wc_cur->n_pass = n;
+        A.ctl->n[0] = n;
+        A.ctl->n[1] = 0;
+        A.ctl->ticket = 0;
+        A.ctl->n_seg = n_seg;
+        A.ctl->max_waves = max_waves;
         for (int i = 0; i < 3; i++) {
             A.clk->start[i] = ~0ull;
             A.clk->end[i] = 0ull;
@@ -541,77 +646,29 @@ __global__ void node_init_kernel(WaveArgs A, const NodeSeg* __restrict__ seg, in
         A.clk->stop = 0;
         A.clk->waves = 0;
         A.clk->iters = 0;
-        A.clk->max_waves = max_waves;
     }
     if (s >= n) return;
-    int lo = 0, hi = n_seg - 1;
-    while (lo < hi) {
-        const int mid = (lo + hi + 1) >> 1;
-        if (seg[mid].slot0 <= s) lo = mid;
-        else hi = mid - 1;
-    }
-    const NodeSeg g = seg[lo];
-    const int64_t idx = g.idx0 + (s - g.slot0);
-    int64_t y = (int64_t)((sqrt(8.0 * (double)idx + 1.0) - 1.0) * 0.5);
-    while (y > 0 && y * (y + 1) / 2 > idx) y--;
-    while ((y + 1) * (y + 2) / 2 <= idx) y++;
-    const int64_t x = idx - y * (y + 1) / 2;
-    const CohortDev& co = A.cohorts[g.job];
-    SlotState& S = A.slots[s];
-    S.k = co.pair_begin + x * co.n_x - x * (x - 1) / 2 + (y - x);
-    S.x = x;
-    S.y = y;
-    S.cohort = g.job;
-    // two units a shape, one for het-het (UNIT in node_weights_kernel)
-    for (int i = 0; i < 5; i++) S.ustart[i] = 2 * i;
-    S.ustart[5] = NODE_UNITS;
-    S.n = 0;
-    S.lists64 = 1;
-    S.fp64 = 1;
-    S.near_count = 0;
-    S.bls = 0;
-    S.escalated = 0;
-    S.gh = 0;
-    S.f64p = 0;
-    S.diffp = 0;
-    S.it = 0;
-    S.f = 0.0;
+    const NodeSeg g = seg_of(A.seg, n_seg, s);
+    int64_t x, y;
+    pair_of(g.idx0 + (s - g.slot0), x, y);
     double x0[9];
     for (int i = 0; i < 9; i++) x0[i] = x == y ? 0.0 : 1.0 / 9.0;
     if (x == y) { x0[0] = 0.5; x0[6] = 0.5; }
     normalise9(x0);
-    for (int i = 0; i < 9; i++) { S.xc[i] = x0[i]; S.xt[i] = x0[i]; }
-    S.ev = EV_INIT;
-    S.kind = co.method == ESTIMATOR_CLS ? PASS_CLS64 : PASS_FP64;
-    make_coef(x0, S.c64);
-    S.status = SLOT_PASS;
-    A.pass_cur[s] = s;
+    double* st = A.state + s;
+#pragma unroll
+    for (int i = 0; i < 9; i++) st[(NS_XT + i) * A.stride] = x0[i];
+    store_coef(st + NS_COEF * A.stride, A.stride, x0);
+    A.count[s] = make_int4(0, 0, 0, 4 * g.job + NP_FIRST);
+    A.list_cur[s] = s;
 }
 
-// 1 / d to an ulp or so: the hardware's approximation and one cubic Newton step.
-__device__ __forceinline__ double node_rcp(double d) {
-    double r;
-    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(d));
-    const double e = fma(-d, r, 1.0);
-    return fma(fma(e, e, e), r, r);
-}
+// ------------------------------------------------------------------- passes
 
-// log d for eps <= d < 2 by table (Tang, ACM TOMS 16, 1990): d = 2^e m, c the
+// log d for 2^-40 <= d < 2 (Tang, ACM TOMS 16, 1990): d = 2^e m, c the
 // reciprocal of the middle of m's 1/128 interval, log d = e log 2 - log c +
 // log1p(m c - 1), the last by its series (|m c - 1| < 2^-8: the first term left
 // out is below 3e-18).  The library's log is 30 FP64 instructions, this 9.
-constexpr int LOG_CELLS = 128, LOG_EXPS = 64;
-struct LogTable {
-    double2 cell[LOG_CELLS];   // {c, -log c}
-    double exp2[LOG_EXPS];     // (e - 40) log 2
-};
-__device__ __forceinline__ void fill_log_table(LogTable& T) {
-    for (int i = threadIdx.x; i < LOG_CELLS; i += blockDim.x) {
-        const double c = 1.0 / (1.0 + (i + 0.5) / LOG_CELLS);
-        T.cell[i] = make_double2(c, -log(c));
-    }
-    for (int i = threadIdx.x; i < LOG_EXPS; i += blockDim.x) T.exp2[i] = (i - 40) * 0.69314718055994530942;
-}
 __device__ __forceinline__ double node_log(double d, const LogTable& T) {
     const int hi = __double2hiint(d);
     const double m = __hiloint2double((hi & 0x000FFFFF) | 0x3FF00000, __double2loint(d));
@@ -625,181 +682,662 @@ __device__ __forceinline__ double node_log(double d, const LogTable& T) {
     return (T.exp2[((hi >> 20) - 1023 + 40) & (LOG_EXPS - 1)] + c.y) + s;
 }
 
-// One genotype pair's nodes for one slot: the moments of its shape (SH) and the
-// sum of W log d; the terms of stream64 with weights.  MIRROR: the pair sees 1
-// - t.  The logarithms of four nodes are added before they join their sum, whose
-// rounding is kept (two-sum): the Armijo test near convergence compares
-// objectives to their last bits.  scale: what an integer weight stands for.
-template <int SH, bool MIRROR>
-__device__ __forceinline__ void node_unit(const NodeDev& N, const double* __restrict__ w, const PassCoef& K, double* P,
-                                          int* cnt, bool write, bool count, const LogTable& T) {
-    constexpr int NG = SH == 0 ? 4 : SH == 3 ? 4 : SH == 4 ? 2 : 3;
-    constexpr int NH = SH == 0 ? 7 : SH == 3 ? 9 : SH == 4 ? 3 : 5;
+// log(d / (d - delta)) = -log(1 - z), z = delta / d: the series for |z| <= 1/64
+// (the first term left out is below 1e-15 of the sum), else the table.
+__device__ __forceinline__ double node_neg_log1m(double z, const LogTable& T) {
+    if (fabs(z) <= 0.015625) {
+        double s = fma(z, 0.125, 1.0 / 7.0);
+        s = fma(z, s, 1.0 / 6.0);
+        s = fma(z, s, 0.2);
+        s = fma(z, s, 0.25);
+        s = fma(z, s, 1.0 / 3.0);
+        s = fma(z, s, 0.5);
+        s = fma(z, s, 1.0);
+        return z * s;
+    }
+    return -node_log(1.0 - z, T);
+}
+
+// d - eps at a node: the shape's polynomial (stream64 of kg_pair.cuh).
+template <int SH>
+__device__ __forceinline__ double node_poly(const double* k, double t, double ty, double q) {
+    if (SH == 0) return t * fma(fma(fma(k[3], t, k[2]), t, k[1]), t, k[0]);
+    if (SH == 1 || SH == 2) return q * fma(fma(k[2], t, k[1]), t, k[0]);
+    if (SH == 3) return q * fma(q, k[3], fma(t, k[2], fma(ty, k[1], k[0])));
+    return q * fma(q, k[1], k[0]);
+}
+
+// One genotype pair's nodes for one slot, every fourth node from part on: the
+// moments of its shape (SH) and the objective sum, sum W log d or (DIFF) sum W
+// log(d / d_old); the terms of stream64 with weights.  MIRROR: the pair sees 1 -
+// t.  out: gradient moments, Hessian moments, objective, sites.
+template <int SH>
+struct NodeShape {
+    static constexpr int NG = SH == 0 ? 4 : SH == 3 ? 4 : SH == 4 ? 2 : 3;
+    static constexpr int NH = SH == 0 ? 7 : SH == 3 ? 9 : SH == 4 ? 3 : 5;
+    static constexpr int NK = SH == 0 || SH == 3 ? 4 : SH == 4 ? 2 : 3;      // coefficients
+    static constexpr int K0 = SH == 0 ? 0 : SH == 1 ? 4 : SH == 2 ? 7 : SH == 3 ? 10 : 14;   // the first in PassCoef
+};
+
+template <int SH, bool MIRROR, bool DIFF>
+__device__ __forceinline__ void node_sums(const NodeDev& N, const double* __restrict__ w, const double* __restrict__ st,
+                                          int64_t stride, int part, const LogTable& T,
+                                          double (&g)[NodeShape<SH>::NG], double (&h)[NodeShape<SH>::NH], double& F) {
+    constexpr int NG = NodeShape<SH>::NG, NH = NodeShape<SH>::NH, NK = NodeShape<SH>::NK, K0 = NodeShape<SH>::K0;
     const double EPS = 1e-8;
-    double k0, k1, k2 = 0.0, k3 = 0.0;
-    if (SH == 0) { k0 = K.a[0]; k1 = K.a[1]; k2 = K.a[2]; k3 = K.a[3]; }
-    if (SH == 1) { k0 = K.b1[0]; k1 = K.b1[1]; k2 = K.b1[2]; }
-    if (SH == 2) { k0 = K.b2[0]; k1 = K.b2[1]; k2 = K.b2[2]; }
-    if (SH == 3) { k0 = K.c[0]; k1 = K.c[1]; k2 = K.c[2]; k3 = K.c[3]; }
-    if (SH == 4) { k0 = K.d[0]; k1 = K.d[1]; }
-    double g[NG], h[NH], F = 0.0, Fl = 0.0;
+    double k[NK], ks[NK];
+#pragma unroll
+    for (int i = 0; i < NK; i++) {
+        k[i] = st[(NS_COEF + K0 + i) * stride];
+        ks[i] = DIFF ? st[(NS_STEP + K0 + i) * stride] : 0.0;
+    }
+    F = 0.0;
 #pragma unroll
     for (int i = 0; i < NG; i++) g[i] = 0.0;
 #pragma unroll
     for (int i = 0; i < NH; i++) h[i] = 0.0;
-    const double2* __restrict__ tab = reinterpret_cast<const double2*>(N.t) + (MIRROR ? (NODE_VALS / 2) * N.nk : 0);
-    const int64_t step = N.stride;
-    auto node = [&](double W, const double2* __restrict__ e) {
-        const double2 e0 = __ldg(e), e1 = __ldg(e + 1);
-        const double t = e0.x, ty = e0.y, q = e1.x, t2 = e1.y;
-        double d;
+    auto node = [&](double W, double tl) {
+        const double tu = 1.0 - tl, t = MIRROR ? tu : tl, ty = MIRROR ? tl : tu, q = t * ty, t2 = t * t;
+        const double d = node_poly<SH>(k, t, ty, q) + EPS;
+        const double rd = recip<true>(d);
         if (SH == 0) {
-            const double2 e2 = __ldg(e + 2), e3 = __ldg(e + 3);
-            d = fma(t, fma(fma(fma(k3, t, k2), t, k1), t, k0), EPS);
-            const double u = t * node_rcp(d), v = u * W;
-            g[0] += v; g[1] = fma(v, t, g[1]); g[2] = fma(v, t2, g[2]); g[3] = fma(v, e2.x, g[3]);
-            const double v2 = v * u;
-            h[0] += v2; h[1] = fma(v2, t, h[1]); h[2] = fma(v2, t2, h[2]); h[3] = fma(v2, e2.x, h[3]);
-            h[4] = fma(v2, e2.y, h[4]); h[5] = fma(v2, e3.x, h[5]); h[6] = fma(v2, e3.y, h[6]);
+            const double t3 = t2 * t, t4 = t2 * t2;
+            const double u = t * rd, v = u * W;
+            g[0] += v; g[1] = fma(v, t, g[1]); g[2] = fma(v, t2, g[2]); g[3] = fma(v, t3, g[3]);
+            const double v2 = v * u, v4 = v2 * t4;
+            h[0] += v2; h[1] = fma(v2, t, h[1]); h[2] = fma(v2, t2, h[2]); h[3] = fma(v2, t3, h[3]);
+            h[4] += v4; h[5] = fma(v4, t, h[5]); h[6] = fma(v4, t2, h[6]);
         } else if (SH == 1 || SH == 2) {
-            const double2 e2 = __ldg(e + 2);
-            d = fma(q, fma(fma(k2, t, k1), t, k0), EPS);
-            const double u = q * node_rcp(d), v = u * W;
+            const double u = q * rd, v = u * W;
             g[0] += v; g[1] = fma(v, t, g[1]); g[2] = fma(v, t2, g[2]);
-            const double v2 = v * u;
-            h[0] += v2; h[1] = fma(v2, t, h[1]); h[2] = fma(v2, t2, h[2]); h[3] = fma(v2, e2.x, h[3]);
-            h[4] = fma(v2, e2.y, h[4]);
+            const double v2 = v * u, v22 = v2 * t2;
+            h[0] += v2; h[1] = fma(v2, t, h[1]); h[2] += v22; h[3] = fma(v22, t, h[3]);
+            h[4] = fma(v22, t2, h[4]);
         } else if (SH == 3) {
-            d = fma(q, fma(q, k3, fma(t, k2, fma(ty, k1, k0))), EPS);
-            const double u = q * node_rcp(d), v = u * W;
+            const double u = q * rd, v = u * W;
             g[0] += v; g[1] = fma(v, ty, g[1]); g[2] = fma(v, t, g[2]); g[3] = fma(v, q, g[3]);
             const double v2 = v * u, vy = v2 * ty, vq = v2 * q;
             h[0] += v2; h[1] += vy; h[2] = fma(v2, t, h[2]); h[3] += vq;
             h[4] = fma(vy, ty, h[4]); h[5] = fma(v2, t2, h[5]);
             h[6] = fma(vq, ty, h[6]); h[7] = fma(vq, t, h[7]); h[8] = fma(vq, q, h[8]);
         } else {
-            d = fma(q, fma(q, k1, k0), EPS);
-            const double u = q * node_rcp(d), v = u * W;
+            const double u = q * rd, v = u * W;
             g[0] += v; g[1] = fma(v, q, g[1]);
             const double v2 = v * u, vq = v2 * q;
             h[0] += v2; h[1] += vq; h[2] = fma(vq, q, h[2]);
         }
-        return W * node_log(d, T);
+        if (DIFF) F = fma(W, node_neg_log1m(node_poly<SH>(ks, t, ty, q) * rd, T), F);
+        else F = fma(W, node_log(d, T), F);
     };
-    static_assert(NODE_J % 4 == 0, "nodes come in fours");
-    const double* wp = w;
-    double W0 = wp[0], W1 = wp[step], W2 = wp[2 * step], W3 = wp[3 * step];
-    for (int i = 0; i < N.nk; i += 4) {
-        const double a0 = W0, a1 = W1, a2 = W2, a3 = W3;
-        if (i + 4 < N.nk) {   // the next four nodes' weights in flight
-            wp += 4 * step;
-            W0 = wp[0]; W1 = wp[step]; W2 = wp[2 * step]; W3 = wp[3 * step];
+    static_assert(NODE_J % 8 == 0, "two nodes a step for each of four parts");
+    const int64_t step = 4 * N.stride;
+    const double* wp = w + part * N.stride;
+    const double* __restrict__ tp = N.t + part;
+    double W0 = wp[0], W1 = wp[step], t0 = __ldg(tp), t1 = __ldg(tp + 4);
+    for (int i = 0; i < N.nk; i += 8) {
+        const double a0 = W0, a1 = W1, b0 = t0, b1 = t1;
+        if (i + 8 < N.nk) {   // the next two nodes' weights and frequencies in flight
+            wp += 2 * step;
+            tp += 8;
+            W0 = wp[0];
+            W1 = wp[step];
+            t0 = __ldg(tp);
+            t1 = __ldg(tp + 4);
         }
-        const double2* e = tab + (NODE_VALS / 2) * i;
-        const double f = (node(a0, e) + node(a1, e + 4)) + (node(a2, e + 8) + node(a3, e + 12));
-        const double s = F + f, z = s - F;
-        Fl += (F - (s - z)) + (f - z);
-        F = s;
+        node(a0, b0);
+        node(a1, b1);
     }
-    if (!write) return;
-    const double scale = N.scale;
-#pragma unroll
-    for (int i = 0; i < NG; i++) P[i] = g[i] * scale;
-#pragma unroll
-    for (int i = 0; i < NH; i++) P[NG + i] = h[i] * scale;
-    P[UNIT_VALS - 1] = (F + Fl) * scale;
-    if (count) {
-        double C = 0.0;
-        for (int i = 0; i < N.nk; i++) C += w[(int64_t)i * step];
-        *cnt = __double2int_rn(C * scale);
-    }
-}
-
-// The CLS moments (cls_stream64) of one genotype pair's nodes.
-template <int SH, bool MIRROR>
-__device__ __forceinline__ void node_unit_cls(const NodeDev& N, const double* __restrict__ w, double* P, int* cnt,
-                                              bool write) {
-    constexpr int NG = SH == 0 ? 4 : SH == 3 ? 4 : SH == 4 ? 2 : 3;
-    constexpr int NH = SH == 0 ? 7 : SH == 3 ? 9 : SH == 4 ? 3 : 5;
-    double g[NG], C = 0.0;
-#pragma unroll
-    for (int i = 0; i < NG; i++) g[i] = 0.0;
-    const double2* __restrict__ tab = reinterpret_cast<const double2*>(N.t) + (MIRROR ? (NODE_VALS / 2) * N.nk : 0);
-    for (int i = 0; i < N.nk; i++) {
-        const double W = w[(int64_t)i * N.stride];
-        const double2 e0 = __ldg(tab + (NODE_VALS / 2) * i), e1 = __ldg(tab + (NODE_VALS / 2) * i + 1);
-        const double t = e0.x, ty = e0.y, q = e1.x, t2 = e1.y;
-        if (SH == 0) {
-            const double v = W * t;
-            g[0] += v; g[1] = fma(v, t, g[1]); g[2] = fma(v, t2, g[2]); g[3] = fma(v * t2, t, g[3]);
-        } else if (SH == 1 || SH == 2) {
-            const double v = W * q;
-            g[0] += v; g[1] = fma(v, t, g[1]); g[2] = fma(v, t2, g[2]);
-        } else if (SH == 3) {
-            const double v = W * q;
-            g[0] += v; g[1] = fma(v, ty, g[1]); g[2] = fma(v, t, g[2]); g[3] = fma(v, q, g[3]);
-        } else {
-            const double v = W * q;
-            g[0] += v; g[1] = fma(v, q, g[1]);
-        }
-        C += W;
-    }
-    if (!write) return;
-    const double scale = N.scale;
-#pragma unroll
-    for (int i = 0; i < NG; i++) P[i] = g[i] * scale;
-#pragma unroll
-    for (int i = 0; i < NH; i++) P[NG + i] = 0.0;
-    P[UNIT_VALS - 1] = 0.0;
-    *cnt = __double2int_rn(C * scale);
 }
 
 template <int SH, bool MIRROR>
-__device__ __forceinline__ void node_task(const WaveArgs& A, const SlotState& S, int s, int u, bool write,
-                                          const LogTable& T) {
-    const NodeDev N = A.nodes[S.cohort];
-    const double* w = N.w + (int64_t)u * N.nk * N.stride + (s - N.slot0);
-    double* P = A.partial + ((int64_t)s * A.max_units + u) * UNIT_VALS;
-    int* cnt = A.node_cnt + (int64_t)s * NODE_UNITS + u;
-    if (S.kind == PASS_CLS64) node_unit_cls<SH, MIRROR>(N, w, P, cnt, write);
-    else node_unit<SH, MIRROR>(N, w, S.c64, P, cnt, write, S.ev == EV_INIT, T);
+__device__ __forceinline__ void node_task(const NodeArgs& A, const NodeDev& N, int s, int u, int kind, int part,
+                                          bool write, const LogTable& T) {
+    constexpr int NG = NodeShape<SH>::NG, NH = NodeShape<SH>::NH;
+    const double* w = N.w + (int64_t)u * N.nk * N.stride + s;
+    const double* st = A.state + s;
+    double g[NG], h[NH], F;
+    if (kind == NP_DIFF) node_sums<SH, MIRROR, true>(N, w, st, A.stride, part, T, g, h, F);
+    else node_sums<SH, MIRROR, false>(N, w, st, A.stride, part, T, g, h, F);
+    // the four parts, in a fixed order
+    auto all = [](double v) {
+        v += __shfl_xor_sync(0xffffffffu, v, 8);
+        return v + __shfl_xor_sync(0xffffffffu, v, 16);
+    };
+    double C = 0.0;
+    const bool first = __any_sync(0xffffffffu, kind == NP_FIRST);
+    if (first) {
+        for (int i = part; i < N.nk; i += 4) C += w[(int64_t)i * N.stride];
+        C = all(C);
+    }
+    const double scale = N.scale;
+    double* P = A.partial + (int64_t)u * UNIT_VALS * A.stride + s;
+#pragma unroll
+    for (int i = 0; i < NG; i++) {
+        const double v = all(g[i]) * scale;
+        if (write && part == (i & 3)) P[i * A.stride] = v;
+    }
+#pragma unroll
+    for (int i = 0; i < NH; i++) {
+        const double v = all(h[i]) * scale;
+        if (write && part == ((NG + i) & 3)) P[(NG + i) * A.stride] = v;
+    }
+    const double f = all(F) * scale;
+    if (write && part == 3) P[(UNIT_VALS - 1) * A.stride] = f;
+    if (first && write && part == 0) A.sites[(int64_t)u * A.stride + s] = __double2int_rn(C * scale);
 }
 
-// A warp per (32 slots of the pass list, genotype pair), a thread per slot:
-// the weights are stored slot-fastest, so a warp's loads are whole sectors,
-// the node's frequency is the same for all lanes, and no sum crosses lanes.
-// Genotype-pair-major, so an SM's warps run one shape's code at a time.  Bound
-// by the FP64 pipe (the reciprocal and the logarithm are most of a node's
-// operations).
-extern "C" __global__ void __launch_bounds__(128, 4) node_pass_kernel(WaveArgs A) {
+// A warp per (8 slots of the pass list, genotype pair): lane l takes every
+// fourth node from l / 8 on of slot l % 8.  The weights are stored slot-fastest,
+// so a warp's loads are whole sectors; four lanes a slot keep a pass over few
+// slots short (a lone lane's 112 nodes took 48 us), two shuffles a moment add
+// them.  Genotype-pair-major, so an SM's warps run one shape's code at a time.
+// Bound by the FP64 pipe's issue.
+extern "C" __global__ void __launch_bounds__(128, 5) node_pass_kernel(NodeArgs A) {
     __shared__ LogTable T;
     if (A.clk->stop) return;   // a device loop past its last wave
-    fill_log_table(T);
-    __syncthreads();
     if (threadIdx.x == 0) atomicMin(&A.clk->start[1], global_ns());
     const int lane = threadIdx.x & 31;
     const PhaseEnd pe{&A.clk->end[1], lane == 0};
-    const int n = A.wc_cur->n_pass, groups = (n + 31) >> 5;
+    const int n = A.ctl->n[A.par], groups = (n + 7) >> 3;
     const int64_t tasks = (int64_t)groups * NODE_UNITS;
+    if ((int64_t)blockIdx.x >= tasks) return;
+    for (int i = threadIdx.x; i < (int)(sizeof(LogTable) / 16); i += blockDim.x)
+        reinterpret_cast<double2*>(&T)[i] = reinterpret_cast<const double2*>(A.log_table)[i];
+    __syncthreads();
+    const int part = lane >> 3;
     // consecutive tasks go to different SMs, so a short list spreads
     for (int64_t task = (int64_t)(threadIdx.x >> 5) * gridDim.x + blockIdx.x; task < tasks;
          task += (int64_t)gridDim.x * (blockDim.x >> 5)) {
-        const int u = (int)(task / groups), i = (int)(task - (int64_t)u * groups) * 32 + lane;
+        const int u = (int)(task / groups), i = (int)(task - (int64_t)u * groups) * 8 + (lane & 7);
         const bool write = i < n;
-        const int s = A.pass_cur[write ? i : n - 1];
-        const SlotState& S = A.slots[s];
+        const int s = A.list_cur[write ? i : n - 1];
+        const int jk = A.count[s].w, kind = jk & 3;
+        const NodeDev N = A.nodes[jk >> 2];
         switch (u) {
-        case 0: node_task<0, false>(A, S, s, u, write, T); break;
-        case 1: node_task<0, true>(A, S, s, u, write, T); break;
-        case 2: node_task<1, false>(A, S, s, u, write, T); break;
-        case 3: node_task<1, true>(A, S, s, u, write, T); break;
-        case 4: node_task<2, false>(A, S, s, u, write, T); break;
-        case 5: node_task<2, true>(A, S, s, u, write, T); break;
-        case 6: node_task<3, false>(A, S, s, u, write, T); break;
-        case 7: node_task<3, true>(A, S, s, u, write, T); break;
-        default: node_task<4, false>(A, S, s, u, write, T); break;
+        case 0: node_task<0, false>(A, N, s, u, kind, part, write, T); break;
+        case 1: node_task<0, true>(A, N, s, u, kind, part, write, T); break;
+        case 2: node_task<1, false>(A, N, s, u, kind, part, write, T); break;
+        case 3: node_task<1, true>(A, N, s, u, kind, part, write, T); break;
+        case 4: node_task<2, false>(A, N, s, u, kind, part, write, T); break;
+        case 5: node_task<2, true>(A, N, s, u, kind, part, write, T); break;
+        case 6: node_task<3, false>(A, N, s, u, kind, part, write, T); break;
+        case 7: node_task<3, true>(A, N, s, u, kind, part, write, T); break;
+        default: node_task<4, false>(A, N, s, u, kind, part, write, T); break;
         }
     }
+}
+
+// --------------------------------------------------------------- the SQP step
+
+// S = sum L r and the upper triangle T = sum L L' r^2 from the moments (rebuild
+// of kg_pair.cuh, its indices known at compile time).
+__device__ __forceinline__ void rebuild_upper(const double (&m)[NMOM], double (&S)[9], double (&T)[QP_Q]) {
+    constexpr int e[9] = {1, 2, 2, 3, 2, 3, 2, 3, 4};
+#pragma unroll
+    for (int i = 0; i < 9; i++) {
+        S[i] = m[e[i] - 1];
+#pragma unroll
+        for (int j = i; j < 9; j++) T[upper_at(i, j)] = m[4 + e[i] + e[j] - 2];
+    }
+    constexpr int cb[4] = {1, 2, 1, 2}, pb[4] = {0, 1, 1, 2}, i1[4] = {2, 3, 7, 8}, i2[4] = {4, 5, 7, 8};
+    constexpr int ic[4] = {1, 3, 5, 8}, hc[4][4] = {{0, 1, 2, 3}, {1, 4, 3, 6}, {2, 3, 5, 7}, {3, 6, 7, 8}};
+    constexpr int id[3] = {6, 7, 8}, cd[3] = {2, 1, 4}, pd[3] = {0, 0, 1};
+#pragma unroll
+    for (int a = 0; a < 4; a++) {
+        S[i1[a]] += cb[a] * m[11 + pb[a]];
+        S[i2[a]] += cb[a] * m[19 + pb[a]];
+        S[ic[a]] += m[27 + a];
+#pragma unroll
+        for (int b = a; b < 4; b++) {
+            T[upper_at(i1[a], i1[b])] += (double)(cb[a] * cb[b]) * m[14 + pb[a] + pb[b]];
+            T[upper_at(i2[a], i2[b])] += (double)(cb[a] * cb[b]) * m[22 + pb[a] + pb[b]];
+            T[upper_at(ic[a], ic[b])] += m[31 + hc[a][b]];
+        }
+    }
+#pragma unroll
+    for (int a = 0; a < 3; a++) {
+        S[id[a]] += cd[a] * m[40 + pd[a]];
+#pragma unroll
+        for (int b = a; b < 3; b++) T[upper_at(id[a], id[b])] += (double)(cd[a] * cd[b]) * m[42 + pd[a] + pd[b]];
+    }
+}
+
+// Column j of the plain LDL^T of the block F (unit pivots and zero columns
+// outside it) and the ones after it.
+template <int j, class HF>
+__device__ __forceinline__ void ldl_plain_columns(const HF& H, unsigned F, double (&L)[36], double (&D)[9],
+                                                  bool& positive) {
+    const bool jf = (F >> j) & 1u;
+    double p[9], sjj = 0.0;
+#pragma unroll
+    for (int s = 0; s < j; s++) {
+        const double l = L[j * (j - 1) / 2 + s];
+        p[s] = D[s] * l;
+        sjj = fma(p[s], l, sjj);
+    }
+    const double dj = H(upper_at(j, j)) - sjj;
+    D[j] = jf ? dj : 1.0;
+    positive = positive && D[j] > 0.0;
+    const double rd = recip<true>(D[j]);
+#pragma unroll
+    for (int i = j + 1; i < 9; i++) {
+        double sij = 0.0;
+#pragma unroll
+        for (int s = 0; s < j; s++) sij = fma(p[s], L[i * (i - 1) / 2 + s], sij);
+        L[i * (i - 1) / 2 + j] = jf && ((F >> i) & 1u) ? quot(H(upper_at(j, i)) - sij, D[j], rd) : 0.0;
+    }
+    if constexpr (j + 1 < 9) ldl_plain_columns<j + 1>(H, F, L, D, positive);
+}
+
+// The reduced Hessian's condition estimate at a KKT point (condition_estimate
+// of kg_solver.cuh, src/sqp.rs:313-391), with zero rows and unit pivots for the
+// variables left out in place of a compacted matrix.  H(k): the upper triangle.
+template <class HF>
+__device__ __forceinline__ double condition_thread(const HF& H, const double (&x)[9], const double (&g)[9], double tol) {
+    double lambda = 0.0;
+#pragma unroll
+    for (int i = 0; i < 9; i++) lambda = fma(x[i], g[i], lambda);
+    unsigned F = 0;
+#pragma unroll
+    for (int i = 0; i < 9; i++)
+        if (!(x[i] == 0.0 && g[i] >= lambda + tol)) F |= 1u << i;
+    if (F == 0) return CUDART_INF;
+    double L[36], D[9];
+    bool positive = true;
+    ldl_plain_columns<0>(H, F, L, D, positive);
+    if (!positive) return CUDART_INF;
+    int imax = -1, imin = -1;
+    double dmax = 0.0, dmin = 0.0;
+#pragma unroll
+    for (int i = 0; i < 9; i++) {
+        if (!((F >> i) & 1u)) continue;
+        if (imax < 0 || D[i] >= dmax) { imax = i; dmax = D[i]; }
+        if (imin < 0 || D[i] < dmin) { imin = i; dmin = D[i]; }
+    }
+    // |L e_max| and |L^-T e_min|
+    double wmax = 0.0, wmin = 0.0, z[9];
+#pragma unroll
+    for (int i = 0; i < 9; i++) {
+        double l = i == imax ? 1.0 : 0.0;
+#pragma unroll
+        for (int j = 0; j < i; j++)
+            if (j == imax) l = L[i * (i - 1) / 2 + j];
+        wmax = fma(l, l, wmax);
+    }
+#pragma unroll
+    for (int i = 8; i >= 0; i--) {
+        double s = 0.0;
+#pragma unroll
+        for (int j = i + 1; j < 9; j++) s = fma(z[j], L[j * (j - 1) / 2 + i], s);
+        z[i] = (i == imin ? 1.0 : 0.0) - s;
+        wmin = fma(z[i], z[i], wmin);
+    }
+    return sqrt(wmax) * sqrt(wmin) * (dmax / dmin);
+}
+
+constexpr int NA_THREADS = 32;   // one warp a block: few slots spread over the SMs
+
+// One slot: returns the kind of its next pass, or -1 when its row is written.
+// my: the thread's column of the shared memory; sum: the block's counters.
+__device__ __forceinline__ int node_advance(const NodeArgs& A, int s, double* my, unsigned long long* sum) {
+    const Tune& tu = A.tune;
+    const int64_t SD = A.stride;
+    double* st = A.state + s;
+    const int4 ct = A.count[s];
+    const int kind = ct.w & 3;
+    // ---- the pair's moments: two genotype pairs a shape, het-het one
+    double xt[9], g[9], obj, nsites;
+    {
+        double m[NMOM];
+        const double* P = A.partial + s;
+        obj = 0.0;
+#pragma unroll
+        for (int u = 0; u < NODE_UNITS; u++) {
+            const int sh = u >> 1, go = sh == 0 ? 0 : sh == 1 ? 11 : sh == 2 ? 19 : sh == 3 ? 27 : 40;
+            const int nv = sh == 0 ? 11 : sh == 3 ? 13 : sh == 4 ? 5 : 8;
+#pragma unroll
+            for (int v = 0; v < 13; v++)
+                if (v < nv) {
+                    const double p = P[((int64_t)u * UNIT_VALS + v) * SD];
+                    m[go + v] = (u & 1) ? m[go + v] + p : p;
+                }
+            obj += P[((int64_t)u * UNIT_VALS + UNIT_VALS - 1) * SD];
+        }
+        if (kind == NP_FIRST) {
+            int64_t c = 0;
+            for (int u = 0; u < NODE_UNITS; u++) c += A.sites[(int64_t)u * SD + s];
+            nsites = (double)c;
+            st[NS_N * SD] = nsites;
+        } else {
+            nsites = st[NS_N * SD];
+        }
+        double T[QP_Q];
+        rebuild_upper(m, g, T);
+        const double rn = 1.0 / nsites;
+#pragma unroll
+        for (int k = 0; k < QP_Q; k++) my[k * NA_THREADS] = quot(T[k], nsites, rn);
+#pragma unroll
+        for (int k = 0; k < 9; k++) g[k] = quot(-g[k], nsites, rn);
+    }
+#pragma unroll
+    for (int k = 0; k < 9; k++) xt[k] = st[(NS_XT + k) * SD];
+    const int gh = ct.z + 1;
+    int it = ct.x;
+    double f;
+    int next = -1;   // the kind of the next pass (-1: the pair is done)
+    bool trial_again = false;
+    if (kind == NP_FIRST) {
+        f = -obj / nsites;
+    } else {
+        // Armijo (src/sqp.rs:294): a difference pass has the objective's
+        // change itself, which the test resolves far below an ulp of f
+        const double f0 = st[NS_F * SD], alpha = st[NS_ALPHA * SD], gp = st[NS_GP * SD];
+        const double bar = alpha * (tu.bls_sufficient_decrease * gp);
+        const double df = -obj / nsites;
+        f = kind == NP_DIFF ? f0 + df : df;
+        const bool accept = kind == NP_DIFF ? df <= bar : f <= f0 + bar;
+        if (!accept && ct.y + 1 != tu.bls_max_iter) {
+            trial_again = true;
+            const double a2 = alpha * tu.bls_step_size_reduce;
+            double xc[9], sum_x = 0.0;
+#pragma unroll
+            for (int k = 0; k < 9; k++) {
+                xc[k] = st[(NS_XC + k) * SD];
+                xt[k] = xc[k] + a2 * st[(NS_P + k) * SD];
+                sum_x += xt[k];
+            }
+#pragma unroll
+            for (int k = 0; k < 9; k++) {
+                xt[k] = xt[k] / sum_x;
+                st[(NS_XT + k) * SD] = xt[k];
+            }
+            st[NS_ALPHA * SD] = a2;
+            next = fabs(a2 * gp) < DIFF_BELOW ? NP_DIFF : NP_DIRECT;
+            store_coef(st + NS_COEF * SD, SD, xt);
+            if (next == NP_DIFF) store_step(st + NS_STEP * SD, SD, xt, xc);
+            A.count[s] = make_int4(it, ct.y + 1, gh, (ct.w & ~3) | next);
+        } else {
+            it++;
+        }
+    }
+    if (!trial_again) {
+        // ---- the accepted point
+        const CohortDev& co = A.cohorts[ct.w >> 2];
+        double resid;
+        const bool none = nsites == 0.0, last = (uint64_t)it >= co.max_iter;
+        if (none || last || kkt_ok(xt, g, tu.sqp_conv_tol, &resid)) {
+            const NodeSeg sg = seg_of(A.seg, A.ctl->n_seg, s);
+            int64_t x, y;
+            pair_of(sg.idx0 + (s - sg.slot0), x, y);
+            double cond = CUDART_NAN;
+            if (!none && !last) cond = condition_thread([my](int k) { return my[k * NA_THREADS]; }, xt, g, tu.sqp_conv_tol);
+            if (none) {
+#pragma unroll
+                for (int k = 0; k < 9; k++) xt[k] = CUDART_NAN;
+                f = CUDART_NAN;
+            }
+            node_write_row(co, x, y, xt, f, none ? 0 : last ? co.max_iter : (uint64_t)it, cond);
+            // the counters of the call
+            unsigned long long evals = 0, shapes[5];
+#pragma unroll
+            for (int sh = 0; sh < 5; sh++) {
+                shapes[sh] = (unsigned long long)A.sites[(int64_t)(2 * sh) * SD + s];
+                if (sh < 4) shapes[sh] += (unsigned long long)A.sites[(int64_t)(2 * sh + 1) * SD + s];
+                evals += (unsigned long long)((sh == 4 ? 1 : 2) * flops_fp64(sh));
+                atomicAdd(&sum[7 + sh], none ? 0ull : shapes[sh]);
+            }
+            if (none) {
+                atomicAdd(&sum[0], 1ull);
+            } else {
+                atomicAdd(&sum[1], (unsigned long long)gh);
+                atomicAdd(&sum[2], (unsigned long long)nsites);
+                atomicAdd(&sum[3], (unsigned long long)nsites * (unsigned long long)gh);
+                if (last) atomicAdd(&sum[4], 1ull);
+                if (!last && !(cond <= COND_RECHECK)) atomicAdd(&sum[5], 1ull);
+                atomicAdd(&sum[6], evals * (unsigned long long)A.nodes[sg.job].nk * (unsigned long long)gh);
+            }
+        } else {
+            // ---- the QP and the step (src/sqp.rs:78-90)
+            auto H = [my](int i2, int j2) { return my[(i2 <= j2 ? upper_at(i2, j2) : upper_at(j2, i2)) * NA_THREADS]; };
+#pragma unroll
+            for (int r = 0; r < 9; r++) {
+                double hx = 0.0;
+#pragma unroll
+                for (int j = 0; j < 9; j++) hx = fma(H(r, j), xt[j], hx);
+                my[(QP_Q + r) * NA_THREADS] = g[r] - hx;
+                st[(NS_XC + r) * SD] = xt[r];
+            }
+            st[NS_F * SD] = f;
+            double y[9];
+#pragma unroll
+            for (int k = 0; k < 9; k++) y[k] = xt[k];
+            qp_simplex_thread<true>([my](int v) { return my[v * NA_THREADS]; }, tu, y);
+            // g . p with p = y - x; the first trial point x + p, normalised
+            double gp = 0.0, sum_x = 0.0, p[9];
+#pragma unroll
+            for (int k = 0; k < 9; k++) {
+                p[k] = y[k] - xt[k];
+                gp = fma(g[k], p[k], gp);
+                y[k] = xt[k] + p[k];
+                sum_x += y[k];
+            }
+#pragma unroll
+            for (int k = 0; k < 9; k++) {
+                st[(NS_P + k) * SD] = p[k];
+                y[k] = y[k] / sum_x;
+                st[(NS_XT + k) * SD] = y[k];
+            }
+            st[NS_GP * SD] = gp;
+            st[NS_ALPHA * SD] = 1.0;
+            next = fabs(gp) < DIFF_BELOW ? NP_DIFF : NP_DIRECT;
+            store_coef(st + NS_COEF * SD, SD, y);
+            if (next == NP_DIFF) store_step(st + NS_STEP * SD, SD, y, xt);
+            A.count[s] = make_int4(it, 0, gh, (ct.w & ~3) | next);
+        }
+    }
+    return next;
+}
+
+// Everything between two passes of a slot, a thread per slot: its moments,
+// the Armijo accept test (a rejected trial backs off and takes the next pass),
+// the KKT test, at convergence the condition estimate and the row, else the
+// simplex QP and the next trial point.  The state and the sums are stored
+// value-major, so a warp's loads and stores are whole sectors; H and c go
+// through shared memory (432 bytes a thread) into the QP.  One kernel instead
+// of the list form's solve, QP and step kernels: nothing is written between
+// them and a wave over few slots waits for one launch.  Bound by the FP64
+// chains of the QP (nine pivots one after the other, up to ten times).  The
+// last block to finish ends the wave: it adds the phase times and decides
+// whether the loop goes on.
+extern "C" __global__ void __launch_bounds__(NA_THREADS) node_advance_kernel(NodeArgs A, int in_loop,
+                                                                            cudaGraphConditionalHandle loop) {
+    __shared__ double in[QP_IN * NA_THREADS];
+    __shared__ unsigned long long sum[12];
+    if (A.clk->stop) {   // a device loop past its last wave
+        if (in_loop && A.par && blockIdx.x == 0 && threadIdx.x == 0) {
+            A.clk->iters++;
+            cudaGraphSetConditional(loop, 0u);
+        }
+        return;
+    }
+    const int n = A.ctl->n[A.par];
+    if (threadIdx.x < 12) sum[threadIdx.x] = 0ull;
+    if (threadIdx.x == 0 && (int)blockIdx.x * NA_THREADS < n) atomicMin(&A.clk->start[2], global_ns());
+    __syncwarp();
+    double* my = in + threadIdx.x;
+    for (int base = blockIdx.x * NA_THREADS; base < n; base += gridDim.x * NA_THREADS) {
+        const bool live = base + (int)threadIdx.x < n;
+        const int s = A.list_cur[live ? base + threadIdx.x : n - 1];
+        const int next = live ? node_advance(A, s, my, sum) : -1;
+        __syncwarp();
+        // slots with another pass join the next wave's list, in this list's order
+        const unsigned more = __ballot_sync(0xffffffffu, next >= 0);
+        int at = 0;
+        if (threadIdx.x == 0 && more) at = atomicAdd(&A.ctl->n[A.par ^ 1], __popc(more));
+        at = __shfl_sync(0xffffffffu, at, 0);
+        if (next >= 0) A.list_next[at + __popc(more & ((1u << threadIdx.x) - 1u))] = s;
+    }
+    __syncwarp();
+    if (threadIdx.x < 12 && sum[threadIdx.x]) {
+        RunCounters* C = A.counters;
+        const unsigned long long v = sum[threadIdx.x];
+        switch (threadIdx.x) {
+        case 0: atomicAdd(&C->nosite_pairs, v); break;
+        case 1: atomicAdd(&C->gh_passes, v); break;
+        case 2: atomicAdd(&C->pair_sites, v); break;
+        case 3: atomicAdd(&C->work_units, v); break;
+        case 4: atomicAdd(&C->nonconverged, v); break;
+        case 5: atomicAdd(&C->fp64_pairs, v); break;
+        case 6: atomicAdd(&C->flops_fp64, v); break;
+        default: atomicAdd(&C->shape_sites[threadIdx.x - 7], v); break;
+        }
+    }
+    __syncwarp();
+    if (threadIdx.x != 0) return;
+    __threadfence();
+    if (atomicAdd(&A.ctl->ticket, 1u) != gridDim.x - 1) return;
+    // ---- the wave's end
+    __threadfence();
+    WaveClock* c = A.clk;
+    volatile NodeCtl* ctl = A.ctl;
+    const unsigned long long now = global_ns();
+    const unsigned long long p0 = *reinterpret_cast<volatile unsigned long long*>(&c->start[1]);
+    const unsigned long long p1 = *reinterpret_cast<volatile unsigned long long*>(&c->end[1]);
+    const unsigned long long s0 = *reinterpret_cast<volatile unsigned long long*>(&c->start[2]);
+    if (p1 > p0) c->acc[1] += p1 - p0;
+    if (now > s0) c->acc[2] += now - s0;
+    c->waves++;
+    unsigned int stop = 0;
+    if (ctl->n[A.par ^ 1] == 0) {
+        stop = 1;
+    } else if (c->waves >= ctl->max_waves) {
+        stop = 1;
+        c->limit_hit = 1;
+    }
+    c->stop = stop;
+    ctl->n[A.par] = 0;
+    ctl->ticket = 0;
+    for (int k = 0; k < 3; k++) {
+        c->start[k] = ~0ull;
+        c->end[k] = 0ull;
+    }
+    if (in_loop && A.par) {
+        c->iters++;
+        cudaGraphSetConditional(loop, stop ? 0u : 1u);
+    }
+}
+
+// ---------------------------------------------------------------------- CLS
+
+// The CLS estimator of a pair (cls_finish of kg_wave.cu, src/coefficients.rs:
+// 218-268), a thread per pair: the pair's summed likelihood rows are cubic and
+// quartic in the frequency, so its nodes give them exactly; c = rows / (-M),
+// the simplex QP on the cohort's Q (two-variable for a self pair), the Brier
+// score and the condition estimate.
+extern "C" __global__ void __launch_bounds__(NA_THREADS) node_cls_kernel(NodeArgs A, int n_seg, int n) {
+    __shared__ double in[QP_IN * NA_THREADS];
+    __shared__ unsigned long long sum[7];
+    if (threadIdx.x < 7) sum[threadIdx.x] = 0ull;
+    __syncwarp();
+    double* my = in + threadIdx.x;
+    for (int s = blockIdx.x * NA_THREADS + threadIdx.x; s < n; s += gridDim.x * NA_THREADS) {
+        const NodeSeg sg = seg_of(A.seg, n_seg, s);
+        const CohortDev& co = A.cohorts[sg.job];
+        const NodeDev N = A.nodes[sg.job];
+        int64_t x, y;
+        pair_of(sg.idx0 + (s - sg.slot0), x, y);
+        // sums of the shapes' monomials: A t^1..4, B w t^0..2, C w {1, ty, t, w}, D w {1, w}
+        double m[16], sites[5];
+#pragma unroll
+        for (int k = 0; k < 16; k++) m[k] = 0.0;
+#pragma unroll
+        for (int k = 0; k < 5; k++) sites[k] = 0.0;
+        for (int i = 0; i < N.nk; i++) {
+            const double* w = N.w + (int64_t)i * N.stride + s;
+            const int64_t un = (int64_t)N.nk * N.stride;
+            const double t = __ldg(N.t + i), u = 1.0 - t, q = t * u, t2 = t * t, u2 = u * u;
+            const double W[9] = {w[0], w[un], w[2 * un], w[3 * un], w[4 * un], w[5 * un], w[6 * un], w[7 * un], w[8 * un]};
+            m[0] = fma(W[0], t, fma(W[1], u, m[0]));
+            m[1] = fma(W[0], t2, fma(W[1], u2, m[1]));
+            m[2] = fma(W[0], t2 * t, fma(W[1], u2 * u, m[2]));
+            m[3] = fma(W[0], t2 * t2, fma(W[1], u2 * u2, m[3]));
+#pragma unroll
+            for (int b = 0; b < 2; b++) {
+                const double v0 = W[2 + 2 * b] * q, v1 = W[3 + 2 * b] * q;
+                m[4 + 3 * b] += v0 + v1;
+                m[5 + 3 * b] = fma(v0, t, fma(v1, u, m[5 + 3 * b]));
+                m[6 + 3 * b] = fma(v0, t2, fma(v1, u2, m[6 + 3 * b]));
+            }
+            const double c0 = W[6] * q, c1 = W[7] * q, d0 = W[8] * q;
+            m[10] += c0 + c1;
+            m[11] = fma(c0, u, fma(c1, t, m[11]));
+            m[12] = fma(c0, t, fma(c1, u, m[12]));
+            m[13] = fma(c0 + c1, q, m[13]);
+            m[14] += d0;
+            m[15] = fma(d0, q, m[15]);
+#pragma unroll
+            for (int k = 0; k < 4; k++) sites[k] += W[2 * k] + W[2 * k + 1];
+            sites[4] += W[8];
+        }
+        double S[9] = {m[0], m[1] + m[10], m[1] + m[4], m[2] + 2.0 * m[5] + m[11], m[1] + m[7],
+                       m[2] + 2.0 * m[8] + m[12], m[1] + 2.0 * m[14], m[2] + m[5] + m[8] + m[14],
+                       m[3] + 2.0 * (m[6] + m[9]) + m[13] + 4.0 * m[15]};
+        const int64_t row = x * co.n_x - x * (x - 1) / 2 + (y - x);
+        Tune tq = A.tune;
+        tq.qp_max_iter = co.max_iter > (uint64_t)INT_MAX ? INT_MAX : (int)co.max_iter;
+#pragma unroll
+        for (int k = 0; k < 9; k++) {
+            double v = S[k] * N.scale;
+            if (co.cls_cmulti) v += co.cls_cmulti[row * 9 + k];   // its tri- and tetra-allelic rows
+            my[(QP_Q + k) * NA_THREADS] = v / -co.cls_m;
+#pragma unroll
+            for (int j = k; j < 9; j++) my[upper_at(k, j) * NA_THREADS] = co.cls_q[k * 9 + j];
+        }
+        auto Q = [my](int i2, int j2) { return my[(i2 <= j2 ? upper_at(i2, j2) : upper_at(j2, i2)) * NA_THREADS]; };
+        double d[9];
+        int iters;
+        if (x == y) {
+            double e0 = 0.0, e6 = 0.0;
+            iters = qp_simplex2(Q(0, 0), Q(0, 6), Q(0, 6), Q(6, 6), my[QP_Q * NA_THREADS], my[(QP_Q + 6) * NA_THREADS],
+                                0.5, 0.5, tq, e0, e6);
+#pragma unroll
+            for (int k = 0; k < 9; k++) d[k] = k == 0 ? e0 : k == 6 ? e6 : 0.0;
+        } else {
+#pragma unroll
+            for (int k = 0; k < 9; k++) d[k] = 1.0 / 9.0;
+            iters = qp_simplex_thread<true>([my](int v) { return my[v * NA_THREADS]; }, tq, d);
+        }
+        double g[9], quad = 0.0, lin = 0.0;
+#pragma unroll
+        for (int r = 0; r < 9; r++) {
+            double qd = 0.0;
+#pragma unroll
+            for (int j = 0; j < 9; j++) qd = fma(Q(r, j), d[j], qd);
+            quad = fma(d[r], qd, quad);
+            const double c = my[(QP_Q + r) * NA_THREADS];
+            lin = fma(c, d[r], lin);
+            g[r] = qd + c;
+        }
+        const double cond = condition_thread([my](int k) { return my[k * NA_THREADS]; }, d, g, tq.sqp_conv_tol);
+        node_write_row(co, x, y, d, (quad + 2.0 * lin) + 1.0, (uint64_t)iters, cond);
+        unsigned long long all = 0;
+#pragma unroll
+        for (int k = 0; k < 5; k++) {
+            const unsigned long long c = (unsigned long long)__double2ll_rn(sites[k] * N.scale);
+            all += c;
+            atomicAdd(&sum[k], c);
+        }
+        atomicAdd(&sum[5], all);
+        if ((uint64_t)iters >= co.max_iter) atomicAdd(&sum[6], 1ull);
+    }
+    __syncwarp();
+    RunCounters* C = A.counters;
+    if (threadIdx.x < 5) atomicAdd(&C->shape_sites[threadIdx.x], sum[threadIdx.x]);
+    if (threadIdx.x == 5) {
+        atomicAdd(&C->pair_sites, sum[5]);
+        atomicAdd(&C->work_units, sum[5]);
+    }
+    if (threadIdx.x == 6 && sum[6]) atomicAdd(&C->nonconverged, sum[6]);
 }
 
 // ------------------------------------------------------------------- host
@@ -810,29 +1348,28 @@ struct NodeEngine {
     cudaGraph_t g = nullptr;
     cudaGraphExec_t x = nullptr;
     cudaEvent_t ev[2] = {nullptr, nullptr};
-    std::vector<void*> key_bufs;
+    std::vector<void*> key;
     uint64_t key_iterations = 0;
     int key_dev = -1;
     cudaStream_t key_st = nullptr;
-    WaveArgs args[2]{};
-    int pass_blocks = 0, solve_blocks = 0, qp_blocks = 0, step_blocks = 0;
+    DevBuf log_table;
+    NodeArgs args[2]{};
+    int pass_blocks = 0, advance_blocks = 0, cls_blocks = 0;
     void drop() {
         if (x) cudaGraphExecDestroy(x);
         if (g) cudaGraphDestroy(g);
         x = nullptr;
         g = nullptr;
+        key.clear();
     }
     ~NodeEngine() {
         drop();
         for (auto& e : ev)
             if (e) cudaEventDestroy(e);
     }
-    void wave(int par, cudaStream_t st) const {
-        const WaveArgs& A = args[par];
-        node_pass_kernel<<<pass_blocks, 128, 0, st>>>(A);
-        wave_solve_kernel<<<solve_blocks, 128, WAVE_WPB * WARP_SMEM, st>>>(A);
-        wave_qp_kernel<<<qp_blocks, QP_THREADS, 0, st>>>(A);
-        wave_step_kernel<<<step_blocks, 128, 0, st>>>(A);
+    void wave(int par, int in_loop, cudaGraphConditionalHandle h, cudaStream_t st) const {
+        node_pass_kernel<<<pass_blocks, 128, 0, st>>>(args[par]);
+        node_advance_kernel<<<advance_blocks, NA_THREADS, 0, st>>>(args[par], in_loop, h);
     }
 };
 
@@ -845,6 +1382,7 @@ int run_nodes(const std::vector<PairJob>& jobs, const RunConfig& cfg, Workspace&
     if (ws.sm_count == 0) KG_NODE_TRY(cudaDeviceGetAttribute(&ws.sm_count, cudaDevAttrMultiProcessorCount, dev));
     const int n_jobs = (int)jobs.size();
     constexpr int J = NODE_J;
+    const bool cls = jobs[0].method == ESTIMATOR_CLS;
     std::vector<CohortDev> table((size_t)n_jobs);
     int64_t total = 0;
     int nk_max = 0;
@@ -858,27 +1396,23 @@ int run_nodes(const std::vector<PairJob>& jobs, const RunConfig& cfg, Workspace&
     }
     // pairs in flight: all of them up to 2^20, or what half the free memory
     // (with what the workspace holds already) takes
-    const size_t per_slot = sizeof(double) * NODE_UNITS * ((size_t)nk_max + UNIT_VALS) + sizeof(SlotState) +
-                            sizeof(double) * QP_VALS + sizeof(int) * (3 + NODE_UNITS);
-    size_t fr = 0, tot = 0;
+    const size_t slot_bytes = sizeof(double) * (NODE_UNITS * UNIT_VALS + NS_VALS + 2) + sizeof(int4) +
+                              sizeof(int) * (2 + NODE_UNITS);
+    const size_t per_slot = sizeof(double) * NODE_UNITS * (size_t)nk_max + slot_bytes;
     int64_t cap = std::min<int64_t>(total, cfg.slots > 0 ? cfg.slots : (int64_t)1 << 20);
-    const size_t held = ws.scratch.bytes + ws.slots.bytes + ws.partial.bytes + ws.qp.bytes;
+    const size_t held = ws.scratch.bytes + ws.slots.bytes;
     if ((size_t)cap * per_slot > held) {
+        size_t fr = 0, tot = 0;
         KG_NODE_TRY(cudaMemGetInfo(&fr, &tot));
         cap = std::max<int64_t>(1, std::min<int64_t>(cap, (int64_t)((fr + held) / 2 / per_slot)));
     }
     const int64_t stride = (cap + 31) / 32 * 32;
     KG_NODE_TRY((cudaError_t)ws.scratch.reserve(sizeof(double) * NODE_UNITS * (size_t)nk_max * stride));
-    KG_NODE_TRY((cudaError_t)ws.partial.reserve(sizeof(double) * NODE_UNITS * UNIT_VALS * (size_t)cap));
-    KG_NODE_TRY((cudaError_t)ws.slots.reserve(sizeof(SlotState) * (size_t)cap));
-    KG_NODE_TRY((cudaError_t)ws.qp.reserve((sizeof(double) * QP_VALS + sizeof(int)) * (size_t)cap));
-    KG_NODE_TRY((cudaError_t)ws.lists_a.reserve(sizeof(int) * 2 * (size_t)cap));
-    KG_NODE_TRY((cudaError_t)ws.lists_b.reserve(sizeof(int) * NODE_UNITS * (size_t)cap));
-    // counters, one buffer: {wave counts x 2, task and queue words, live, clock,
-    // run counters, finished pairs per job}
-    const size_t off_live = sizeof(WaveCounts) * 2 + 64, off_clk = (off_live + sizeof(LiveQueue) + 15) & ~(size_t)15;
-    const size_t off_run = off_clk + sizeof(WaveClock), off_done = off_run + sizeof(RunCounters);
-    KG_NODE_TRY((cudaError_t)ws.node_counts.reserve(off_done + sizeof(unsigned long long) * n_jobs));
+    KG_NODE_TRY((cudaError_t)ws.slots.reserve(slot_bytes * (size_t)stride));
+    // control words, one buffer: {control, clock, run counters}
+    const size_t off_clk = sizeof(NodeCtl), off_run = off_clk + sizeof(WaveClock);
+    const size_t ctl_bytes = off_run + sizeof(RunCounters);
+    KG_NODE_TRY((cudaError_t)ws.node_counts.reserve(ctl_bytes));
     const size_t off_nodes = sizeof(CohortDev) * n_jobs, off_seg = off_nodes + sizeof(NodeDev) * n_jobs;
     const size_t blob = off_seg + sizeof(NodeSeg) * n_jobs;
     KG_NODE_TRY((cudaError_t)ws.node_table.reserve(blob));
@@ -893,54 +1427,52 @@ int run_nodes(const std::vector<PairJob>& jobs, const RunConfig& cfg, Workspace&
     const unsigned long long bound = 2ull * (max_iter + 2) * 16ull + 64ull;
     const char* hw = std::getenv("KESTREL_HOST_WAVES");
     const bool host_waves = hw && hw[0] == '1';
-    const std::vector<void*> bufs{ws.scratch.p, ws.partial.p, ws.slots.p, ws.qp.p, ws.lists_a.p, ws.lists_b.p,
-                                  ws.node_counts.p, ws.node_table.p, reinterpret_cast<void*>(off_nodes), reinterpret_cast<void*>((size_t)cap)};
-    const bool same = E.key_bufs == bufs && E.key_iterations == cfg.iterations &&
-                      E.key_dev == dev && E.key_st == st;
-    if (!same) {
+    const std::vector<void*> key{ws.scratch.p, ws.slots.p, ws.node_counts.p, ws.node_table.p,
+                                 reinterpret_cast<void*>(off_nodes), reinterpret_cast<void*>((size_t)stride)};
+    if (E.key != key || E.key_iterations != cfg.iterations || E.key_dev != dev || E.key_st != st) {
         E.drop();
-        WaveArgs A{};
+        if (!E.log_table.p || E.key_dev != dev) {
+            LogTable T;
+            for (int i = 0; i < LOG_CELLS; i++) {
+                const double c = 1.0 / (1.0 + (i + 0.5) / LOG_CELLS);
+                T.cell[i] = make_double2(c, -std::log(c));
+            }
+            for (int i = 0; i < LOG_EXPS; i++) T.exp2[i] = (i - 40) * 0.69314718055994530942;
+            E.log_table.release();
+            KG_NODE_TRY((cudaError_t)E.log_table.reserve(sizeof(T)));
+            KG_NODE_TRY(cudaMemcpy(E.log_table.p, &T, sizeof(T), cudaMemcpyHostToDevice));
+        }
+        NodeArgs A{};
         A.cohorts = reinterpret_cast<CohortDev*>(dtab);
         A.nodes = reinterpret_cast<NodeDev*>(dtab + off_nodes);
-        A.live = reinterpret_cast<LiveQueue*>(counts + off_live);
-        unsigned long long* words = reinterpret_cast<unsigned long long*>(counts + sizeof(WaveCounts) * 2);
-        A.admit_task = reinterpret_cast<int*>(words);
-        A.queue = words + 1;
-        A.pass_task = words + 2;
+        A.seg = reinterpret_cast<NodeSeg*>(dtab + off_seg);
+        A.stride = stride;
+        A.state = ws.slots.as<double>();
+        A.partial = A.state + (size_t)(NS_VALS + 2) * stride;
+        A.count = reinterpret_cast<int4*>(A.partial + (size_t)NODE_UNITS * UNIT_VALS * stride);
+        A.sites = reinterpret_cast<int*>(A.count + stride);
+        int* lists = A.sites + NODE_UNITS * stride;
+        A.ctl = reinterpret_cast<NodeCtl*>(counts);
         A.clk = reinterpret_cast<WaveClock*>(counts + off_clk);
         A.counters = reinterpret_cast<RunCounters*>(counts + off_run);
-        A.cohort_done = reinterpret_cast<unsigned long long*>(counts + off_done);
-        A.precision = KG_PREC_FP32C;
-        A.slots = ws.slots.as<SlotState>();
-        A.n_slots = (int)cap;
-        A.partial = ws.partial.as<double>();
-        A.max_units = NODE_UNITS;
+        A.log_table = E.log_table.as<LogTable>();
         A.tune = make_tune(cfg.iterations);
-        A.qp_buf = ws.qp.as<double>();
-        A.qp_list = reinterpret_cast<int*>(A.qp_buf + (size_t)QP_VALS * cap);
-        A.unit_elems = UNIT_ELEMS;
-        A.node_cnt = ws.lists_b.as<int>();
         for (int par = 0; par < 2; par++) {
-            WaveArgs& W = E.args[par];
-            W = A;
-            W.pass_cur = ws.lists_a.as<int>() + (par ? cap : 0);
-            W.pass_next = ws.lists_a.as<int>() + (par ? 0 : cap);
-            W.wc_cur = reinterpret_cast<WaveCounts*>(counts) + par;
-            W.wc_next = reinterpret_cast<WaveCounts*>(counts) + (par ^ 1);
+            E.args[par] = A;
+            E.args[par].par = par;
+            E.args[par].list_cur = lists + (par ? stride : 0);
+            E.args[par].list_next = lists + (par ? 0 : stride);
         }
         int occ = 0;
         KG_NODE_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, node_pass_kernel, 128, 0));
         E.pass_blocks = ws.sm_count * std::max(1, occ);
-        KG_NODE_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, wave_solve_kernel, 128, WAVE_WPB * WARP_SMEM));
-        E.solve_blocks = ws.sm_count * std::max(1, occ);
-        KG_NODE_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, wave_qp_kernel, QP_THREADS, 0));
-        E.qp_blocks = ws.sm_count * std::max(1, occ);
-        KG_NODE_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, wave_step_kernel, 128, 0));
-        E.step_blocks = ws.sm_count * std::max(1, occ);
+        KG_NODE_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, node_advance_kernel, NA_THREADS, 0));
+        E.advance_blocks = ws.sm_count * std::max(1, occ);
+        KG_NODE_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, node_cls_kernel, NA_THREADS, 0));
+        E.cls_blocks = ws.sm_count * std::max(1, occ);
         KG_NODE_TRY(cudaFuncSetAttribute(node_weights_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, NW_SMEM));
         for (auto& e : E.ev)
             if (!e) KG_NODE_TRY(cudaEventCreate(&e));
-        E.key_bufs.clear();
         KG_NODE_TRY(cudaGraphCreate(&E.g, 0));
         cudaGraphConditionalHandle h;
         KG_NODE_TRY(cudaGraphConditionalHandleCreate(&h, E.g, 1, cudaGraphCondAssignDefault));
@@ -953,36 +1485,33 @@ int run_nodes(const std::vector<PairJob>& jobs, const RunConfig& cfg, Workspace&
         KG_NODE_TRY(cudaGraphAddNode(&node, E.g, nullptr, 0, &np));
         cudaGraph_t body = np.conditional.phGraph_out[0];
         KG_NODE_TRY(cudaStreamBeginCaptureToGraph(st, body, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal));
-        for (int par = 0; par < 2; par++) {
-            E.wave(par, st);
-            wave_end_kernel<<<1, 32, 0, st>>>(E.args[par], par, h, 0);
-        }
+        for (int par = 0; par < 2; par++) E.wave(par, 1, h, st);
         cudaGraph_t captured = nullptr;
         const cudaError_t ce = cudaGetLastError();
         const cudaError_t ee = cudaStreamEndCapture(st, &captured);
         KG_NODE_TRY(ce);
         KG_NODE_TRY(ee);
         KG_NODE_TRY(cudaGraphInstantiate(&E.x, E.g, 0));
-        E.key_bufs = bufs;
+        E.key = key;
         E.key_iterations = cfg.iterations;
         E.key_dev = dev;
         E.key_st = st;
     }
     std::memcpy(htab, table.data(), sizeof(CohortDev) * n_jobs);
-    KG_NODE_TRY(cudaMemsetAsync(counts, 0, off_done + sizeof(unsigned long long) * n_jobs, st));
+    KG_NODE_TRY(cudaMemsetAsync(counts, 0, ctl_bytes, st));
     NodeDev* h_nodes = reinterpret_cast<NodeDev*>(htab + off_nodes);
     NodeSeg* h_seg = reinterpret_cast<NodeSeg*>(htab + off_seg);
     RunCounters* d_run = reinterpret_cast<RunCounters*>(counts + off_run);
+    const WaveClock* d_clk = reinterpret_cast<const WaveClock*>(counts + off_clk);
     int job = 0;
     int64_t at = 0;   // the job's next pair, y-major
     bool limit_hit = false;
-    double build_ms = 0.0, pass_ms = 0.0, solve_ms = 0.0;
+    double build_ms = 0.0;
     uint64_t waves = 0, launches = 0;
     while (job < n_jobs && !limit_hit) {
         // the next chunk of pairs
         int n_seg = 0;
         int64_t n = 0;
-        std::vector<int> in;
         while (job < n_jobs && n < cap) {
             const int64_t np = table[job].n_pairs, take = std::min<int64_t>(np - at, cap - n);
             if (take > 0) {
@@ -991,11 +1520,9 @@ int run_nodes(const std::vector<PairJob>& jobs, const RunConfig& cfg, Workspace&
                 NodeDev& nd = h_nodes[job];
                 nd.w = ws.scratch.as<double>();
                 nd.stride = stride;
-                nd.slot0 = 0;
                 nd.nk = c.nd_n * J;
                 nd.t = c.nd_t.as<double>();
                 nd.scale = std::ldexp(1.0, -(8 * NODE_L - 2));
-                in.push_back(job);
                 n_seg++;
                 n += take;
                 at += take;
@@ -1008,8 +1535,8 @@ int run_nodes(const std::vector<PairJob>& jobs, const RunConfig& cfg, Workspace&
         KG_NODE_TRY(cudaMemcpyAsync(dtab, htab, blob, cudaMemcpyHostToDevice, st));
         KG_NODE_TRY(cudaEventRecord(E.ev[0], st));
         for (int k = 0; k < n_seg; k++) {
-            const Cohort& c = *jobs[in[k]].panel;
             const NodeSeg& g = h_seg[k];
+            const Cohort& c = *jobs[g.job].panel;
             NodeProduct P;
             P.planes = c.nd_planes.as<uint2>();
             P.dig = c.nd_dig.as<int8_t>();
@@ -1021,73 +1548,69 @@ int run_nodes(const std::vector<PairJob>& jobs, const RunConfig& cfg, Workspace&
             P.idx0 = g.idx0;
             P.idx1 = g.idx0 + g.n;
             P.slot0 = g.slot0;
-            auto y_of = [](int64_t idx) {
-                int64_t y = (int64_t)((std::sqrt(8.0 * (double)idx + 1.0) - 1.0) * 0.5);
-                while (y > 0 && y * (y + 1) / 2 > idx) y--;
-                while ((y + 1) * (y + 2) / 2 <= idx) y++;
-                return y;
-            };
-            P.y0 = y_of(P.idx0);
-            P.first_unit = yx_before(P.y0);
-            P.n_yx = yx_before(y_of(P.idx1 - 1) + 1) - P.first_unit;
+            int64_t x, y0, y1;
+            pair_of(P.idx0, x, y0);
+            pair_of(P.idx1 - 1, x, y1);
+            P.first_unit = yx_before(y0);
+            P.n_yx = yx_before(y1 + 1) - P.first_unit;
             P.w = ws.scratch.as<double>();
             P.stride = stride;
             P.stalled = &d_run->stalled_waits;
             const int grid = (int)std::min<int64_t>(ws.sm_count, P.n_yx * P.bins);
             node_weights_kernel<<<grid, NW_THREADS, NW_SMEM, st>>>(P);
         }
-        node_init_kernel<<<(int)((n + 127) / 128), 128, 0, st>>>(
-            E.args[0], reinterpret_cast<const NodeSeg*>(dtab + off_seg), n_seg, (int)n,
-            cfg.max_waves ? cfg.max_waves - waves : bound);
+        launches += n_seg + 1;
         KG_NODE_TRY(cudaGetLastError());
         KG_NODE_TRY(cudaEventRecord(E.ev[1], st));
-        launches += n_seg + 1;
-        const WaveClock* d_clk = reinterpret_cast<const WaveClock*>(counts + off_clk);
-        if (host_waves) {
-            for (uint64_t k = 0;; k++) {
-                E.wave((int)(k & 1), st);
-                wave_end_kernel<<<1, 32, 0, st>>>(E.args[k & 1], 0, cudaGraphConditionalHandle{}, 0);
-                KG_NODE_TRY(cudaMemcpyAsync(h_clk, d_clk, sizeof(WaveClock), cudaMemcpyDeviceToHost, st));
-                KG_NODE_TRY(cudaStreamSynchronize(st));
-                launches += 5;
-                if (h_clk->stop) break;
-            }
+        if (cls) {
+            const int grid = (int)std::min<int64_t>(E.cls_blocks, (n + NA_THREADS - 1) / NA_THREADS);
+            node_cls_kernel<<<grid, NA_THREADS, 0, st>>>(E.args[0], n_seg, (int)n);
         } else {
-            KG_NODE_TRY(cudaGraphLaunch(E.x, st));
+            node_init_kernel<<<(int)((n + 127) / 128), 128, 0, st>>>(E.args[0], n_seg, (int)n,
+                                                                     cfg.max_waves ? cfg.max_waves - waves : bound);
+            if (host_waves) {
+                for (uint64_t k = 0;; k++) {
+                    E.wave((int)(k & 1), 0, cudaGraphConditionalHandle{}, st);
+                    KG_NODE_TRY(cudaMemcpyAsync(h_clk, d_clk, sizeof(WaveClock), cudaMemcpyDeviceToHost, st));
+                    KG_NODE_TRY(cudaStreamSynchronize(st));
+                    launches += 2;
+                    if (h_clk->stop) break;
+                }
+            } else {
+                KG_NODE_TRY(cudaGraphLaunch(E.x, st));
+            }
         }
+        KG_NODE_TRY(cudaGetLastError());
         KG_NODE_TRY(cudaMemcpyAsync(h_clk, d_clk, sizeof(WaveClock) + sizeof(RunCounters), cudaMemcpyDeviceToHost, st));
         KG_NODE_TRY(cudaStreamSynchronize(st));
-        if (!host_waves) launches += 10 * h_clk->iters;
+        if (!host_waves && !cls) launches += 4 * h_clk->iters;
         float ms = 0.f;
         KG_NODE_TRY(cudaEventElapsedTime(&ms, E.ev[0], E.ev[1]));
         build_ms += ms;
-        waves += h_clk->waves;
-        limit_hit = h_clk->limit_hit != 0 || (cfg.max_waves && waves >= cfg.max_waves && job < n_jobs);
+        waves += cls ? 1 : h_clk->waves;
+        limit_hit = !cls && (h_clk->limit_hit != 0 || (cfg.max_waves && waves >= cfg.max_waves && job < n_jobs));
         if (h_run->stalled_waits) {
             err = "a device wait of the node weights ran out of its limit";
             return KG_ETIMEOUT;
         }
     }
-    pass_ms = (double)h_clk->acc[1] * 1e-6;
-    solve_ms = (double)h_clk->acc[2] * 1e-6;
     const RunCounters& rc = *h_run;
-    stats.gh_passes = rc.gh_passes;
-    stats.obj_passes = rc.obj_passes;
-    stats.fp64_passes = rc.fp64_passes;
+    stats.gh_passes = cls ? (uint64_t)total : rc.gh_passes;
+    stats.obj_passes = stats.gh_passes;
+    stats.fp64_passes = cls ? 0 : rc.gh_passes;   // every pass over nodes is FP64
     stats.fp64_pairs = rc.fp64_pairs;
     stats.pair_sites = rc.pair_sites;
     stats.work_units = rc.work_units;
     stats.launches = launches;
-    stats.flops_fp32 = rc.flops_fp32;
     stats.flops_fp64 = rc.flops_fp64;
     for (int k = 0; k < 5; k++) stats.shape_sites[k] = rc.shape_sites[k];
     stats.nonconverged = rc.nonconverged;
     stats.waves = waves;
     stats.slots = (uint64_t)cap;
     stats.admit_ms = build_ms;
-    stats.pass_ms = pass_ms;
-    stats.solve_ms = solve_ms;
-    stats.pair_kernel_ms = build_ms + pass_ms + solve_ms;
+    stats.pass_ms = (double)h_clk->acc[1] * 1e-6;
+    stats.solve_ms = (double)h_clk->acc[2] * 1e-6;
+    stats.pair_kernel_ms = stats.admit_ms + stats.pass_ms + stats.solve_ms;
     if (limit_hit) {
         err = "the wave loop reached its wave limit";
         return KG_ETIMEOUT;

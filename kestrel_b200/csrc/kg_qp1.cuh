@@ -7,8 +7,8 @@
 //
 // It computes what the row-parallel form (qp_simplex_rows in kg_rowsolve.cuh)
 // computes, operation for operation and in the same order (the same FMAs,
-// quotients and sequential sums), so both give the same bits; with a thread
-// per slot a warp serves 32 pairs' QPs instead of two.
+// quotients and sequential sums), so both give the same bits (FAST: to an ulp of
+// each quotient); with a thread per slot a warp serves 32 pairs' QPs instead of two.
 //
 // The lanes' free sets differ, so the code has no branch on them: a fixed
 // variable's rows and columns are zeros and its pivot 1, which adds exact
@@ -31,7 +31,24 @@ __host__ __device__ __forceinline__ int popc9(unsigned v) {
     return n;
 }
 
-// c / d, given r = 1 / d correctly rounded.
+// 1 / d: the correctly rounded quotient, or (FAST) the hardware's approximation
+// and one cubic Newton step, to an ulp, at a third of the latency (a division
+// is a chain of 127 cycles, and an iteration has a pivot's in each of its nine
+// columns one after the other).
+template <bool FAST>
+__host__ __device__ __forceinline__ double recip(double d) {
+#ifdef __CUDA_ARCH__
+    if (FAST) {
+        double r;
+        asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(d));
+        const double e = fma(-d, r, 1.0);
+        return fma(fma(e, e, e), r, r);
+    }
+#endif
+    return 1.0 / d;
+}
+
+// c / d, given r = 1 / d; correctly rounded when r is.
 __host__ __device__ __forceinline__ double quot(double c, double d, double r) {
     const double q = c * r;
     return fma(fma(-q, d, c), r, q);
@@ -42,10 +59,42 @@ __host__ __device__ constexpr int upper_at(int i, int j) { return i * 9 - i * (i
 constexpr int QP_Q = 45;   // upper triangle of Q, then c
 constexpr int QP_IN = 54;
 
+// Column j of the factorisation and the ones after it.
+template <int j, bool FAST, class QF>
+__host__ __device__ __forceinline__ void ldl_columns(const QF& Q, unsigned F, double beta2, double rbeta2, double delta,
+                                                     double (&L)[36], double (&d)[9], double (&rd)[9]) {
+    const bool jf = (F >> j) & 1u;
+    double p[9];
+    double sjj = 0.0;
+#pragma unroll
+    for (int s = 0; s < j; s++) {
+        const double ljs = L[j * (j - 1) / 2 + s];
+        p[s] = d[s] * ljs;
+        sjj = fma(p[s], ljs, sjj);
+    }
+    const double cjj = Q(j, j) - sjj;
+    double theta = 0.0;
+#pragma unroll
+    for (int i = j + 1; i < 9; i++) {
+        double sij = 0.0;
+#pragma unroll
+        for (int s = 0; s < j; s++) sij = fma(p[s], L[i * (i - 1) / 2 + s], sij);
+        const double cij = jf && ((F >> i) & 1u) ? Q(j, i) - sij : 0.0;
+        L[i * (i - 1) / 2 + j] = cij;
+        theta = fmax(theta, fabs(cij));
+    }
+    const double dj = fmax(fmax(fabs(cjj), quot(theta * theta, beta2, rbeta2)), delta);
+    d[j] = jf ? dj : 1.0;
+    rd[j] = recip<FAST>(d[j]);
+#pragma unroll
+    for (int i = j + 1; i < 9; i++) L[i * (i - 1) / 2 + j] = quot(L[i * (i - 1) / 2 + j], d[j], rd[j]);
+    if constexpr (j + 1 < 9) ldl_columns<j + 1, FAST>(Q, F, beta2, rbeta2, delta, L, d, rd);
+}
+
 // GMW81-modified LDL^T of the free block (mask F, nf free): L strictly lower
 // (row i at i (i - 1) / 2), d the pivots, rd their reciprocals; fixed variables
 // have zero rows and columns and pivot 1.  Q(i, j) reads the upper triangle.
-template <class QF>
+template <bool FAST, class QF>
 __host__ __device__ __forceinline__ void ldl_gmw_thread(const QF& Q, unsigned F, int nf, double (&L)[36],
                                                         double (&d)[9], double (&rd)[9]) {
     double gamma = 0.0, xi = 0.0;
@@ -61,38 +110,8 @@ __host__ __device__ __forceinline__ void ldl_gmw_thread(const QF& Q, unsigned F,
     const double t = sqrt((double)nf * (double)nf - 1.0);
     const double ratio = (nf <= 1) ? 0.0 : xi / t;
     const double beta2 = fmax(fmax(gamma, ratio), eps);
-    const double rbeta2 = 1.0 / beta2;
-#pragma unroll
-    for (int j = 0; j < 9; j++) {
-        const bool jf = (F >> j) & 1u;
-        double p[9];
-        double sjj = 0.0;
-#pragma unroll
-        for (int s = 0; s < j; s++) {
-            const double ljs = L[j * (j - 1) / 2 + s];
-            p[s] = d[s] * ljs;
-            sjj = fma(p[s], ljs, sjj);
-        }
-        const double cjj = Q(j, j) - sjj;
-        double theta = 0.0;
-#pragma unroll
-        for (int i = j + 1; i < 9; i++) {
-            double sij = 0.0;
-#pragma unroll
-            for (int s = 0; s < j; s++) sij = fma(p[s], L[i * (i - 1) / 2 + s], sij);
-            const double cij = jf && ((F >> i) & 1u) ? Q(j, i) - sij : 0.0;
-            L[i * (i - 1) / 2 + j] = cij;
-            theta = fmax(theta, fabs(cij));
-        }
-        const double dj = fmax(fmax(fabs(cjj), quot(theta * theta, beta2, rbeta2)), delta);
-        d[j] = jf ? dj : 1.0;
-        rd[j] = 1.0 / d[j];
-#pragma unroll
-        for (int i = j + 1; i < 9; i++) {
-            double& l = L[i * (i - 1) / 2 + j];
-            l = quot(l, d[j], rd[j]);
-        }
-    }
+    const double rbeta2 = recip<FAST>(beta2);
+    ldl_columns<0, FAST>(Q, F, beta2, rbeta2, delta, L, d, rd);
 }
 
 // L D L^T z = b for two right-hand sides (zero at fixed variables), in the
@@ -130,7 +149,7 @@ __host__ __device__ __forceinline__ void ldl_solve2_thread(const double (&L)[36]
 
 // The QP from y (in) to y (out); in(k): the upper triangle of Q (row-major,
 // k < 45), then c.  Returns the iteration count.
-template <class In>
+template <bool FAST, class In>
 __host__ __device__ __forceinline__ int qp_simplex_thread(const In& in, const Tune& tu, double (&y)[9]) {
     auto Q = [&](int i, int j) { return in(i <= j ? upper_at(i, j) : upper_at(j, i)); };
     unsigned work = 0;
@@ -142,7 +161,7 @@ __host__ __device__ __forceinline__ int qp_simplex_thread(const In& in, const Tu
             double s = 0.0;
 #pragma unroll
             for (int i = 0; i < 9; i++) s += y[i];
-            const double rs = 1.0 / s;
+            const double rs = recip<FAST>(s);
 #pragma unroll
             for (int i = 0; i < 9; i++) y[i] = quot(y[i], s, rs);
         }
@@ -164,7 +183,7 @@ __host__ __device__ __forceinline__ int qp_simplex_thread(const In& in, const Tu
         }
         {
             double L[36], d[9], rd[9];
-            ldl_gmw_thread(Q, F, nf, L, d, rd);
+            ldl_gmw_thread<FAST>(Q, F, nf, L, d, rd);
             ldl_solve2_thread(L, d, rd, gf, on);
         }
         double sg = 0.0, so = 0.0;
@@ -196,7 +215,8 @@ __host__ __device__ __forceinline__ int qp_simplex_thread(const In& in, const Tu
             for (int i = 0; i < 9; i++) {
                 const double pv = ((work >> i) & 1u) ? 0.0 : gf[i];
                 gf[i] = pv;
-                const double a = -y[i] / (pv < 0.0 ? pv : -1.0);
+                const double den = pv < 0.0 ? pv : -1.0;
+                const double a = FAST ? -y[i] * recip<FAST>(den) : -y[i] / den;
                 if (pv < 0.0 && a < alpha) { alpha = a; block = i; }
             }
 #pragma unroll

@@ -7,7 +7,6 @@
 
 #include "kg_engine.h"
 #include "kg_bulk.cuh"
-#include "kg_node.h"
 #include "kg_qp1.cuh"
 #include "kg_wave.cuh"
 
@@ -21,6 +20,8 @@ namespace kg {
             return e_ == cudaErrorMemoryAllocation ? KG_ENOMEM : KG_ECUDA;      \
         }                                                                       \
     } while (0)
+
+constexpr int WAVE_WPB = 4;   // warps per block of the three wave kernels
 
 // ------------------------------------------------------------------ admit
 
@@ -1003,20 +1004,15 @@ __device__ inline void finish_slot(const WaveArgs& A, SlotState& S, int s, const
         if (iters >= co.max_iter) atomicAdd(&C->nonconverged, 1ull);
         const int p32 = co.method == ESTIMATOR_CLS ? 0 : S.gh - S.f64p;   // the ML site arithmetic only
         unsigned long long f32 = 0, f64 = 0;
-        const unsigned long long nk = A.nodes ? (unsigned long long)A.nodes[S.cohort].nk : 0ull;
         for (int sh = 0; sh < 5; sh++) {
             atomicAdd(&C->shape_sites[sh], (unsigned long long)S.cnt[sh]);
-            if (A.nodes) {   // evaluations at nodes, two genotype pairs a shape (het-het: one)
-                if (co.method != ESTIMATOR_CLS) f64 += nk * (unsigned long long)((sh == 4 ? 1 : 2) * S.f64p * flops_fp64(sh));
-                continue;
-            }
             f32 += (unsigned long long)S.cnt[sh] * (unsigned long long)(p32 * flops4_fp32_hi(sh) + S.diffp * flops4_diff_extra(sh));
             f64 += (unsigned long long)S.cnt[sh] * (unsigned long long)(S.f64p * flops_fp64(sh));
         }
         atomicAdd(&C->flops_fp32, f32 / 4);
         atomicAdd(&C->flops_fp64, f64);
         S.status = SLOT_FREE;
-        if (!A.nodes) A.free_next[atomicAdd(&A.wc_next->n_free, 1)] = s;
+        A.free_next[atomicAdd(&A.wc_next->n_free, 1)] = s;
         atomicAdd(&A.cohort_done[S.cohort], 1ull);
     }
 }
@@ -1094,7 +1090,7 @@ __device__ inline void schedule_pass(const WaveArgs& A, SlotState& S, int s, int
         S.ev = ev;
         set_coefficients(S, kind);
     }
-    if (!A.nodes && kind == PASS_FP64 && !S.lists64) {
+    if (kind == PASS_FP64 && !S.lists64) {
         if (lane == 0) {
             S.status = SLOT_RESORT;
             A.free_next[atomicAdd(&A.wc_next->n_free, 1)] = s;
@@ -1103,42 +1099,28 @@ __device__ inline void schedule_pass(const WaveArgs& A, SlotState& S, int s, int
         return;
     }
     if (lane == 0) S.status = SLOT_PASS;
-    if (A.nodes) {
-        if (lane == 0) A.pass_next[atomicAdd(&A.wc_next->n_pass, 1)] = s;
-        return;
-    }
     grp.sync();
     enqueue_pass<16>(A.pass_next, A.tasks_next, A.task_cap, A.wc_next, s, S, lane, grp.mask, A.unit_elems);
 }
 
-// The pair's sites per shape from the counts of its genotype pairs (two a
-// shape, het-het one).
-__device__ __forceinline__ void node_counts(const WaveArgs& A, SlotState& S, int s) {
-    const int* c = A.node_cnt + (int64_t)s * NODE_UNITS;
-    int64_t n = 0;
-    for (int sh = 0; sh < 5; sh++) {
-        S.cnt[sh] = c[2 * sh] + (sh < 4 ? c[2 * sh + 1] : 0);
-        n += S.cnt[sh];
-    }
-    S.n = n;
-}
-
-// A pair without a jointly called site: a row of NaN.
-__device__ inline void finish_nosite(const WaveArgs& A, SlotState& S, int lane) {
-    const CohortDev& co = A.cohorts[S.cohort];
-    double nan9[9];
-    for (int i = 0; i < 9; i++) nan9[i] = CUDART_NAN;
-    write_row(co.out + (S.k - co.pair_begin), S.x, S.y, nan9, CUDART_NAN, 0, CUDART_NAN, lane);
-    if (lane == 0) {
-        S.status = SLOT_FREE;
-        atomicAdd(&A.counters->nosite_pairs, 1ull);
-        atomicAdd(&A.cohort_done[S.cohort], 1ull);
-    }
-}
-
-__device__ __forceinline__ void solve_slot(const WaveArgs& A, int i, int lane, const HalfGrp& grp, double* mom_s) {
+// Two slots per warp, one per half-warp (the row-parallel solver needs nine
+// lanes), four blocks of four warps per SM (at most 128 registers a thread):
+// the solver is latency-bound, so warps count for more than the few spilled
+// values.  `lane` below is the lane's index in its half.
+extern "C" __global__ void __launch_bounds__(128, 4) wave_solve_kernel(WaveArgs A) {
+    extern __shared__ __align__(16) char smem[];
+    const int wib = threadIdx.x >> 5, half = (threadIdx.x >> 4) & 1;
+    const int lane = threadIdx.x & 15;
+    const HalfGrp grp{half ? 0xFFFF0000u : 0x0000FFFFu};
+    const int i = (blockIdx.x * WAVE_WPB + wib) * 2 + half;
+    if (A.clk->stop) return;   // a device loop past its last wave
+    if (threadIdx.x == 0) atomicMin(&A.clk->start[2], global_ns());
+    const PhaseEnd pe{&A.clk->end[2], (threadIdx.x & 31) == 0};
+    if (i >= A.wc_cur->n_pass) return;
     const int s = A.pass_cur[i];
     SlotState& S = A.slots[s];
+    char* wsm = smem + wib * WARP_SMEM;
+    double* mom_s = reinterpret_cast<double*>(wsm) + half * 64;
     const Tune& tu = A.tune;
     // ---- sum the units' partials in unit order: lane owns moments lane,
     // lane + 16 and lane + 32 (45 = the objective); a moment's units are those
@@ -1170,20 +1152,9 @@ __device__ __forceinline__ void solve_slot(const WaveArgs& A, int i, int lane, c
     grp.sync();
     const int kind = S.kind;
     if (kind == PASS_CLS || kind == PASS_CLS64) {
-        if (A.nodes && lane == 0) node_counts(A, S, s);
         if (lane == 0) S.gh++;
-        grp.sync();
         cls_finish(A, S, s, mom_s, lane, grp);
         return;
-    }
-    if (A.nodes && S.ev == EV_INIT && S.kind == PASS_FP64) {
-        // the pair's first pass over its nodes gave its site counts
-        if (lane == 0) node_counts(A, S, s);
-        grp.sync();
-        if (S.n == 0) {
-            finish_nosite(A, S, lane);
-            return;
-        }
     }
     const double n = (double)S.n;
     double corr = 0.0;
@@ -1309,10 +1280,7 @@ __device__ __forceinline__ void solve_slot(const WaveArgs& A, int i, int lane, c
         }
     }
     if (conv) {
-        const double cond = condition_rows(grp, x, g, Hr, tu.sqp_conv_tol);
-        // on nodes every pass is FP64: the pairs that FP32 passes would hand over are counted
-        if (A.nodes && A.precision == KG_PREC_FP32C && lane == 0 && !(cond <= COND_RECHECK)) S.escalated = 1;
-        finish_slot(A, S, s, x, f, it, cond, lane);
+        finish_slot(A, S, s, x, f, it, condition_rows(grp, x, g, Hr, tu.sqp_conv_tol), lane);
         return;
     }
     // ---- QP step (src/sqp.rs:78-83): c = g - H x, y = QP(H, c, x).  Its
@@ -1336,26 +1304,6 @@ __device__ __forceinline__ void solve_slot(const WaveArgs& A, int i, int lane, c
     }
 }
 
-// Two slots per warp, one per half-warp (the row-parallel solver needs nine
-// lanes), four blocks of four warps per SM (at most 128 registers a thread):
-// the solver is latency-bound, so warps count for more than the few spilled
-// values.  `lane` is the lane's index in its half.
-extern "C" __global__ void __launch_bounds__(128, 4) wave_solve_kernel(WaveArgs A) {
-    extern __shared__ __align__(16) char smem[];
-    const int wib = threadIdx.x >> 5, half = (threadIdx.x >> 4) & 1;
-    const int lane = threadIdx.x & 15;
-    const HalfGrp grp{half ? 0xFFFF0000u : 0x0000FFFFu};
-    if (A.clk->stop) return;   // a device loop past its last wave
-    if (threadIdx.x == 0) atomicMin(&A.clk->start[2], global_ns());
-    const PhaseEnd pe{&A.clk->end[2], (threadIdx.x & 31) == 0};
-    double* mom_s = reinterpret_cast<double*>(smem + wib * WARP_SMEM) + half * 64;
-    const int n = A.wc_cur->n_pass;
-    for (int i = (blockIdx.x * WAVE_WPB + wib) * 2 + half; i < n; i += gridDim.x * WAVE_WPB * 2) {
-        solve_slot(A, i, lane, grp, mom_s);
-        grp.sync();   // the moments are read before the next slot's
-    }
-}
-
 // The QP of every slot in this wave's QP list, a thread per slot (kg_qp1.cuh,
 // the same arithmetic as the row-parallel form).  The list's QPs lie
 // value-major in memory, so a warp's loads are whole sectors; Q and c stay in
@@ -1365,20 +1313,19 @@ extern "C" __global__ void __launch_bounds__(QP_THREADS) wave_qp_kernel(WaveArgs
     __shared__ double in[QP_IN * QP_THREADS];
     if (A.clk->stop) return;   // a device loop past its last wave
     const PhaseEnd pe{&A.clk->end[2], (threadIdx.x & 31) == 0};   // timed as part of the solve phase
-    const int n = A.wc_cur->n_qp;
+    const int i = blockIdx.x * QP_THREADS + threadIdx.x;
+    if (i >= A.wc_cur->n_qp) return;
     const int64_t st = A.n_slots;
     double* my = in + threadIdx.x;
-    for (int i = blockIdx.x * QP_THREADS + threadIdx.x; i < n; i += gridDim.x * QP_THREADS) {
-        double* Qb = A.qp_buf + i;
+    double* Qb = A.qp_buf + i;
 #pragma unroll
-        for (int v = 0; v < QP_IN; v++) my[v * QP_THREADS] = Qb[v * st];
-        double y[9];
+    for (int v = 0; v < QP_IN; v++) my[v * QP_THREADS] = Qb[v * st];
+    double y[9];
 #pragma unroll
-        for (int k = 0; k < 9; k++) y[k] = Qb[(QP_IN + k) * st];
-        qp_simplex_thread([my](int v) { return my[v * QP_THREADS]; }, A.tune, y);
+    for (int k = 0; k < 9; k++) y[k] = Qb[(QP_IN + k) * st];
+    qp_simplex_thread<false>([my](int v) { return my[v * QP_THREADS]; }, A.tune, y);
 #pragma unroll
-        for (int k = 0; k < 9; k++) Qb[(QP_IN + k) * st] = y[k];
-    }
+    for (int k = 0; k < 9; k++) Qb[(QP_IN + k) * st] = y[k];
 }
 
 // The step after each QP (src/sqp.rs:78-90): p = y - x, the first trial point
@@ -1387,36 +1334,35 @@ extern "C" __global__ void __launch_bounds__(128) wave_step_kernel(WaveArgs A) {
     const int wib = threadIdx.x >> 5, half = (threadIdx.x >> 4) & 1;
     const int lane = threadIdx.x & 15;
     const HalfGrp grp{half ? 0xFFFF0000u : 0x0000FFFFu};
+    const int i = (blockIdx.x * WAVE_WPB + wib) * 2 + half;
     if (A.clk->stop) return;   // a device loop past its last wave
     const PhaseEnd pe{&A.clk->end[2], (threadIdx.x & 31) == 0};
-    const int n = A.wc_cur->n_qp;
-    for (int i = (blockIdx.x * WAVE_WPB + wib) * 2 + half; i < n; i += gridDim.x * WAVE_WPB * 2) {
-        const int s = A.qp_list[i];
-        SlotState& S = A.slots[s];
-        const double* Qb = A.qp_buf + i;
-        double x[9], g[9], p[9];
+    if (i >= A.wc_cur->n_qp) return;
+    const int s = A.qp_list[i];
+    SlotState& S = A.slots[s];
+    const double* Qb = A.qp_buf + i;
+    double x[9], g[9], p[9];
 #pragma unroll
-        for (int k = 0; k < 9; k++) {
-            x[k] = S.xc[k];
-            g[k] = S.g[k];
-            p[k] = Qb[(QP_IN + k) * (int64_t)A.n_slots] - x[k];
-        }
-        const double gp = dot_fma(9, g, p);
-        double xn[9];
-#pragma unroll
-        for (int k = 0; k < 9; k++) xn[k] = x[k] + 1.0 * p[k];
-        normalise9(xn);
-        const bool fp64 = S.fp64 != 0;
-        const int nkind = fp64 ? PASS_FP64 : (fabs(gp) < DIFF_BELOW ? PASS_FP32_DIFF : PASS_FP32_DIRECT);
-        grp.sync();   // every lane has read S before lane 0 writes it
-        if (lane == 0) {
-            for (int k = 0; k < 9; k++) { S.p[k] = p[k]; S.xt[k] = xn[k]; }
-            S.gp = gp;
-            S.alpha = 1.0;
-            S.bls = 0;
-        }
-        schedule_pass(A, S, s, nkind, EV_TRIAL, lane, grp);
+    for (int k = 0; k < 9; k++) {
+        x[k] = S.xc[k];
+        g[k] = S.g[k];
+        p[k] = Qb[(QP_IN + k) * (int64_t)A.n_slots] - x[k];
     }
+    const double gp = dot_fma(9, g, p);
+    double xn[9];
+#pragma unroll
+    for (int k = 0; k < 9; k++) xn[k] = x[k] + 1.0 * p[k];
+    normalise9(xn);
+    const bool fp64 = S.fp64 != 0;
+    const int nkind = fp64 ? PASS_FP64 : (fabs(gp) < DIFF_BELOW ? PASS_FP32_DIFF : PASS_FP32_DIRECT);
+    grp.sync();   // every lane has read S before lane 0 writes it
+    if (lane == 0) {
+        for (int k = 0; k < 9; k++) { S.p[k] = p[k]; S.xt[k] = xn[k]; }
+        S.gp = gp;
+        S.alpha = 1.0;
+        S.bls = 0;
+    }
+    schedule_pass(A, S, s, nkind, EV_TRIAL, lane, grp);
 }
 
 // ------------------------------------------------------------------- host
@@ -1446,7 +1392,7 @@ __global__ void wave_end_kernel(WaveArgs A, int last, cudaGraphConditionalHandle
         const WaveCounts& n = *A.wc_next;
         if (n.n_pass == 0 && n.n_resort == 0 && *A.queue >= (unsigned long long)A.live->total_pairs) {
             c->stop = 1;
-        } else if (c->waves >= (c->max_waves ? c->max_waves : max_waves)) {
+        } else if (c->waves >= max_waves) {
             c->stop = 1;
             c->limit_hit = 1;
         }

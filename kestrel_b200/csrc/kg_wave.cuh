@@ -82,7 +82,6 @@ struct WaveClock {
     unsigned long long acc[3];     // summed over the waves of the device loop
     unsigned long long waves;      // waves the device loop ran
     unsigned long long iters;      // loop bodies (two wave slots each)
-    unsigned long long max_waves;  // kg_node.cu: waves this loop may run (0: wave_end_kernel's argument)
     unsigned int stop;             // set once the job is done or the limit is hit
     unsigned int limit_hit;
 };
@@ -137,29 +136,7 @@ struct WaveArgs {
     double* qp_buf;                // value v of the wave's QP i at [v * n_slots + i]: Q's upper triangle, c, y (in: x)
     int* qp_list;                  // the slots of this wave's QPs (wc_cur->n_qp of them)
     int unit_elems;                // list entries per pass work unit
-    // pairs on frequency nodes (kg_node.cu) instead of site lists: no admit
-    // step, no task lists, every pass FP64 over the pair's nodes
-    const struct NodeDev* nodes;   // per job of the table (NULL: site lists)
-    int* node_cnt;                 // per slot and unit: the pair's sites, from its first pass
 };
-
-// A job's nodes in the current chunk of pairs: W of slot s at w[(u nk + i) *
-// stride + s - slot0], u a genotype pair, i a node.
-struct NodeDev {
-    const double* w;
-    int64_t stride;
-    int32_t slot0;
-    int32_t nk;           // nodes per genotype pair (bins x nodes per bin)
-    const double* t;      // their table (kg_node.cu), genotypes folded to the rarer allele
-    double scale;         // what a unit of an (integer) weight stands for
-};
-
-// The steps after a pass, also launched by kg_node.cu (kg_wave.cu).
-extern "C" __global__ void wave_solve_kernel(WaveArgs A);
-extern "C" __global__ void wave_qp_kernel(WaveArgs A);
-extern "C" __global__ void wave_step_kernel(WaveArgs A);
-__global__ void wave_end_kernel(WaveArgs A, int last, cudaGraphConditionalHandle loop, unsigned long long max_waves);
-constexpr int WAVE_WPB = 4;   // warps per block of the wave kernels
 
 // Work units of the ML path's tri- and tetra-allelic sites: at most ML_CHUNK
 // kept sites each, the largest cohort's sites split evenly; per unit 9
