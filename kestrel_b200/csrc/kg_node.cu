@@ -260,13 +260,22 @@ int prepare_nodes(Cohort& c, const uint8_t* codes, int64_t stride, int bins, dou
 // into shared memory in the 128-byte swizzle.  With A in shared memory its
 // 48 KB a stage would be written and read again through the 128 B/clk port,
 // which B's 12 KB written and 36 KB read already keep busy half the time.
-// Per stage of 128 sites: 12 instructions of 48 cycles; two stages, so the
-// expansion of one runs under the products of the other.
-constexpr int NW_THREADS = 416;          // 4 warps expand A, 4 expand B, 4 read out, 1 issues
+// Per stage of 128 sites: 12 instructions of 48 cycles.  Expanding A takes a
+// warp longer than that (250 instructions, half of them at half rate, and the
+// tensor-memory stores behind a wait), so two groups of four warps take half a
+// stage each, into four half-stage buffers, and every expansion is in registers
+// before its buffer is waited for.  A lone issuing thread was what bound the
+// first form (18.2 ms at 1024 samples x 100,000 sites against 7.6 ms of
+// instructions): a wait on a barrier that is long complete takes it 270 cycles,
+// an instruction 30.  So three warps issue, one a genotype of x (their
+// accumulators are apart), all lanes converged (one thread of a diverged warp
+// took 25.5 ms), with one wait and one commit a half-stage.
+constexpr int NW_THREADS = 608;          // 2 x 4 warps expand A, 4 expand B, 4 read out, 3 issue
 constexpr int NW_N = 96;                 // B's rows: 3 genotypes of y x 32 columns
 constexpr int NW_BSTAGE = NW_N * NODE_STAGE;
 constexpr int NW_STAGES = 2;
-constexpr uint32_t NW_TM_A = 320;        // tensor-memory column of A's stages (D: 0 .. 287)
+constexpr int NW_AHEAD = 2;              // stages whose planes and digits a thread has in flight
+constexpr uint32_t NW_TM_A = 320;        // tensor-memory column of A's half-stages, 48 each (D: 0 .. 287)
 constexpr int NW_SMEM = 120 * 1024;      // more than half an SM's: one block (it owns the tensor memory)
 
 struct NodeProduct {
@@ -318,22 +327,24 @@ __device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
 __global__ void __launch_bounds__(NW_THREADS, 1) node_weights_kernel(NodeProduct P) {
     constexpr int J = NODE_J, L = NODE_L;
     extern __shared__ __align__(1024) unsigned char nw_smem[];
-    __shared__ __align__(8) uint64_t full[NW_STAGES], empty[NW_STAGES], acc_full, acc_empty;
+    // buffer 2 stage + half; B's stage arrives with its first half and is free
+    // with its second
+    __shared__ __align__(8) uint64_t full[2 * NW_STAGES], empty[2 * NW_STAGES], acc_full, acc_empty;
     __shared__ uint32_t tm_slot;
     __shared__ int gave_up;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const uint32_t b0 = (smem_u32(nw_smem) + 1023u) & ~1023u;
     if (threadIdx.x == 0) {
-        for (int i = 0; i < NW_STAGES; i++) {
-            mbar_init(&full[i], 8);     // the eight expanding warps
-            mbar_init(&empty[i], 1);
+        for (int i = 0; i < 2 * NW_STAGES; i++) {
+            mbar_init(&full[i], (i & 1) ? 4 : 8);   // four warps of A's, with the first half four of B's
+            mbar_init(&empty[i], 3);                // the issuing warps
         }
-        mbar_init(&acc_full, 1);
+        mbar_init(&acc_full, 3);
         mbar_init(&acc_empty, 4);
         gave_up = 0;
         fence_mbar_init();
     }
-    if (warp == 12) tmem_alloc<512>(smem_u32(&tm_slot));
+    if (warp == 16) tmem_alloc<512>(smem_u32(&tm_slot));
     tmem_fence_before();
     __syncthreads();
     tmem_fence_after();
@@ -341,49 +352,58 @@ __global__ void __launch_bounds__(NW_THREADS, 1) node_weights_kernel(NodeProduct
     const int64_t n_units = P.n_yx * P.bins;
     uint32_t seq = 0;    // stages so far
     bool ok = true;
-    if (warp < 4) {
-        // ---- A: a thread per sample x
-        const uint32_t my = tm + ((uint32_t)(warp * 32) << 16) + NW_TM_A;
+    if (warp < 8) {
+        // ---- A: a thread per sample x; group warp / 4 expands that half of
+        // every stage, into buffers (2 stage + half) % 4
+        const uint32_t half = warp >> 2;
+        const uint32_t my = tm + ((uint32_t)((warp & 3) * 32) << 16) + NW_TM_A + half * 48;
         for (int64_t un = blockIdx.x; ok && un < n_units; un += gridDim.x) {
             const int k = (int)(un / P.n_yx);
             int y, xb;
             decode_yx(P.first_unit + (un - k * P.n_yx), y, xb);
             const NodeBin bn = P.bin[k];
-            const int x = xb * 128 + warp * 32 + lane;
-            const bool live = x < P.n_samples;
-            const uint4* src = reinterpret_cast<const uint4*>(P.planes + (int64_t)(live ? x : 0) * P.words + (bn.start >> 5));
-            uint4 v0 = src[0], v1 = src[1];
-            for (int i = 0; i < bn.stages; i++, seq++) {
-                const uint32_t lo[4] = {v0.x, v0.z, v1.x, v1.z}, hi[4] = {v0.y, v0.w, v1.y, v1.w};
-                if (i + 1 < bn.stages) {
-                    v0 = src[2 * i + 2];
-                    v1 = src[2 * i + 3];
+            const int x = xb * 128 + (warp & 3) * 32 + lane;
+            const uint32_t live = x < P.n_samples ? ~0u : 0u;
+            const uint4* src =
+                reinterpret_cast<const uint4*>(P.planes + (int64_t)(live ? x : 0) * P.words + (bn.start >> 5)) + half;
+            uint4 v[NW_AHEAD];
+#pragma unroll
+            for (int j = 0; j < NW_AHEAD; j++)
+                if (j < bn.stages) v[j] = src[2 * j];
+            for (int i0 = 0; ok && i0 < bn.stages; i0 += NW_AHEAD) {
+#pragma unroll
+                for (int j = 0; j < NW_AHEAD; j++) {
+                    const int i = i0 + j;
+                    if (i >= bn.stages) break;
+                    const uint32_t lo[2] = {v[j].x, v[j].z}, hi[2] = {v[j].y, v[j].w};
+                    if (i + NW_AHEAD < bn.stages) v[j] = src[2 * (i + NW_AHEAD)];
+                    uint32_t r[48];
+#pragma unroll
+                    for (int a = 0; a < 3; a++)
+#pragma unroll
+                        for (int w = 0; w < 2; w++) {
+                            const uint32_t m =
+                                (a == 0 ? ~(lo[w] | hi[w]) : a == 1 ? lo[w] & ~hi[w] : hi[w] & ~lo[w]) & live;
+#pragma unroll
+                            for (int q = 0; q < 8; q++) r[16 * a + 8 * w + q] = (m >> q) & 0x01010101u;
+                        }
+                    const uint32_t st = seq % NW_STAGES;
+                    if (!nw_wait_warp(&empty[2 * st + half], ((seq / NW_STAGES) & 1u) ^ 1u, &gave_up)) { ok = false; break; }
+                    tmem_fence_after();
+#pragma unroll
+                    for (int a = 0; a < 3; a++) tmem_store16(my + st * 96 + a * 16, r + 16 * a);
+                    tmem_store_wait();
+                    tmem_fence_before();
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(&full[2 * st + half]);
+                    seq++;
                 }
-                const uint32_t st = seq % NW_STAGES;
-                if (!nw_wait_warp(&empty[st], ((seq / NW_STAGES) & 1u) ^ 1u, &gave_up)) { ok = false; break; }
-                tmem_fence_after();
-#pragma unroll
-                for (int a = 0; a < 3; a++) {
-                    uint32_t r[32];
-#pragma unroll
-                    for (int w = 0; w < 4; w++) {
-                        uint32_t m = a == 0 ? ~(lo[w] | hi[w]) : a == 1 ? lo[w] & ~hi[w] : hi[w] & ~lo[w];
-                        if (!live) m = 0u;
-#pragma unroll
-                        for (int q = 0; q < 8; q++) r[8 * w + q] = (m >> q) & 0x01010101u;
-                    }
-                    tmem_store32(my + st * 96 + a * 32, r);
-                }
-                tmem_store_wait();
-                tmem_fence_before();
-                __syncwarp();
-                if (lane == 0) mbar_arrive(&full[st]);
             }
         }
-    } else if (warp < 8) {
+    } else if (warp < 12) {
         // ---- B: thread (row, 16-site piece); rows row and row + 16 of the
         // 32 columns, for the three genotypes of y
-        const int tid = threadIdx.x - 128, c = tid & 7, row = tid >> 3;
+        const int tid = threadIdx.x - 256, c = tid & 7, row = tid >> 3;
         for (int64_t un = blockIdx.x; ok && un < n_units; un += gridDim.x) {
             const int k = (int)(un / P.n_yx);
             int y, xb;
@@ -391,42 +411,57 @@ __global__ void __launch_bounds__(NW_THREADS, 1) node_weights_kernel(NodeProduct
             const NodeBin bn = P.bin[k];
             const int8_t* d0 = P.dig + (int64_t)row * P.mp + bn.start + 16 * c;
             const uint2* py = P.planes + (int64_t)y * P.words + (bn.start >> 5) + (c >> 1);
-            uint4 va = *reinterpret_cast<const uint4*>(d0), vb = *reinterpret_cast<const uint4*>(d0 + 16 * P.mp);
-            uint2 pl = py[0];
-            for (int i = 0; i < bn.stages; i++, seq++) {
-                const uint4 da = va, db = vb;
-                const uint32_t lo = pl.x, hi = pl.y;
-                if (i + 1 < bn.stages) {
-                    va = *reinterpret_cast<const uint4*>(d0 + (int64_t)(i + 1) * NODE_STAGE);
-                    vb = *reinterpret_cast<const uint4*>(d0 + 16 * P.mp + (int64_t)(i + 1) * NODE_STAGE);
-                    pl = py[4 * (i + 1)];
-                }
-                const uint32_t st = seq % NW_STAGES;
-                if (!nw_wait_warp(&empty[st], ((seq / NW_STAGES) & 1u) ^ 1u, &gave_up)) { ok = false; break; }
-                const uint32_t base = b0 + st * NW_BSTAGE + ((uint32_t)(c ^ (row & 7)) << 4);
+            uint4 va[NW_AHEAD], vb[NW_AHEAD];
+            uint2 pl[NW_AHEAD];
+            auto fetch = [&](int i, uint4& a4, uint4& b4, uint2& p2) {
+                a4 = *reinterpret_cast<const uint4*>(d0 + (int64_t)i * NODE_STAGE);
+                b4 = *reinterpret_cast<const uint4*>(d0 + 16 * P.mp + (int64_t)i * NODE_STAGE);
+                p2 = py[4 * i];
+            };
 #pragma unroll
-                for (int b = 0; b < 3; b++) {
-                    const uint32_t m = (b == 0 ? ~(lo | hi) : b == 1 ? lo & ~hi : hi & ~lo) >> (4 * (c & 1));
-                    uint32_t f[4];
+            for (int j = 0; j < NW_AHEAD; j++)
+                if (j < bn.stages) fetch(j, va[j], vb[j], pl[j]);
+            for (int i0 = 0; ok && i0 < bn.stages; i0 += NW_AHEAD) {
 #pragma unroll
-                    for (int q = 0; q < 4; q++) f[q] = ((m >> q) & 0x01010101u) * 255u;
-                    const uint32_t at = base + (uint32_t)(b * 32 + row) * 128u;
-                    asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(at), "r"(da.x & f[0]),
-                                 "r"(da.y & f[1]), "r"(da.z & f[2]), "r"(da.w & f[3])
-                                 : "memory");
-                    asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(at + 16u * 128u), "r"(db.x & f[0]),
-                                 "r"(db.y & f[1]), "r"(db.z & f[2]), "r"(db.w & f[3])
-                                 : "memory");
+                for (int j = 0; j < NW_AHEAD; j++) {
+                    const int i = i0 + j;
+                    if (i >= bn.stages) break;
+                    const uint32_t lo = pl[j].x, hi = pl[j].y;
+                    uint4 va3[3], vb3[3];
+#pragma unroll
+                    for (int b = 0; b < 3; b++) {
+                        const uint32_t m = (b == 0 ? ~(lo | hi) : b == 1 ? lo & ~hi : hi & ~lo) >> (4 * (c & 1));
+                        uint32_t f[4];
+#pragma unroll
+                        for (int q = 0; q < 4; q++) f[q] = ((m >> q) & 0x01010101u) * 255u;
+                        va3[b] = make_uint4(va[j].x & f[0], va[j].y & f[1], va[j].z & f[2], va[j].w & f[3]);
+                        vb3[b] = make_uint4(vb[j].x & f[0], vb[j].y & f[1], vb[j].z & f[2], vb[j].w & f[3]);
+                    }
+                    if (i + NW_AHEAD < bn.stages) fetch(i + NW_AHEAD, va[j], vb[j], pl[j]);
+                    const uint32_t st = seq % NW_STAGES;
+                    if (!nw_wait_warp(&empty[2 * st + 1], ((seq / NW_STAGES) & 1u) ^ 1u, &gave_up)) { ok = false; break; }
+                    const uint32_t base = b0 + st * NW_BSTAGE + ((uint32_t)(c ^ (row & 7)) << 4);
+#pragma unroll
+                    for (int b = 0; b < 3; b++) {
+                        const uint32_t at = base + (uint32_t)(b * 32 + row) * 128u;
+                        asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(at), "r"(va3[b].x),
+                                     "r"(va3[b].y), "r"(va3[b].z), "r"(va3[b].w)
+                                     : "memory");
+                        asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(at + 16u * 128u), "r"(vb3[b].x),
+                                     "r"(vb3[b].y), "r"(vb3[b].z), "r"(vb3[b].w)
+                                     : "memory");
+                    }
+                    fence_proxy_async_smem();
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(&full[2 * st]);
+                    seq++;
                 }
-                fence_proxy_async_smem();
-                __syncwarp();
-                if (lane == 0) mbar_arrive(&full[st]);
             }
         }
-    } else if (warp < 12) {
+    } else if (warp < 16) {
         // ---- read-out: a thread per sample x; lanes of consecutive x are
         // consecutive slots
-        const uint32_t my = tm + ((uint32_t)((warp - 8) * 32) << 16);
+        const uint32_t my = tm + ((uint32_t)((warp - 12) * 32) << 16);
         // the genotype pair's number u (see the file comment) of (gx, gy) = (a, b)
         constexpr int UNIT[9] = {0, 2, 6, 4, 8, 5, 7, 3, 1};
         uint32_t n_acc = 0;
@@ -437,7 +472,7 @@ __global__ void __launch_bounds__(NW_THREADS, 1) node_weights_kernel(NodeProduct
             decode_yx(P.first_unit + (un - k * P.n_yx), y, xb);
             if (P.bin[k].stages == 0) {
                 // an empty bin: zero weights, no product
-                const int x = xb * 128 + (warp - 8) * 32 + lane;
+                const int x = xb * 128 + (warp - 12) * 32 + lane;
                 const int64_t idx = (int64_t)y * (y + 1) / 2 + x;
                 if (x <= y && idx >= P.idx0 && idx < P.idx1)
                     for (int u = 0; u < 9; u++)
@@ -448,7 +483,7 @@ __global__ void __launch_bounds__(NW_THREADS, 1) node_weights_kernel(NodeProduct
             if (!nw_wait_warp(&acc_full, n_acc & 1u, &gave_up)) { ok = false; break; }
             n_acc++;
             tmem_fence_after();
-            const int x = xb * 128 + (warp - 8) * 32 + lane;
+            const int x = xb * 128 + (warp - 12) * 32 + lane;
             const int64_t idx = (int64_t)y * (y + 1) / 2 + x;
             const bool store = x <= y && idx >= P.idx0 && idx < P.idx1;
             double* out = P.w + (int64_t)(k * J) * P.stride + P.slot0 + (idx - P.idx0);
@@ -471,30 +506,36 @@ __global__ void __launch_bounds__(NW_THREADS, 1) node_weights_kernel(NodeProduct
                 }
             }
         }
-    } else if (lane == 0) {
-        // ---- the issuing thread
+    } else {
+        // ---- the issuing warps, a genotype of x each: every lane waits, one issues
         constexpr uint32_t idesc = idesc_i8(128, NW_N);
+        const uint32_t a = warp - 16, d = tm + a * NW_N, a0 = tm + NW_TM_A + a * 16;
         uint32_t n_acc = 0;
         for (int64_t un = blockIdx.x; ok && un < n_units; un += gridDim.x) {
             const NodeBin bn = P.bin[un / P.n_yx];
             if (bn.stages == 0) continue;
-            if (!nw_wait(&acc_empty, (n_acc & 1u) ^ 1u, &gave_up)) { ok = false; break; }
+            if (!nw_wait_warp(&acc_empty, (n_acc & 1u) ^ 1u, &gave_up)) { ok = false; break; }
             n_acc++;
             tmem_fence_after();
-            for (int i = 0; i < bn.stages; i++, seq++) {
-                const uint32_t st = seq % NW_STAGES;
-                if (!nw_wait(&full[st], (seq / NW_STAGES) & 1u, &gave_up)) { ok = false; break; }
-                tmem_fence_after();
+            bool add = false;
+            for (int i = 0; ok && i < bn.stages; i++, seq++) {
+                const uint32_t st = seq % NW_STAGES, phase = (seq / NW_STAGES) & 1u;
                 const uint64_t bd = smem_desc_sw128(b0 + st * NW_BSTAGE);
 #pragma unroll
-                for (int q = 0; q < 4; q++)
-#pragma unroll
-                    for (int a = 0; a < 3; a++)
-                        mma_i8_ts(tm + a * NW_N, tm + NW_TM_A + st * 96 + a * 32 + 8 * q, bd + 2 * q, idesc,
-                                  (i | q) != 0);
-                mma_commit(smem_u32(&empty[st]));
+                for (uint32_t half = 0; half < 2; half++) {
+                    if (!nw_wait_warp(&full[2 * st + half], phase, &gave_up)) { ok = false; break; }
+                    tmem_fence_after();
+                    if (elect_one()) {
+                        mma_i8_ts(d, a0 + st * 96 + half * 48, bd + 4 * half, idesc, add);
+                        mma_i8_ts(d, a0 + st * 96 + half * 48 + 8, bd + 4 * half + 2, idesc, true);
+                        mma_commit(smem_u32(&empty[2 * st + half]));
+                    }
+                    __syncwarp();
+                    add = true;
+                }
             }
-            if (ok) mma_commit(smem_u32(&acc_full));
+            if (ok && elect_one()) mma_commit(smem_u32(&acc_full));
+            __syncwarp();
         }
     }
     if (!ok && lane == 0) atomicAdd(P.stalled, 1ull);
@@ -502,7 +543,7 @@ __global__ void __launch_bounds__(NW_THREADS, 1) node_weights_kernel(NodeProduct
     tmem_fence_before();
     __syncthreads();
     tmem_fence_after();
-    if (warp == 12) tmem_free<512>(tm);
+    if (warp == 16) tmem_free<512>(tm);
 }
 
 // --------------------------------------------------------- a chunk's slots
