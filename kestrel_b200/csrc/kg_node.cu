@@ -288,8 +288,8 @@ struct NodeProduct {
     int64_t idx0, idx1;        // the pairs (x <= y) of this chunk: y (y + 1) / 2 + x
     int64_t slot0;             // slot of pair idx0 within w's columns
     int64_t first_unit, n_yx;  // the first (y, x block) in the count from y = 0, how many
-    double* w;
-    int64_t stride;
+    double* w;                 // see NodeDev
+    int64_t group;
     unsigned long long* stalled;
 };
 
@@ -474,10 +474,11 @@ __global__ void __launch_bounds__(NW_THREADS, 1) node_weights_kernel(NodeProduct
                 // an empty bin: zero weights, no product
                 const int x = xb * 128 + (warp - 12) * 32 + lane;
                 const int64_t idx = (int64_t)y * (y + 1) / 2 + x;
+                const int64_t s = P.slot0 + (idx - P.idx0);
                 if (x <= y && idx >= P.idx0 && idx < P.idx1)
                     for (int u = 0; u < 9; u++)
                         for (int j = 0; j < J; j++)
-                            P.w[((int64_t)u * nk + k * J + j) * P.stride + P.slot0 + (idx - P.idx0)] = 0.0;
+                            P.w[(s >> 3) * P.group + ((int64_t)u * nk + k * J + j) * 8 + (s & 7)] = 0.0;
                 continue;
             }
             if (!nw_wait_warp(&acc_full, n_acc & 1u, &gave_up)) { ok = false; break; }
@@ -486,7 +487,8 @@ __global__ void __launch_bounds__(NW_THREADS, 1) node_weights_kernel(NodeProduct
             const int x = xb * 128 + (warp - 12) * 32 + lane;
             const int64_t idx = (int64_t)y * (y + 1) / 2 + x;
             const bool store = x <= y && idx >= P.idx0 && idx < P.idx1;
-            double* out = P.w + (int64_t)(k * J) * P.stride + P.slot0 + (idx - P.idx0);
+            const int64_t s = P.slot0 + (idx - P.idx0);
+            double* out = P.w + (s >> 3) * P.group + (int64_t)(k * J) * 8 + (s & 7);
 #pragma unroll
             for (int ab = 0; ab < 9; ab++) {
                 uint32_t r[32];
@@ -502,7 +504,7 @@ __global__ void __launch_bounds__(NW_THREADS, 1) node_weights_kernel(NodeProduct
                     long long v = (int)r[j * L];
 #pragma unroll
                     for (int d = 1; d < L; d++) v += (long long)(int)r[j * L + d] * (1ll << (8 * d));
-                    if (store) out[((int64_t)UNIT[ab] * nk + j) * P.stride] = (double)v;
+                    if (store) out[((int64_t)UNIT[ab] * nk + j) * 8] = (double)v;
                 }
             }
         }
@@ -554,10 +556,14 @@ struct NodeSeg {
     int32_t slot0, n, job, pad;
 };
 
-// A job's nodes: W of slot s at w[(u nk + i) stride + s], u a genotype pair, i a node.
+// A job's nodes.  The weights of eight slots lie together (64 KB for 14 bins):
+// W of slot s at w[(s / 8) group + (u nk + i) 8 + s % 8], u a genotype pair, i a
+// node.  With the slots of a node together instead (rows of 4 MB at 1024
+// samples) every load of a pass went to another page: 25 ms of passes against
+// 19 ms.
 struct NodeDev {
     const double* w;
-    int64_t stride;
+    int64_t group;
     const double* t;      // the nodes' frequencies (at most 1/2)
     double scale;         // what a unit of the (integer) weights stands for
     int32_t nk;           // nodes per genotype pair: bins x NODE_J
@@ -571,8 +577,14 @@ struct LogTable {
     double exp2[LOG_EXPS];     // (e - 40) log 2
 };
 
-// A slot's SQP state (src/sqp.rs:49-93) between its passes, value-major:
-// value v of slot s at [v * stride + s].
+// Per-slot values lie in blocks of 32 slots, value-major inside: value v of
+// slot s, of V values, at [(s / 32) V 32 + v 32 + s % 32].
+constexpr int NS_LANES = 32;
+__host__ __device__ __forceinline__ int64_t slot_at(int s, int values) {
+    return (int64_t)(s >> 5) * (values * NS_LANES) + (s & 31);
+}
+
+// A slot's SQP state (src/sqp.rs:49-93) between its passes.
 enum : int {
     NS_XC = 0,        // accepted point
     NS_XT = 9,        // point of the pending pass
@@ -600,11 +612,10 @@ struct NodeArgs {
     const CohortDev* cohorts;
     const NodeDev* nodes;      // per job
     const NodeSeg* seg;        // the chunk's runs (ctl->n_seg)
-    int64_t stride;            // slots
-    double* state;             // NS_VALS
-    double* partial;           // UNIT_VALS x NODE_UNITS, value-major
+    double* state;             // NS_VALS values a slot
+    double* partial;           // NODE_PART values a slot
     int4* count;               // {iterations, backtracks, passes, job * 4 + kind} per slot
-    int* sites;                // NODE_UNITS per slot, value-major: the pair's sites by genotype pair
+    int* sites;                // NODE_UNITS values a slot: the pair's sites by genotype pair
     int* list_cur;             // slots with a pending pass
     int* list_next;
     int par;                   // 0: even waves
@@ -614,6 +625,8 @@ struct NodeArgs {
     const LogTable* log_table;
     Tune tune;
 };
+
+constexpr int NODE_PART = UNIT_VALS * NODE_UNITS;   // a pass's sums
 
 // Kinds of a pending pass: the pair's first, direct objective, objective change.
 enum : int { NP_FIRST = 0, NP_DIRECT = 1, NP_DIFF = 2 };
@@ -647,18 +660,18 @@ __device__ __forceinline__ void node_write_row(const CohortDev& co, int64_t x, i
     o->cond = cond;
 }
 
-__device__ __forceinline__ void store_coef(double* v, int64_t stride, const double* x) {
+__device__ __forceinline__ void store_coef(double* v, const double* x) {
     PassCoef k;
     make_coef(x, k);
     const double* c = reinterpret_cast<const double*>(&k);
 #pragma unroll
-    for (int i = 0; i < NS_COEFS; i++) v[i * stride] = c[i];
+    for (int i = 0; i < NS_COEFS; i++) v[i * NS_LANES] = c[i];
 }
 
 // The step xt - xc of a difference pass, less its part along xc: both points
 // add up to 1 only to an ulp, and the objective would change by that ulp (its
 // slope along x itself is -1) where the step's own change is smaller still.
-__device__ __forceinline__ void store_step(double* v, int64_t stride, const double* xt, const double* xc) {
+__device__ __forceinline__ void store_step(double* v, const double* xt, const double* xc) {
     double d[9], s = 0.0;
 #pragma unroll
     for (int i = 0; i < 9; i++) {
@@ -667,7 +680,7 @@ __device__ __forceinline__ void store_step(double* v, int64_t stride, const doub
     }
 #pragma unroll
     for (int i = 0; i < 9; i++) d[i] = fma(-s, xc[i], d[i]);
-    store_coef(v, stride, d);
+    store_coef(v, d);
 }
 
 // Thread per slot: the pair's state before its first pass; thread 0 readies
@@ -696,10 +709,10 @@ __global__ void node_init_kernel(NodeArgs A, int n_seg, int n, unsigned long lon
     for (int i = 0; i < 9; i++) x0[i] = x == y ? 0.0 : 1.0 / 9.0;
     if (x == y) { x0[0] = 0.5; x0[6] = 0.5; }
     normalise9(x0);
-    double* st = A.state + s;
+    double* st = A.state + slot_at(s, NS_VALS);
 #pragma unroll
-    for (int i = 0; i < 9; i++) st[(NS_XT + i) * A.stride] = x0[i];
-    store_coef(st + NS_COEF * A.stride, A.stride, x0);
+    for (int i = 0; i < 9; i++) st[(NS_XT + i) * NS_LANES] = x0[i];
+    store_coef(st + NS_COEF * NS_LANES, x0);
     A.count[s] = make_int4(0, 0, 0, 4 * g.job + NP_FIRST);
     A.list_cur[s] = s;
 }
@@ -762,15 +775,15 @@ struct NodeShape {
 
 template <int SH, bool MIRROR, bool DIFF>
 __device__ __forceinline__ void node_sums(const NodeDev& N, const double* __restrict__ w, const double* __restrict__ st,
-                                          int64_t stride, int part, const LogTable& T,
+                                          int part, const LogTable& T,
                                           double (&g)[NodeShape<SH>::NG], double (&h)[NodeShape<SH>::NH], double& F) {
     constexpr int NG = NodeShape<SH>::NG, NH = NodeShape<SH>::NH, NK = NodeShape<SH>::NK, K0 = NodeShape<SH>::K0;
     const double EPS = 1e-8;
     double k[NK], ks[NK];
 #pragma unroll
     for (int i = 0; i < NK; i++) {
-        k[i] = st[(NS_COEF + K0 + i) * stride];
-        ks[i] = DIFF ? st[(NS_STEP + K0 + i) * stride] : 0.0;
+        k[i] = st[(NS_COEF + K0 + i) * NS_LANES];
+        ks[i] = DIFF ? st[(NS_STEP + K0 + i) * NS_LANES] : 0.0;
     }
     F = 0.0;
 #pragma unroll
@@ -811,8 +824,8 @@ __device__ __forceinline__ void node_sums(const NodeDev& N, const double* __rest
         else F = fma(W, node_log(d, T), F);
     };
     static_assert(NODE_J % 8 == 0, "two nodes a step for each of four parts");
-    const int64_t step = 4 * N.stride;
-    const double* wp = w + part * N.stride;
+    constexpr int step = 4 * 8;
+    const double* wp = w + part * 8;
     const double* __restrict__ tp = N.t + part;
     double W0 = wp[0], W1 = wp[step], t0 = __ldg(tp), t1 = __ldg(tp + 4);
     for (int i = 0; i < N.nk; i += 8) {
@@ -834,11 +847,11 @@ template <int SH, bool MIRROR>
 __device__ __forceinline__ void node_task(const NodeArgs& A, const NodeDev& N, int s, int u, int kind, int part,
                                           bool write, const LogTable& T) {
     constexpr int NG = NodeShape<SH>::NG, NH = NodeShape<SH>::NH;
-    const double* w = N.w + (int64_t)u * N.nk * N.stride + s;
-    const double* st = A.state + s;
+    const double* w = N.w + (s >> 3) * N.group + (int64_t)u * N.nk * 8 + (s & 7);
+    const double* st = A.state + slot_at(s, NS_VALS);
     double g[NG], h[NH], F;
-    if (kind == NP_DIFF) node_sums<SH, MIRROR, true>(N, w, st, A.stride, part, T, g, h, F);
-    else node_sums<SH, MIRROR, false>(N, w, st, A.stride, part, T, g, h, F);
+    if (kind == NP_DIFF) node_sums<SH, MIRROR, true>(N, w, st, part, T, g, h, F);
+    else node_sums<SH, MIRROR, false>(N, w, st, part, T, g, h, F);
     // the four parts, in a fixed order
     auto all = [](double v) {
         v += __shfl_xor_sync(0xffffffffu, v, 8);
@@ -847,29 +860,29 @@ __device__ __forceinline__ void node_task(const NodeArgs& A, const NodeDev& N, i
     double C = 0.0;
     const bool first = __any_sync(0xffffffffu, kind == NP_FIRST);
     if (first) {
-        for (int i = part; i < N.nk; i += 4) C += w[(int64_t)i * N.stride];
+        for (int i = part; i < N.nk; i += 4) C += w[i * 8];
         C = all(C);
     }
     const double scale = N.scale;
-    double* P = A.partial + (int64_t)u * UNIT_VALS * A.stride + s;
+    double* P = A.partial + slot_at(s, NODE_PART) + u * UNIT_VALS * NS_LANES;
 #pragma unroll
     for (int i = 0; i < NG; i++) {
         const double v = all(g[i]) * scale;
-        if (write && part == (i & 3)) P[i * A.stride] = v;
+        if (write && part == (i & 3)) P[i * NS_LANES] = v;
     }
 #pragma unroll
     for (int i = 0; i < NH; i++) {
         const double v = all(h[i]) * scale;
-        if (write && part == ((NG + i) & 3)) P[(NG + i) * A.stride] = v;
+        if (write && part == ((NG + i) & 3)) P[(NG + i) * NS_LANES] = v;
     }
     const double f = all(F) * scale;
-    if (write && part == 3) P[(UNIT_VALS - 1) * A.stride] = f;
-    if (first && write && part == 0) A.sites[(int64_t)u * A.stride + s] = __double2int_rn(C * scale);
+    if (write && part == 3) P[(UNIT_VALS - 1) * NS_LANES] = f;
+    if (first && write && part == 0) A.sites[slot_at(s, NODE_UNITS) + u * NS_LANES] = __double2int_rn(C * scale);
 }
 
 // A warp per (8 slots of the pass list, genotype pair): lane l takes every
-// fourth node from l / 8 on of slot l % 8.  The weights are stored slot-fastest,
-// so a warp's loads are whole sectors; four lanes a slot keep a pass over few
+// fourth node from l / 8 on of slot l % 8, so a warp's load of weights is 256
+// bytes in a row while its slots are neighbours; four lanes a slot keep a pass over few
 // slots short (a lone lane's 112 nodes took 48 us), two shuffles a moment add
 // them.  Genotype-pair-major, so an SM's warps run one shape's code at a time.
 // Bound by the FP64 pipe's issue.
@@ -1022,15 +1035,16 @@ constexpr int NA_THREADS = 32;   // one warp a block: few slots spread over the 
 // my: the thread's column of the shared memory; sum: the block's counters.
 __device__ __forceinline__ int node_advance(const NodeArgs& A, int s, double* my, unsigned long long* sum) {
     const Tune& tu = A.tune;
-    const int64_t SD = A.stride;
-    double* st = A.state + s;
+    constexpr int SD = NS_LANES;
+    double* st = A.state + slot_at(s, NS_VALS);
+    const int* sites = A.sites + slot_at(s, NODE_UNITS);
     const int4 ct = A.count[s];
     const int kind = ct.w & 3;
     // ---- the pair's moments: two genotype pairs a shape, het-het one
     double xt[9], g[9], obj, nsites;
     {
         double m[NMOM];
-        const double* P = A.partial + s;
+        const double* P = A.partial + slot_at(s, NODE_PART);
         obj = 0.0;
 #pragma unroll
         for (int u = 0; u < NODE_UNITS; u++) {
@@ -1039,14 +1053,14 @@ __device__ __forceinline__ int node_advance(const NodeArgs& A, int s, double* my
 #pragma unroll
             for (int v = 0; v < 13; v++)
                 if (v < nv) {
-                    const double p = P[((int64_t)u * UNIT_VALS + v) * SD];
+                    const double p = P[(u * UNIT_VALS + v) * SD];
                     m[go + v] = (u & 1) ? m[go + v] + p : p;
                 }
-            obj += P[((int64_t)u * UNIT_VALS + UNIT_VALS - 1) * SD];
+            obj += P[(u * UNIT_VALS + UNIT_VALS - 1) * SD];
         }
         if (kind == NP_FIRST) {
             int64_t c = 0;
-            for (int u = 0; u < NODE_UNITS; u++) c += A.sites[(int64_t)u * SD + s];
+            for (int u = 0; u < NODE_UNITS; u++) c += sites[u * SD];
             nsites = (double)c;
             st[NS_N * SD] = nsites;
         } else {
@@ -1094,8 +1108,8 @@ __device__ __forceinline__ int node_advance(const NodeArgs& A, int s, double* my
             }
             st[NS_ALPHA * SD] = a2;
             next = fabs(a2 * gp) < DIFF_BELOW ? NP_DIFF : NP_DIRECT;
-            store_coef(st + NS_COEF * SD, SD, xt);
-            if (next == NP_DIFF) store_step(st + NS_STEP * SD, SD, xt, xc);
+            store_coef(st + NS_COEF * SD, xt);
+            if (next == NP_DIFF) store_step(st + NS_STEP * SD, xt, xc);
             A.count[s] = make_int4(it, ct.y + 1, gh, (ct.w & ~3) | next);
         } else {
             it++;
@@ -1122,8 +1136,8 @@ __device__ __forceinline__ int node_advance(const NodeArgs& A, int s, double* my
             unsigned long long evals = 0, shapes[5];
 #pragma unroll
             for (int sh = 0; sh < 5; sh++) {
-                shapes[sh] = (unsigned long long)A.sites[(int64_t)(2 * sh) * SD + s];
-                if (sh < 4) shapes[sh] += (unsigned long long)A.sites[(int64_t)(2 * sh + 1) * SD + s];
+                shapes[sh] = (unsigned long long)sites[2 * sh * SD];
+                if (sh < 4) shapes[sh] += (unsigned long long)sites[(2 * sh + 1) * SD];
                 evals += (unsigned long long)((sh == 4 ? 1 : 2) * flops_fp64(sh));
                 atomicAdd(&sum[7 + sh], none ? 0ull : shapes[sh]);
             }
@@ -1171,8 +1185,8 @@ __device__ __forceinline__ int node_advance(const NodeArgs& A, int s, double* my
             st[NS_GP * SD] = gp;
             st[NS_ALPHA * SD] = 1.0;
             next = fabs(gp) < DIFF_BELOW ? NP_DIFF : NP_DIRECT;
-            store_coef(st + NS_COEF * SD, SD, y);
-            if (next == NP_DIFF) store_step(st + NS_STEP * SD, SD, y, xt);
+            store_coef(st + NS_COEF * SD, y);
+            if (next == NP_DIFF) store_step(st + NS_STEP * SD, y, xt);
             A.count[s] = make_int4(it, 0, gh, (ct.w & ~3) | next);
         }
     }
@@ -1182,8 +1196,8 @@ __device__ __forceinline__ int node_advance(const NodeArgs& A, int s, double* my
 // Everything between two passes of a slot, a thread per slot: its moments,
 // the Armijo accept test (a rejected trial backs off and takes the next pass),
 // the KKT test, at convergence the condition estimate and the row, else the
-// simplex QP and the next trial point.  The state and the sums are stored
-// value-major, so a warp's loads and stores are whole sectors; H and c go
+// simplex QP and the next trial point.  The state and the sums are blocked by 32
+// slots, so a warp's loads and stores are whole sectors; H and c go
 // through shared memory (432 bytes a thread) into the QP.  One kernel instead
 // of the list form's solve, QP and step kernels: nothing is written between
 // them and a wave over few slots waits for one launch.  Bound by the FP64
@@ -1294,8 +1308,8 @@ extern "C" __global__ void __launch_bounds__(NA_THREADS) node_cls_kernel(NodeArg
 #pragma unroll
         for (int k = 0; k < 5; k++) sites[k] = 0.0;
         for (int i = 0; i < N.nk; i++) {
-            const double* w = N.w + (int64_t)i * N.stride + s;
-            const int64_t un = (int64_t)N.nk * N.stride;
+            const double* w = N.w + (s >> 3) * N.group + i * 8 + (s & 7);
+            const int un = N.nk * 8;
             const double t = __ldg(N.t + i), u = 1.0 - t, q = t * u, t2 = t * t, u2 = u * u;
             const double W[9] = {w[0], w[un], w[2 * un], w[3 * un], w[4 * un], w[5 * un], w[6 * un], w[7 * un], w[8 * un]};
             m[0] = fma(W[0], t, fma(W[1], u, m[0]));
@@ -1448,7 +1462,8 @@ int run_nodes(const std::vector<PairJob>& jobs, const RunConfig& cfg, Workspace&
         cap = std::max<int64_t>(1, std::min<int64_t>(cap, (int64_t)((fr + held) / 2 / per_slot)));
     }
     const int64_t stride = (cap + 31) / 32 * 32;
-    KG_NODE_TRY((cudaError_t)ws.scratch.reserve(sizeof(double) * NODE_UNITS * (size_t)nk_max * stride));
+    const int64_t group = (int64_t)NODE_UNITS * nk_max * 8;
+    KG_NODE_TRY((cudaError_t)ws.scratch.reserve(sizeof(double) * (size_t)group * (stride / 8)));
     KG_NODE_TRY((cudaError_t)ws.slots.reserve(slot_bytes * (size_t)stride));
     // control words, one buffer: {control, clock, run counters}
     const size_t off_clk = sizeof(NodeCtl), off_run = off_clk + sizeof(WaveClock);
@@ -1487,7 +1502,6 @@ int run_nodes(const std::vector<PairJob>& jobs, const RunConfig& cfg, Workspace&
         A.cohorts = reinterpret_cast<CohortDev*>(dtab);
         A.nodes = reinterpret_cast<NodeDev*>(dtab + off_nodes);
         A.seg = reinterpret_cast<NodeSeg*>(dtab + off_seg);
-        A.stride = stride;
         A.state = ws.slots.as<double>();
         A.partial = A.state + (size_t)(NS_VALS + 2) * stride;
         A.count = reinterpret_cast<int4*>(A.partial + (size_t)NODE_UNITS * UNIT_VALS * stride);
@@ -1560,7 +1574,7 @@ int run_nodes(const std::vector<PairJob>& jobs, const RunConfig& cfg, Workspace&
                 h_seg[n_seg] = NodeSeg{at, (int32_t)n, (int32_t)take, job, 0};
                 NodeDev& nd = h_nodes[job];
                 nd.w = ws.scratch.as<double>();
-                nd.stride = stride;
+                nd.group = group;
                 nd.nk = c.nd_n * J;
                 nd.t = c.nd_t.as<double>();
                 nd.scale = std::ldexp(1.0, -(8 * NODE_L - 2));
@@ -1595,7 +1609,7 @@ int run_nodes(const std::vector<PairJob>& jobs, const RunConfig& cfg, Workspace&
             P.first_unit = yx_before(y0);
             P.n_yx = yx_before(y1 + 1) - P.first_unit;
             P.w = ws.scratch.as<double>();
-            P.stride = stride;
+            P.group = group;
             P.stalled = &d_run->stalled_waits;
             const int grid = (int)std::min<int64_t>(ws.sm_count, P.n_yx * P.bins);
             node_weights_kernel<<<grid, NW_THREADS, NW_SMEM, st>>>(P);
