@@ -499,7 +499,7 @@ static int grid_for(int64_t n, int threads) { return (int)std::max<int64_t>(1, c
 
 int prepare_cohort(Cohort& c, const uint8_t* codes, int64_t n_samples, int64_t n_sites,
                    int64_t row_stride, bool codes_on_device, const double* af, double maf,
-                   cudaStream_t st, std::string& err, bool cls, uint64_t iterations, bool nodes) {
+                   cudaStream_t st, std::string& err, bool cls, uint64_t iterations, bool nodes, bool both) {
     if (n_samples <= 0 || n_sites <= 0 || row_stride < n_sites) {
         err = "n_samples and n_sites must be positive and row_stride >= n_sites";
         return KG_EINVAL;
@@ -601,7 +601,10 @@ int prepare_cohort(Cohort& c, const uint8_t* codes, int64_t n_samples, int64_t n
             std::memcpy(&t_min, &key, sizeof(t_min));
         }
         const int bins = node_bins(cls, c.n_kept, n_samples, t_min);
-        if (bins > 0) return prepare_nodes(c, draw, stride, bins, t_min, st, err);
+        if (bins > 0) {
+            const int r = prepare_nodes(c, draw, stride, bins, t_min, st, err);
+            if (r || !both) return r;
+        }
     }
     KG_CUDA_TRY((cudaError_t)c.planes.reserve(sizeof(uint2) * n_samples * c.plane_stride));
     const int64_t work = n_samples * c.plane_stride;

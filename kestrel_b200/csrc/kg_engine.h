@@ -121,11 +121,11 @@ struct Cohort {
 // the sites are those every sample calls, frequencies are counts over all
 // samples (or af), nothing is filtered by frequency, and Q is computed.  With
 // nodes the cohort is laid out for pairs on frequency nodes where that pays
-// (node_bins), else for site lists.
+// (node_bins), else for site lists; with both, for lists in either case.
 int prepare_cohort(Cohort& c, const uint8_t* codes, int64_t n_samples, int64_t n_sites,
                    int64_t row_stride, bool codes_on_device, const double* af, double maf,
                    cudaStream_t st, std::string& err, bool cls = false, uint64_t iterations = 100,
-                   bool nodes = false);
+                   bool nodes = false, bool both = false);
 
 // After prepare_cohort(..., cls = true): adds the cohort's tri- and
 // tetra-allelic sites (c.mg, c.malleles, c.maf uploaded, c.n_multi set) to the

@@ -68,10 +68,6 @@ int node_bins(bool cls, int64_t n_kept, int64_t n_samples, double t_min) {
     const double need = std::ceil(std::log(0.5 / t_min) / std::log(NODE_RATIO));
     if (!(need <= (double)NODE_MAX_BINS)) return 0;
     const int bins = std::max(1, (int)need);
-    // below ten sites per node the lists win: 64 samples x 10,000 sites (14
-    // bins, 1,008 nodes a pair) took 2.73 ms on lists and 3.28 ms on nodes, 201
-    // x 33,333 (2,016 nodes of 24 bins) 41.6 against 6.6 ms
-    if (n_kept < (int64_t)10 * NODE_UNITS * NODE_J * bins) return 0;
     return bins;
 }
 
@@ -191,9 +187,10 @@ __global__ void node_scatter_kernel(NodeGrid G, const double* __restrict__ p64, 
 }
 
 // A block per (sample, part): warps build the folded {lo, hi} planes of 32
-// placed sites a time; the sample's codes are read through L1.
-__global__ void node_pack_kernel(const uint8_t* __restrict__ raw, int64_t stride, const uint32_t* __restrict__ place,
-                                 int64_t words, uint2* __restrict__ planes) {
+// placed sites a time; the sample's codes are read through L1.  mask: sites to
+// keep (NULL: all).
+__global__ void node_pack_kernel(const uint8_t* __restrict__ raw, int64_t stride, const uint8_t* __restrict__ mask,
+                                 const uint32_t* __restrict__ place, int64_t words, uint2* __restrict__ planes) {
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, nw = blockDim.x >> 5;
     const uint8_t* row = raw + (int64_t)blockIdx.x * stride;
     uint2* out = planes + (int64_t)blockIdx.x * words;
@@ -202,11 +199,21 @@ __global__ void node_pack_kernel(const uint8_t* __restrict__ raw, int64_t stride
         unsigned c = 3u;
         if (e != 0xFFFFFFFFu) {
             c = row[e & 0x7FFFFFFFu];
+            if (mask && !mask[e & 0x7FFFFFFFu]) c = 3u;
             if ((e >> 31) && c < 3u) c = 2u - c;
         }
         const unsigned lo = __ballot_sync(0xffffffffu, c & 1u), hi = __ballot_sync(0xffffffffu, (c >> 1) & 1u);
         if (lane == 0) out[k] = make_uint2(lo, hi);
     }
+}
+
+static void pack_placed(const uint8_t* codes, int64_t rows, int64_t stride, const uint8_t* mask, const DevBuf& place,
+                        int64_t mp, const DevBuf& planes, cudaStream_t st) {
+    // enough blocks to fill the SMs, few enough that a sample's row is read by few
+    const int64_t words = mp / 32;
+    const int parts = (int)std::max<int64_t>(1, std::min<int64_t>((words + 63) / 64, 1184 / rows + 1));
+    node_pack_kernel<<<dim3((unsigned)rows, parts), 256, 0, st>>>(codes, stride, mask, place.as<uint32_t>(), words,
+                                                                  planes.as<uint2>());
 }
 
 int prepare_nodes(Cohort& c, const uint8_t* codes, int64_t stride, int bins, double t_min, cudaStream_t st,
@@ -236,14 +243,33 @@ int prepare_nodes(Cohort& c, const uint8_t* codes, int64_t stride, int bins, dou
     node_layout_kernel<<<1, 256, 0, st>>>(G, hist, bin, c.nd_t.as<double>());
     node_scatter_kernel<<<grid, 256, 0, st>>>(G, c.p64.as<double>(), c.site_of.as<int32_t>(), hist,
                                               c.nd_place.as<uint32_t>(), c.nd_dig.as<int8_t>(), mp);
-    // enough blocks to fill the SMs, few enough that a sample's row is read by few
-    const int64_t words = mp / 32;
-    const int parts = (int)std::max<int64_t>(1, std::min<int64_t>((words + 63) / 64, 1184 / c.n_samples + 1));
-    node_pack_kernel<<<dim3((unsigned)c.n_samples, parts), 256, 0, st>>>(codes, stride, c.nd_place.as<uint32_t>(),
-                                                                         words, c.nd_planes.as<uint2>());
+    pack_placed(codes, c.n_samples, stride, nullptr, c.nd_place, mp, c.nd_planes, st);
     KG_NODE_TRY(cudaGetLastError());
     c.nd_n = bins;
     c.nd_mp = mp;
+    return KG_OK;
+}
+
+int prepare_query_nodes(const Cohort& panel, QueryPlanes& q, const uint8_t* codes, int64_t n_rows, int64_t row_stride,
+                        const uint8_t* site_mask, cudaStream_t st, std::string& err) {
+    if (n_rows <= 0 || row_stride < panel.n_sites || !codes || panel.nd_n <= 0) {
+        err = "query rows must be positive and cover the panel's sites";
+        return KG_EINVAL;
+    }
+    const int64_t ns = panel.n_sites;
+    q.n_rows = n_rows;
+    KG_NODE_TRY((cudaError_t)q.raw.reserve((size_t)(n_rows * ns)));
+    KG_NODE_TRY(cudaMemcpy2DAsync(q.raw.p, (size_t)ns, codes, (size_t)row_stride, (size_t)ns, (size_t)n_rows,
+                                  cudaMemcpyHostToDevice, st));
+    const uint8_t* dmask = nullptr;
+    if (site_mask) {
+        KG_NODE_TRY((cudaError_t)q.mask.reserve((size_t)ns));
+        KG_NODE_TRY(cudaMemcpyAsync(q.mask.p, site_mask, (size_t)ns, cudaMemcpyHostToDevice, st));
+        dmask = q.mask.as<uint8_t>();
+    }
+    KG_NODE_TRY((cudaError_t)q.planes.reserve(sizeof(uint2) * (panel.nd_mp / 32) * n_rows));
+    pack_placed(q.raw.as<uint8_t>(), n_rows, ns, dmask, panel.nd_place, panel.nd_mp, q.planes, st);
+    KG_NODE_TRY(cudaGetLastError());
     return KG_OK;
 }
 
@@ -279,13 +305,15 @@ constexpr uint32_t NW_TM_A = 320;        // tensor-memory column of A's half-sta
 constexpr int NW_SMEM = 120 * 1024;      // more than half an SM's: one block (it owns the tensor memory)
 
 struct NodeProduct {
-    const uint2* planes;       // [sample][words]
+    const uint2* planes;       // [sample][words] of the A operand's samples
+    const uint2* planes_b;     // of the B operand's (a triangle: the same)
     const int8_t* dig;         // [32][mp]
     const NodeBin* bin;
     int64_t words, mp;
-    int32_t n_samples;         // rows of the planes
+    int32_t n_samples;         // rows of planes
+    int32_t rect;              // query x panel: A's samples are the panel's (y), B's the query's (x)
     int32_t bins;
-    int64_t idx0, idx1;        // the pairs (x <= y) of this chunk: y (y + 1) / 2 + x
+    int64_t idx0, idx1;        // the pairs of this chunk: y (y + 1) / 2 + x, x <= y (rect: x n_samples + y)
     int64_t slot0;             // slot of pair idx0 within w's columns
     int64_t first_unit, n_yx;  // the first (y, x block) in the count from y = 0, how many
     double* w;                 // see NodeDev
@@ -298,7 +326,14 @@ __host__ __device__ inline int64_t yx_before(int64_t y) {
     const int64_t q = y >> 7;
     return 64 * q * (q + 1) + (y - (q << 7)) * (q + 1);
 }
-__device__ __forceinline__ void decode_yx(int64_t u, int& y, int& xb) {
+// (B's sample, block of A's samples)
+__device__ __forceinline__ void decode_yx(const NodeProduct& P, int64_t u, int& y, int& xb) {
+    if (P.rect) {
+        const int64_t nb = (P.n_samples + 127) >> 7;
+        y = (int)(u / nb);
+        xb = (int)(u - y * nb);
+        return;
+    }
     int64_t q = (int64_t)((sqrt(1.0 + (double)u / 16.0) - 1.0) * 0.5);
     while (q > 0 && 64 * q * (q + 1) > u) q--;
     while (64 * (q + 1) * (q + 2) <= u) q++;
@@ -360,7 +395,7 @@ __global__ void __launch_bounds__(NW_THREADS, 1) node_weights_kernel(NodeProduct
         for (int64_t un = blockIdx.x; ok && un < n_units; un += gridDim.x) {
             const int k = (int)(un / P.n_yx);
             int y, xb;
-            decode_yx(P.first_unit + (un - k * P.n_yx), y, xb);
+            decode_yx(P, P.first_unit + (un - k * P.n_yx), y, xb);
             const NodeBin bn = P.bin[k];
             const int x = xb * 128 + (warp & 3) * 32 + lane;
             const uint32_t live = x < P.n_samples ? ~0u : 0u;
@@ -407,10 +442,10 @@ __global__ void __launch_bounds__(NW_THREADS, 1) node_weights_kernel(NodeProduct
         for (int64_t un = blockIdx.x; ok && un < n_units; un += gridDim.x) {
             const int k = (int)(un / P.n_yx);
             int y, xb;
-            decode_yx(P.first_unit + (un - k * P.n_yx), y, xb);
+            decode_yx(P, P.first_unit + (un - k * P.n_yx), y, xb);
             const NodeBin bn = P.bin[k];
             const int8_t* d0 = P.dig + (int64_t)row * P.mp + bn.start + 16 * c;
-            const uint2* py = P.planes + (int64_t)y * P.words + (bn.start >> 5) + (c >> 1);
+            const uint2* py = P.planes_b + (int64_t)y * P.words + (bn.start >> 5) + (c >> 1);
             uint4 va[NW_AHEAD], vb[NW_AHEAD];
             uint2 pl[NW_AHEAD];
             auto fetch = [&](int i, uint4& a4, uint4& b4, uint2& p2) {
@@ -463,19 +498,20 @@ __global__ void __launch_bounds__(NW_THREADS, 1) node_weights_kernel(NodeProduct
         // consecutive slots
         const uint32_t my = tm + ((uint32_t)((warp - 12) * 32) << 16);
         // the genotype pair's number u (see the file comment) of (gx, gy) = (a, b)
-        constexpr int UNIT[9] = {0, 2, 6, 4, 8, 5, 7, 3, 1};
+        // and, query x panel, of (b, a)
+        constexpr int UNIT[9] = {0, 2, 6, 4, 8, 5, 7, 3, 1}, UNIT_T[9] = {0, 4, 7, 2, 8, 3, 6, 5, 1};
         uint32_t n_acc = 0;
         const int nk = P.bins * J;
         for (int64_t un = blockIdx.x; ok && un < n_units; un += gridDim.x) {
             const int k = (int)(un / P.n_yx);
             int y, xb;
-            decode_yx(P.first_unit + (un - k * P.n_yx), y, xb);
+            decode_yx(P, P.first_unit + (un - k * P.n_yx), y, xb);
             if (P.bin[k].stages == 0) {
                 // an empty bin: zero weights, no product
                 const int x = xb * 128 + (warp - 12) * 32 + lane;
-                const int64_t idx = (int64_t)y * (y + 1) / 2 + x;
+                const int64_t idx = P.rect ? (int64_t)y * P.n_samples + x : (int64_t)y * (y + 1) / 2 + x;
                 const int64_t s = P.slot0 + (idx - P.idx0);
-                if (x <= y && idx >= P.idx0 && idx < P.idx1)
+                if (x < (P.rect ? P.n_samples : y + 1) && idx >= P.idx0 && idx < P.idx1)
                     for (int u = 0; u < 9; u++)
                         for (int j = 0; j < J; j++)
                             P.w[(s >> 3) * P.group + ((int64_t)u * nk + k * J + j) * 8 + (s & 7)] = 0.0;
@@ -485,8 +521,8 @@ __global__ void __launch_bounds__(NW_THREADS, 1) node_weights_kernel(NodeProduct
             n_acc++;
             tmem_fence_after();
             const int x = xb * 128 + (warp - 12) * 32 + lane;
-            const int64_t idx = (int64_t)y * (y + 1) / 2 + x;
-            const bool store = x <= y && idx >= P.idx0 && idx < P.idx1;
+            const int64_t idx = P.rect ? (int64_t)y * P.n_samples + x : (int64_t)y * (y + 1) / 2 + x;
+            const bool store = x < (P.rect ? P.n_samples : y + 1) && idx >= P.idx0 && idx < P.idx1;
             const int64_t s = P.slot0 + (idx - P.idx0);
             double* out = P.w + (s >> 3) * P.group + (int64_t)(k * J) * 8 + (s & 7);
 #pragma unroll
@@ -504,7 +540,7 @@ __global__ void __launch_bounds__(NW_THREADS, 1) node_weights_kernel(NodeProduct
                     long long v = (int)r[j * L];
 #pragma unroll
                     for (int d = 1; d < L; d++) v += (long long)(int)r[j * L + d] * (1ll << (8 * d));
-                    if (store) out[((int64_t)UNIT[ab] * nk + j) * 8] = (double)v;
+                    if (store) out[((int64_t)(P.rect ? UNIT_T[ab] : UNIT[ab]) * nk + j) * 8] = (double)v;
                 }
             }
         }
@@ -550,7 +586,8 @@ __global__ void __launch_bounds__(NW_THREADS, 1) node_weights_kernel(NodeProduct
 
 // --------------------------------------------------------- a chunk's slots
 
-// A run of one job's pairs (y-major: y (y + 1) / 2 + x) in consecutive slots.
+// A run of one job's pairs (y-major: y (y + 1) / 2 + x; query x panel: x n_y +
+// y) in consecutive slots.
 struct NodeSeg {
     int64_t idx0;
     int32_t slot0, n, job, pad;
@@ -648,9 +685,19 @@ __host__ __device__ inline void pair_of(int64_t idx, int64_t& x, int64_t& y) {
     x = idx - y * (y + 1) / 2;
 }
 
-__device__ __forceinline__ void node_write_row(const CohortDev& co, int64_t x, int64_t y, const double* d, double obj,
+// The samples of a job's pair idx, and its output row.
+__device__ __forceinline__ int64_t job_pair(const CohortDev& co, int64_t idx, int64_t& x, int64_t& y) {
+    if (co.kind == COHORT_RECT) {
+        x = idx / co.n_y;
+        y = idx - x * co.n_y;
+        return idx;
+    }
+    pair_of(idx, x, y);
+    return x * co.n_x - x * (x - 1) / 2 + (y - x);
+}
+
+__device__ __forceinline__ void node_write_row(kg_output* o, int64_t x, int64_t y, const double* d, double obj,
                                                uint64_t iters, double cond) {
-    kg_output* o = co.out + (x * co.n_x - x * (x - 1) / 2 + (y - x));
     o->x = (uint64_t)x;
     o->y = (uint64_t)y;
 #pragma unroll
@@ -703,11 +750,13 @@ __global__ void node_init_kernel(NodeArgs A, int n_seg, int n, unsigned long lon
     }
     if (s >= n) return;
     const NodeSeg g = seg_of(A.seg, n_seg, s);
+    const CohortDev& co = A.cohorts[g.job];
     int64_t x, y;
-    pair_of(g.idx0 + (s - g.slot0), x, y);
+    job_pair(co, g.idx0 + (s - g.slot0), x, y);
+    const bool self_pair = co.kind == COHORT_TRIANGLE && x == y;
     double x0[9];
-    for (int i = 0; i < 9; i++) x0[i] = x == y ? 0.0 : 1.0 / 9.0;
-    if (x == y) { x0[0] = 0.5; x0[6] = 0.5; }
+    for (int i = 0; i < 9; i++) x0[i] = self_pair ? 0.0 : 1.0 / 9.0;
+    if (self_pair) { x0[0] = 0.5; x0[6] = 0.5; }
     normalise9(x0);
     double* st = A.state + slot_at(s, NS_VALS);
 #pragma unroll
@@ -1123,7 +1172,7 @@ __device__ __forceinline__ int node_advance(const NodeArgs& A, int s, double* my
         if (none || last || kkt_ok(xt, g, tu.sqp_conv_tol, &resid)) {
             const NodeSeg sg = seg_of(A.seg, A.ctl->n_seg, s);
             int64_t x, y;
-            pair_of(sg.idx0 + (s - sg.slot0), x, y);
+            const int64_t row = job_pair(co, sg.idx0 + (s - sg.slot0), x, y);
             double cond = CUDART_NAN;
             if (!none && !last) cond = condition_thread([my](int k) { return my[k * NA_THREADS]; }, xt, g, tu.sqp_conv_tol);
             if (none) {
@@ -1131,7 +1180,7 @@ __device__ __forceinline__ int node_advance(const NodeArgs& A, int s, double* my
                 for (int k = 0; k < 9; k++) xt[k] = CUDART_NAN;
                 f = CUDART_NAN;
             }
-            node_write_row(co, x, y, xt, f, none ? 0 : last ? co.max_iter : (uint64_t)it, cond);
+            node_write_row(co.out + row, x, y, xt, f, none ? 0 : last ? co.max_iter : (uint64_t)it, cond);
             // the counters of the call
             unsigned long long evals = 0, shapes[5];
 #pragma unroll
@@ -1300,7 +1349,7 @@ extern "C" __global__ void __launch_bounds__(NA_THREADS) node_cls_kernel(NodeArg
         const CohortDev& co = A.cohorts[sg.job];
         const NodeDev N = A.nodes[sg.job];
         int64_t x, y;
-        pair_of(sg.idx0 + (s - sg.slot0), x, y);
+        const int64_t row = job_pair(co, sg.idx0 + (s - sg.slot0), x, y);
         // sums of the shapes' monomials: A t^1..4, B w t^0..2, C w {1, ty, t, w}, D w {1, w}
         double m[16], sites[5];
 #pragma unroll
@@ -1337,7 +1386,6 @@ extern "C" __global__ void __launch_bounds__(NA_THREADS) node_cls_kernel(NodeArg
         double S[9] = {m[0], m[1] + m[10], m[1] + m[4], m[2] + 2.0 * m[5] + m[11], m[1] + m[7],
                        m[2] + 2.0 * m[8] + m[12], m[1] + 2.0 * m[14], m[2] + m[5] + m[8] + m[14],
                        m[3] + 2.0 * (m[6] + m[9]) + m[13] + 4.0 * m[15]};
-        const int64_t row = x * co.n_x - x * (x - 1) / 2 + (y - x);
         Tune tq = A.tune;
         tq.qp_max_iter = co.max_iter > (uint64_t)INT_MAX ? INT_MAX : (int)co.max_iter;
 #pragma unroll
@@ -1374,7 +1422,7 @@ extern "C" __global__ void __launch_bounds__(NA_THREADS) node_cls_kernel(NodeArg
             g[r] = qd + c;
         }
         const double cond = condition_thread([my](int k) { return my[k * NA_THREADS]; }, d, g, tq.sqp_conv_tol);
-        node_write_row(co, x, y, d, (quad + 2.0 * lin) + 1.0, (uint64_t)iters, cond);
+        node_write_row(co.out + row, x, y, d, (quad + 2.0 * lin) + 1.0, (uint64_t)iters, cond);
         unsigned long long all = 0;
 #pragma unroll
         for (int k = 0; k < 5; k++) {
@@ -1593,7 +1641,9 @@ int run_nodes(const std::vector<PairJob>& jobs, const RunConfig& cfg, Workspace&
             const NodeSeg& g = h_seg[k];
             const Cohort& c = *jobs[g.job].panel;
             NodeProduct P;
+            P.rect = jobs[g.job].kind == COHORT_RECT ? 1 : 0;
             P.planes = c.nd_planes.as<uint2>();
+            P.planes_b = P.rect ? jobs[g.job].query->planes.as<uint2>() : P.planes;
             P.dig = c.nd_dig.as<int8_t>();
             P.bin = reinterpret_cast<const NodeBin*>(c.nd_bins.as<int>() + NODE_MAX_BINS);
             P.mp = c.nd_mp;
@@ -1604,10 +1654,18 @@ int run_nodes(const std::vector<PairJob>& jobs, const RunConfig& cfg, Workspace&
             P.idx1 = g.idx0 + g.n;
             P.slot0 = g.slot0;
             int64_t x, y0, y1;
-            pair_of(P.idx0, x, y0);
-            pair_of(P.idx1 - 1, x, y1);
-            P.first_unit = yx_before(y0);
-            P.n_yx = yx_before(y1 + 1) - P.first_unit;
+            if (P.rect) {
+                const int64_t nb = (P.n_samples + 127) >> 7;
+                y0 = P.idx0 / P.n_samples;
+                y1 = (P.idx1 - 1) / P.n_samples;
+                P.first_unit = y0 * nb;
+                P.n_yx = (y1 + 1) * nb - P.first_unit;
+            } else {
+                pair_of(P.idx0, x, y0);
+                pair_of(P.idx1 - 1, x, y1);
+                P.first_unit = yx_before(y0);
+                P.n_yx = yx_before(y1 + 1) - P.first_unit;
+            }
             P.w = ws.scratch.as<double>();
             P.group = group;
             P.stalled = &d_run->stalled_waits;
