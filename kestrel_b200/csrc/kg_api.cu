@@ -676,8 +676,8 @@ int kg_relatedness(kg_ctx* c, int64_t num_samples, uint64_t iterations, double m
         if (cudaEventElapsedTime(&dms, ev0, ev1) == cudaSuccess) stats.device_ms = dms;
         cudaEventDestroy(ev0);
         cudaEventDestroy(ev1);
-        stats.launches += 7;  // count, freq, two scans, compact, pad, pack
         const kg::Cohort& co = c->cohort;
+        stats.launches += co.nd_n ? 10 : 7;  // count, freq, two scans, compact, pad(, three for the nodes' places), pack
         if (co.n_multi > 0) stats.launches += 3 + (co.ml_nk > 0 ? 2 : 0);   // fit, two scans, rows, codes
         stats.sites_used[0] = (uint64_t)(co.n_kept + co.ml_by_alleles[0]);
         stats.sites_used[1] = (uint64_t)co.ml_by_alleles[1];
@@ -745,7 +745,8 @@ int kg_relatedness_gt(kg_ctx* c, int64_t num_samples, uint64_t iterations, kg_ou
         if (cudaEventElapsedTime(&dms, ev0, ev1) == cudaSuccess) stats.device_ms = dms;
         cudaEventDestroy(ev0);
         cudaEventDestroy(ev1);
-        stats.launches += 9;  // count, freq, two scans, compact, pad, pack, Gram, Gram total
+        // count, freq, two scans, compact, pad(, three for the nodes' places), pack, Gram, Gram total
+        stats.launches += c->cohort.nd_n ? 12 : 9;
         if (c->cohort.n_multi > 0) stats.launches += 5;   // multi-allelic frequencies, Gram, Gram total, transpose, rows
         stats.sites_used[0] = (uint64_t)c->cohort.n_kept;
         stats.sites_discarded = (uint64_t)(c->cohort.n_sites - c->cohort.n_kept +
@@ -835,7 +836,7 @@ int kg_relatedness_gl(kg_ctx* c, int64_t num_samples, uint64_t iterations, doubl
         cudaEventCreate(&ev1);
         cudaEventRecord(ev0, c->stream);
         int64_t kept = 0, used[3] = {0, 0, 0};
-        uint64_t sc[5] = {0, 0, 0, 0, 0};
+        uint64_t sc[6] = {0, 0, 0, 0, 0, 0};
         kg::SoftMultiInput mi;
         mi.gl3 = c->soft_n3 ? c->soft_gl3.as<double>() : nullptr;
         mi.n3 = c->soft_n3;
@@ -850,7 +851,7 @@ int kg_relatedness_gl(kg_ctx* c, int64_t num_samples, uint64_t iterations, doubl
         if (cudaEventElapsedTime(&dms, ev0, ev1) == cudaSuccess) stats.device_ms = dms;
         cudaEventDestroy(ev0);
         cudaEventDestroy(ev1);
-        stats.launches = c->precision == KG_PREC_FP64 ? 2 : 3;   // frequencies, (FP32 packing,) pairs
+        stats.launches = (c->precision == KG_PREC_FP64 ? 1 : 2) + (sc[5] ? sc[5] : 1);   // frequencies, (FP32 packing,) pairs
         stats.gh_passes = sc[0];
         stats.obj_passes = sc[0];
         stats.fp64_passes = sc[1];

@@ -154,7 +154,9 @@ int prepare_ml_multi(Cohort& c, bool have_af, double maf, uint64_t iterations, c
 // kept with 2, 3 and 4 alleles after the frequency cut.
 // Device buffers of the soft-likelihood estimator, kept between calls (they
 // only grow, so repeated calls allocate nothing).
+struct SoftWaves;
 struct SoftWork {
+    std::shared_ptr<SoftWaves> waves;   // the pairs' slots and their graph
     DevBuf pf, qf, keep, idx, kp, kq, ctr, g32, pq32, mgk, mgidx, mrows, mused, mscratch;
 };
 struct SoftMultiInput {

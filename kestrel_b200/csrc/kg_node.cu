@@ -31,6 +31,7 @@
 #include <cstdlib>
 #include <cstring>
 
+#include "kg_advance.cuh"
 #include "kg_bulk.cuh"
 #include "kg_engine.h"
 #include "kg_node.h"
@@ -586,13 +587,6 @@ __global__ void __launch_bounds__(NW_THREADS, 1) node_weights_kernel(NodeProduct
 
 // --------------------------------------------------------- a chunk's slots
 
-// A run of one job's pairs (y-major: y (y + 1) / 2 + x; query x panel: x n_y +
-// y) in consecutive slots.
-struct NodeSeg {
-    int64_t idx0;
-    int32_t slot0, n, job, pad;
-};
-
 // A job's nodes.  The weights of eight slots lie together (64 KB for 14 bins):
 // W of slot s at w[(s / 8) group + (u nk + i) 8 + s % 8], u a genotype pair, i a
 // node.  With the slots of a node together instead (rows of 4 MB at 1024
@@ -614,156 +608,16 @@ struct LogTable {
     double exp2[LOG_EXPS];     // (e - 40) log 2
 };
 
-// Per-slot values lie in blocks of 32 slots, value-major inside: value v of
-// slot s, of V values, at [(s / 32) V 32 + v 32 + s % 32].
-constexpr int NS_LANES = 32;
-__host__ __device__ __forceinline__ int64_t slot_at(int s, int values) {
-    return (int64_t)(s >> 5) * (values * NS_LANES) + (s & 31);
-}
-
-// A slot's SQP state (src/sqp.rs:49-93) between its passes.
-enum : int {
-    NS_XC = 0,        // accepted point
-    NS_XT = 9,        // point of the pending pass
-    NS_P = 18,        // search direction
-    NS_F = 27,        // objective at xc
-    NS_GP = 28,       // g . p
-    NS_ALPHA = 29,
-    NS_N = 30,        // the pair's sites
-    NS_COEF = 31,     // PassCoef at xt (16)
-    NS_STEP = 47,     // PassCoef of xt - xc (16): difference passes
-    NS_VALS = 63
-};
-constexpr int NS_COEFS = (int)(sizeof(PassCoef) / sizeof(double));
-static_assert(NS_COEFS == 16, "PassCoef: a 4, b1 3, b2 3, c 4, d 2");
-
-// The waves' control words.
-struct NodeCtl {
-    int n[2];              // pending passes of the even and the odd waves
-    unsigned int ticket;   // blocks of the advance kernel that are done
-    int n_seg;             // runs of the chunk
-    unsigned long long max_waves;
-};
-
-struct NodeArgs {
-    const CohortDev* cohorts;
+struct NodeArgs : SlotArgs {
     const NodeDev* nodes;      // per job
-    const NodeSeg* seg;        // the chunk's runs (ctl->n_seg)
-    double* state;             // NS_VALS values a slot
     double* partial;           // NODE_PART values a slot
-    int4* count;               // {iterations, backtracks, passes, job * 4 + kind} per slot
     int* sites;                // NODE_UNITS values a slot: the pair's sites by genotype pair
-    int* list_cur;             // slots with a pending pass
-    int* list_next;
-    int par;                   // 0: even waves
-    NodeCtl* ctl;
-    WaveClock* clk;
-    RunCounters* counters;
     const LogTable* log_table;
-    Tune tune;
 };
-
 constexpr int NODE_PART = UNIT_VALS * NODE_UNITS;   // a pass's sums
 
-// Kinds of a pending pass: the pair's first, direct objective, objective change.
-enum : int { NP_FIRST = 0, NP_DIRECT = 1, NP_DIFF = 2 };
-
-__device__ __forceinline__ NodeSeg seg_of(const NodeSeg* seg, int n_seg, int s) {
-    int lo = 0, hi = n_seg - 1;
-    while (lo < hi) {
-        const int mid = (lo + hi + 1) >> 1;
-        if (seg[mid].slot0 <= s) lo = mid;
-        else hi = mid - 1;
-    }
-    return seg[lo];
-}
-
-__host__ __device__ inline void pair_of(int64_t idx, int64_t& x, int64_t& y) {
-    y = (int64_t)((sqrt(8.0 * (double)idx + 1.0) - 1.0) * 0.5);
-    while (y > 0 && y * (y + 1) / 2 > idx) y--;
-    while ((y + 1) * (y + 2) / 2 <= idx) y++;
-    x = idx - y * (y + 1) / 2;
-}
-
-// The samples of a job's pair idx, and its output row.
-__device__ __forceinline__ int64_t job_pair(const CohortDev& co, int64_t idx, int64_t& x, int64_t& y) {
-    if (co.kind == COHORT_RECT) {
-        x = idx / co.n_y;
-        y = idx - x * co.n_y;
-        return idx;
-    }
-    pair_of(idx, x, y);
-    return x * co.n_x - x * (x - 1) / 2 + (y - x);
-}
-
-__device__ __forceinline__ void node_write_row(kg_output* o, int64_t x, int64_t y, const double* d, double obj,
-                                               uint64_t iters, double cond) {
-    o->x = (uint64_t)x;
-    o->y = (uint64_t)y;
-#pragma unroll
-    for (int i = 0; i < 9; i++) o->jacquard[i] = d[i];
-    o->obj = obj;
-    o->iters = iters;
-    o->cond = cond;
-}
-
-__device__ __forceinline__ void store_coef(double* v, const double* x) {
-    PassCoef k;
-    make_coef(x, k);
-    const double* c = reinterpret_cast<const double*>(&k);
-#pragma unroll
-    for (int i = 0; i < NS_COEFS; i++) v[i * NS_LANES] = c[i];
-}
-
-// The step xt - xc of a difference pass, less its part along xc: both points
-// add up to 1 only to an ulp, and the objective would change by that ulp (its
-// slope along x itself is -1) where the step's own change is smaller still.
-__device__ __forceinline__ void store_step(double* v, const double* xt, const double* xc) {
-    double d[9], s = 0.0;
-#pragma unroll
-    for (int i = 0; i < 9; i++) {
-        d[i] = xt[i] - xc[i];
-        s += d[i];
-    }
-#pragma unroll
-    for (int i = 0; i < 9; i++) d[i] = fma(-s, xc[i], d[i]);
-    store_coef(v, d);
-}
-
-// Thread per slot: the pair's state before its first pass; thread 0 readies
-// the control words and the clock.
 __global__ void node_init_kernel(NodeArgs A, int n_seg, int n, unsigned long long max_waves) {
-    const int s = blockIdx.x * blockDim.x + threadIdx.x;
-    if (s == 0) {
-        A.ctl->n[0] = n;
-        A.ctl->n[1] = 0;
-        A.ctl->ticket = 0;
-        A.ctl->n_seg = n_seg;
-        A.ctl->max_waves = max_waves;
-        for (int i = 0; i < 3; i++) {
-            A.clk->start[i] = ~0ull;
-            A.clk->end[i] = 0ull;
-        }
-        A.clk->stop = 0;
-        A.clk->waves = 0;
-        A.clk->iters = 0;
-    }
-    if (s >= n) return;
-    const NodeSeg g = seg_of(A.seg, n_seg, s);
-    const CohortDev& co = A.cohorts[g.job];
-    int64_t x, y;
-    job_pair(co, g.idx0 + (s - g.slot0), x, y);
-    const bool self_pair = co.kind == COHORT_TRIANGLE && x == y;
-    double x0[9];
-    for (int i = 0; i < 9; i++) x0[i] = self_pair ? 0.0 : 1.0 / 9.0;
-    if (self_pair) { x0[0] = 0.5; x0[6] = 0.5; }
-    normalise9(x0);
-    double* st = A.state + slot_at(s, NS_VALS);
-#pragma unroll
-    for (int i = 0; i < 9; i++) st[(NS_XT + i) * NS_LANES] = x0[i];
-    store_coef(st + NS_COEF * NS_LANES, x0);
-    A.count[s] = make_int4(0, 0, 0, 4 * g.job + NP_FIRST);
-    A.list_cur[s] = s;
+    init_slot(A, n_seg, n, max_waves);
 }
 
 // ------------------------------------------------------------------- passes
@@ -954,8 +808,8 @@ extern "C" __global__ void __launch_bounds__(128, 5) node_pass_kernel(NodeArgs A
         const int u = (int)(task / groups), i = (int)(task - (int64_t)u * groups) * 8 + (lane & 7);
         const bool write = i < n;
         const int s = A.list_cur[write ? i : n - 1];
-        const int jk = A.count[s].w, kind = jk & 3;
-        const NodeDev N = A.nodes[jk >> 2];
+        const int jk = A.count[s].w, kind = jk & 7;
+        const NodeDev N = A.nodes[jk >> 3];
         switch (u) {
         case 0: node_task<0, false>(A, N, s, u, kind, part, write, T); break;
         case 1: node_task<0, true>(A, N, s, u, kind, part, write, T); break;
@@ -1005,95 +859,17 @@ __device__ __forceinline__ void rebuild_upper(const double (&m)[NMOM], double (&
     }
 }
 
-// Column j of the plain LDL^T of the block F (unit pivots and zero columns
-// outside it) and the ones after it.
-template <int j, class HF>
-__device__ __forceinline__ void ldl_plain_columns(const HF& H, unsigned F, double (&L)[36], double (&D)[9],
-                                                  bool& positive) {
-    const bool jf = (F >> j) & 1u;
-    double p[9], sjj = 0.0;
-#pragma unroll
-    for (int s = 0; s < j; s++) {
-        const double l = L[j * (j - 1) / 2 + s];
-        p[s] = D[s] * l;
-        sjj = fma(p[s], l, sjj);
-    }
-    const double dj = H(upper_at(j, j)) - sjj;
-    D[j] = jf ? dj : 1.0;
-    positive = positive && D[j] > 0.0;
-    const double rd = recip<true>(D[j]);
-#pragma unroll
-    for (int i = j + 1; i < 9; i++) {
-        double sij = 0.0;
-#pragma unroll
-        for (int s = 0; s < j; s++) sij = fma(p[s], L[i * (i - 1) / 2 + s], sij);
-        L[i * (i - 1) / 2 + j] = jf && ((F >> i) & 1u) ? quot(H(upper_at(j, i)) - sij, D[j], rd) : 0.0;
-    }
-    if constexpr (j + 1 < 9) ldl_plain_columns<j + 1>(H, F, L, D, positive);
-}
-
-// The reduced Hessian's condition estimate at a KKT point (condition_estimate
-// of kg_solver.cuh, src/sqp.rs:313-391), with zero rows and unit pivots for the
-// variables left out in place of a compacted matrix.  H(k): the upper triangle.
-template <class HF>
-__device__ __forceinline__ double condition_thread(const HF& H, const double (&x)[9], const double (&g)[9], double tol) {
-    double lambda = 0.0;
-#pragma unroll
-    for (int i = 0; i < 9; i++) lambda = fma(x[i], g[i], lambda);
-    unsigned F = 0;
-#pragma unroll
-    for (int i = 0; i < 9; i++)
-        if (!(x[i] == 0.0 && g[i] >= lambda + tol)) F |= 1u << i;
-    if (F == 0) return CUDART_INF;
-    double L[36], D[9];
-    bool positive = true;
-    ldl_plain_columns<0>(H, F, L, D, positive);
-    if (!positive) return CUDART_INF;
-    int imax = -1, imin = -1;
-    double dmax = 0.0, dmin = 0.0;
-#pragma unroll
-    for (int i = 0; i < 9; i++) {
-        if (!((F >> i) & 1u)) continue;
-        if (imax < 0 || D[i] >= dmax) { imax = i; dmax = D[i]; }
-        if (imin < 0 || D[i] < dmin) { imin = i; dmin = D[i]; }
-    }
-    // |L e_max| and |L^-T e_min|
-    double wmax = 0.0, wmin = 0.0, z[9];
-#pragma unroll
-    for (int i = 0; i < 9; i++) {
-        double l = i == imax ? 1.0 : 0.0;
-#pragma unroll
-        for (int j = 0; j < i; j++)
-            if (j == imax) l = L[i * (i - 1) / 2 + j];
-        wmax = fma(l, l, wmax);
-    }
-#pragma unroll
-    for (int i = 8; i >= 0; i--) {
-        double s = 0.0;
-#pragma unroll
-        for (int j = i + 1; j < 9; j++) s = fma(z[j], L[j * (j - 1) / 2 + i], s);
-        z[i] = (i == imin ? 1.0 : 0.0) - s;
-        wmin = fma(z[i], z[i], wmin);
-    }
-    return sqrt(wmax) * sqrt(wmin) * (dmax / dmin);
-}
-
-constexpr int NA_THREADS = 32;   // one warp a block: few slots spread over the SMs
-
-// One slot: returns the kind of its next pass, or -1 when its row is written.
-// my: the thread's column of the shared memory; sum: the block's counters.
-__device__ __forceinline__ int node_advance(const NodeArgs& A, int s, double* my, unsigned long long* sum) {
-    const Tune& tu = A.tune;
-    constexpr int SD = NS_LANES;
-    double* st = A.state + slot_at(s, NS_VALS);
-    const int* sites = A.sites + slot_at(s, NODE_UNITS);
-    const int4 ct = A.count[s];
-    const int kind = ct.w & 3;
-    // ---- the pair's moments: two genotype pairs a shape, het-het one
-    double xt[9], g[9], obj, nsites;
-    {
+// A pass's sums over nodes: two genotype pairs a shape, het-het one.
+struct NodeSums {
+    static constexpr bool FP32 = false, COEF = true;
+    const NodeArgs& A;
+    static __device__ double none() { return CUDART_NAN; }
+    __device__ __forceinline__ void load(int s, int kind, double* st, double& obj, double (&g)[9], double (&T)[QP_Q],
+                                         double& nsites) const {
         double m[NMOM];
         const double* P = A.partial + slot_at(s, NODE_PART);
+        const int* sites = A.sites + slot_at(s, NODE_UNITS);
+        constexpr int SD = NS_LANES;
         obj = 0.0;
 #pragma unroll
         for (int u = 0; u < NODE_UNITS; u++) {
@@ -1115,220 +891,26 @@ __device__ __forceinline__ int node_advance(const NodeArgs& A, int s, double* my
         } else {
             nsites = st[NS_N * SD];
         }
-        double T[QP_Q];
         rebuild_upper(m, g, T);
-        const double rn = 1.0 / nsites;
-#pragma unroll
-        for (int k = 0; k < QP_Q; k++) my[k * NA_THREADS] = quot(T[k], nsites, rn);
-#pragma unroll
-        for (int k = 0; k < 9; k++) g[k] = quot(-g[k], nsites, rn);
     }
+    __device__ __forceinline__ void count(int s, int job, int gh, int, double, bool ill, unsigned long long* sum) const {
+        const int* sites = A.sites + slot_at(s, NODE_UNITS);
+        unsigned long long evals = 0;
 #pragma unroll
-    for (int k = 0; k < 9; k++) xt[k] = st[(NS_XT + k) * SD];
-    const int gh = ct.z + 1;
-    int it = ct.x;
-    double f;
-    int next = -1;   // the kind of the next pass (-1: the pair is done)
-    bool trial_again = false;
-    if (kind == NP_FIRST) {
-        f = -obj / nsites;
-    } else {
-        // Armijo (src/sqp.rs:294): a difference pass has the objective's
-        // change itself, which the test resolves far below an ulp of f
-        const double f0 = st[NS_F * SD], alpha = st[NS_ALPHA * SD], gp = st[NS_GP * SD];
-        const double bar = alpha * (tu.bls_sufficient_decrease * gp);
-        const double df = -obj / nsites;
-        f = kind == NP_DIFF ? f0 + df : df;
-        const bool accept = kind == NP_DIFF ? df <= bar : f <= f0 + bar;
-        if (!accept && ct.y + 1 != tu.bls_max_iter) {
-            trial_again = true;
-            const double a2 = alpha * tu.bls_step_size_reduce;
-            double xc[9], sum_x = 0.0;
-#pragma unroll
-            for (int k = 0; k < 9; k++) {
-                xc[k] = st[(NS_XC + k) * SD];
-                xt[k] = xc[k] + a2 * st[(NS_P + k) * SD];
-                sum_x += xt[k];
-            }
-#pragma unroll
-            for (int k = 0; k < 9; k++) {
-                xt[k] = xt[k] / sum_x;
-                st[(NS_XT + k) * SD] = xt[k];
-            }
-            st[NS_ALPHA * SD] = a2;
-            next = fabs(a2 * gp) < DIFF_BELOW ? NP_DIFF : NP_DIRECT;
-            store_coef(st + NS_COEF * SD, xt);
-            if (next == NP_DIFF) store_step(st + NS_STEP * SD, xt, xc);
-            A.count[s] = make_int4(it, ct.y + 1, gh, (ct.w & ~3) | next);
-        } else {
-            it++;
+        for (int sh = 0; sh < 5; sh++) {
+            int c = sites[2 * sh * NS_LANES];
+            if (sh < 4) c += sites[(2 * sh + 1) * NS_LANES];
+            atomicAdd(&sum[7 + sh], (unsigned long long)c);
+            evals += (unsigned long long)((sh == 4 ? 1 : 2) * flops_fp64(sh));
         }
+        if (ill) atomicAdd(&sum[5], 1ull);   // the pairs that FP32 passes would hand to FP64
+        atomicAdd(&sum[6], evals * (unsigned long long)A.nodes[job].nk * (unsigned long long)gh);
     }
-    if (!trial_again) {
-        // ---- the accepted point
-        const CohortDev& co = A.cohorts[ct.w >> 2];
-        double resid;
-        const bool none = nsites == 0.0, last = (uint64_t)it >= co.max_iter;
-        if (none || last || kkt_ok(xt, g, tu.sqp_conv_tol, &resid)) {
-            const NodeSeg sg = seg_of(A.seg, A.ctl->n_seg, s);
-            int64_t x, y;
-            const int64_t row = job_pair(co, sg.idx0 + (s - sg.slot0), x, y);
-            double cond = CUDART_NAN;
-            if (!none && !last) cond = condition_thread([my](int k) { return my[k * NA_THREADS]; }, xt, g, tu.sqp_conv_tol);
-            if (none) {
-#pragma unroll
-                for (int k = 0; k < 9; k++) xt[k] = CUDART_NAN;
-                f = CUDART_NAN;
-            }
-            node_write_row(co.out + row, x, y, xt, f, none ? 0 : last ? co.max_iter : (uint64_t)it, cond);
-            // the counters of the call
-            unsigned long long evals = 0, shapes[5];
-#pragma unroll
-            for (int sh = 0; sh < 5; sh++) {
-                shapes[sh] = (unsigned long long)sites[2 * sh * SD];
-                if (sh < 4) shapes[sh] += (unsigned long long)sites[(2 * sh + 1) * SD];
-                evals += (unsigned long long)((sh == 4 ? 1 : 2) * flops_fp64(sh));
-                atomicAdd(&sum[7 + sh], none ? 0ull : shapes[sh]);
-            }
-            if (none) {
-                atomicAdd(&sum[0], 1ull);
-            } else {
-                atomicAdd(&sum[1], (unsigned long long)gh);
-                atomicAdd(&sum[2], (unsigned long long)nsites);
-                atomicAdd(&sum[3], (unsigned long long)nsites * (unsigned long long)gh);
-                if (last) atomicAdd(&sum[4], 1ull);
-                if (!last && !(cond <= COND_RECHECK)) atomicAdd(&sum[5], 1ull);
-                atomicAdd(&sum[6], evals * (unsigned long long)A.nodes[sg.job].nk * (unsigned long long)gh);
-            }
-        } else {
-            // ---- the QP and the step (src/sqp.rs:78-90)
-            auto H = [my](int i2, int j2) { return my[(i2 <= j2 ? upper_at(i2, j2) : upper_at(j2, i2)) * NA_THREADS]; };
-#pragma unroll
-            for (int r = 0; r < 9; r++) {
-                double hx = 0.0;
-#pragma unroll
-                for (int j = 0; j < 9; j++) hx = fma(H(r, j), xt[j], hx);
-                my[(QP_Q + r) * NA_THREADS] = g[r] - hx;
-                st[(NS_XC + r) * SD] = xt[r];
-            }
-            st[NS_F * SD] = f;
-            double y[9];
-#pragma unroll
-            for (int k = 0; k < 9; k++) y[k] = xt[k];
-            qp_simplex_thread<true>([my](int v) { return my[v * NA_THREADS]; }, tu, y);
-            // g . p with p = y - x; the first trial point x + p, normalised
-            double gp = 0.0, sum_x = 0.0, p[9];
-#pragma unroll
-            for (int k = 0; k < 9; k++) {
-                p[k] = y[k] - xt[k];
-                gp = fma(g[k], p[k], gp);
-                y[k] = xt[k] + p[k];
-                sum_x += y[k];
-            }
-#pragma unroll
-            for (int k = 0; k < 9; k++) {
-                st[(NS_P + k) * SD] = p[k];
-                y[k] = y[k] / sum_x;
-                st[(NS_XT + k) * SD] = y[k];
-            }
-            st[NS_GP * SD] = gp;
-            st[NS_ALPHA * SD] = 1.0;
-            next = fabs(gp) < DIFF_BELOW ? NP_DIFF : NP_DIRECT;
-            store_coef(st + NS_COEF * SD, y);
-            if (next == NP_DIFF) store_step(st + NS_STEP * SD, y, xt);
-            A.count[s] = make_int4(it, 0, gh, (ct.w & ~3) | next);
-        }
-    }
-    return next;
-}
+};
 
-// Everything between two passes of a slot, a thread per slot: its moments,
-// the Armijo accept test (a rejected trial backs off and takes the next pass),
-// the KKT test, at convergence the condition estimate and the row, else the
-// simplex QP and the next trial point.  The state and the sums are blocked by 32
-// slots, so a warp's loads and stores are whole sectors; H and c go
-// through shared memory (432 bytes a thread) into the QP.  One kernel instead
-// of the list form's solve, QP and step kernels: nothing is written between
-// them and a wave over few slots waits for one launch.  Bound by the FP64
-// chains of the QP (nine pivots one after the other, up to ten times).  The
-// last block to finish ends the wave: it adds the phase times and decides
-// whether the loop goes on.
 extern "C" __global__ void __launch_bounds__(NA_THREADS) node_advance_kernel(NodeArgs A, int in_loop,
                                                                             cudaGraphConditionalHandle loop) {
-    __shared__ double in[QP_IN * NA_THREADS];
-    __shared__ unsigned long long sum[12];
-    if (A.clk->stop) {   // a device loop past its last wave
-        if (in_loop && A.par && blockIdx.x == 0 && threadIdx.x == 0) {
-            A.clk->iters++;
-            cudaGraphSetConditional(loop, 0u);
-        }
-        return;
-    }
-    const int n = A.ctl->n[A.par];
-    if (threadIdx.x < 12) sum[threadIdx.x] = 0ull;
-    if (threadIdx.x == 0 && (int)blockIdx.x * NA_THREADS < n) atomicMin(&A.clk->start[2], global_ns());
-    __syncwarp();
-    double* my = in + threadIdx.x;
-    for (int base = blockIdx.x * NA_THREADS; base < n; base += gridDim.x * NA_THREADS) {
-        const bool live = base + (int)threadIdx.x < n;
-        const int s = A.list_cur[live ? base + threadIdx.x : n - 1];
-        const int next = live ? node_advance(A, s, my, sum) : -1;
-        __syncwarp();
-        // slots with another pass join the next wave's list, in this list's order
-        const unsigned more = __ballot_sync(0xffffffffu, next >= 0);
-        int at = 0;
-        if (threadIdx.x == 0 && more) at = atomicAdd(&A.ctl->n[A.par ^ 1], __popc(more));
-        at = __shfl_sync(0xffffffffu, at, 0);
-        if (next >= 0) A.list_next[at + __popc(more & ((1u << threadIdx.x) - 1u))] = s;
-    }
-    __syncwarp();
-    if (threadIdx.x < 12 && sum[threadIdx.x]) {
-        RunCounters* C = A.counters;
-        const unsigned long long v = sum[threadIdx.x];
-        switch (threadIdx.x) {
-        case 0: atomicAdd(&C->nosite_pairs, v); break;
-        case 1: atomicAdd(&C->gh_passes, v); break;
-        case 2: atomicAdd(&C->pair_sites, v); break;
-        case 3: atomicAdd(&C->work_units, v); break;
-        case 4: atomicAdd(&C->nonconverged, v); break;
-        case 5: atomicAdd(&C->fp64_pairs, v); break;
-        case 6: atomicAdd(&C->flops_fp64, v); break;
-        default: atomicAdd(&C->shape_sites[threadIdx.x - 7], v); break;
-        }
-    }
-    __syncwarp();
-    if (threadIdx.x != 0) return;
-    __threadfence();
-    if (atomicAdd(&A.ctl->ticket, 1u) != gridDim.x - 1) return;
-    // ---- the wave's end
-    __threadfence();
-    WaveClock* c = A.clk;
-    volatile NodeCtl* ctl = A.ctl;
-    const unsigned long long now = global_ns();
-    const unsigned long long p0 = *reinterpret_cast<volatile unsigned long long*>(&c->start[1]);
-    const unsigned long long p1 = *reinterpret_cast<volatile unsigned long long*>(&c->end[1]);
-    const unsigned long long s0 = *reinterpret_cast<volatile unsigned long long*>(&c->start[2]);
-    if (p1 > p0) c->acc[1] += p1 - p0;
-    if (now > s0) c->acc[2] += now - s0;
-    c->waves++;
-    unsigned int stop = 0;
-    if (ctl->n[A.par ^ 1] == 0) {
-        stop = 1;
-    } else if (c->waves >= ctl->max_waves) {
-        stop = 1;
-        c->limit_hit = 1;
-    }
-    c->stop = stop;
-    ctl->n[A.par] = 0;
-    ctl->ticket = 0;
-    for (int k = 0; k < 3; k++) {
-        c->start[k] = ~0ull;
-        c->end[k] = 0ull;
-    }
-    if (in_loop && A.par) {
-        c->iters++;
-        cudaGraphSetConditional(loop, stop ? 0u : 1u);
-    }
+    advance_wave(A, NodeSums{A}, in_loop, loop);
 }
 
 // ---------------------------------------------------------------------- CLS
@@ -1345,7 +927,7 @@ extern "C" __global__ void __launch_bounds__(NA_THREADS) node_cls_kernel(NodeArg
     __syncwarp();
     double* my = in + threadIdx.x;
     for (int s = blockIdx.x * NA_THREADS + threadIdx.x; s < n; s += gridDim.x * NA_THREADS) {
-        const NodeSeg sg = seg_of(A.seg, n_seg, s);
+        const PairSeg sg = seg_of(A.seg, n_seg, s);
         const CohortDev& co = A.cohorts[sg.job];
         const NodeDev N = A.nodes[sg.job];
         int64_t x, y;
@@ -1514,11 +1096,11 @@ int run_nodes(const std::vector<PairJob>& jobs, const RunConfig& cfg, Workspace&
     KG_NODE_TRY((cudaError_t)ws.scratch.reserve(sizeof(double) * (size_t)group * (stride / 8)));
     KG_NODE_TRY((cudaError_t)ws.slots.reserve(slot_bytes * (size_t)stride));
     // control words, one buffer: {control, clock, run counters}
-    const size_t off_clk = sizeof(NodeCtl), off_run = off_clk + sizeof(WaveClock);
+    const size_t off_clk = sizeof(SlotCtl), off_run = off_clk + sizeof(WaveClock);
     const size_t ctl_bytes = off_run + sizeof(RunCounters);
     KG_NODE_TRY((cudaError_t)ws.node_counts.reserve(ctl_bytes));
     const size_t off_nodes = sizeof(CohortDev) * n_jobs, off_seg = off_nodes + sizeof(NodeDev) * n_jobs;
-    const size_t blob = off_seg + sizeof(NodeSeg) * n_jobs;
+    const size_t blob = off_seg + sizeof(PairSeg) * n_jobs;
     KG_NODE_TRY((cudaError_t)ws.node_table.reserve(blob));
     KG_NODE_TRY((cudaError_t)ws.host.reserve(blob + sizeof(WaveClock) + sizeof(RunCounters)));
     char* counts = ws.node_counts.as<char>();
@@ -1549,13 +1131,13 @@ int run_nodes(const std::vector<PairJob>& jobs, const RunConfig& cfg, Workspace&
         NodeArgs A{};
         A.cohorts = reinterpret_cast<CohortDev*>(dtab);
         A.nodes = reinterpret_cast<NodeDev*>(dtab + off_nodes);
-        A.seg = reinterpret_cast<NodeSeg*>(dtab + off_seg);
+        A.seg = reinterpret_cast<PairSeg*>(dtab + off_seg);
         A.state = ws.slots.as<double>();
         A.partial = A.state + (size_t)(NS_VALS + 2) * stride;
         A.count = reinterpret_cast<int4*>(A.partial + (size_t)NODE_UNITS * UNIT_VALS * stride);
         A.sites = reinterpret_cast<int*>(A.count + stride);
         int* lists = A.sites + NODE_UNITS * stride;
-        A.ctl = reinterpret_cast<NodeCtl*>(counts);
+        A.ctl = reinterpret_cast<SlotCtl*>(counts);
         A.clk = reinterpret_cast<WaveClock*>(counts + off_clk);
         A.counters = reinterpret_cast<RunCounters*>(counts + off_run);
         A.log_table = E.log_table.as<LogTable>();
@@ -1576,25 +1158,8 @@ int run_nodes(const std::vector<PairJob>& jobs, const RunConfig& cfg, Workspace&
         KG_NODE_TRY(cudaFuncSetAttribute(node_weights_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, NW_SMEM));
         for (auto& e : E.ev)
             if (!e) KG_NODE_TRY(cudaEventCreate(&e));
-        KG_NODE_TRY(cudaGraphCreate(&E.g, 0));
-        cudaGraphConditionalHandle h;
-        KG_NODE_TRY(cudaGraphConditionalHandleCreate(&h, E.g, 1, cudaGraphCondAssignDefault));
-        cudaGraphNodeParams np{};
-        np.type = cudaGraphNodeTypeConditional;
-        np.conditional.handle = h;
-        np.conditional.type = cudaGraphCondTypeWhile;
-        np.conditional.size = 1;
-        cudaGraphNode_t node;
-        KG_NODE_TRY(cudaGraphAddNode(&node, E.g, nullptr, 0, &np));
-        cudaGraph_t body = np.conditional.phGraph_out[0];
-        KG_NODE_TRY(cudaStreamBeginCaptureToGraph(st, body, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal));
-        for (int par = 0; par < 2; par++) E.wave(par, 1, h, st);
-        cudaGraph_t captured = nullptr;
-        const cudaError_t ce = cudaGetLastError();
-        const cudaError_t ee = cudaStreamEndCapture(st, &captured);
-        KG_NODE_TRY(ce);
-        KG_NODE_TRY(ee);
-        KG_NODE_TRY(cudaGraphInstantiate(&E.x, E.g, 0));
+        KG_NODE_TRY(wave_loop_graph(
+            st, [&](int par, int in_loop, cudaGraphConditionalHandle h) { E.wave(par, in_loop, h, st); }, &E.g, &E.x));
         E.key = key;
         E.key_iterations = cfg.iterations;
         E.key_dev = dev;
@@ -1603,7 +1168,7 @@ int run_nodes(const std::vector<PairJob>& jobs, const RunConfig& cfg, Workspace&
     std::memcpy(htab, table.data(), sizeof(CohortDev) * n_jobs);
     KG_NODE_TRY(cudaMemsetAsync(counts, 0, ctl_bytes, st));
     NodeDev* h_nodes = reinterpret_cast<NodeDev*>(htab + off_nodes);
-    NodeSeg* h_seg = reinterpret_cast<NodeSeg*>(htab + off_seg);
+    PairSeg* h_seg = reinterpret_cast<PairSeg*>(htab + off_seg);
     RunCounters* d_run = reinterpret_cast<RunCounters*>(counts + off_run);
     const WaveClock* d_clk = reinterpret_cast<const WaveClock*>(counts + off_clk);
     int job = 0;
@@ -1619,7 +1184,7 @@ int run_nodes(const std::vector<PairJob>& jobs, const RunConfig& cfg, Workspace&
             const int64_t np = table[job].n_pairs, take = std::min<int64_t>(np - at, cap - n);
             if (take > 0) {
                 const Cohort& c = *jobs[job].panel;
-                h_seg[n_seg] = NodeSeg{at, (int32_t)n, (int32_t)take, job, 0};
+                h_seg[n_seg] = PairSeg{at, (int32_t)n, (int32_t)take, job, 0};
                 NodeDev& nd = h_nodes[job];
                 nd.w = ws.scratch.as<double>();
                 nd.group = group;
@@ -1638,7 +1203,7 @@ int run_nodes(const std::vector<PairJob>& jobs, const RunConfig& cfg, Workspace&
         KG_NODE_TRY(cudaMemcpyAsync(dtab, htab, blob, cudaMemcpyHostToDevice, st));
         KG_NODE_TRY(cudaEventRecord(E.ev[0], st));
         for (int k = 0; k < n_seg; k++) {
-            const NodeSeg& g = h_seg[k];
+            const PairSeg& g = h_seg[k];
             const Cohort& c = *jobs[g.job].panel;
             NodeProduct P;
             P.rect = jobs[g.job].kind == COHORT_RECT ? 1 : 0;

@@ -1004,6 +1004,7 @@ enum : int { PASS_FP32_DIRECT = 0, PASS_FP32_DIFF = 1, PASS_FP64 = 2, PASS_CLS =
 
 struct PairEval {
     double f;       // objective at the evaluated point
+    double df;      // soft likelihoods: its change, in a difference pass
     double g[9];    // gradient (warp-uniform)
     double Hr[9];   // this lane's row of the Hessian (lanes 0..8)
 };

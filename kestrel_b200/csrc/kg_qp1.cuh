@@ -20,6 +20,8 @@
 // three instructions instead of a division.
 #pragma once
 
+#include <math_constants.h>
+
 #include "kg_solver.cuh"
 
 namespace kg {
@@ -229,5 +231,79 @@ __host__ __device__ __forceinline__ int qp_simplex_thread(const In& in, const Tu
     }
     return tu.qp_max_iter;
 }
+
+// Column j of the plain LDL^T of the block F (unit pivots and zero columns
+// outside it) and the ones after it.
+template <int j, class HF>
+__device__ __forceinline__ void ldl_plain_columns(const HF& H, unsigned F, double (&L)[36], double (&D)[9],
+                                                  bool& positive) {
+    const bool jf = (F >> j) & 1u;
+    double p[9], sjj = 0.0;
+#pragma unroll
+    for (int s = 0; s < j; s++) {
+        const double l = L[j * (j - 1) / 2 + s];
+        p[s] = D[s] * l;
+        sjj = fma(p[s], l, sjj);
+    }
+    const double dj = H(upper_at(j, j)) - sjj;
+    D[j] = jf ? dj : 1.0;
+    positive = positive && D[j] > 0.0;
+    const double rd = recip<true>(D[j]);
+#pragma unroll
+    for (int i = j + 1; i < 9; i++) {
+        double sij = 0.0;
+#pragma unroll
+        for (int s = 0; s < j; s++) sij = fma(p[s], L[i * (i - 1) / 2 + s], sij);
+        L[i * (i - 1) / 2 + j] = jf && ((F >> i) & 1u) ? quot(H(upper_at(j, i)) - sij, D[j], rd) : 0.0;
+    }
+    if constexpr (j + 1 < 9) ldl_plain_columns<j + 1>(H, F, L, D, positive);
+}
+
+// The reduced Hessian's condition estimate at a KKT point (condition_estimate
+// of kg_solver.cuh, src/sqp.rs:313-391), with zero rows and unit pivots for the
+// variables left out in place of a compacted matrix.  H(k): the upper triangle.
+template <class HF>
+__device__ __forceinline__ double condition_thread(const HF& H, const double (&x)[9], const double (&g)[9], double tol) {
+    double lambda = 0.0;
+#pragma unroll
+    for (int i = 0; i < 9; i++) lambda = fma(x[i], g[i], lambda);
+    unsigned F = 0;
+#pragma unroll
+    for (int i = 0; i < 9; i++)
+        if (!(x[i] == 0.0 && g[i] >= lambda + tol)) F |= 1u << i;
+    if (F == 0) return CUDART_INF;
+    double L[36], D[9];
+    bool positive = true;
+    ldl_plain_columns<0>(H, F, L, D, positive);
+    if (!positive) return CUDART_INF;
+    int imax = -1, imin = -1;
+    double dmax = 0.0, dmin = 0.0;
+#pragma unroll
+    for (int i = 0; i < 9; i++) {
+        if (!((F >> i) & 1u)) continue;
+        if (imax < 0 || D[i] >= dmax) { imax = i; dmax = D[i]; }
+        if (imin < 0 || D[i] < dmin) { imin = i; dmin = D[i]; }
+    }
+    // |L e_max| and |L^-T e_min|
+    double wmax = 0.0, wmin = 0.0, z[9];
+#pragma unroll
+    for (int i = 0; i < 9; i++) {
+        double l = i == imax ? 1.0 : 0.0;
+#pragma unroll
+        for (int j = 0; j < i; j++)
+            if (j == imax) l = L[i * (i - 1) / 2 + j];
+        wmax = fma(l, l, wmax);
+    }
+#pragma unroll
+    for (int i = 8; i >= 0; i--) {
+        double s = 0.0;
+#pragma unroll
+        for (int j = i + 1; j < 9; j++) s = fma(z[j], L[j * (j - 1) / 2 + i], s);
+        z[i] = (i == imin ? 1.0 : 0.0) - s;
+        wmin = fma(z[i], z[i], wmin);
+    }
+    return sqrt(wmax) * sqrt(wmin) * (dmax / dmin);
+}
+
 
 }  // namespace kg

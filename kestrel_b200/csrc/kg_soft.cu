@@ -6,20 +6,26 @@
 //
 // Layout: biallelic likelihoods double [sample][site][3] (0/0, 0/1, 1/1;
 // linear scale; a NaN marks a missing sample) as loaded; the kept sites'
-// likelihoods are also packed as FP32 [sample][kept site] float4 records
-// (the three likelihoods and a zero; all three NaN when missing), beside the
-// kept sites' FP32 (REF, ALT) frequency pairs.  Tri- and tetra-allelic sites: double [sample][site][6] and
+// likelihoods are also packed as FP32, two sites a record [sample][site pair]
+// {l0a, l0b, l1a, l1b}, {l2a, l2b, 0, 0} (NaN where a sample is missing and
+// past the last site), beside {pa, pb, qa, qb} of the kept frequencies.  Tri- and tetra-allelic sites: double [sample][site][6] and
 // [sample][site][10] in the VCF genotype order.
 //
-// A warp per pair, lanes over the kept sites; the SQP itself is FP64.  Its
-// evaluations (f, g and H at a point) of the biallelic sites run in one of two
-// forms:
+// A warp per pair, lanes over the kept sites; the SQP itself is FP64.  FP32C
+// pairs without tri- and tetra-allelic sites run in waves: the evaluations in
+// soft_pass_kernel, the solver between them in soft_advance_kernel, a thread per
+// pair (kg_advance.cuh).  In one kernel the solver's 1,300 straight instructions an
+// iteration pushed the site loop out of the instruction caches (its warps waited
+// for instructions twice as long as they issued) and took 145,000 cycles a QP.
+// The other pairs run in soft_pairs_kernel, from a counter.  The evaluations (f,
+// g and H at a point) of the biallelic sites have one of two forms:
 //   * FP32 (the default, KG_PREC_FP32C): from the FP32 likelihoods, which stay
 //     L2-resident for cohorts of a few hundred samples, each site's row L is
-//     formed from the pair's nine likelihood products in closed form; d =
-//     eps + L.x with the FP32 hi parts of x, the sums in FP32 promoted to FP64
-//     (gradient and objective every 8 sites, Hessian every 32 into the lane's
-//     shared memory), and the lo parts of x restored to first order in FP64;
+//     formed from the pair's nine likelihood products in closed form, two sites
+//     an instruction (packed FP32); d = eps + L.x with the FP32 hi parts of x,
+//     the sums in FP32 promoted to FP64 (per site parity: gradient and
+//     objective every 8 sites, Hessian every 32 into the lane's shared memory),
+//     and the lo parts of x restored to first order in FP64;
 //     near convergence the objective change is summed as log(d / d_old), as
 //     on the hard-call path.  A pair whose FP32 condition estimate exceeds
 //     COND_RECHECK, or whose KKT residual stalls below 1e-6 three times, is
@@ -36,16 +42,18 @@
 #include <math_constants.h>
 
 #include <algorithm>
+#include <cstdlib>
 #include <string>
 #include <vector>
 
 #include "kestrel_gpu.h"
+#include "kg_advance.cuh"
 #include "kg_allele.cuh"
 #include "kg_alleleN.cuh"
 #include "kg_bulk.cuh"
 #include "kg_engine.h"
 #include "kg_pair.cuh"
-#include "kg_rowsolve.cuh"
+#include "kg_qp1.cuh"
 #include "kg_solver.cuh"
 
 namespace kg {
@@ -134,11 +142,13 @@ __global__ void soft_freq_kernel(const double* __restrict__ gl, int64_t n_sample
 constexpr int SOFT_WARPS = 4;
 constexpr int HS = 33;   // shared-memory stride of the Hessian sums: 32 lane partials, then the warp total
 // A warp's shared memory: the Hessian sums (45 rows of HS doubles, padded to
-// 16 bytes), then per lane SOFT_STAGES slots of 48 bytes for the FP32 form's
-// prefetched site (the two samples' float4 records and the (p, q) pair).
-constexpr int SOFT_STAGES = 3;
+// 16 bytes), then per lane SOFT_STAGES slots of 80 bytes for the FP32 form's
+// prefetched sites (the two samples' records of a site pair and its
+// frequencies).
+constexpr int SOFT_STAGES = 2;
+constexpr int SOFT_SLOT = 5;   // float4 of a slot
 constexpr int SOFT_SUMS_BYTES = (45 * HS * 8 + 15) / 16 * 16;
-constexpr int SOFT_WARP_SMEM = SOFT_SUMS_BYTES + 32 * SOFT_STAGES * 48;
+constexpr int SOFT_WARP_SMEM = SOFT_SUMS_BYTES + 32 * SOFT_STAGES * SOFT_SLOT * 16;
 constexpr int SOFT_SMEM = SOFT_WARPS * SOFT_WARP_SMEM;
 
 // ---------------------------------------------------------- tri / tetra
@@ -351,21 +361,20 @@ __device__ __forceinline__ void hessian_totals(double* hs, int lane) {
     __syncwarp();
 }
 
-// f, g and this lane's Hessian row at x over the pair's rows (-(1/n) sum log(eps
-// + L.x), -(1/n) sum L r, (1/n) sum L L' r^2, r = 1/(eps + L.x)); n = rows
-// without a NaN.  hs: the warp's Hessian sums in shared memory; R, nm: the
-// pair's multi-allelic rows.
-__device__ __noinline__ int64_t soft_evaluate(const double* __restrict__ gl, int64_t n_sites,
-                                              const int32_t* __restrict__ kept, const double* __restrict__ kp,
-                                              const double* __restrict__ kq, int64_t nk, int64_t x, int64_t y,
-                                              const double* xv, double eps, int lane, double* hs, const double* R,
-                                              int64_t nm, PairEval& ev) {
-    double f = 0.0, g[9];
+// The FP64 site loop over every parts-th group of 32 kept sites from part on:
+// this lane's sums of log d, L r and (in shared memory) L L' r^2, r = 1/(eps +
+// L.x), and its rows without a NaN.
+__device__ __forceinline__ void soft_sites64(const double* __restrict__ gl, int64_t n_sites,
+                                             const int32_t* __restrict__ kept, const double* __restrict__ kp,
+                                             const double* __restrict__ kq, int64_t nk, int64_t x, int64_t y,
+                                             const double* xv, double eps, int lane, int part, int parts, double* hs,
+                                             double (&g)[9], double& f, int64_t& n) {
+    f = 0.0;
 #pragma unroll
     for (int i = 0; i < 9; i++) g[i] = 0.0;
     for (int a = 0; a < 45; a++) hs[a * HS + lane] = 0.0;
-    int64_t n = 0;
-    for (int64_t k = lane; k < nk; k += 32) {
+    n = 0;
+    for (int64_t k = lane + 32 * part; k < nk; k += 32 * parts) {
         const int64_t v = kept[k];
         const double* lx = gl + (x * n_sites + v) * 3;
         const double* ly = gl + (y * n_sites + v) * 3;
@@ -403,6 +412,20 @@ __device__ __noinline__ int64_t soft_evaluate(const double* __restrict__ gl, int
             for (int j = i; j < 9; j++, a++) hs[a * HS + lane] = fma(b[i], b[j], hs[a * HS + lane]);
         n++;
     }
+}
+
+// f, g and this lane's Hessian row at x over the pair's rows (-(1/n) sum log(eps
+// + L.x), -(1/n) sum L r, (1/n) sum L L' r^2, r = 1/(eps + L.x)); n = rows
+// without a NaN.  hs: the warp's Hessian sums in shared memory; R, nm: the
+// pair's multi-allelic rows.
+__device__ __noinline__ int64_t soft_evaluate(const double* __restrict__ gl, int64_t n_sites,
+                                              const int32_t* __restrict__ kept, const double* __restrict__ kp,
+                                              const double* __restrict__ kq, int64_t nk, int64_t x, int64_t y,
+                                              const double* xv, double eps, int lane, double* hs, const double* R,
+                                              int64_t nm, PairEval& ev) {
+    double f, g[9];
+    int64_t n;
+    soft_sites64(gl, n_sites, kept, kp, kq, nk, x, y, xv, eps, lane, 0, 1, hs, g, f, n);
     // warp sums (fixed butterfly order)
     for (int off = 16; off > 0; off >>= 1) {
         f += __shfl_xor_sync(0xffffffffu, f, off);
@@ -423,153 +446,208 @@ __device__ __noinline__ int64_t soft_evaluate(const double* __restrict__ gl, int
     return n;
 }
 
-// Packs the kept sites' likelihoods as FP32 [sample][kept][3], all three NaN
-// for a missing sample, and the kept frequencies as FP32.
+// Packs the kept sites' likelihoods and frequencies as FP32, two sites a record
+// (see the file comment).
 __global__ void soft_pack32_kernel(const double* __restrict__ gl, int64_t n_samples, int64_t n_sites,
                                    const int32_t* __restrict__ kept, const double* __restrict__ kp,
                                    const double* __restrict__ kq, int64_t nk, float4* __restrict__ g32,
-                                   float2* __restrict__ pq32) {
-    const int64_t total = n_samples * nk;
+                                   float4* __restrict__ pq32) {
+    const int64_t np = (nk + 1) / 2, total = n_samples * np;
     for (int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; t < total; t += (int64_t)gridDim.x * blockDim.x) {
-        const int64_t s = t / nk, k = t - s * nk;
-        const double* r = gl + (s * n_sites + kept[k]) * 3;
-        const bool miss = isnan(r[0]) || isnan(r[1]) || isnan(r[2]);
-        g32[t] = miss ? make_float4(CUDART_NAN_F, CUDART_NAN_F, CUDART_NAN_F, 0.f)
-                      : make_float4((float)r[0], (float)r[1], (float)r[2], 0.f);
-        if (s == 0) pq32[k] = make_float2((float)kp[k], (float)kq[k]);
+        const int64_t s = t / np, j = t - s * np;
+        float l[2][3];
+#pragma unroll
+        for (int h = 0; h < 2; h++) {
+            const int64_t k = 2 * j + h;
+            const double* r = gl + (s * n_sites + (k < nk ? kept[k] : 0)) * 3;
+            const bool miss = k >= nk || isnan(r[0]) || isnan(r[1]) || isnan(r[2]);
+#pragma unroll
+            for (int g = 0; g < 3; g++) l[h][g] = miss ? CUDART_NAN_F : (float)r[g];
+        }
+        g32[2 * t] = make_float4(l[0][0], l[1][0], l[0][1], l[1][1]);
+        g32[2 * t + 1] = make_float4(l[0][2], l[1][2], 0.f, 0.f);
+        if (s == 0) {
+            const int64_t k1 = 2 * j + 1 < nk ? 2 * j + 1 : 2 * j;
+            pq32[j] = make_float4((float)kp[2 * j], (float)kp[k1], (float)kq[2 * j], (float)kq[k1]);
+        }
     }
 }
 
-// The FP32 evaluation (see the file comment) at xt; in a difference pass
-// (DIFF) the objective is f_old - (1/n) sum log(d / d_old) with d_old at xc.
-// hs: the warp's FP64 Hessian sums in shared memory; R, nm: the pair's
-// multi-allelic rows, added in FP64 after the lo correction of the biallelic
-// sums.  Returns n.  Not inlined: the site loop gets the registers the pair's
-// SQP state would hold.
+// The FP32 site loop (see the file comment) over every parts-th group of 32
+// site pairs from part on, at xt: this lane's FP64 sums G of L r and F of log2 d
+// or (DIFF: step = xt - xc less its part along xc, difference_step) of log(d /
+// d_old), in shared memory of L L' r^2, and its sites.
 template <bool DIFF>
-__device__ __noinline__ int64_t soft_evaluate32(const float4* __restrict__ g32, const float2* __restrict__ pq32,
-                                                int64_t nk, int64_t x, int64_t y,
-                                                const double* xt, const double* xc, double f_old, double eps,
-                                                int lane, double* hs, float4* slots, const double* R, int64_t nm,
-                                                PairEval& ev) {
+__device__ __forceinline__ void soft_sites32(const float4* __restrict__ g32, const float4* __restrict__ pq32, int64_t nk,
+                                             int64_t x, int64_t y, const double* xt, const double* step, double eps,
+                                             int lane, int part, int parts, double* hs, float4* slots, double (&G)[9],
+                                             double& F, int64_t& n) {
     const bool diff = DIFF;
     float xh[9], sd[9];
 #pragma unroll
     for (int i = 0; i < 9; i++) {
         xh[i] = (float)xt[i];
-        sd[i] = DIFF ? (float)(xt[i] - xc[i]) : 0.f;
+        sd[i] = DIFF ? (float)step[i] : 0.f;
     }
-    double G[9], F = 0.0;
-    float g[9], h[45], o = 0.f;
+    F = 0.0;
+    float2 g[9], h[45], o = dup2(0.f);
 #pragma unroll
-    for (int i = 0; i < 9; i++) { G[i] = 0.0; g[i] = 0.f; }
+    for (int i = 0; i < 9; i++) { G[i] = 0.0; g[i] = dup2(0.f); }
 #pragma unroll
-    for (int a = 0; a < 45; a++) h[a] = 0.f;
+    for (int a = 0; a < 45; a++) h[a] = dup2(0.f);
     for (int a = 0; a < 45; a++) hs[a * HS + lane] = 0.0;
-    const float4* lx = g32 + x * nk;
-    const float4* ly = g32 + y * nk;
-    const float e32 = (float)eps;
-    const int nk32 = (int)nk;
-    int64_t n = 0;
-    // Warp-uniform iterations (a lane past the end or at a missing sample
-    // skips the site), so that the FP64 flushes below run once per warp.  The
-    // site two iterations ahead is copied by cp.async into the lane's slots:
-    // the prefetch holds no registers.
-    float4* my = slots + lane * (3 * SOFT_STAGES);
+    const int np = (int)((nk + 1) >> 1);   // site pairs
+    const float4* lx = g32 + x * 2 * (int64_t)np;
+    const float4* ly = g32 + y * 2 * (int64_t)np;
+    const float2 e32 = dup2((float)eps);
+    n = 0;
+    // Warp-uniform iterations over site pairs (a lane past the end has NaN
+    // records), so that the FP64 flushes below run once per warp.  The pair of
+    // the next iteration is copied by cp.async into the lane's slots: the
+    // prefetch holds no registers.  Two sites an instruction, because the loop is
+    // bound by fetching and issuing it: with one site the warps waited for
+    // instructions twice as long as they issued (277 a site, three warps a
+    // scheduler at different places of the kernel).
+    float4* my = slots + lane * (SOFT_SLOT * SOFT_STAGES);
     const uint32_t my0 = smem_u32(my);
     auto issue = [&](int it2) {
-        const int k2 = lane + 32 * it2;
-        if (k2 < nk32) {
-            const uint32_t d = my0 + 48u * (uint32_t)(it2 % SOFT_STAGES);
-            cp_async16(d, lx + k2);
-            cp_async16(d + 16u, ly + k2);
-            cp_async8(d + 32u, pq32 + k2);
+        const int k2 = lane + 32 * (it2 * parts + part);
+        if (k2 < np) {
+            const uint32_t d = my0 + 16u * SOFT_SLOT * (uint32_t)(it2 & 1);
+            cp_async16(d, lx + 2 * k2);
+            cp_async16(d + 16u, lx + 2 * k2 + 1);
+            cp_async16(d + 32u, ly + 2 * k2);
+            cp_async16(d + 48u, ly + 2 * k2 + 1);
+            cp_async16(d + 64u, pq32 + k2);
         }
         cp_async_commit();
     };
-    const int iters = (nk32 + 31) >> 5;
+    const int iters = max(0, (((np + 31) >> 5) - part + parts - 1) / parts);
     issue(0);
-    issue(1);
     for (int it = 0; it < iters; it++) {
-        issue(it + 2);
-        cp_async_wait<2>();   // this iteration's site has landed
-        const int k = lane + 32 * it;
-        const float4* st = my + 3 * (it % SOFT_STAGES);
-        float4 X = make_float4(CUDART_NAN_F, 0.f, 0.f, 0.f), Y = X;
-        float2 PQ = make_float2(0.f, 0.f);
-        if (k < nk32) {
-            X = st[0];
-            Y = st[1];
-            PQ = *reinterpret_cast<const float2*>(st + 2);
+        issue(it + 1);
+        cp_async_wait<1>();   // this iteration's pair has landed
+        const float4* st = my + SOFT_SLOT * (it & 1);
+        const bool in = lane + 32 * (it * parts + part) < np;
+        float2 X0 = dup2(CUDART_NAN_F), X1 = X0, X2 = X0, Y0 = X0, Y1 = X0, Y2 = X0, p = dup2(0.f), q = p;
+        if (in) {
+            const float4 a0 = st[0], c0 = st[2], f0 = st[4];
+            X0 = make_float2(a0.x, a0.y);
+            X1 = make_float2(a0.z, a0.w);
+            X2 = *reinterpret_cast<const float2*>(st + 1);
+            Y0 = make_float2(c0.x, c0.y);
+            Y1 = make_float2(c0.z, c0.w);
+            Y2 = *reinterpret_cast<const float2*>(st + 3);
+            p = make_float2(f0.x, f0.y);
+            q = make_float2(f0.z, f0.w);
         }
-        const float X0 = X.x, X1 = X.y, X2 = X.z, Y0 = Y.x, Y1 = Y.y, Y2 = Y.z;
-        const float p = PQ.x, q = PQ.y;
-        // a missing sample has all three NaN (and so has a lane past the end)
-        if (!isnan(X0) && !isnan(Y0)) {
-            // L = sum over (gx, gy) of GLx(gx) GLy(gy) m(gx, gy), the nine rows
-            // of the biallelic conditional table (cls_row) gathered by entry
-            const float A = X0 * Y0, B = X2 * Y2, C = X0 * Y2, D = X2 * Y0, E = X0 * Y1;
-            const float Fx = X2 * Y1, Gx = X1 * Y0, Hx = X1 * Y2, I = X1 * Y1;
-            const float p2 = p * p, q2 = q * q, pq = p * q;
-            const float p2q = p2 * q, pq2 = p * q2;
-            const float S2 = fmaf(A, p2, B * q2);
-            const float S3 = fmaf(A, p2 * p, B * (q2 * q));
-            float L[9];
-            L[0] = fmaf(A, p, B * q);
-            L[1] = fmaf(C + D, pq, S2);
-            L[2] = fmaf(E + Fx, pq, S2);
-            L[3] = fmaf(2.0f * E, p2q, fmaf(2.0f * Fx, pq2, fmaf(C, pq2, fmaf(D, p2q, S3))));
-            L[4] = fmaf(Gx + Hx, pq, S2);
-            L[5] = fmaf(2.0f * Gx, p2q, fmaf(2.0f * Hx, pq2, fmaf(C, p2q, fmaf(D, pq2, S3))));
-            L[6] = fmaf(2.0f * I, pq, S2);
-            L[7] = fmaf(I, p2q + pq2, fmaf(Fx + Hx, pq2, fmaf(E + Gx, p2q, S3)));
-            L[8] = fmaf(4.0f * I, p2 * q2,
-                        fmaf(2.0f * (Fx + Hx), pq2 * q,
-                             fmaf(2.0f * (E + Gx), p2q * p, fmaf(C + D, p2 * q2, fmaf(A, p2 * p2, B * (q2 * q2))))));
-            const float d = dot9_eps(L, xh, e32);
-            const float r = rcp_approx(d);
-            float b[9];
+        // L = sum over (gx, gy) of GLx(gx) GLy(gy) m(gx, gy), the nine rows of
+        // the biallelic conditional table (cls_row) gathered by entry
+        const float2 A = mul2(X0, Y0), B = mul2(X2, Y2), C = mul2(X0, Y2), D = mul2(X2, Y0);
+        const float2 E = mul2(X0, Y1), Fx = mul2(X2, Y1), Gx = mul2(X1, Y0), Hx = mul2(X1, Y2), I = mul2(X1, Y1);
+        // a site where either sample is missing has NaN products
+        const bool v0 = !isnan(A.x), v1 = !isnan(A.y);
+        const float2 two = dup2(2.0f);
+        const float2 p2 = mul2(p, p), q2 = mul2(q, q), pq = mul2(p, q), p2q = mul2(p2, q), pq2 = mul2(p, q2);
+        const float2 S2 = fma2(A, p2, mul2(B, q2)), S3 = fma2(A, mul2(p2, p), mul2(B, mul2(q2, q)));
+        float2 L[9];
+        L[0] = fma2(A, p, mul2(B, q));
+        L[1] = fma2(add2(C, D), pq, S2);
+        L[2] = fma2(add2(E, Fx), pq, S2);
+        L[3] = fma2(mul2(two, E), p2q, fma2(mul2(two, Fx), pq2, fma2(C, pq2, fma2(D, p2q, S3))));
+        L[4] = fma2(add2(Gx, Hx), pq, S2);
+        L[5] = fma2(mul2(two, Gx), p2q, fma2(mul2(two, Hx), pq2, fma2(C, p2q, fma2(D, pq2, S3))));
+        L[6] = fma2(mul2(two, I), pq, S2);
+        const float2 FH = add2(Fx, Hx), EG = add2(E, Gx);
+        L[7] = fma2(I, add2(p2q, pq2), fma2(FH, pq2, fma2(EG, p2q, S3)));
+        const float2 p2q2 = mul2(p2, q2);
+        L[8] = fma2(mul2(dup2(4.0f), I), p2q2,
+                    fma2(mul2(two, FH), mul2(pq2, q),
+                         fma2(mul2(two, EG), mul2(p2q, p),
+                              fma2(add2(C, D), p2q2, fma2(A, mul2(p2, p2), mul2(B, mul2(q2, q2)))))));
+        // d = eps + L.x in three chains (dot9_eps)
+        const float2 da = fma2(L[0], dup2(xh[0]), fma2(L[3], dup2(xh[3]), fma2(L[6], dup2(xh[6]), e32)));
+        const float2 db = fma2(L[1], dup2(xh[1]), fma2(L[4], dup2(xh[4]), mul2(L[7], dup2(xh[7]))));
+        const float2 dc = fma2(L[2], dup2(xh[2]), fma2(L[5], dup2(xh[5]), mul2(L[8], dup2(xh[8]))));
+        const float2 d = add2(da, add2(db, dc));
+        const float2 r = make_float2(v0 ? rcp_approx(d.x) : 0.f, v1 ? rcp_approx(d.y) : 0.f);
+        if (!v0 || !v1) {
 #pragma unroll
-            for (int i = 0; i < 9; i++) {
-                b[i] = L[i] * r;
-                g[i] += b[i];
-            }
+            for (int i = 0; i < 9; i++) L[i] = make_float2(v0 ? L[i].x : 0.f, v1 ? L[i].y : 0.f);
+        }
+        if (!diff) {
+            o = add2(o, make_float2(v0 ? lg2_approx(d.x) : 0.f, v1 ? lg2_approx(d.y) : 0.f));
+        } else {
+            float2 dl = mul2(L[0], dup2(sd[0]));
+#pragma unroll
+            for (int i = 1; i < 9; i++) dl = fma2(L[i], dup2(sd[i]), dl);
+            dl = mul2(dl, r);
+            o = add2(o, make_float2(neg_log1m(dl.x), neg_log1m(dl.y)));
+        }
+#pragma unroll
+        for (int i = 0; i < 9; i++) {
+            g[i] = fma2(L[i], r, g[i]);
+            L[i] = mul2(L[i], r);
+        }
+        {
             int a = 0;
 #pragma unroll
             for (int i = 0; i < 9; i++)
 #pragma unroll
-                for (int j = i; j < 9; j++, a++) h[a] = fmaf(b[i], b[j], h[a]);
-            if (!diff) {
-                o += lg2_approx(d);
-            } else {
-                float dl = 0.f;
-#pragma unroll
-                for (int i = 0; i < 9; i++) dl = fmaf(L[i], sd[i], dl);
-                o += neg_log1m(dl * r);
-            }
-            n++;
+                for (int j = i; j < 9; j++, a++) h[a] = fma2(L[i], L[j], h[a]);
         }
+        n += (v0 ? 1 : 0) + (v1 ? 1 : 0);
         if ((it & 7) == 7) {
 #pragma unroll
-            for (int i = 0; i < 9; i++) { G[i] += (double)g[i]; g[i] = 0.f; }
-            F += (double)o;
-            o = 0.f;
+            for (int i = 0; i < 9; i++) {
+                G[i] += (double)g[i].x;
+                G[i] += (double)g[i].y;
+                g[i] = dup2(0.f);
+            }
+            F += (double)o.x;
+            F += (double)o.y;
+            o = dup2(0.f);
         }
-        if ((it & 31) == 31) {
+        if ((it & 15) == 15) {
 #pragma unroll
             for (int a2 = 0; a2 < 45; a2++) {
-                hs[a2 * HS + lane] += (double)h[a2];
-                h[a2] = 0.f;
+                hs[a2 * HS + lane] += (double)(h[a2].x + h[a2].y);
+                h[a2] = dup2(0.f);
                 asm volatile("" ::: "memory");   // one read-modify-write at a time: no register peak
             }
         }
     }
     cp_async_wait<0>();   // no copy outstanding into the slots (they are past the last site)
 #pragma unroll
-    for (int i = 0; i < 9; i++) G[i] += (double)g[i];
-    F += (double)o;
+    for (int i = 0; i < 9; i++) {
+        G[i] += (double)g[i].x;
+        G[i] += (double)g[i].y;
+    }
+    F += (double)o.x;
+    F += (double)o.y;
 #pragma unroll
-    for (int a = 0; a < 45; a++) hs[a * HS + lane] += (double)h[a];
+    for (int a = 0; a < 45; a++) hs[a * HS + lane] += (double)(h[a].x + h[a].y);
+}
+
+// The FP32 evaluation (see the file comment) at xt; in a difference pass
+// (DIFF) the objective is f_old - (1/n) sum log(d / d_old) with d_old at xc,
+// step = xt - xc less its part along xc (difference_step).  // hs: the warp's FP64 Hessian sums in shared memory; R, nm: the pair's
+// multi-allelic rows, added in FP64 after the lo correction of the biallelic
+// sums.  Returns n.  Not inlined: the site loop gets the registers the pair's
+// SQP state would hold.
+template <bool DIFF>
+__device__ __noinline__ int64_t soft_evaluate32(const float4* __restrict__ g32, const float4* __restrict__ pq32,
+                                                int64_t nk, int64_t x, int64_t y,
+                                                const double* xt, const double* step, const double* xc, double f_old,
+                                                double eps, int lane, double* hs, float4* slots, const double* R,
+                                                int64_t nm, PairEval& ev) {
+    const bool diff = DIFF;
+    float xh[9];
+#pragma unroll
+    for (int i = 0; i < 9; i++) xh[i] = (float)xt[i];
+    double G[9], F;
+    int64_t n;
+    soft_sites32<DIFF>(g32, pq32, nk, x, y, xt, step, eps, lane, 0, 1, hs, slots, G, F, n);
     // warp sums (fixed butterfly order)
     for (int off = 16; off > 0; off >>= 1) {
         F += __shfl_xor_sync(0xffffffffu, F, off);
@@ -598,7 +676,8 @@ __device__ __noinline__ int64_t soft_evaluate32(const float4* __restrict__ g32, 
     double fsum = diff ? F : F * 0.69314718055994530942 + corr;
     if (nm > 0) soft_multi_add(R, nm, xt, xc, diff, eps, lane, hs, Gc, fsum, n);
     const double dn = (double)n;
-    ev.f = diff ? f_old - fsum / dn : -fsum / dn;
+    ev.df = -fsum / dn;   // in a difference pass the objective's change
+    ev.f = diff ? f_old + ev.df : ev.df;
 #pragma unroll
     for (int i = 0; i < 9; i++) ev.g[i] = -Gc[i] / dn;
 #pragma unroll
@@ -607,14 +686,41 @@ __device__ __noinline__ int64_t soft_evaluate32(const float4* __restrict__ g32, 
     return n;
 }
 
+// The QP and the condition estimate of the warp's pair, by every lane alike
+// (kg_qp1.cuh) from its shared memory: in holds H's upper triangle and, for the
+// QP, c.  One thread's straight chain takes a fifth of the row-parallel form's
+// 145,000 cycles of shuffles and divisions.
+__device__ __noinline__ void soft_qp(const double* in, const Tune& tu, double* y) {
+    double v[9];
+#pragma unroll
+    for (int i = 0; i < 9; i++) v[i] = y[i];
+    qp_simplex_thread<true>([in](int k) { return in[k]; }, tu, v);
+#pragma unroll
+    for (int i = 0; i < 9; i++) y[i] = v[i];
+}
+__device__ __noinline__ double soft_condition(const double* in, const double* x, const double* g, double tol) {
+    double xv[9], gv[9];
+#pragma unroll
+    for (int i = 0; i < 9; i++) { xv[i] = x[i]; gv[i] = g[i]; }
+    return condition_thread([in](int k) { return in[k]; }, xv, gv, tol);
+}
+// Lane i < 9's row of H to the upper triangle in shared memory.
+__device__ __forceinline__ void soft_share_hessian(const double* Hr, int lane, double* in) {
+    __syncwarp();
+#pragma unroll
+    for (int j = 0; j < 9; j++)
+        if (lane < 9 && j >= lane) in[lane * 9 - lane * (lane - 1) / 2 + (j - lane)] = Hr[j];
+    __syncwarp();
+}
+
 // Warp per output row of the first ns samples (x-major, y >= x), taken from a
 // counter; the Jacquard SQP of src/sqp.rs:49-93 in FP64 on FP32 evaluations
 // (prec64 = 0) or FP64 ones.  stats: [0] grad-Hessian evaluations, [1] of them
 // in FP64, [2] pairs escalated to FP64, [3] pair-sites evaluated (summed over
 // evaluations), [4] of them in FP64.
-__global__ void __launch_bounds__(SOFT_WARPS * 32, 3) soft_pairs_kernel(
+__global__ void __launch_bounds__(SOFT_WARPS * 32, 2) soft_pairs_kernel(
     const double* __restrict__ gl, int64_t n_sites, const int32_t* __restrict__ kept, const double* __restrict__ kp,
-    const double* __restrict__ kq, const float4* __restrict__ g32, const float2* __restrict__ pq32, int prec64, int64_t nk, int64_t ns, int64_t n_rows, uint64_t iterations,
+    const double* __restrict__ kq, const float4* __restrict__ g32, const float4* __restrict__ pq32, int prec64, int64_t nk, int64_t ns, int64_t n_rows, uint64_t iterations,
     kg_output* out, unsigned long long* next, int* no_rows, unsigned long long* stats, SoftMultiDev M) {
     extern __shared__ __align__(16) unsigned char soft_smem[];   // SOFT_WARP_SMEM per warp
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
@@ -654,10 +760,12 @@ __global__ void __launch_bounds__(SOFT_WARPS * 32, 3) soft_pairs_kernel(
                 m = soft_evaluate(gl, n_sites, kept, kp, kq, nk, x, y, xt, tu.epsilon, lane, hs, R, M.total, ev);
                 c_sites64 += (unsigned long long)m;
             } else {
-                m = diff ? soft_evaluate32<true>(g32, pq32, nk, x, y, xt, xc, f_old, tu.epsilon, lane, hs, slots, R,
-                                                 M.total, ev)
-                         : soft_evaluate32<false>(g32, pq32, nk, x, y, xt, xc, f_old, tu.epsilon, lane, hs, slots, R,
-                                                  M.total, ev);
+                double step[9];
+                difference_step(xt, xc, step);
+                m = diff ? soft_evaluate32<true>(g32, pq32, nk, x, y, xt, step, xc, f_old, tu.epsilon, lane, hs, slots,
+                                                 R, M.total, ev)
+                         : soft_evaluate32<false>(g32, pq32, nk, x, y, xt, step, xc, f_old, tu.epsilon, lane, hs, slots,
+                                                  R, M.total, ev);
             }
             c_sites += (unsigned long long)m;
             return m;
@@ -687,7 +795,8 @@ __global__ void __launch_bounds__(SOFT_WARPS * 32, 3) soft_pairs_kernel(
             bool conv = kkt_ok(xv, g, tu.sqp_conv_tol, &resid);
             if (!fp64 && (conv || resid < 1e-6)) {
                 if (!conv) near_count++;
-                const double c32 = conv ? condition_rows(xv, g, Hr, tu.sqp_conv_tol) : 0.0;
+                soft_share_hessian(Hr, lane, hs);
+                const double c32 = conv ? soft_condition(hs, xv, g, tu.sqp_conv_tol) : 0.0;
                 if (conv ? !(c32 <= COND_RECHECK) : (near_count >= 3)) {
                     // FP64 re-evaluation at the same point; the pair stays FP64
                     fp64 = true;
@@ -705,14 +814,20 @@ __global__ void __launch_bounds__(SOFT_WARPS * 32, 3) soft_pairs_kernel(
             }
             if (conv) {
                 iters = it;
-                cond = condition_rows(xv, g, Hr, tu.sqp_conv_tol);
+                soft_share_hessian(Hr, lane, hs);
+                cond = soft_condition(hs, xv, g, tu.sqp_conv_tol);
                 break;
             }
             double cr = 0.0;
             if (lane < 9) cr = pick9(g, lane) - dot_fma(9, Hr, xv);
-            double c[9], yv[9], p[9];
-            gather9(cr, c);
-            qp_simplex_rows(WarpGrp{FULL_MASK}, Hr, c, xv, tu, lane, yv);
+            double yv[9], p[9];
+            soft_share_hessian(Hr, lane, hs);
+            if (lane < 9) hs[QP_Q + lane] = cr;
+            __syncwarp();
+#pragma unroll
+            for (int i = 0; i < 9; i++) yv[i] = xv[i];
+            soft_qp(hs, tu, yv);
+            __syncwarp();   // every lane has read hs before the next sums
 #pragma unroll
             for (int i = 0; i < 9; i++) p[i] = yv[i] - xv[i];
             const double gp = dot_fma(9, g, p);
@@ -722,8 +837,10 @@ __global__ void __launch_bounds__(SOFT_WARPS * 32, 3) soft_pairs_kernel(
 #pragma unroll
                 for (int i = 0; i < 9; i++) xn[i] = xv[i] + alpha * p[i];
                 normalise9(xn);
-                eval(xn, xv, fabs(alpha * gp) < DIFF_BELOW, f);
-                const bool accept = ev.f <= f + alpha * tt;
+                const bool change = fabs(alpha * gp) < DIFF_BELOW;
+                eval(xn, xv, change, f);
+                // the change itself resolves the test far below an ulp of f
+                const bool accept = change && !fp64 ? ev.df <= alpha * tt : ev.f <= f + alpha * tt;
                 bls++;
                 if (accept || bls == tu.bls_max_iter) break;
                 alpha *= tu.bls_step_size_reduce;
@@ -748,6 +865,282 @@ __global__ void __launch_bounds__(SOFT_WARPS * 32, 3) soft_pairs_kernel(
         atomicAdd(&stats[3], c_sites);
         atomicAdd(&stats[4], c_sites64);
     }
+}
+
+// ------------------------------------------------------------------- waves
+
+// what changes from call to call, in device memory (the launches are a graph)
+struct SoftCall {
+    const double* gl;
+    const int32_t* kept;
+    const double *kp, *kq;
+    const float4 *g32, *pq32;
+    int64_t n_sites, nk;
+};
+
+__global__ void soft_init_kernel(SlotArgs A, int n, unsigned long long max_waves) { init_slot(A, 1, n, max_waves); }
+
+// A pass's sums of a slot: sum L L' r^2 (45, upper triangle), sum L r (9), the
+// objective sum, the sites.
+constexpr int SOFT_PART = 56;
+
+// A block per slot of the pass list, its warps every fourth group of 32 sites
+// (or site pairs): a wave over few slots lasts a quarter of a warp's site loop.
+// The warps' sums are added in a fixed order; two blocks per SM (255 registers,
+// no spills: with three, 168 registers, 200 samples x 15,000 sites took 20.2
+// against 15.0 ms).
+__global__ void __launch_bounds__(SOFT_WARPS * 32, 2) soft_pass_kernel(SlotArgs A, const SoftCall* call,
+                                                                      double* partial) {
+    extern __shared__ __align__(16) unsigned char soft_smem[];   // SOFT_WARP_SMEM per warp
+    __shared__ double part_sum[SOFT_WARPS][11];
+    __shared__ double total[45];
+    if (A.clk->stop) return;   // a device loop past its last wave
+    if (threadIdx.x == 0) atomicMin(&A.clk->start[1], global_ns());
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const PhaseEnd pe{&A.clk->end[1], lane == 0};
+    double* hs = reinterpret_cast<double*>(soft_smem + w * SOFT_WARP_SMEM);
+    float4* slots = reinterpret_cast<float4*>(soft_smem + w * SOFT_WARP_SMEM + SOFT_SUMS_BYTES);
+    const SoftCall C = *call;
+    const int n_list = A.ctl->n[A.par];
+    const PairSeg sg = A.seg[0];
+    for (int i = blockIdx.x; i < n_list; i += gridDim.x) {
+        const int s = A.list_cur[i];
+        const int kind = A.count[s].w & 7;
+        int64_t x, y;
+        pair_of(sg.idx0 + (s - sg.slot0), x, y);
+        const double* st = A.state + slot_at(s, NS_VALS);
+        double xt[9], step[9], G[9], F;
+        int64_t n;
+#pragma unroll
+        for (int k = 0; k < 9; k++) {
+            xt[k] = st[(NS_XT + k) * NS_LANES];
+            step[k] = kind == NP_DIFF ? st[(NS_STEP + k) * NS_LANES] : 0.0;
+        }
+        if (kind >= NP_FP64)
+            soft_sites64(C.gl, C.n_sites, C.kept, C.kp, C.kq, C.nk, x, y, xt, A.tune.epsilon, lane, w, SOFT_WARPS, hs, G,
+                         F, n);
+        else if (kind == NP_DIFF)
+            soft_sites32<true>(C.g32, C.pq32, C.nk, x, y, xt, step, A.tune.epsilon, lane, w, SOFT_WARPS, hs, slots, G, F, n);
+        else
+            soft_sites32<false>(C.g32, C.pq32, C.nk, x, y, xt, step, A.tune.epsilon, lane, w, SOFT_WARPS, hs, slots, G, F,
+                                n);
+        // warp sums (fixed butterfly order), then the block's
+        for (int off = 16; off > 0; off >>= 1) {
+            F += __shfl_xor_sync(0xffffffffu, F, off);
+            n += __shfl_xor_sync(0xffffffffu, n, off);
+#pragma unroll
+            for (int k = 0; k < 9; k++) G[k] += __shfl_xor_sync(0xffffffffu, G[k], off);
+        }
+        if (lane < 9) part_sum[w][lane] = pick9(G, lane);
+        if (lane == 9) part_sum[w][9] = F;
+        if (lane == 10) part_sum[w][10] = (double)n;
+        __syncthreads();
+        double* P = partial + slot_at(s, SOFT_PART);
+        for (int a = w; a < 45; a += SOFT_WARPS) {
+            double h = 0.0;
+#pragma unroll
+            for (int v = 0; v < SOFT_WARPS; v++)
+                h += reinterpret_cast<const double*>(soft_smem + v * SOFT_WARP_SMEM)[a * HS + lane];
+            for (int off = 16; off > 0; off >>= 1) h += __shfl_xor_sync(0xffffffffu, h, off);
+            if (lane == 0) {
+                total[a] = h;
+                P[a * NS_LANES] = h;
+            }
+        }
+        __syncthreads();
+        if (w == 0 && lane < 11) {
+            double v = 0.0;
+#pragma unroll
+            for (int u = 0; u < SOFT_WARPS; u++) v += part_sum[u][lane];
+            if (kind < NP_FP64) {
+                // the lo parts of x to first order: sum log d gains sum_j lo_j
+                // G_j, and G_i loses sum_j H_ij lo_j (a difference pass's
+                // objective uses the step's FP32 values)
+                double corr = 0.0;
+#pragma unroll
+                for (int j = 0; j < 9; j++) {
+                    const double lo = xt[j] - (double)(float)xt[j], gj = __shfl_sync(0x7FFu, v, j);
+                    const int r = min(lane, 8);
+                    corr = fma(lane < 9 ? total[r <= j ? upper_at(r, j) : upper_at(j, r)] : gj, lo, corr);
+                }
+                if (lane < 9) v -= corr;
+                else if (lane == 9 && kind != NP_DIFF) v = v * 0.69314718055994530942 + corr;
+            }
+            P[(45 + lane) * NS_LANES] = v;
+        }
+        __syncthreads();   // the sums are read before the next slot's
+    }
+}
+
+struct SoftSums {
+    static constexpr bool FP32 = true, COEF = false;
+    const double* partial;
+    static __device__ double none() { return 0.0; }
+    __device__ __forceinline__ void load(int s, int, double*, double& obj, double (&g)[9], double (&T)[QP_Q],
+                                         double& nsites) const {
+        const double* P = partial + slot_at(s, SOFT_PART);
+#pragma unroll
+        for (int k = 0; k < QP_Q; k++) T[k] = P[k * NS_LANES];
+#pragma unroll
+        for (int k = 0; k < 9; k++) g[k] = P[(45 + k) * NS_LANES];
+        obj = P[54 * NS_LANES];
+        nsites = P[55 * NS_LANES];
+    }
+    // (soft_relatedness reads them back: FP64 passes and their sites)
+    __device__ __forceinline__ void count(int, int, int, int f64p, double nsites, bool, unsigned long long* sum) const {
+        atomicAdd(&sum[7], (unsigned long long)f64p);
+        atomicAdd(&sum[6], (unsigned long long)nsites * (unsigned long long)f64p);
+    }
+};
+
+__global__ void __launch_bounds__(NA_THREADS) soft_advance_kernel(SlotArgs A, const double* partial, int in_loop,
+                                                                  cudaGraphConditionalHandle loop) {
+    advance_wave(A, SoftSums{partial}, in_loop, loop);
+}
+
+// The waves' graph and buffers, kept between calls.
+struct SoftWaves {
+    cudaGraph_t g = nullptr;
+    cudaGraphExec_t x = nullptr;
+    DevBuf slots, words;
+    PinBuf host;
+    int64_t cap = 0;
+    uint64_t iterations = 0;
+    int dev = -1;
+    cudaStream_t st = nullptr;
+    SlotArgs args[2]{};
+    double* partial = nullptr;
+    int pass_blocks = 0, advance_blocks = 0;
+    void drop() {
+        if (x) cudaGraphExecDestroy(x);
+        if (g) cudaGraphDestroy(g);
+        x = nullptr;
+        g = nullptr;
+        cap = 0;
+    }
+    ~SoftWaves() { drop(); }
+};
+
+// What a call's waves read and write beside the slots, one buffer on the device
+// and its copy on the host.
+struct SoftWords {
+    CohortDev co;
+    PairSeg seg;
+    SoftCall call;
+    SlotCtl ctl;
+    WaveClock clk;
+    RunCounters run;
+};
+
+static void launch_soft_wave(const SoftWaves& E, const SoftWords* D, int par, int in_loop, cudaGraphConditionalHandle h,
+                             cudaStream_t st) {
+    soft_pass_kernel<<<E.pass_blocks, SOFT_WARPS * 32, SOFT_SMEM, st>>>(E.args[par], &D->call, E.partial);
+    soft_advance_kernel<<<E.advance_blocks, NA_THREADS, 0, st>>>(E.args[par], E.partial, in_loop, h);
+}
+
+static int run_soft_waves(SoftWork& w, const SoftCall& call, int64_t ns, uint64_t iterations, kg_output* d_out,
+                          cudaStream_t st, std::string& err, uint64_t* counters) {
+    if (!w.waves) w.waves = std::make_shared<SoftWaves>();
+    SoftWaves& E = *w.waves;
+    int dev = 0, sms = 148;
+    KG_SOFT_TRY(cudaGetDevice(&dev));
+    KG_SOFT_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+    const int64_t total = ns * (ns + 1) / 2;
+    const size_t per_slot = sizeof(double) * (NS_VALS + SOFT_PART) + sizeof(int4) + 2 * sizeof(int);
+    const int64_t cap = (std::min<int64_t>(total, (int64_t)1 << 20) + 31) / 32 * 32;
+    if (E.cap < cap || E.iterations != iterations || E.dev != dev || E.st != st) {
+        const int64_t keep = E.dev == dev ? std::max<int64_t>(E.cap, cap) : cap;
+        E.drop();
+        KG_SOFT_TRY((cudaError_t)E.slots.reserve(per_slot * (size_t)keep));
+        KG_SOFT_TRY((cudaError_t)E.words.reserve(sizeof(SoftWords)));
+        KG_SOFT_TRY((cudaError_t)E.host.reserve(sizeof(SoftWords)));
+        SoftWords* D = E.words.as<SoftWords>();
+        SlotArgs A{};
+        A.cohorts = &D->co;
+        A.seg = &D->seg;
+        A.state = E.slots.as<double>();
+        E.partial = A.state + (size_t)NS_VALS * keep;
+        A.count = reinterpret_cast<int4*>(E.partial + (size_t)SOFT_PART * keep);
+        int* lists = reinterpret_cast<int*>(A.count + keep);
+        A.ctl = &D->ctl;
+        A.clk = &D->clk;
+        A.counters = &D->run;
+        A.tune = make_tune(iterations);
+        for (int par = 0; par < 2; par++) {
+            E.args[par] = A;
+            E.args[par].par = par;
+            E.args[par].list_cur = lists + (par ? keep : 0);
+            E.args[par].list_next = lists + (par ? 0 : keep);
+        }
+        int occ = 0;
+        KG_SOFT_TRY(cudaFuncSetAttribute(soft_pass_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SOFT_SMEM));
+        KG_SOFT_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, soft_pass_kernel, SOFT_WARPS * 32, SOFT_SMEM));
+        E.pass_blocks = sms * std::max(1, occ);
+        KG_SOFT_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, soft_advance_kernel, NA_THREADS, 0));
+        E.advance_blocks = sms * std::max(1, occ);
+        KG_SOFT_TRY(wave_loop_graph(
+            st,
+            [&](int par, int in_loop, cudaGraphConditionalHandle h) {
+                launch_soft_wave(E, D, par, in_loop, h, st);
+            },
+            &E.g, &E.x));
+        E.cap = keep;
+        E.iterations = iterations;
+        E.dev = dev;
+        E.st = st;
+    }
+    SoftWords* D = E.words.as<SoftWords>();
+    SoftWords* H = E.host.as<SoftWords>();
+    *H = SoftWords{};
+    H->co.kind = COHORT_TRIANGLE;
+    H->co.n_x = ns;
+    H->co.n_pairs = total;
+    H->co.out = d_out;
+    H->co.max_iter = iterations;
+    H->call = call;
+    const char* hw = std::getenv("KESTREL_HOST_WAVES");
+    const bool host_waves = hw && hw[0] == '1';   // for kernel profilers, as in run_nodes
+    uint64_t launches = 0;
+    const unsigned long long bound = 4ull * (iterations + 2) * 16ull + 64ull;   // FP32, then once more in FP64
+    for (int64_t at = 0; at < total; at += E.cap) {
+        const int n = (int)std::min<int64_t>(E.cap, total - at);
+        H->seg = PairSeg{at, 0, n, 0, 0};
+        // the counters go on from chunk to chunk
+        KG_SOFT_TRY(cudaMemcpyAsync(D, H, sizeof(SoftWords), cudaMemcpyHostToDevice, st));
+        soft_init_kernel<<<(n + 127) / 128, 128, 0, st>>>(E.args[0], n, bound);
+        KG_SOFT_TRY(cudaGetLastError());
+        if (host_waves) {
+            for (int par = 0;; par ^= 1) {
+                launch_soft_wave(E, D, par, 0, cudaGraphConditionalHandle{}, st);
+                launches += 2;
+                KG_SOFT_TRY(cudaMemcpyAsync(H, D, sizeof(SoftWords), cudaMemcpyDeviceToHost, st));
+                KG_SOFT_TRY(cudaStreamSynchronize(st));
+                if (H->clk.stop) break;
+            }
+        } else {
+            KG_SOFT_TRY(cudaGraphLaunch(E.x, st));
+        }
+        KG_SOFT_TRY(cudaMemcpyAsync(H, D, sizeof(SoftWords), cudaMemcpyDeviceToHost, st));
+        KG_SOFT_TRY(cudaStreamSynchronize(st));
+        if (H->clk.limit_hit) {
+            err = "the wave loop reached its wave limit";
+            return KG_ETIMEOUT;
+        }
+        launches += 1 + (host_waves ? 0 : 4 * H->clk.iters);
+    }
+    if (counters) {
+        counters[0] = H->run.gh_passes;
+        counters[1] = H->run.shape_sites[0];   // SoftSums::count
+        counters[2] = H->run.fp64_pairs;
+        counters[3] = H->run.work_units;
+        counters[4] = H->run.flops_fp64;
+        counters[5] = launches;
+    }
+    if (H->run.nosite_pairs) {
+        err = "a pair shares no called segregating site";
+        return KG_ENOSITES;
+    }
+    return KG_OK;
 }
 
 int soft_relatedness(SoftWork& w, const DevBuf& gl, int64_t n_samples, int64_t n_sites, int64_t ns,
@@ -826,15 +1219,21 @@ int soft_relatedness(SoftWork& w, const DevBuf& gl, int64_t n_samples, int64_t n
     int* no_rows = reinterpret_cast<int*>(next + 6);
     const bool fp64 = precision == KG_PREC_FP64;
     if (!fp64) {
-        KG_SOFT_TRY((cudaError_t)g32.reserve(sizeof(float4) * (size_t)(n_samples * nk1)));
-        KG_SOFT_TRY((cudaError_t)pq32.reserve(sizeof(float2) * nk1));
-        const int64_t total = n_samples * nk;
+        const int64_t pairs = (nk1 + 1) / 2;   // of sites
+        KG_SOFT_TRY((cudaError_t)g32.reserve(sizeof(float4) * 2 * (size_t)(n_samples * pairs)));
+        KG_SOFT_TRY((cudaError_t)pq32.reserve(sizeof(float4) * pairs));
+        const int64_t total = n_samples * ((nk + 1) / 2);
         if (total > 0) {
             const unsigned blocks = (unsigned)std::min<int64_t>((total + 255) / 256, 148 * 16);
             soft_pack32_kernel<<<blocks, 256, 0, st>>>(gl.as<double>(), n_samples, n_sites, idx.as<int32_t>(),
                                                        kp.as<double>(), kq.as<double>(), nk, g32.as<float4>(),
-                                                       pq32.as<float2>());
+                                                       pq32.as<float4>());
         }
+    }
+    if (!fp64 && M.total == 0) {
+        const SoftCall call{gl.as<double>(),    idx.as<int32_t>(),  kp.as<double>(), kq.as<double>(),
+                            g32.as<float4>(),   pq32.as<float4>(), n_sites,         nk};
+        return run_soft_waves(w, call, ns, iterations, d_out, st, err, counters);
     }
     const int64_t rows = ns * (ns + 1) / 2;
     int dev = 0, sms = 148;
@@ -850,7 +1249,7 @@ int soft_relatedness(SoftWork& w, const DevBuf& gl, int64_t n_samples, int64_t n
     }
     soft_pairs_kernel<<<(unsigned)grid, SOFT_WARPS * 32, SOFT_SMEM, st>>>(
         gl.as<double>(), n_sites, idx.as<int32_t>(), kp.as<double>(), kq.as<double>(), g32.as<float4>(),
-        pq32.as<float2>(), fp64 ? 1 : 0, nk, ns, rows, iterations, d_out, next, no_rows, stats, M);
+        pq32.as<float4>(), fp64 ? 1 : 0, nk, ns, rows, iterations, d_out, next, no_rows, stats, M);
     KG_SOFT_TRY(cudaGetLastError());
     int h_no_rows = 0;
     unsigned long long hs[5] = {0, 0, 0, 0, 0};
