@@ -444,7 +444,8 @@ def run_gl_soft(args, local):
     peak = ctypes_peak(local)
     achieved = st["flops_fp32"] / (t * 1e-3) / 1e12
     roof = {"bound": "fp32", "achieved": achieved, "peak": peak, "unit": "TFLOP/s",
-            "frac": achieved / peak if peak else None, "traffic": None, "kernel": "soft_pairs_kernel",
+            "frac": achieved / peak if peak else None, "traffic": None,
+            "kernel": "soft_pass_kernel" if args.precision == "fp32c" else "soft_pairs_kernel",
             "peak_source": "kg_fp32_peak (FFMA loop over all SMs, measured in this run)",
             "flops_counted": "FP32 evaluations at 204 FLOP per pair-site (the row from the nine likelihood "
                              "products, d, gradient, 45 Hessian terms, objective; FMA = 2) over the device time "
@@ -580,18 +581,21 @@ def run_gt_cls(args, local):
         est.relatedness_gt(out=out_pin)
         e2e_ms.append((time.perf_counter() - t0) * 1e3)
     te = float(np.mean(e2e_ms))
-    # the list-building (admit) kernel dominates: HBM-bound, 4 bytes written per
-    # listed pair-site; the moment pass reads them once
     pair_sites = float(st["pair_sites"])
     admit_ms, pass_ms = st["admit_ms"], st["pass_ms"]
-    top = "wave_admit_kernel" if admit_ms >= pass_ms else "wave_pass_kernel"
-    top_ms = max(admit_ms, pass_ms)
-    achieved = 4.0 * pair_sites / (top_ms * 1e-3) / 1e9
-    peak = measured_hbm_peak()
-    roof = {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
-            "frac": achieved / peak if peak else None, "traffic": None, "kernel": top,
-            "algorithmic_bytes": 4.0 * pair_sites / max(1, int(st["waves"])),
-            "note": "4 bytes per listed pair-site (written by the admit kernel, read once by the moment pass)"}
+    if args.precision == "fp32c" and mg is None:
+        roof = node_weights_roof(admit_ms, pair_sites)
+    else:
+        # on site lists: HBM-bound, 4 bytes written per listed pair-site by the
+        # admit kernel, which the moment pass reads once
+        top_ms = max(admit_ms, pass_ms)
+        achieved = 4.0 * pair_sites / (top_ms * 1e-3) / 1e9
+        peak = measured_hbm_peak()
+        roof = {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
+                "frac": achieved / peak if peak else None, "traffic": None,
+                "kernel": "wave_admit_kernel" if admit_ms >= pass_ms else "wave_pass_kernel",
+                "algorithmic_bytes": 4.0 * pair_sites / max(1, int(st["waves"])),
+                "note": "4 bytes per listed pair-site (written by the admit kernel, read once by the moment pass)"}
     cpu = None
     if not args.no_cpu:
         sub = min(n_s, 192)
@@ -665,7 +669,7 @@ def main():
     clocks = ClockSampler(local)
     barrier()
     clocks.start()
-    dev_ms, kern_ms, fl32, phases, stats = [], [], [], [], None
+    dev_ms, kern_ms, phases, stats = [], [], [], None
     for _ in range(args.steps):
         flush.zero_()          # evict L2 between steps
         torch.cuda.synchronize()
@@ -673,7 +677,6 @@ def main():
         stats = est.run_stats()
         dev_ms.append(stats["device_ms"])
         kern_ms.append(stats["pass_ms"])
-        fl32.append(stats["flops_fp32"])
         phases.append([stats["admit_ms"], stats["pass_ms"], stats["solve_ms"], stats["pair_kernel_ms"]])
     barrier()
     clk = clocks.stop()
@@ -710,37 +713,32 @@ def main():
                "ms_per_step": tm, "timing": "host wall clock around the synchronous C-ABI calls per step "
                                             "(packed genotypes up from pinned memory, estimate, all rows to "
                                             "pinned memory)"}
-    # ---- roofline of the site-pass kernel (FP32 CUDA-core bound; FP64 for the FP64 form)
+    # ---- roofline of the kernel that takes the most time: the node passes (FP64
+    # CUDA cores); the FP64 form's passes over site lists
     peak32 = ctypes_peak(local)
+    peak = peak32 / 2.0 if peak32 else None
     kms = float(np.mean(kern_ms))
     launches = max(1, int(stats["waves"]))           # one pass launch per wave
-    pass_sites = float(stats["work_units"])          # pair-site evaluations of the step
     fp64_form = args.precision == "fp64"
-    flops = float(stats["flops_fp64"]) if fp64_form else float(np.mean(fl32))
-    peak = (peak32 / 2.0 if peak32 else None) if fp64_form else peak32
+    flops = float(stats["flops_fp64"])
     achieved = flops / (kms * 1e-3) / 1e12
-    ref_equiv = pass_sites * 156.0 / (kms * 1e-3) / 1e12
-    list_bytes = 8.0 if fp64_form else 4.0
-    roof = {"bound": "fp64" if fp64_form else "fp32", "achieved": achieved, "peak": peak,
-            "unit": "TFLOP/s", "frac": achieved / peak if peak else None,
-            # DRAM bytes per pair-site-pass from one ncu capture (a 96-sample
-            # cohort), times the pair-sites of an average pass launch of this step
-            "traffic": (PASS_DRAM_BYTES_PER_SITE * pass_sites / launches) if not fp64_form else None,
-            "traffic_unit": "bytes per launch",
-            "algorithmic_bytes": list_bytes * pass_sites / launches,
-            "hbm_achieved_gbs": list_bytes * pass_sites / (kms * 1e-3) / 1e9,
+    # bytes of a pass: the FP64 form's 8 bytes a listed site; on nodes the nine
+    # weights of every node and two words of their sum
+    nbytes = 8.0 * float(stats["work_units"]) if fp64_form else flops / NODE_FLOPS * 72.0
+    roof = {"bound": "fp64", "achieved": achieved, "peak": peak, "unit": "TFLOP/s",
+            "frac": achieved / peak if peak else None, "traffic": None,
+            "algorithmic_bytes": nbytes / launches,
+            "hbm_achieved_gbs": nbytes / (kms * 1e-3) / 1e9,
             "hbm_peak_gbs": measured_hbm_peak(),
-            "kernel": "wave_pass_kernel", "kernel_ms": kms, "launches": launches,
+            "kernel": "wave_pass_kernel" if fp64_form else "node_pass_kernel", "kernel_ms": kms, "launches": launches,
             "kernel_timing": "device clock (%globaltimer) from the first block's start to the last warp's end "
-                             "of every wave's site-pass launch, summed per step",
-            "peak_source": ("half of kg_fp32_peak (B200 FP64 CUDA-core rate)" if fp64_form else
-                            "kg_fp32_peak (FFMA loop over all SMs, measured in this run)"),
-            "flops_counted": ("executed site arithmetic of the shape-moment passes (FMA = 2, MUFU = 1) "
-                              "per shape and pass kind; FP64 re-evaluation passes excluded" if not fp64_form
-                              else "executed FP64 site arithmetic of the shape-moment passes (FMA = 2)"),
-            "ref_formulation_tflops": ref_equiv,
-            "ref_formulation_note": "the same pair-site-passes counted at the reference formulation's "
-                                    "136 + 20 FLOP (dense 9 + 45 sums); the shape moments need 19-41"}
+                             "of every wave's pass launch, summed per step",
+            "peak_source": "half of kg_fp32_peak (FFMA loop over all SMs, measured in this run): the FP64 "
+                           "CUDA-core rate",
+            "flops_counted": "executed FP64 arithmetic of the passes (FMA = 2): "
+                             + ("per listed site" if fp64_form else f"{NODE_FLOPS} per frequency node and pass")}
+    if not fp64_form:
+        roof["node_weights"] = node_weights_roof(float(np.mean([p[0] for p in phases])), float(stats["pair_sites"]))
     line = {"metric": METRIC, "value": value, "unit": "pairs/s", "n_gpus": world,
             "steps": args.steps, "warmup": args.warmup, "ms_per_step": t_mean,
             "higher_is_better": True, "scaling": "weak", "vs_baseline": None,
@@ -790,10 +788,28 @@ def measure_fp64_form(est, fp32c_value, steps=2):
             "timing": "device time (CUDA events in the library) of kg_relatedness with KG_PREC_FP64"}
 
 
-# DRAM bytes (read + write) per pair-site-pass of wave_pass_kernel: the ncu
-# capture of one launch on a 96-sample x 100,000-site cohort read and wrote
-# 1.912 GB over 447,339,158 pair-site-passes.
-PASS_DRAM_BYTES_PER_SITE = 4.27
+# FP64 operations of a pass at one frequency node: the nine genotype pairs'
+# site arithmetic (two orientations of four shapes and the double heterozygote).
+NODE_FLOPS = 2 * (50 + 39 + 39 + 55) + 27
+
+
+def node_weights_roof(ms, pair_sites):
+    """The weights kernel on the int8 tensor cores: per pair and site nine
+    genotype pairs by 32 digit columns (eight nodes' four signed digits), two
+    operations each, against twice the measured bf16 rate."""
+    ops = 2.0 * 9 * 32 * pair_sites
+    peak = None
+    try:
+        with open(os.path.join(ROOT, "MEASURED_PEAKS.json")) as f:
+            peak = 2.0 * float(json.load(f)["bf16_tflops"])
+    except (OSError, KeyError, ValueError):
+        pass
+    achieved = ops / (ms * 1e-3) / 1e12
+    return {"bound": "int8 tensor", "achieved": achieved, "peak": peak, "unit": "TOP/s",
+            "frac": achieved / peak if peak else None, "traffic": None, "kernel": "node_weights_kernel",
+            "kernel_ms": ms, "peak_source": "twice the measured cuBLAS bf16 rate",
+            "note": "jointly observed pair-sites only; the tiles also cover both triangles' diagonal blocks, the "
+                    "bins' padding and missing sites"}
 
 
 def ctypes_peak(device):
