@@ -27,21 +27,25 @@
 namespace kg {
 
 // Nodes per bin, signed 8-bit digits of l's fixed-point value (2^-30), and the
-// largest ratio of a bin's ends.  The interpolation error of the gradient
-// terms is then below 1.3e-9 of a term anywhere on the simplex (1e-11 over a
-// pair's sum), under the 6e-8 of a FP32 site term.  The FP64 form keeps its site
+// largest ratio of a bin's ends.  The interpolation error is then below 2e-10
+// of a site's log d and 1.1e-10 of its gradient term x_i L_i / d anywhere on the
+// simplex, and its mean over a bin's sites below 5e-13, against the 6e-8 of a FP32
+// site term.  (With 2^(1/4) it is ten times lower, and no row of 1,024 samples x
+// 100,000 sites is nearer to the FP64 form's, 9.6e-9 at most on both: where the two stop
+// decides; but a third more nodes: 18.8 against 15.0 ms of passes, 13.3 against
+// 13.0 ms of weights.)  The FP64 form keeps its site
 // lists: with 12 nodes and 5 digits it ran 2.4 times as fast and 1e-13
 // accurate, but within 1e-9 of the list form's rows only where no pair's last
 // line search hangs on an ulp of the objective.
 constexpr int NODE_J = 8, NODE_L = 4;
-constexpr double NODE_RATIO = 1.189207115002721;   // 2^(1/4)
+constexpr double NODE_RATIO = 1.2599210498948732;   // 2^(1/3)
 constexpr int NODE_MAX_BINS = 64;
 constexpr int NODE_UNITS = 9;        // genotype pairs (gx, gy)
 constexpr int NODE_STAGE = 128;      // sites per tile of the product; a bin's sites are padded to it
 
 // Whether a prepared cohort's pairs run on nodes, given its kept sites and
 // their smallest min(p, 1 - p), and the bins that takes (0: it does not: a
-// frequency outside 0..1, or below 1/2 x 2^(-64/4) = 7.6e-6, the end of 64 bins).
+// frequency outside 0..1, or below 1/2 x 2^(-64/3) = 1.9e-7, the end of 64 bins).
 // Nodes win at any size: whole calls of 2 samples x 300 sites took 0.50 ms
 // against 1.35 ms on lists, 64 x 1,200 0.95 against 1.93, 600 x 300 9.0 against
 // 30.4, 600 x 10,000 11.3 against 43.2 ms.

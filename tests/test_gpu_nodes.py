@@ -3,7 +3,7 @@ the tiles can go wrong: one sample, sample counts around the 128-row tile, site
 counts around the padded bins, a narrow and a wide range of frequencies, a
 chunk boundary inside a row, a pair without a common site.
 
-The objective's bar: the interpolation error of log d is below 2e-11 of a
+The objective's bar: the interpolation error of log d is below 2e-10 of a
 site's term (FP32C's eight nodes a bin) and the fixed-point weights add less than
 2^-30, averaged over the pair's sites, on an objective of order 1, and the two
 sides stop within a KKT residual of 1e-8 of the same optimum, where the
