@@ -64,6 +64,9 @@ struct kg_ctx {
     int64_t soft_n3 = 0, soft_n4 = 0;
     kg::Workspace ws;
     kg::DevBuf dout;
+    // kg_relatedness_batch: its cohorts' device buffers, kept between calls up to
+    // kBatchKeep of them and kBatchKeepBytes in all
+    std::vector<std::unique_ptr<kg::Cohort>> batch;
     kg_run_stats last{};
     // serving
     std::mutex mu;
@@ -105,6 +108,10 @@ int use_device(kg_ctx* c) {
     return KG_OK;
 }
 
+// What kg_relatedness_batch keeps: allocating and freeing some 20 buffers a
+// cohort took 9 of a four-cohort call's 20.7 ms.
+constexpr size_t kBatchKeep = 16, kBatchKeepBytes = (size_t)256 << 20;
+
 bool budget_ok(kg_ctx* c, size_t extra) {
     size_t fr = 0, tot = 0;
     if (cudaMemGetInfo(&fr, &tot) != cudaSuccess) return false;
@@ -114,6 +121,14 @@ bool budget_ok(kg_ctx* c, size_t extra) {
         if (used + extra > c->budget) return false;
     }
     return true;
+}
+
+// budget_ok for the calls of the context's own thread, which may give back the
+// buffers kept for batches.
+bool fits(kg_ctx* c, size_t extra) {
+    if (budget_ok(c, extra)) return true;
+    c->batch.clear();
+    return budget_ok(c, extra);
 }
 
 template <class F>
@@ -537,7 +552,7 @@ int kg_load_genotypes(kg_ctx* c, const uint8_t* codes, int64_t n_samples, int64_
     return guarded(c, [&]() -> int {
         int st = use_device(c);
         if (st) return st;
-        if (!budget_ok(c, (size_t)(n_samples * n_sites))) return set_err(c, KG_ENOMEM, "genotypes exceed the memory budget");
+        if (!fits(c, (size_t)(n_samples * n_sites))) return set_err(c, KG_ENOMEM, "genotypes exceed the memory budget");
         if (c->cohort.raw.reserve((size_t)(n_samples * n_sites)) != cudaSuccess)
             return set_err(c, KG_ENOMEM, "cannot allocate device genotypes");
         cudaError_t e = cudaMemcpy2DAsync(c->cohort.raw.p, (size_t)n_sites, codes, (size_t)row_stride,
@@ -590,7 +605,7 @@ int kg_load_multiallelic(kg_ctx* c, const uint8_t* gidx, int64_t n_samples, int6
         int st = use_device(c);
         if (st) return st;
         kg::Cohort& co = c->cohort;
-        if (!budget_ok(c, (size_t)(n_samples * n_sites)))
+        if (!fits(c, (size_t)(n_samples * n_sites)))
             return set_err(c, KG_ENOMEM, "multi-allelic genotypes exceed the memory budget");
         if (co.mg.reserve((size_t)(n_samples * n_sites)) != cudaSuccess || co.malleles.reserve((size_t)n_sites) != cudaSuccess ||
             (af && co.maf.reserve(sizeof(double) * 4 * n_sites) != cudaSuccess))
@@ -768,7 +783,7 @@ int kg_load_likelihoods(kg_ctx* c, const double* gl, int64_t n_samples, int64_t 
         int st = use_device(c);
         if (st) return st;
         const size_t bytes = sizeof(double) * 3 * (size_t)n_samples * (size_t)n_sites;
-        if (!budget_ok(c, bytes)) return set_err(c, KG_ENOMEM, "likelihoods exceed the memory budget");
+        if (!fits(c, bytes)) return set_err(c, KG_ENOMEM, "likelihoods exceed the memory budget");
         if (c->soft_gl.reserve(bytes) != cudaSuccess) return set_err(c, KG_ENOMEM, "cannot allocate device likelihoods");
         cudaError_t e = cudaMemcpyAsync(c->soft_gl.p, gl, bytes, cudaMemcpyHostToDevice, c->stream);
         if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
@@ -800,7 +815,7 @@ int kg_load_likelihoods_multiallelic(kg_ctx* c, const double* gl, int64_t n_samp
         if (st) return st;
         const int ng = n_alleles * (n_alleles + 1) / 2;
         const size_t bytes = sizeof(double) * ng * (size_t)n_samples * (size_t)n_sites;
-        if (!budget_ok(c, bytes)) return set_err(c, KG_ENOMEM, "likelihoods exceed the memory budget");
+        if (!fits(c, bytes)) return set_err(c, KG_ENOMEM, "likelihoods exceed the memory budget");
         if (buf.reserve(bytes) != cudaSuccess) return set_err(c, KG_ENOMEM, "cannot allocate device likelihoods");
         cudaError_t e = cudaMemcpyAsync(buf.p, gl, bytes, cudaMemcpyHostToDevice, c->stream);
         if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
@@ -903,6 +918,7 @@ int kg_relatedness_batch(kg_ctx* c, kg_cohort* cohorts, int n_cohorts, uint64_t 
         std::vector<int64_t> offs(n_cohorts, 0);
         int64_t total = 0;
         std::string err;
+        kg::DevBuf raw;
         for (int i = 0; i < n_cohorts; i++) {
             kg_cohort& k = cohorts[i];
             k.n_out = 0;
@@ -911,7 +927,14 @@ int kg_relatedness_batch(kg_ctx* c, kg_cohort* cohorts, int n_cohorts, uint64_t 
                 k.status = KG_EINVAL;
                 continue;
             }
-            auto co = std::make_unique<kg::Cohort>();
+            std::unique_ptr<kg::Cohort> co;
+            if (c->batch.empty()) {
+                co = std::make_unique<kg::Cohort>();
+            } else {
+                co = std::move(c->batch.front());   // in order: a repeated call finds its sizes
+                c->batch.erase(c->batch.begin());
+            }
+            if (raw.bytes > co->raw.bytes) std::swap(raw, co->raw);
             std::string e1;
             int s1 = kg::prepare_cohort(*co, k.codes, k.n_samples, k.n_sites, k.row_stride, false,
                                         k.allele_frequencies, std::isnan(maf) ? -1.0 : maf, c->stream, e1, false,
@@ -923,7 +946,10 @@ int kg_relatedness_batch(kg_ctx* c, kg_cohort* cohorts, int n_cohorts, uint64_t 
             }
             if (cudaError_t e = cudaStreamSynchronize(c->stream); e != cudaSuccess)
                 return set_err(c, KG_ECUDA, std::string("prepare: ") + cudaGetErrorString(e));
-            co->raw.release();  // packed planes are all the pair kernel needs
+            // packed planes are all the pair kernels need: the next cohort's codes
+            // go to the same buffer
+            std::swap(raw, co->raw);
+            co->raw.release();
             kg::PairJob jb;
             jb.panel = co.get();
             jb.kind = 0;
@@ -946,13 +972,31 @@ int kg_relatedness_batch(kg_ctx* c, kg_cohort* cohorts, int n_cohorts, uint64_t 
             int64_t np = jobs[job_of[i]].n_pairs();
             cudaError_t e = cudaMemcpyAsync(cohorts[i].out, c->dout.as<kg_output>() + offs[i],
                                             sizeof(kg_output) * np, cudaMemcpyDeviceToHost, c->stream);
-            if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
-            if (e != cudaSuccess) return set_err(c, KG_ECUDA, std::string("copy rows: ") + cudaGetErrorString(e));
+            if (e != cudaSuccess) {
+                cudaStreamSynchronize(c->stream);   // no copy into the caller's rows outlives the call
+                return set_err(c, KG_ECUDA, std::string("copy rows: ") + cudaGetErrorString(e));
+            }
             cohorts[i].n_out = np;
+        }
+        if (cudaError_t e = cudaStreamSynchronize(c->stream); e != cudaSuccess)
+            return set_err(c, KG_ECUDA, std::string("copy rows: ") + cudaGetErrorString(e));
+        for (int i = 0; i < n_cohorts; i++) {
+            if (job_of[i] < 0) continue;
+            const int64_t np = cohorts[i].n_out;
             if (st == KG_ENOSITES) {
                 for (int64_t r = 0; r < np; r++)
                     if (std::isnan(cohorts[i].out[r].obj)) { cohorts[i].status = KG_ENOSITES; break; }
             }
+        }
+        // nothing is in flight: keep the buffers for the next call, as far as they fit
+        if (!prep.empty()) std::swap(prep.back()->raw, raw);
+        size_t kept = 0;
+        for (const auto& b : c->batch) kept += b->device_bytes();
+        for (auto& b : prep) {
+            const size_t n = b->device_bytes();
+            if (c->batch.size() >= kBatchKeep || kept + n > kBatchKeepBytes) continue;
+            kept += n;
+            c->batch.push_back(std::move(b));
         }
         stats.total_ms = std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - t0).count();
         c->last = stats;
