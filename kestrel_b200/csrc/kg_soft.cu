@@ -998,6 +998,10 @@ __global__ void __launch_bounds__(NA_THREADS) soft_advance_kernel(SlotArgs A, co
     advance_wave(A, SoftSums{partial}, in_loop, loop);
 }
 
+// Pairs in flight at most (0.26 GB of slots): far more than the SMs hold, and a
+// chunk's tail of waves over few pairs is short beside its first ones.
+constexpr int64_t SOFT_SLOTS = (int64_t)1 << 18;
+
 // The waves' graph and buffers, kept between calls.
 struct SoftWaves {
     cudaGraph_t g = nullptr;
@@ -1047,11 +1051,17 @@ static int run_soft_waves(SoftWork& w, const SoftCall& call, int64_t ns, uint64_
     KG_SOFT_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
     const int64_t total = ns * (ns + 1) / 2;
     const size_t per_slot = sizeof(double) * (NS_VALS + SOFT_PART) + sizeof(int4) + 2 * sizeof(int);
-    const int64_t cap = (std::min<int64_t>(total, (int64_t)1 << 20) + 31) / 32 * 32;
+    const int64_t cap = (std::min<int64_t>(total, SOFT_SLOTS) + 31) / 32 * 32;
     if (E.cap < cap || E.iterations != iterations || E.dev != dev || E.st != st) {
-        const int64_t keep = E.dev == dev ? std::max<int64_t>(E.cap, cap) : cap;
+        int64_t keep = E.dev == dev ? std::max<int64_t>(E.cap, cap) : cap;
         E.drop();
-        KG_SOFT_TRY((cudaError_t)E.slots.reserve(per_slot * (size_t)keep));
+        // fewer pairs in flight where the memory is short
+        cudaError_t e;
+        while ((e = (cudaError_t)E.slots.reserve(per_slot * (size_t)keep)) == cudaErrorMemoryAllocation && keep > 4096) {
+            cudaGetLastError();
+            keep = keep / 64 * 32;
+        }
+        KG_SOFT_TRY(e);
         KG_SOFT_TRY((cudaError_t)E.words.reserve(sizeof(SoftWords)));
         KG_SOFT_TRY((cudaError_t)E.host.reserve(sizeof(SoftWords)));
         SoftWords* D = E.words.as<SoftWords>();

@@ -39,6 +39,19 @@ def test_sizes(oracle, n, m):
         print(compare(rows, ref))
 
 
+def test_more_pairs_than_slots(oracle):
+    """725 samples: 262,144 pairs in flight and 1,031 after them."""
+    gl = likelihoods(725, 64, 31)
+    ref, _ = oracle.gl_relatedness(gl, maf=0.02)
+    with kb.Estimator() as est:
+        est.load_likelihoods(np.ascontiguousarray(gl.transpose(1, 0, 2)))
+        rows = est.relatedness_gl(maf=0.02)
+        few = est.relatedness_gl(maf=0.02, num_samples=30)
+    assert (np.abs(rows["obj"] - ref["obj"]) / np.abs(ref["obj"])).max() <= OBJ
+    same = rows[(rows["x"] < 30) & (rows["y"] < 30)]
+    assert np.array_equal(few.view(np.uint8), same.view(np.uint8))
+
+
 def test_sample_without_data():
     gl = likelihoods(6, 1500, 77)
     gl[:, 2] = np.nan
