@@ -81,9 +81,10 @@ const char *kg_version(void);
 /* Arithmetic of the per-site sums (kg_precision). */
 int kg_set_precision(kg_ctx *ctx, int precision);
 
-/* Launch shape of the pair engine: pairs in flight per wave (slots; 0 = a
- * fifth of the pairs, from 4096 to 131072, as memory allows) and blocks per SM
- * of the site-pass kernel (0 = the occupancy limit).  Exposed for the
+/* Launch shape of the pair engine: pairs in flight per wave (slots; 0 = on
+ * site lists a fifth of the pairs, from 4096 to 131072, on frequency nodes all
+ * pairs, as memory allows) and blocks per SM of the site-pass kernel (0 = the
+ * occupancy limit; site lists only).  Exposed for the
  * autotuner and tests; results do not depend on it. */
 int kg_set_launch(kg_ctx *ctx, int slots, int blocks_per_sm);
 
@@ -316,7 +317,8 @@ typedef struct {
     uint64_t gh_passes;
     uint64_t obj_passes;
     uint64_t fp64_passes;
-    uint64_t fp64_pairs;
+    uint64_t fp64_pairs;       /* pairs above the condition estimate where FP32 passes give way to FP64 ones
+                                  (on frequency nodes every pass is FP64: counted, not run again) */
     uint64_t pair_sites;       /* sum over pairs of jointly observed sites */
     uint64_t work_units;       /* sum over passes of sites visited */
     uint64_t launches;         /* kernels launched by the call */
@@ -324,11 +326,11 @@ typedef struct {
     uint64_t flops_fp64;       /* executed FP64 site arithmetic */
     uint64_t shape_sites[5];   /* pair-sites per genotype-pair shape A,B1,B2,C,D */
     uint64_t nonconverged;     /* pairs that stopped at the iteration limit */
-    uint64_t waves;            /* admit / pass / solve waves of the pair engine */
+    uint64_t waves;            /* waves of the pair engine */
     uint64_t slots;            /* pairs in flight per wave */
-    double admit_ms;           /* CUDA-event time of the admit kernels (list build) */
-    double pass_ms;            /* CUDA-event time of the site-pass kernels */
-    double solve_ms;           /* CUDA-event time of the solve kernels (SQP steps) */
+    double admit_ms;           /* device time of the admit kernels (list build) or of the node weights */
+    double pass_ms;            /* device time of the pass kernels */
+    double solve_ms;           /* device time of the solver between the passes (SQP steps) */
     double pair_kernel_ms;     /* CUDA-event time of all pair-engine waves */
     double device_ms;          /* CUDA-event time of preparation + pair kernel */
     double total_ms;           /* host time of the call */
