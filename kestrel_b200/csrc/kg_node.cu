@@ -60,6 +60,8 @@ struct NodeBin {
 
 int node_bins(bool cls, int64_t n_kept, int64_t n_samples, double t_min) {
     if (n_kept <= 0 || n_samples <= 0) return 0;
+    // places, padding included, are 32-bit
+    if (n_kept > (int64_t)INT_MAX - (NODE_MAX_BINS + 1) * NODE_STAGE) return 0;
     if (cls) {
         if (!(t_min >= 0.0)) return 0;
         const int64_t by_work = (n_kept + 1023) / 1024, by_sms = 296 / n_samples + 1;
@@ -68,8 +70,7 @@ int node_bins(bool cls, int64_t n_kept, int64_t n_samples, double t_min) {
     if (!(t_min > 0.0) || t_min > 0.5) return 0;
     const double need = std::ceil(std::log(0.5 / t_min) / std::log(NODE_RATIO));
     if (!(need <= (double)NODE_MAX_BINS)) return 0;
-    const int bins = std::max(1, (int)need);
-    return bins;
+    return std::max(1, (int)need);
 }
 
 // What places a folded frequency: bin edges 1/2 * q^k (q < 1), or equal runs.
@@ -297,6 +298,9 @@ int prepare_query_nodes(const Cohort& panel, QueryPlanes& q, const uint8_t* code
 // an instruction 30.  So three warps issue, one a genotype of x (their
 // accumulators are apart), all lanes converged (one thread of a diverged warp
 // took 25.5 ms), with one wait and one commit a half-stage.
+// A sum of NODE_SEG_STAGES stages of digits fits the 32-bit accumulators
+// whatever the digits (sites of one frequency have the same ones); a bin that
+// may be longer is done in segments, which add up in 64 bits in memory.
 constexpr int NW_THREADS = 608;          // 2 x 4 warps expand A, 4 expand B, 4 read out, 3 issue
 constexpr int NW_N = 96;                 // B's rows: 3 genotypes of y x 32 columns
 constexpr int NW_BSTAGE = NW_N * NODE_STAGE;
@@ -317,6 +321,7 @@ struct NodeProduct {
     int64_t idx0, idx1;        // the pairs of this chunk: y (y + 1) / 2 + x, x <= y (rect: x n_samples + y)
     int64_t slot0;             // slot of pair idx0 within w's columns
     int64_t first_unit, n_yx;  // the first (y, x block) in the count from y = 0, how many
+    int32_t seg, segs;         // stages of a unit at most, units a bin takes at most
     double* w;                 // see NodeDev
     int64_t group;
     unsigned long long* stalled;
@@ -327,6 +332,11 @@ __host__ __device__ inline int64_t yx_before(int64_t y) {
     const int64_t q = y >> 7;
     return 64 * q * (q + 1) + (y - (q << 7)) * (q + 1);
 }
+// A unit: segment un % segs of bin k for a (y, x block) pair.
+struct NodeUnit {
+    int y, xb, k;
+    int start, stages;   // its first site and its stages (0: past the bin's end)
+};
 // (B's sample, block of A's samples)
 __device__ __forceinline__ void decode_yx(const NodeProduct& P, int64_t u, int& y, int& xb) {
     if (P.rect) {
@@ -341,6 +351,19 @@ __device__ __forceinline__ void decode_yx(const NodeProduct& P, int64_t u, int& 
     const int64_t r = u - 64 * q * (q + 1);
     y = (int)((q << 7) + r / (q + 1));
     xb = (int)(r % (q + 1));
+}
+
+__device__ __forceinline__ NodeUnit node_unit(const NodeProduct& P, int64_t un) {
+    const int64_t t = P.segs == 1 ? un : un / P.segs;
+    const int sg = (int)(un - t * P.segs);
+    NodeUnit U;
+    U.k = (int)(t / P.n_yx);
+    decode_yx(P, P.first_unit + (t - U.k * P.n_yx), U.y, U.xb);
+    const NodeBin bn = P.bin[U.k];
+    const int64_t first = (int64_t)sg * P.seg;
+    U.stages = (int)max((long long)0, min((long long)P.seg, (long long)bn.stages - first));
+    U.start = U.stages > 0 ? bn.start + (int)first * NODE_STAGE : bn.start;
+    return U;
 }
 
 // Bounded wait: false once the limit or another warp's has run out.
@@ -385,7 +408,7 @@ __global__ void __launch_bounds__(NW_THREADS, 1) node_weights_kernel(NodeProduct
     __syncthreads();
     tmem_fence_after();
     const uint32_t tm = tm_slot;
-    const int64_t n_units = P.n_yx * P.bins;
+    const int64_t n_units = P.n_yx * P.bins * P.segs;
     uint32_t seq = 0;    // stages so far
     bool ok = true;
     if (warp < 8) {
@@ -394,25 +417,22 @@ __global__ void __launch_bounds__(NW_THREADS, 1) node_weights_kernel(NodeProduct
         const uint32_t half = warp >> 2;
         const uint32_t my = tm + ((uint32_t)((warp & 3) * 32) << 16) + NW_TM_A + half * 48;
         for (int64_t un = blockIdx.x; ok && un < n_units; un += gridDim.x) {
-            const int k = (int)(un / P.n_yx);
-            int y, xb;
-            decode_yx(P, P.first_unit + (un - k * P.n_yx), y, xb);
-            const NodeBin bn = P.bin[k];
-            const int x = xb * 128 + (warp & 3) * 32 + lane;
+            const NodeUnit U = node_unit(P, un);
+            const int x = U.xb * 128 + (warp & 3) * 32 + lane;
             const uint32_t live = x < P.n_samples ? ~0u : 0u;
             const uint4* src =
-                reinterpret_cast<const uint4*>(P.planes + (int64_t)(live ? x : 0) * P.words + (bn.start >> 5)) + half;
+                reinterpret_cast<const uint4*>(P.planes + (int64_t)(live ? x : 0) * P.words + (U.start >> 5)) + half;
             uint4 v[NW_AHEAD];
 #pragma unroll
             for (int j = 0; j < NW_AHEAD; j++)
-                if (j < bn.stages) v[j] = src[2 * j];
-            for (int i0 = 0; ok && i0 < bn.stages; i0 += NW_AHEAD) {
+                if (j < U.stages) v[j] = src[2 * j];
+            for (int i0 = 0; ok && i0 < U.stages; i0 += NW_AHEAD) {
 #pragma unroll
                 for (int j = 0; j < NW_AHEAD; j++) {
                     const int i = i0 + j;
-                    if (i >= bn.stages) break;
+                    if (i >= U.stages) break;
                     const uint32_t lo[2] = {v[j].x, v[j].z}, hi[2] = {v[j].y, v[j].w};
-                    if (i + NW_AHEAD < bn.stages) v[j] = src[2 * (i + NW_AHEAD)];
+                    if (i + NW_AHEAD < U.stages) v[j] = src[2 * (i + NW_AHEAD)];
                     uint32_t r[48];
 #pragma unroll
                     for (int a = 0; a < 3; a++)
@@ -441,12 +461,9 @@ __global__ void __launch_bounds__(NW_THREADS, 1) node_weights_kernel(NodeProduct
         // 32 columns, for the three genotypes of y
         const int tid = threadIdx.x - 256, c = tid & 7, row = tid >> 3;
         for (int64_t un = blockIdx.x; ok && un < n_units; un += gridDim.x) {
-            const int k = (int)(un / P.n_yx);
-            int y, xb;
-            decode_yx(P, P.first_unit + (un - k * P.n_yx), y, xb);
-            const NodeBin bn = P.bin[k];
-            const int8_t* d0 = P.dig + (int64_t)row * P.mp + bn.start + 16 * c;
-            const uint2* py = P.planes_b + (int64_t)y * P.words + (bn.start >> 5) + (c >> 1);
+            const NodeUnit U = node_unit(P, un);
+            const int8_t* d0 = P.dig + (int64_t)row * P.mp + U.start + 16 * c;
+            const uint2* py = P.planes_b + (int64_t)U.y * P.words + (U.start >> 5) + (c >> 1);
             uint4 va[NW_AHEAD], vb[NW_AHEAD];
             uint2 pl[NW_AHEAD];
             auto fetch = [&](int i, uint4& a4, uint4& b4, uint2& p2) {
@@ -456,12 +473,12 @@ __global__ void __launch_bounds__(NW_THREADS, 1) node_weights_kernel(NodeProduct
             };
 #pragma unroll
             for (int j = 0; j < NW_AHEAD; j++)
-                if (j < bn.stages) fetch(j, va[j], vb[j], pl[j]);
-            for (int i0 = 0; ok && i0 < bn.stages; i0 += NW_AHEAD) {
+                if (j < U.stages) fetch(j, va[j], vb[j], pl[j]);
+            for (int i0 = 0; ok && i0 < U.stages; i0 += NW_AHEAD) {
 #pragma unroll
                 for (int j = 0; j < NW_AHEAD; j++) {
                     const int i = i0 + j;
-                    if (i >= bn.stages) break;
+                    if (i >= U.stages) break;
                     const uint32_t lo = pl[j].x, hi = pl[j].y;
                     uint4 va3[3], vb3[3];
 #pragma unroll
@@ -473,7 +490,7 @@ __global__ void __launch_bounds__(NW_THREADS, 1) node_weights_kernel(NodeProduct
                         va3[b] = make_uint4(va[j].x & f[0], va[j].y & f[1], va[j].z & f[2], va[j].w & f[3]);
                         vb3[b] = make_uint4(vb[j].x & f[0], vb[j].y & f[1], vb[j].z & f[2], vb[j].w & f[3]);
                     }
-                    if (i + NW_AHEAD < bn.stages) fetch(i + NW_AHEAD, va[j], vb[j], pl[j]);
+                    if (i + NW_AHEAD < U.stages) fetch(i + NW_AHEAD, va[j], vb[j], pl[j]);
                     const uint32_t st = seq % NW_STAGES;
                     if (!nw_wait_warp(&empty[2 * st + 1], ((seq / NW_STAGES) & 1u) ^ 1u, &gave_up)) { ok = false; break; }
                     const uint32_t base = b0 + st * NW_BSTAGE + ((uint32_t)(c ^ (row & 7)) << 4);
@@ -504,28 +521,22 @@ __global__ void __launch_bounds__(NW_THREADS, 1) node_weights_kernel(NodeProduct
         uint32_t n_acc = 0;
         const int nk = P.bins * J;
         for (int64_t un = blockIdx.x; ok && un < n_units; un += gridDim.x) {
-            const int k = (int)(un / P.n_yx);
-            int y, xb;
-            decode_yx(P, P.first_unit + (un - k * P.n_yx), y, xb);
-            if (P.bin[k].stages == 0) {
-                // an empty bin: zero weights, no product
-                const int x = xb * 128 + (warp - 12) * 32 + lane;
-                const int64_t idx = P.rect ? (int64_t)y * P.n_samples + x : (int64_t)y * (y + 1) / 2 + x;
-                const int64_t s = P.slot0 + (idx - P.idx0);
-                if (x < (P.rect ? P.n_samples : y + 1) && idx >= P.idx0 && idx < P.idx1)
+            const NodeUnit U = node_unit(P, un);
+            const int y = U.y, k = U.k, x = U.xb * 128 + (warp - 12) * 32 + lane;
+            const int64_t idx = P.rect ? (int64_t)y * P.n_samples + x : (int64_t)y * (y + 1) / 2 + x;
+            const bool store = x < (P.rect ? P.n_samples : y + 1) && idx >= P.idx0 && idx < P.idx1;
+            const int64_t s = P.slot0 + (idx - P.idx0);
+            double* out = P.w + (s >> 3) * P.group + (int64_t)(k * J) * 8 + (s & 7);
+            if (U.stages == 0) {
+                // an empty bin: zero weights, no product (in segments they are zero already)
+                if (store && P.segs == 1)
                     for (int u = 0; u < 9; u++)
-                        for (int j = 0; j < J; j++)
-                            P.w[(s >> 3) * P.group + ((int64_t)u * nk + k * J + j) * 8 + (s & 7)] = 0.0;
+                        for (int j = 0; j < J; j++) out[((int64_t)u * nk + j) * 8] = 0.0;
                 continue;
             }
             if (!nw_wait_warp(&acc_full, n_acc & 1u, &gave_up)) { ok = false; break; }
             n_acc++;
             tmem_fence_after();
-            const int x = xb * 128 + (warp - 12) * 32 + lane;
-            const int64_t idx = P.rect ? (int64_t)y * P.n_samples + x : (int64_t)y * (y + 1) / 2 + x;
-            const bool store = x < (P.rect ? P.n_samples : y + 1) && idx >= P.idx0 && idx < P.idx1;
-            const int64_t s = P.slot0 + (idx - P.idx0);
-            double* out = P.w + (s >> 3) * P.group + (int64_t)(k * J) * 8 + (s & 7);
 #pragma unroll
             for (int ab = 0; ab < 9; ab++) {
                 uint32_t r[32];
@@ -541,7 +552,9 @@ __global__ void __launch_bounds__(NW_THREADS, 1) node_weights_kernel(NodeProduct
                     long long v = (int)r[j * L];
 #pragma unroll
                     for (int d = 1; d < L; d++) v += (long long)(int)r[j * L + d] * (1ll << (8 * d));
-                    if (store) out[((int64_t)(P.rect ? UNIT_T[ab] : UNIT[ab]) * nk + j) * 8] = (double)v;
+                    double* o = out + ((int64_t)(P.rect ? UNIT_T[ab] : UNIT[ab]) * nk + j) * 8;
+                    if (store && P.segs == 1) *o = (double)v;
+                    else if (store) atomicAdd(reinterpret_cast<unsigned long long*>(o), (unsigned long long)v);
                 }
             }
         }
@@ -551,13 +564,13 @@ __global__ void __launch_bounds__(NW_THREADS, 1) node_weights_kernel(NodeProduct
         const uint32_t a = warp - 16, d = tm + a * NW_N, a0 = tm + NW_TM_A + a * 16;
         uint32_t n_acc = 0;
         for (int64_t un = blockIdx.x; ok && un < n_units; un += gridDim.x) {
-            const NodeBin bn = P.bin[un / P.n_yx];
-            if (bn.stages == 0) continue;
+            const int stages = node_unit(P, un).stages;
+            if (stages == 0) continue;
             if (!nw_wait_warp(&acc_empty, (n_acc & 1u) ^ 1u, &gave_up)) { ok = false; break; }
             n_acc++;
             tmem_fence_after();
             bool add = false;
-            for (int i = 0; ok && i < bn.stages; i++, seq++) {
+            for (int i = 0; ok && i < stages; i++, seq++) {
                 const uint32_t st = seq % NW_STAGES, phase = (seq / NW_STAGES) & 1u;
                 const uint64_t bd = smem_desc_sw128(b0 + st * NW_BSTAGE);
 #pragma unroll
@@ -583,6 +596,19 @@ __global__ void __launch_bounds__(NW_THREADS, 1) node_weights_kernel(NodeProduct
     __syncthreads();
     tmem_fence_after();
     if (warp == 16) tmem_free<512>(tm);
+}
+
+// Weights formed in segments: 64-bit integers that start at zero and become
+// doubles when every segment has been added.
+template <bool CONVERT>
+__global__ void node_segments_kernel(double* w, int64_t group, int32_t nk, int64_t slot0, int64_t n) {
+    const int64_t per = (int64_t)NODE_UNITS * nk;
+    for (int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; e < n * per; e += (int64_t)gridDim.x * blockDim.x) {
+        // slots fastest, as they lie
+        const int64_t s = slot0 + e % n;
+        double* p = w + (s >> 3) * group + (e / n) * 8 + (s & 7);
+        *p = CONVERT ? (double)*reinterpret_cast<const long long*>(p) : 0.0;
+    }
 }
 
 // --------------------------------------------------------- a chunk's slots
@@ -1234,8 +1260,17 @@ int run_nodes(const std::vector<PairJob>& jobs, const RunConfig& cfg, Workspace&
             P.w = ws.scratch.as<double>();
             P.group = group;
             P.stalled = &d_run->stalled_waits;
-            const int grid = (int)std::min<int64_t>(ws.sm_count, P.n_yx * P.bins);
+            P.seg = NODE_SEG_STAGES;
+            P.segs = node_segments(c.nd_mp / NODE_STAGE, P.seg);
+            const int grid = (int)std::min<int64_t>(ws.sm_count, P.n_yx * P.bins * P.segs);
+            const int sgrid = (int)std::min<int64_t>(((int64_t)g.n * NODE_UNITS * c.nd_n * J + 255) / 256, ws.sm_count * 8);
+            if (P.segs > 1)
+                node_segments_kernel<false><<<sgrid, 256, 0, st>>>(P.w, group, c.nd_n * J, g.slot0, g.n);
             node_weights_kernel<<<grid, NW_THREADS, NW_SMEM, st>>>(P);
+            if (P.segs > 1) {
+                node_segments_kernel<true><<<sgrid, 256, 0, st>>>(P.w, group, c.nd_n * J, g.slot0, g.n);
+                launches += 2;
+            }
         }
         launches += n_seg + 1;
         KG_NODE_TRY(cudaGetLastError());

@@ -43,6 +43,13 @@ constexpr int NODE_MAX_BINS = 64;
 constexpr int NODE_UNITS = 9;        // genotype pairs (gx, gy)
 constexpr int NODE_STAGE = 128;      // sites per tile of the product; a bin's sites are padded to it
 
+// Stages that one 32-bit accumulator adds up at most: a site's digit is -128 at
+// the least, and 2^16 x 128 x 128 = 2^30.  And the segments that a bin of up to
+// `stages` stages takes at `seg` a segment.
+constexpr int NODE_SEG_STAGES = 1 << 16;
+inline int node_segments(int64_t stages, int64_t seg) { return (int)((stages + seg - 1) / seg); }
+static_assert((int64_t)NODE_SEG_STAGES * NODE_STAGE * 128 < ((int64_t)1 << 31), "32-bit sums");
+
 // Whether a prepared cohort's pairs run on nodes, given its kept sites and
 // their smallest min(p, 1 - p), and the bins that takes (0: it does not: a
 // frequency outside 0..1, or below 1/2 x 2^(-64/3) = 1.9e-7, the end of 64 bins).

@@ -93,3 +93,26 @@ def test_cls_sizes(oracle, n, m):
         est.load(codes)
         rows = est.relatedness_gt()
     compare(rows, ref)
+
+
+def test_more_sites_of_a_frequency_than_a_32_bit_sum_holds():
+    """17.3 million sites of one frequency and one genotype pair: the digit of -128
+    that this frequency has in two of its columns adds up to -2.2e9.  The FP64 form
+    (site lists) is the reference: the same sites, the objective at the shared bar
+    (the overflow moved it by 1e-3, and its count of sites by 8e5)."""
+    m, called = 17_600_000, 300_000
+    codes = np.zeros((2, m), np.uint8)
+    codes[:, :called] = np.random.default_rng(1).integers(0, 3, (2, called))
+    af = np.empty((m, 2))
+    af[:, 0] = 0.2622113028257064
+    af[:, 1] = 1.0 - af[:, 0]
+    got = {}
+    for precision in ("fp32c", "fp64"):
+        with kb.Estimator(precision=precision) as est:
+            est.load(codes, af)
+            got[precision] = est.relatedness(maf=0.0), est.run_stats()
+    rows, st = got["fp32c"]
+    ref, sr = got["fp64"]
+    assert st["fp64_passes"] == st["gh_passes"] > 0 and st["pass_ms"] > 0, "the cohort should run on nodes"
+    assert st["pair_sites"] == sr["pair_sites"] == 3 * m
+    assert (np.abs(rows["obj"] - ref["obj"]) / np.abs(ref["obj"])).max() <= 1e-6
