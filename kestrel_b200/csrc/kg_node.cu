@@ -321,7 +321,7 @@ struct NodeProduct {
     int64_t idx0, idx1;        // the pairs of this chunk: y (y + 1) / 2 + x, x <= y (rect: x n_samples + y)
     int64_t slot0;             // slot of pair idx0 within w's columns
     int64_t first_unit, n_yx;  // the first (y, x block) in the count from y = 0, how many
-    int32_t seg, segs;         // stages of a unit at most, units a bin takes at most
+    int32_t seg, segs;         // stages of a unit at most, units a bin takes at most (1: no segments)
     double* w;                 // see NodeDev
     int64_t group;
     unsigned long long* stalled;
@@ -332,10 +332,11 @@ __host__ __device__ inline int64_t yx_before(int64_t y) {
     const int64_t q = y >> 7;
     return 64 * q * (q + 1) + (y - (q << 7)) * (q + 1);
 }
-// A unit: segment un % segs of bin k for a (y, x block) pair.
+// A unit: a segment of bin k for a (y, x block) pair; a segment's pairs follow
+// one another.
 struct NodeUnit {
     int y, xb, k;
-    int start, stages;   // its first site and its stages (0: past the bin's end)
+    int start, stages;   // its first site and its stages (0: an empty bin)
 };
 // (B's sample, block of A's samples)
 __device__ __forceinline__ void decode_yx(const NodeProduct& P, int64_t u, int& y, int& xb) {
@@ -353,16 +354,28 @@ __device__ __forceinline__ void decode_yx(const NodeProduct& P, int64_t u, int& 
     xb = (int)(r % (q + 1));
 }
 
-__device__ __forceinline__ NodeUnit node_unit(const NodeProduct& P, int64_t un) {
-    const int64_t t = P.segs == 1 ? un : un / P.segs;
-    const int sg = (int)(un - t * P.segs);
+// SEGS: bins in segments (seg0: each bin's first, then their number), else each
+// bin a unit.
+template <bool SEGS>
+__device__ __forceinline__ NodeUnit node_unit(const NodeProduct& P, const int* seg0, int64_t un) {
     NodeUnit U;
-    U.k = (int)(t / P.n_yx);
-    decode_yx(P, P.first_unit + (t - U.k * P.n_yx), U.y, U.xb);
+    U.k = (int)(un / P.n_yx);
+    decode_yx(P, P.first_unit + (un - U.k * P.n_yx), U.y, U.xb);
+    int first = 0;
+    if (SEGS) {
+        const int q = U.k;
+        int lo = 0, hi = P.bins - 1;
+        while (lo < hi) {
+            const int mid = (lo + hi + 1) >> 1;
+            if (seg0[mid] <= q) lo = mid;
+            else hi = mid - 1;
+        }
+        U.k = lo;
+        first = (q - seg0[lo]) * P.seg;
+    }
     const NodeBin bn = P.bin[U.k];
-    const int64_t first = (int64_t)sg * P.seg;
-    U.stages = (int)max((long long)0, min((long long)P.seg, (long long)bn.stages - first));
-    U.start = U.stages > 0 ? bn.start + (int)first * NODE_STAGE : bn.start;
+    U.stages = SEGS ? min(P.seg, bn.stages - first) : bn.stages;
+    U.start = bn.start + first * NODE_STAGE;
     return U;
 }
 
@@ -383,6 +396,7 @@ __device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
     asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
 }
 
+template <bool SEGS>
 __global__ void __launch_bounds__(NW_THREADS, 1) node_weights_kernel(NodeProduct P) {
     constexpr int J = NODE_J, L = NODE_L;
     extern __shared__ __align__(1024) unsigned char nw_smem[];
@@ -391,6 +405,7 @@ __global__ void __launch_bounds__(NW_THREADS, 1) node_weights_kernel(NodeProduct
     __shared__ __align__(8) uint64_t full[2 * NW_STAGES], empty[2 * NW_STAGES], acc_full, acc_empty;
     __shared__ uint32_t tm_slot;
     __shared__ int gave_up;
+    __shared__ int seg0[SEGS ? NODE_MAX_BINS + 1 : 1];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const uint32_t b0 = (smem_u32(nw_smem) + 1023u) & ~1023u;
     if (threadIdx.x == 0) {
@@ -402,13 +417,21 @@ __global__ void __launch_bounds__(NW_THREADS, 1) node_weights_kernel(NodeProduct
         mbar_init(&acc_empty, 4);
         gave_up = 0;
         fence_mbar_init();
+        if (SEGS) {
+            int at = 0;
+            for (int k = 0; k < P.bins; k++) {
+                seg0[k] = at;
+                at += (P.bin[k].stages + P.seg - 1) / P.seg;
+            }
+            seg0[P.bins] = at;
+        }
     }
     if (warp == 16) tmem_alloc<512>(smem_u32(&tm_slot));
     tmem_fence_before();
     __syncthreads();
     tmem_fence_after();
     const uint32_t tm = tm_slot;
-    const int64_t n_units = P.n_yx * P.bins * P.segs;
+    const int64_t n_units = P.n_yx * (SEGS ? seg0[P.bins] : P.bins);
     uint32_t seq = 0;    // stages so far
     bool ok = true;
     if (warp < 8) {
@@ -417,7 +440,7 @@ __global__ void __launch_bounds__(NW_THREADS, 1) node_weights_kernel(NodeProduct
         const uint32_t half = warp >> 2;
         const uint32_t my = tm + ((uint32_t)((warp & 3) * 32) << 16) + NW_TM_A + half * 48;
         for (int64_t un = blockIdx.x; ok && un < n_units; un += gridDim.x) {
-            const NodeUnit U = node_unit(P, un);
+            const NodeUnit U = node_unit<SEGS>(P, seg0, un);
             const int x = U.xb * 128 + (warp & 3) * 32 + lane;
             const uint32_t live = x < P.n_samples ? ~0u : 0u;
             const uint4* src =
@@ -461,7 +484,7 @@ __global__ void __launch_bounds__(NW_THREADS, 1) node_weights_kernel(NodeProduct
         // 32 columns, for the three genotypes of y
         const int tid = threadIdx.x - 256, c = tid & 7, row = tid >> 3;
         for (int64_t un = blockIdx.x; ok && un < n_units; un += gridDim.x) {
-            const NodeUnit U = node_unit(P, un);
+            const NodeUnit U = node_unit<SEGS>(P, seg0, un);
             const int8_t* d0 = P.dig + (int64_t)row * P.mp + U.start + 16 * c;
             const uint2* py = P.planes_b + (int64_t)U.y * P.words + (U.start >> 5) + (c >> 1);
             uint4 va[NW_AHEAD], vb[NW_AHEAD];
@@ -521,15 +544,15 @@ __global__ void __launch_bounds__(NW_THREADS, 1) node_weights_kernel(NodeProduct
         uint32_t n_acc = 0;
         const int nk = P.bins * J;
         for (int64_t un = blockIdx.x; ok && un < n_units; un += gridDim.x) {
-            const NodeUnit U = node_unit(P, un);
+            const NodeUnit U = node_unit<SEGS>(P, seg0, un);
             const int y = U.y, k = U.k, x = U.xb * 128 + (warp - 12) * 32 + lane;
             const int64_t idx = P.rect ? (int64_t)y * P.n_samples + x : (int64_t)y * (y + 1) / 2 + x;
             const bool store = x < (P.rect ? P.n_samples : y + 1) && idx >= P.idx0 && idx < P.idx1;
             const int64_t s = P.slot0 + (idx - P.idx0);
             double* out = P.w + (s >> 3) * P.group + (int64_t)(k * J) * 8 + (s & 7);
             if (U.stages == 0) {
-                // an empty bin: zero weights, no product (in segments they are zero already)
-                if (store && P.segs == 1)
+                // an empty bin: zero weights, no product
+                if (store)
                     for (int u = 0; u < 9; u++)
                         for (int j = 0; j < J; j++) out[((int64_t)u * nk + j) * 8] = 0.0;
                 continue;
@@ -553,8 +576,10 @@ __global__ void __launch_bounds__(NW_THREADS, 1) node_weights_kernel(NodeProduct
 #pragma unroll
                     for (int d = 1; d < L; d++) v += (long long)(int)r[j * L + d] * (1ll << (8 * d));
                     double* o = out + ((int64_t)(P.rect ? UNIT_T[ab] : UNIT[ab]) * nk + j) * 8;
-                    if (store && P.segs == 1) *o = (double)v;
-                    else if (store) atomicAdd(reinterpret_cast<unsigned long long*>(o), (unsigned long long)v);
+                    if (store) {
+                        if (SEGS) atomicAdd(reinterpret_cast<unsigned long long*>(o), (unsigned long long)v);
+                        else *o = (double)v;
+                    }
                 }
             }
         }
@@ -564,7 +589,7 @@ __global__ void __launch_bounds__(NW_THREADS, 1) node_weights_kernel(NodeProduct
         const uint32_t a = warp - 16, d = tm + a * NW_N, a0 = tm + NW_TM_A + a * 16;
         uint32_t n_acc = 0;
         for (int64_t un = blockIdx.x; ok && un < n_units; un += gridDim.x) {
-            const int stages = node_unit(P, un).stages;
+            const int stages = node_unit<SEGS>(P, seg0, un).stages;
             if (stages == 0) continue;
             if (!nw_wait_warp(&acc_empty, (n_acc & 1u) ^ 1u, &gave_up)) { ok = false; break; }
             n_acc++;
@@ -1181,7 +1206,8 @@ int run_nodes(const std::vector<PairJob>& jobs, const RunConfig& cfg, Workspace&
         E.advance_blocks = ws.sm_count * std::max(1, occ);
         KG_NODE_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, node_cls_kernel, NA_THREADS, 0));
         E.cls_blocks = ws.sm_count * std::max(1, occ);
-        KG_NODE_TRY(cudaFuncSetAttribute(node_weights_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, NW_SMEM));
+        KG_NODE_TRY(cudaFuncSetAttribute(node_weights_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, NW_SMEM));
+        KG_NODE_TRY(cudaFuncSetAttribute(node_weights_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, NW_SMEM));
         for (auto& e : E.ev)
             if (!e) KG_NODE_TRY(cudaEventCreate(&e));
         KG_NODE_TRY(wave_loop_graph(
@@ -1260,14 +1286,15 @@ int run_nodes(const std::vector<PairJob>& jobs, const RunConfig& cfg, Workspace&
             P.w = ws.scratch.as<double>();
             P.group = group;
             P.stalled = &d_run->stalled_waits;
-            P.seg = NODE_SEG_STAGES;
+            P.seg = (int32_t)node_seg_stages(c.nd_mp / NODE_STAGE, P.n_yx, ws.sm_count);
             P.segs = node_segments(c.nd_mp / NODE_STAGE, P.seg);
-            const int grid = (int)std::min<int64_t>(ws.sm_count, P.n_yx * P.bins * P.segs);
+            const int grid = (int)std::min<int64_t>(ws.sm_count, P.n_yx * (P.bins + P.segs - 1));
             const int sgrid = (int)std::min<int64_t>(((int64_t)g.n * NODE_UNITS * c.nd_n * J + 255) / 256, ws.sm_count * 8);
-            if (P.segs > 1)
+            if (P.segs == 1) {
+                node_weights_kernel<false><<<grid, NW_THREADS, NW_SMEM, st>>>(P);
+            } else {
                 node_segments_kernel<false><<<sgrid, 256, 0, st>>>(P.w, group, c.nd_n * J, g.slot0, g.n);
-            node_weights_kernel<<<grid, NW_THREADS, NW_SMEM, st>>>(P);
-            if (P.segs > 1) {
+                node_weights_kernel<true><<<grid, NW_THREADS, NW_SMEM, st>>>(P);
                 node_segments_kernel<true><<<sgrid, 256, 0, st>>>(P.w, group, c.nd_n * J, g.slot0, g.n);
                 launches += 2;
             }

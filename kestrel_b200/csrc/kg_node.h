@@ -44,9 +44,19 @@ constexpr int NODE_UNITS = 9;        // genotype pairs (gx, gy)
 constexpr int NODE_STAGE = 128;      // sites per tile of the product; a bin's sites are padded to it
 
 // Stages that one 32-bit accumulator adds up at most: a site's digit is -128 at
-// the least, and 2^16 x 128 x 128 = 2^30.  And the segments that a bin of up to
-// `stages` stages takes at `seg` a segment.
+// the least, and 2^16 x 128 x 128 = 2^30.
 constexpr int NODE_SEG_STAGES = 1 << 16;
+// The stages of a segment for a cohort of `stages` stages and `units` (y, x block)
+// pairs.  With few pairs the fullest bin is one SM's work from end to end: 2
+// samples x 3,000,000 sites took 3.9 ms of weights, in segments for two units an SM
+// 0.33 ms.  Below 2,048 stages, or with more pairs than half the SMs, the
+// segments' two further passes over the weights cost what they save.
+inline int64_t node_seg_stages(int64_t stages, int64_t units, int sms) {
+    if (stages < 2048 || 2 * units > sms) return NODE_SEG_STAGES;
+    const int64_t fair = (stages * units + 2 * sms - 1) / (2 * sms);
+    return fair < 256 ? 256 : fair > NODE_SEG_STAGES ? NODE_SEG_STAGES : fair;
+}
+// The segments that a bin of up to `stages` stages takes at `seg` a segment.
 inline int node_segments(int64_t stages, int64_t seg) { return (int)((stages + seg - 1) / seg); }
 static_assert((int64_t)NODE_SEG_STAGES * NODE_STAGE * 128 < ((int64_t)1 << 31), "32-bit sums");
 

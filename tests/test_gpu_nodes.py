@@ -116,3 +116,17 @@ def test_more_sites_of_a_frequency_than_a_32_bit_sum_holds():
     assert st["fp64_passes"] == st["gh_passes"] > 0 and st["pass_ms"] > 0, "the cohort should run on nodes"
     assert st["pair_sites"] == sr["pair_sites"] == 3 * m
     assert (np.abs(rows["obj"] - ref["obj"]) / np.abs(ref["obj"])).max() <= 1e-6
+
+
+def test_split_bins_leave_the_rows_unchanged():
+    """From 262,144 sites on, chunks of few pairs form a bin's weights in segments;
+    the whole triangle (140 samples) does not: the sums are integers, so the rows
+    are the same bit for bit."""
+    codes = cohort(140, 270_000, 12)
+    with kb.Estimator() as est:
+        est.load(codes)
+        whole = est.relatedness()
+        assert est.run_stats()["fp64_passes"] == est.run_stats()["gh_passes"] > 0
+        est.set_launch(1000)
+        parts = est.relatedness()
+    assert np.array_equal(whole.view(np.uint8), parts.view(np.uint8))
