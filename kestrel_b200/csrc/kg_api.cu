@@ -692,7 +692,7 @@ int kg_relatedness(kg_ctx* c, int64_t num_samples, uint64_t iterations, double m
         cudaEventDestroy(ev0);
         cudaEventDestroy(ev1);
         const kg::Cohort& co = c->cohort;
-        stats.launches += co.nd_n ? 10 : 7;  // count, freq, two scans, compact, pad(, three for the nodes' places), pack
+        stats.launches += co.nd_n ? 11 : 7;  // count, freq, two scans, compact, pad(, four for the nodes' places), pack
         if (co.n_multi > 0) stats.launches += 3 + (co.ml_nk > 0 ? 2 : 0);   // fit, two scans, rows, codes
         stats.sites_used[0] = (uint64_t)(co.n_kept + co.ml_by_alleles[0]);
         stats.sites_used[1] = (uint64_t)co.ml_by_alleles[1];
@@ -760,8 +760,8 @@ int kg_relatedness_gt(kg_ctx* c, int64_t num_samples, uint64_t iterations, kg_ou
         if (cudaEventElapsedTime(&dms, ev0, ev1) == cudaSuccess) stats.device_ms = dms;
         cudaEventDestroy(ev0);
         cudaEventDestroy(ev1);
-        // count, freq, two scans, compact, pad(, three for the nodes' places), pack, Gram, Gram total
-        stats.launches += c->cohort.nd_n ? 12 : 9;
+        // count, freq, two scans, compact, pad(, four for the nodes' places), pack, Gram, Gram total
+        stats.launches += c->cohort.nd_n ? 13 : 9;
         if (c->cohort.n_multi > 0) stats.launches += 5;   // multi-allelic frequencies, Gram, Gram total, transpose, rows
         stats.sites_used[0] = (uint64_t)c->cohort.n_kept;
         stats.sites_discarded = (uint64_t)(c->cohort.n_sites - c->cohort.n_kept +

@@ -206,17 +206,27 @@ __global__ void compact_kernel(const uint8_t* __restrict__ keep, const int32_t* 
                                float* __restrict__ p32, double* __restrict__ p64,
                                double* __restrict__ q64, unsigned long long* __restrict__ t_min) {
     int64_t v = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (v >= n || !keep[v]) return;
+    const bool kept = v < n && keep[v];
+    unsigned long long key = ~0ull;
+    if (kept) {
+        const double t = fmin(pf[v], 1.0 - pf[v]);
+        key = pf[v] >= 0.0 && pf[v] <= 1.0 ? (unsigned long long)__double_as_longlong(t) + 1ull : 0ull;
+    }
+    // the smallest min(p, 1 - p), as 1 + its bits (0: some p is not within 0..1)
+    if (t_min != nullptr) {
+        for (int off = 16; off > 0; off >>= 1) {
+            const unsigned long long o = __shfl_xor_sync(0xffffffffu, key, off);
+            key = o < key ? o : key;
+        }
+        if ((threadIdx.x & 31) == 0 && key < *reinterpret_cast<volatile unsigned long long*>(t_min))
+            atomicMin(t_min, key);
+    }
+    if (!kept) return;
     int64_t k = (int64_t)kidx[v] + bsum[v / SCAN_BLOCK];
     site_of[k] = (int32_t)v;
     p64[freq_index(k)] = pf[v];
     q64[k] = qf[v];
     p32[freq_index(k)] = (float)pf[v];
-    // the smallest min(p, 1 - p), as 1 + its bits (0: some p is not within 0..1)
-    if (t_min == nullptr) return;
-    const double t = fmin(pf[v], 1.0 - pf[v]);
-    const unsigned long long key = pf[v] >= 0.0 && pf[v] <= 1.0 ? (unsigned long long)__double_as_longlong(t) + 1ull : 0ull;
-    if (key < *reinterpret_cast<volatile unsigned long long*>(t_min)) atomicMin(t_min, key);
 }
 
 __global__ void pad_kernel(const int32_t* __restrict__ nkept, int64_t cap, float* __restrict__ p32,

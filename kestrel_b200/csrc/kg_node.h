@@ -49,7 +49,7 @@ constexpr int NODE_SEG_STAGES = 1 << 16;
 // The stages of a segment for a cohort of `stages` stages and `units` (y, x block)
 // pairs.  With few pairs the fullest bin is one SM's work from end to end: 2
 // samples x 3,000,000 sites took 3.9 ms of weights, in segments for two units an SM
-// 0.33 ms.  Below 2,048 stages, or with more pairs than half the SMs, the
+// 0.29 ms.  Below 2,048 stages, or with more pairs than half the SMs, the
 // segments' two further passes over the weights cost what they save.
 inline int64_t node_seg_stages(int64_t stages, int64_t units, int sms) {
     if (stages < 2048 || 2 * units > sms) return NODE_SEG_STAGES;
