@@ -545,8 +545,9 @@ __device__ __forceinline__ void soft_sites32(const float4* __restrict__ g32, con
         // the biallelic conditional table (cls_row) gathered by entry
         const float2 A = mul2(X0, Y0), B = mul2(X2, Y2), C = mul2(X0, Y2), D = mul2(X2, Y0);
         const float2 E = mul2(X0, Y1), Fx = mul2(X2, Y1), Gx = mul2(X1, Y0), Hx = mul2(X1, Y2), I = mul2(X1, Y1);
-        // a site where either sample is missing has NaN products
-        const bool v0 = !isnan(A.x), v1 = !isnan(A.y);
+        // a missing sample's record is NaN (the product is one too where a
+        // likelihood is beyond FP32: such a pair's sums become NaN and it goes on in FP64)
+        const bool v0 = !(isnan(X0.x) || isnan(Y0.x)), v1 = !(isnan(X0.y) || isnan(Y0.y));
         const float2 two = dup2(2.0f);
         const float2 p2 = mul2(p, p), q2 = mul2(q, q), pq = mul2(p, q), p2q = mul2(p2, q), pq2 = mul2(p, q2);
         const float2 S2 = fma2(A, p2, mul2(B, q2)), S3 = fma2(A, mul2(p2, p), mul2(B, mul2(q2, q)));

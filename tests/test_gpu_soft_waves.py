@@ -60,3 +60,20 @@ def test_sample_without_data():
         with pytest.raises(kb.KestrelError) as e:
             est.relatedness_gl(maf=0.02)
     assert e.value.status == kb.KG_ENOSITES
+
+
+@pytest.mark.parametrize("scale", [1e60, 1e39, 1e25])
+def test_likelihoods_beyond_fp32(scale):
+    """Likelihoods of any scale: one that FP32 holds as an infinity is no missing
+    sample (infinity times zero is a NaN product); its pairs are estimated from all
+    their sites, as in the FP64 form.  The bars of this file."""
+    gl = likelihoods(4, 1500, 41).transpose(1, 0, 2).copy()
+    gl[0, 700], gl[1, 700], gl[2, 700] = (scale, 0, 0), (0, 1, 0), (scale, 0.5 * scale, 0)
+    got = {}
+    for precision in ("fp32c", "fp64"):
+        with kb.Estimator(precision=precision) as est:
+            est.load_likelihoods(gl)
+            got[precision] = est.relatedness_gl(maf=0.02)
+    a, b = got["fp32c"], got["fp64"]
+    assert (np.abs(a["obj"] - b["obj"]) / np.abs(b["obj"])).max() <= OBJ
+    print(compare(a, b))
