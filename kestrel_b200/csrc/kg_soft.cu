@@ -285,9 +285,10 @@ __device__ __noinline__ int64_t soft_multi_build(const SoftMultiDev M, int64_t x
 
 // Adds the pair's multi-allelic rows at xt to the warp's totals, in FP64:
 // G (warp-uniform), the 45 Hessian totals at hs[a * HS + 32], F (sum log d, or
-// sum log(d / d_old) with d_old at xc in a difference pass) and n.
-__device__ __noinline__ void soft_multi_add(const double* R, int64_t total, const double* xt, const double* xc,
-                                            bool diff, double eps, int lane, double* hs, double* G, double& F,
+// sum log(d / d_old) with d_old at xc, d - d_old from step (difference_step), in a
+// difference pass) and n.
+__device__ __noinline__ void soft_multi_add(const double* R, int64_t total, const double* xt, const double* step,
+                                            const double* xc, bool diff, double eps, int lane, double* hs, double* G, double& F,
                                             int64_t& n) {
     double g[9], f = 0.0;
 #pragma unroll
@@ -319,7 +320,7 @@ __device__ __noinline__ void soft_multi_add(const double* R, int64_t total, cons
 #pragma unroll
             for (int i = 0; i < 9; i++) {
                 dc = fma(xc[i], L[i], dc);
-                dl = fma(xt[i] - xc[i], L[i], dl);
+                dl = fma(step[i], L[i], dl);
             }
             f += log1p(dl / dc);
         }
@@ -434,7 +435,7 @@ __device__ __noinline__ int64_t soft_evaluate(const double* __restrict__ gl, int
         for (int i = 0; i < 9; i++) g[i] += __shfl_xor_sync(0xffffffffu, g[i], off);
     }
     hessian_totals(hs, lane);
-    if (nm > 0) soft_multi_add(R, nm, xv, xv, false, eps, lane, hs, g, f, n);
+    if (nm > 0) soft_multi_add(R, nm, xv, xv, xv, false, eps, lane, hs, g, f, n);
     const double dn = (double)n;
     ev.f = -f / dn;
 #pragma unroll
@@ -675,7 +676,7 @@ __device__ __noinline__ int64_t soft_evaluate32(const float4* __restrict__ g32, 
     }
     // objective so far in natural-log units (direct: F counted log2 d)
     double fsum = diff ? F : F * 0.69314718055994530942 + corr;
-    if (nm > 0) soft_multi_add(R, nm, xt, xc, diff, eps, lane, hs, Gc, fsum, n);
+    if (nm > 0) soft_multi_add(R, nm, xt, step, xc, diff, eps, lane, hs, Gc, fsum, n);
     const double dn = (double)n;
     ev.df = -fsum / dn;   // in a difference pass the objective's change
     ev.f = diff ? f_old + ev.df : ev.df;

@@ -186,3 +186,29 @@ def test_cli_soft_pl_with_multiallelic_records(oracle):
     assert f"Found {len(pls[3])} tri-allelic sites" in r.stderr
     assert len(rows) == len(ref)
     print(check_values(*_tsv_values(rows), ref))
+
+
+def test_difference_passes_with_multiallelic_sites():
+    """A pair's rows at tri- and tetra-allelic sites see the same step in a difference
+    pass as its biallelic ones (the step less its part along the iterate).  The FP64
+    form compares objectives, whose ulp rejects some last trials; a difference
+    pass rejects only what does not go down, so that where nearly all sites are
+    multi-allelic (FP64 sums in both forms) the iterations are the same and the
+    passes are no more."""
+    rng = np.random.default_rng(1)
+    codes = synth.make_cohort(150, 100, 72, missing=0.02, planted={"parent_offspring": 9, "full_sib": 9}).codes
+    gl = rng.uniform(0, 0.08, codes.shape + (3,))
+    for k in range(3):
+        gl[..., k] = np.where(codes == k, 1.0, gl[..., k])
+    gl[codes == 3] = np.nan
+    g, al = synth.make_multiallelic(150, 3000, 14, missing=0.02)
+    m = _soft_multi(g, al, rng)
+    got = {}
+    for prec in ("fp64", "fp32c"):
+        with kb.Estimator(precision=prec) as e:
+            e.load_likelihoods(gl)
+            e.load_likelihoods_multiallelic(m[3], 3)
+            e.load_likelihoods_multiallelic(m[4], 4)
+            got[prec] = e.relatedness_gl(), e.run_stats()
+    assert np.array_equal(got["fp32c"][0]["iters"], got["fp64"][0]["iters"])
+    assert got["fp32c"][1]["gh_passes"] <= got["fp64"][1]["gh_passes"]
