@@ -23,7 +23,8 @@ CUDA_SOURCES = ["kg_engine.cu", "kg_wave.cu", "kg_api.cu", "kg_noalloc.cu", "kg_
                 "kg_node.cu"]
 HOST_SOURCES = ["kg_cli.cpp", "kg_vcf.cpp"]
 HEADERS = ["kg_engine.h", "kg_pair.cuh", "kg_solver.cuh", "kg_rowsolve.cuh", "kg_wave.cuh", "kg_bulk.cuh",
-           "kg_vcf.h", "kg_threads.h", "kg_allele.cuh", "kg_alleleN.cuh", "kg_qp1.cuh", "kg_node.h", "kg_tmem.cuh", "kg_advance.cuh"]
+           "kg_vcf.h", "kg_threads.h", "kg_allele.cuh", "kg_alleleN.cuh", "kg_qp1.cuh", "kg_node.h", "kg_tmem.cuh", "kg_advance.cuh",
+           "kg_log.cuh"]
 
 
 def nvcc() -> str:

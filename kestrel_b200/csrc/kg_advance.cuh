@@ -121,7 +121,7 @@ __device__ __forceinline__ void store_coef(double* v, const double* x) {
 // The step xt - xc of a difference pass, less its part along xc: both points
 // add up to 1 only to an ulp, and the objective would change by that ulp (its
 // slope along x itself is -1) where the step's own change is smaller still.
-__device__ __forceinline__ void difference_step(const double* xt, const double* xc, double (&d)[9]) {
+__host__ __device__ __forceinline__ void difference_step(const double* xt, const double* xc, double (&d)[9]) {
     double s = 0.0;
 #pragma unroll
     for (int i = 0; i < 9; i++) {

@@ -34,6 +34,7 @@
 #include "kg_advance.cuh"
 #include "kg_bulk.cuh"
 #include "kg_engine.h"
+#include "kg_log.cuh"
 #include "kg_node.h"
 #include "kg_pair.cuh"
 #include "kg_qp1.cuh"
@@ -693,13 +694,6 @@ struct NodeDev {
     int32_t pad;
 };
 
-// log d by table (node_log).
-constexpr int LOG_CELLS = 128, LOG_EXPS = 64;
-struct LogTable {
-    double2 cell[LOG_CELLS];   // {c, -log c}
-    double exp2[LOG_EXPS];     // (e - 40) log 2
-};
-
 struct NodeArgs : SlotArgs {
     const NodeDev* nodes;      // per job
     double* partial;           // NODE_PART values a slot
@@ -713,39 +707,6 @@ __global__ void node_init_kernel(NodeArgs A, int n_seg, int n, unsigned long lon
 }
 
 // ------------------------------------------------------------------- passes
-
-// log d for 2^-40 <= d < 2 (Tang, ACM TOMS 16, 1990): d = 2^e m, c the
-// reciprocal of the middle of m's 1/128 interval, log d = e log 2 - log c +
-// log1p(m c - 1), the last by its series (|m c - 1| < 2^-8: the first term left
-// out is below 3e-18).  The library's log is 30 FP64 instructions, this 9.
-__device__ __forceinline__ double node_log(double d, const LogTable& T) {
-    const int hi = __double2hiint(d);
-    const double m = __hiloint2double((hi & 0x000FFFFF) | 0x3FF00000, __double2loint(d));
-    const double2 c = T.cell[(hi >> 13) & (LOG_CELLS - 1)];
-    const double r = fma(m, c.x, -1.0);
-    double s = fma(r, -1.0 / 6.0, 0.2);
-    s = fma(r, s, -0.25);
-    s = fma(r, s, 1.0 / 3.0);
-    s = fma(r, s, -0.5);
-    s = fma(r * r, s, r);
-    return (T.exp2[((hi >> 20) - 1023 + 40) & (LOG_EXPS - 1)] + c.y) + s;
-}
-
-// log(d / (d - delta)) = -log(1 - z), z = delta / d: the series for |z| <= 1/64
-// (the first term left out is below 1e-15 of the sum), else the table.
-__device__ __forceinline__ double node_neg_log1m(double z, const LogTable& T) {
-    if (fabs(z) <= 0.015625) {
-        double s = fma(z, 0.125, 1.0 / 7.0);
-        s = fma(z, s, 1.0 / 6.0);
-        s = fma(z, s, 0.2);
-        s = fma(z, s, 0.25);
-        s = fma(z, s, 1.0 / 3.0);
-        s = fma(z, s, 0.5);
-        s = fma(z, s, 1.0);
-        return z * s;
-    }
-    return -node_log(1.0 - z, T);
-}
 
 // d - eps at a node: the shape's polynomial (stream64 of kg_pair.cuh).
 template <int SH>
@@ -1211,11 +1172,7 @@ int run_nodes(const std::vector<PairJob>& jobs, const RunConfig& cfg, Workspace&
         E.drop();
         if (!E.log_table.p || E.key_dev != dev) {
             LogTable T;
-            for (int i = 0; i < LOG_CELLS; i++) {
-                const double c = 1.0 / (1.0 + (i + 0.5) / LOG_CELLS);
-                T.cell[i] = make_double2(c, -std::log(c));
-            }
-            for (int i = 0; i < LOG_EXPS; i++) T.exp2[i] = (i - 40) * 0.69314718055994530942;
+            fill_log_table(T);
             E.log_table.release();
             KG_NODE_TRY((cudaError_t)E.log_table.reserve(sizeof(T)));
             KG_NODE_TRY(cudaMemcpy(E.log_table.p, &T, sizeof(T), cudaMemcpyHostToDevice));
