@@ -1081,7 +1081,10 @@ extern "C" __global__ void __launch_bounds__(NA_THREADS) node_cls_kernel(NodeArg
 // ------------------------------------------------------------------- host
 
 // The waves of a chunk as one graph launch (a WHILE node over two waves), kept
-// between calls: it depends on the workspace's buffers only, not on the cohort.
+// between calls: it depends on the workspace's buffers and on what they are laid
+// out for (slots and jobs, grown in powers of two), not on the cohort.  Capturing
+// and instantiating it takes 0.25 ms: with the layout of the call itself, 64 x
+// 10,000 sites took 1.01 ms again and again, and 1.26 ms among other sizes.
 struct NodeEngine {
     cudaGraph_t g = nullptr;
     cudaGraphExec_t x = nullptr;
@@ -1090,6 +1093,8 @@ struct NodeEngine {
     uint64_t key_iterations = 0;
     int key_dev = -1;
     cudaStream_t key_st = nullptr;
+    int64_t stride = 0;   // slots that the layout holds
+    int jobs = 0;         // jobs that the tables hold
     DevBuf log_table;
     NodeArgs args[2]{};
     int pass_blocks = 0, advance_blocks = 0, cls_blocks = 0;
@@ -1144,16 +1149,26 @@ int run_nodes(const std::vector<PairJob>& jobs, const RunConfig& cfg, Workspace&
         KG_NODE_TRY(cudaMemGetInfo(&fr, &tot));
         cap = std::max<int64_t>(1, std::min<int64_t>(cap, (int64_t)((fr + held) / 2 / per_slot)));
     }
-    const int64_t stride = (cap + 31) / 32 * 32;
     const int64_t group = (int64_t)NODE_UNITS * nk_max * 8;
-    KG_NODE_TRY((cudaError_t)ws.scratch.reserve(sizeof(double) * (size_t)group * (stride / 8)));
-    KG_NODE_TRY((cudaError_t)ws.slots.reserve(slot_bytes * (size_t)stride));
+    KG_NODE_TRY((cudaError_t)ws.scratch.reserve(sizeof(double) * (size_t)group * ((cap + 7) / 8)));
+    int64_t stride = 4096;
+    while (stride < cap) stride *= 2;
+    if (stride < E.stride && slot_bytes * (size_t)E.stride <= ws.slots.bytes) stride = E.stride;
+    if (ws.slots.reserve(slot_bytes * (size_t)stride) != cudaSuccess) {
+        cudaGetLastError();
+        stride = (cap + 31) / 32 * 32;
+        KG_NODE_TRY((cudaError_t)ws.slots.reserve(slot_bytes * (size_t)stride));
+    }
+    // (the tables are copied whole: no more than 64 jobs are kept for fewer)
+    int job_cap = 16;
+    while (job_cap < n_jobs) job_cap *= 2;
+    if (job_cap < E.jobs && E.jobs <= 64) job_cap = E.jobs;
     // control words, one buffer: {control, clock, run counters}
     const size_t off_clk = sizeof(SlotCtl), off_run = off_clk + sizeof(WaveClock);
     const size_t ctl_bytes = off_run + sizeof(RunCounters);
     KG_NODE_TRY((cudaError_t)ws.node_counts.reserve(ctl_bytes));
-    const size_t off_nodes = sizeof(CohortDev) * n_jobs, off_seg = off_nodes + sizeof(NodeDev) * n_jobs;
-    const size_t blob = off_seg + sizeof(PairSeg) * n_jobs;
+    const size_t off_nodes = sizeof(CohortDev) * job_cap, off_seg = off_nodes + sizeof(NodeDev) * job_cap;
+    const size_t blob = off_seg + sizeof(PairSeg) * job_cap;
     KG_NODE_TRY((cudaError_t)ws.node_table.reserve(blob));
     KG_NODE_TRY((cudaError_t)ws.host.reserve(blob + sizeof(WaveClock) + sizeof(RunCounters)));
     char* counts = ws.node_counts.as<char>();
@@ -1166,9 +1181,8 @@ int run_nodes(const std::vector<PairJob>& jobs, const RunConfig& cfg, Workspace&
     const unsigned long long bound = 2ull * (max_iter + 2) * 16ull + 64ull;
     const char* hw = std::getenv("KESTREL_HOST_WAVES");
     const bool host_waves = hw && hw[0] == '1';
-    const std::vector<void*> key{ws.scratch.p, ws.slots.p, ws.node_counts.p, ws.node_table.p,
-                                 reinterpret_cast<void*>(off_nodes), reinterpret_cast<void*>((size_t)stride)};
-    if (E.key != key || E.key_iterations != cfg.iterations || E.key_dev != dev || E.key_st != st) {
+    const std::vector<void*> key{ws.slots.p, ws.node_counts.p, ws.node_table.p};
+    if (E.key != key || E.stride != stride || E.jobs != job_cap || E.key_iterations != cfg.iterations || E.key_dev != dev || E.key_st != st) {
         E.drop();
         if (!E.log_table.p || E.key_dev != dev) {
             LogTable T;
@@ -1211,6 +1225,8 @@ int run_nodes(const std::vector<PairJob>& jobs, const RunConfig& cfg, Workspace&
         KG_NODE_TRY(wave_loop_graph(
             st, [&](int par, int in_loop, cudaGraphConditionalHandle h) { E.wave(par, in_loop, h, st); }, &E.g, &E.x));
         E.key = key;
+        E.stride = stride;
+        E.jobs = job_cap;
         E.key_iterations = cfg.iterations;
         E.key_dev = dev;
         E.key_st = st;

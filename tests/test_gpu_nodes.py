@@ -130,3 +130,33 @@ def test_split_bins_leave_the_rows_unchanged():
         est.set_launch(1000)
         parts = est.relatedness()
     assert np.array_equal(whole.view(np.uint8), parts.view(np.uint8))
+
+
+def test_calls_of_other_sizes_on_one_context():
+    """One context keeps its slots, tables and graph while sizes grow and shrink (past
+    4,096 pairs, past 16 and 64 cohorts in a call): the rows are a fresh context's."""
+    sizes = [(5, 900), (130, 2100), (33, 4000), (2, 700), (95, 1000)]
+    cohorts = {s: cohort(*s, 300 + s[0]) for s in sizes}
+    small = [(cohort(3, 400, 900 + k), None, None) for k in range(70)]
+
+    def calls(est, s):
+        est.load(cohorts[s])
+        complete = np.where(cohorts[s] == 3, 0, cohorts[s])
+        ml = est.relatedness(allow_nosites=True)
+        est.load(complete)
+        return [ml, est.relatedness_gt(), est.relatedness(iterations=3, allow_nosites=True)]
+
+    def batch(est, n):
+        return est.relatedness_batch(small[:n])
+
+    def fresh(f, arg):
+        with kb.Estimator() as est:
+            return f(est, arg)
+
+    want = {s: fresh(calls, s) for s in sizes}
+    want |= {n: fresh(batch, n) for n in (3, 20, 70)}
+    with kb.Estimator() as est:
+        for step in [*sizes, 3, *sizes[::-1], 20, sizes[3], 70, 3, sizes[1], 20, sizes[0]]:
+            got = batch(est, step) if isinstance(step, int) else calls(est, step)
+            for g, w in zip(got, want[step]):
+                assert np.array_equal(g.view(np.uint8), w.view(np.uint8)), step
