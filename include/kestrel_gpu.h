@@ -243,9 +243,11 @@ int kg_relatedness_batch(kg_ctx *ctx, kg_cohort *cohorts, int n_cohorts,
 
 /* ------------------------------------------------------------- serving */
 
-/* Serving is continuous batching: worker threads each run a wave engine, and
- * queued requests join a running engine between its waves as memory allows;
- * a request is answered as soon as its own pairs are done. */
+/* Serving is continuous batching: two worker threads each run requests' pairs
+ * together (FP32C on frequency nodes, in runs of up to 131,072 pairs that the
+ * requests share; FP64 in a wave engine), queued requests join between runs or
+ * waves as memory allows, and a request is answered as soon as its own pairs
+ * are done. */
 
 /* Makes `codes` the resident reference panel (packed in HBM with its allele
  * frequencies, estimated unless af is given).  Query requests are scored

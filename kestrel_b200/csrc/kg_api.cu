@@ -81,11 +81,17 @@ struct kg_ctx {
     int64_t served_requests = 0, served_pairs = 0, served_launches = 0;
     int64_t in_flight = 0;               // requests admitted into a serving engine
     int64_t panel_gen = 0;               // bumped by every kg_panel_load
+    // A request's device buffers on frequency nodes.
+    struct ServeBuffers {
+        kg::QueryPlanes query;
+        kg::DevBuf rows;
+        size_t device_bytes() const { return query.device_bytes() + rows.bytes; }
+    };
     struct ServeWorker {
         cudaStream_t stream = nullptr;
         kg::Workspace ws;
-        std::vector<std::unique_ptr<kg::QueryPlanes>> queries;   // on nodes: kept between runs
-        std::vector<std::unique_ptr<kg::DevBuf>> rows;
+        bool busy = false;                                   // has requests in flight (under mu)
+        std::vector<std::unique_ptr<ServeBuffers>> idle;     // kept for the next requests (under mu)
     };
     std::vector<ServeWorker> workers;
 };
@@ -124,10 +130,14 @@ bool budget_ok(kg_ctx* c, size_t extra) {
 }
 
 // budget_ok for the calls of the context's own thread, which may give back the
-// buffers kept for batches.
+// buffers kept for batches and for serving.
 bool fits(kg_ctx* c, size_t extra) {
     if (budget_ok(c, extra)) return true;
     c->batch.clear();
+    {
+        std::lock_guard<std::mutex> lk(c->mu);
+        for (auto& w : c->workers) w.idle.clear();
+    }
     return budget_ok(c, extra);
 }
 
@@ -180,100 +190,143 @@ struct LiveRequest {
 // Serving workers, each with its own stream and engine; their kernels overlap
 // on the device.
 constexpr int kServeWorkers = 2;
-// Query buffers and device rows that a worker keeps for its next requests.
-constexpr size_t kServeKeep = 16;
+// Requests' buffers that a worker keeps for its next ones, and their bytes in all.
+constexpr size_t kServeKeep = 16, kServeKeepBytes = (size_t)64 << 20;
 // Pairs in flight per worker (as memory allows).
 constexpr int64_t kServeSlots = 32768;
 // A worker takes more requests only while fewer than this many of its pairs
 // wait for a slot (its slots stay busy; a burst spreads over the workers).
 constexpr int64_t kWorkerBacklog = 1 << 16;
+// On frequency nodes, the pairs of a worker's run (10 ms at 100,000 sites: what a
+// request that arrives meanwhile waits; with 64 queries x 1,024 panel samples one
+// run still takes a request whole), and the requests that share it.
+constexpr int64_t kServeRunPairs = 1 << 17;
+constexpr size_t kServeRunRequests = 64;
 
-// The requests a worker took, on frequency nodes: one run over all of them
-// (about 0.5 ms for 6,000 pairs, so nothing is gained by joining requests to a
-// run on its way), then every row copied back and answered.
-void serve_nodes(kg_ctx* c, kg_ctx::ServeWorker& w, const std::vector<std::shared_ptr<Request>>& admit) {
-    const cudaStream_t st = w.stream;
-    std::string err;
-    std::vector<kg::PairJob> jobs;
-    std::vector<std::shared_ptr<Request>> in;
-    auto answer = [&](Request& r, int status, const std::string& why, int64_t pairs) {
-        std::lock_guard<std::mutex> lk(c->mu);
-        r.status = status;
-        r.err = why;
-        r.done = true;
-        if (pairs > 0) {
-            c->served_requests++;
-            c->served_pairs += pairs;
-        }
-        c->in_flight--;
-        c->cv.notify_all();
-    };
-    for (const auto& rq : admit) {
-        const size_t k = jobs.size();
-        if (k >= w.queries.size()) {
-            w.queries.emplace_back(new kg::QueryPlanes());
-            w.rows.emplace_back(new kg::DevBuf());
-        }
-        const int64_t np = rq->n_query * c->panel.n_samples;
-        int r = kg::prepare_query_nodes(c->panel, *w.queries[k], rq->codes.data(), rq->n_query, c->panel.n_sites,
-                                        rq->mask.empty() ? nullptr : rq->mask.data(), st, err);
-        if (r == KG_OK && w.rows[k]->reserve(sizeof(kg_output) * np) != cudaSuccess) {
-            r = KG_ENOMEM;
-            err = "request rows do not fit";
-        }
-        if (r != KG_OK) {
-            answer(*rq, r, err, 0);
-            continue;
-        }
-        kg::PairJob jb;
-        jb.panel = &c->panel;
-        jb.query = w.queries[k].get();
-        jb.kind = 1;
-        jb.n_x = rq->n_query;
-        jb.n_y = c->panel.n_samples;
-        jb.d_out = w.rows[k]->as<kg_output>();
-        jb.iterations = rq->iterations;   // each request keeps its own limit
-        jobs.push_back(jb);
-        in.push_back(rq);
+// A request on frequency nodes: its buffers, and the pairs of it that are done.
+struct NodeRequest {
+    std::shared_ptr<Request> r;
+    std::unique_ptr<kg_ctx::ServeBuffers> b;
+    int64_t pairs = 0, next = 0;
+};
+
+// Ends a worker's node request; its buffers stay with the worker as far as they
+// fit.  Nothing of it is in flight.
+void end_request(kg_ctx* c, kg_ctx::ServeWorker& w, NodeRequest& q, int status, const std::string& why) {
+    std::lock_guard<std::mutex> lk(c->mu);
+    q.r->status = status;
+    q.r->err = why;
+    q.r->done = true;
+    if (status == KG_OK) {
+        c->served_requests++;
+        c->served_pairs += q.pairs;
     }
-    if (!jobs.empty()) {
-        kg::RunConfig cfg = run_config(c, 100);
-        cfg.max_waves = 0;
-        kg_run_stats stats{};
-        int r = kg::run_pairs(jobs, cfg, w.ws, st, stats, err);
-        if (r == KG_ENOSITES) r = KG_OK;   // such pairs' rows are NaN
-        {
-            std::lock_guard<std::mutex> lk(c->mu);
-            c->served_launches += (int64_t)stats.waves;
-        }
-        for (size_t k = 0; k < in.size(); k++) {
-            const int64_t np = jobs[k].n_pairs();
-            int rk = r;
-            std::string why = err;
-            if (rk == KG_OK) {
-                in[k]->rows.resize((size_t)np);
-                cudaError_t ce = cudaMemcpyAsync(in[k]->rows.data(), jobs[k].d_out, sizeof(kg_output) * np,
-                                                 cudaMemcpyDeviceToHost, st);
-                if (ce == cudaSuccess) ce = cudaStreamSynchronize(st);
-                if (ce != cudaSuccess) {
-                    rk = KG_ECUDA;
-                    why = cudaGetErrorString(ce);
-                }
-            }
-            answer(*in[k], rk, why, rk == KG_OK ? np : 0);
-        }
-    }
-    if (w.queries.size() > kServeKeep) {
-        w.queries.resize(kServeKeep);
-        w.rows.resize(kServeKeep);
-    }
+    c->in_flight--;
+    size_t kept = 0;
+    for (const auto& b : w.idle) kept += b->device_bytes();
+    if (w.idle.size() < kServeKeep && kept + q.b->device_bytes() <= kServeKeepBytes) w.idle.push_back(std::move(q.b));
+    c->cv.notify_all();
 }
 
-// One serving worker.  Its wave engine runs while it has requests in flight.
-// Between waves, queued requests whose inputs and rows fit the memory budget
-// join the engine's job table, so their pairs take slots as slots free
-// (continuous batching); a request is answered as soon as its own pairs are
-// done.  A pair's result does not depend on which requests share its waves.
+// One run over a worker's node requests (0.5 ms for 6,000 pairs): up to
+// kServeRunPairs pairs, an equal share for each request and what that leaves for
+// the oldest, so that a small request is not held up by a large one.  Those
+// whose pairs are all done are answered and leave `live`.  Returns the run's
+// status; after an error every request has been answered with it.
+int serve_run(kg_ctx* c, kg_ctx::ServeWorker& w, std::vector<NodeRequest>& live, std::string& err) {
+    const cudaStream_t st = w.stream;
+    std::vector<int64_t> take(live.size());
+    int64_t left = kServeRunPairs;
+    const int64_t share = std::max<int64_t>(1, left / (int64_t)live.size());
+    for (size_t k = 0; k < live.size(); k++) {
+        take[k] = std::min(live[k].pairs - live[k].next, share);
+        left -= take[k];
+    }
+    std::vector<kg::PairJob> jobs;
+    for (size_t k = 0; k < live.size(); k++) {
+        const int64_t more = std::min(live[k].pairs - live[k].next - take[k], std::max<int64_t>(0, left));
+        take[k] += more;
+        left -= more;
+        kg::PairJob jb;
+        jb.panel = &c->panel;
+        jb.query = &live[k].b->query;
+        jb.kind = 1;
+        jb.n_x = live[k].r->n_query;
+        jb.n_y = c->panel.n_samples;
+        jb.d_out = live[k].b->rows.as<kg_output>();
+        jb.iterations = live[k].r->iterations;   // each request keeps its own limit
+        jb.first = live[k].next;
+        jb.count = take[k];
+        jobs.push_back(jb);
+    }
+    kg::RunConfig cfg = run_config(c, 100);
+    cfg.max_waves = 0;
+    kg_run_stats stats{};
+    int r = kg::run_pairs(jobs, cfg, w.ws, st, stats, err);
+    if (r == KG_ENOSITES) r = KG_OK;   // such pairs' rows are NaN
+    {
+        std::lock_guard<std::mutex> lk(c->mu);
+        c->served_launches += (int64_t)stats.waves;
+    }
+    for (size_t k = 0; k < live.size(); k++) {
+        NodeRequest& q = live[k];
+        q.next += take[k];
+        if (r == KG_OK && q.next < q.pairs) continue;
+        int rk = r;
+        std::string why = err;
+        if (rk == KG_OK) {
+            q.r->rows.resize((size_t)q.pairs);
+            cudaError_t ce = cudaMemcpyAsync(q.r->rows.data(), q.b->rows.p, sizeof(kg_output) * q.pairs,
+                                             cudaMemcpyDeviceToHost, st);
+            if (ce == cudaSuccess) ce = cudaStreamSynchronize(st);
+            if (ce != cudaSuccess) {
+                rk = KG_ECUDA;
+                why = cudaGetErrorString(ce);
+            }
+        }
+        end_request(c, w, q, rk, why);
+        q.r.reset();
+    }
+    live.erase(std::remove_if(live.begin(), live.end(), [](const NodeRequest& q) { return !q.r; }), live.end());
+    return r;
+}
+
+// A request that joins a worker's node requests: its rows packed on the panel's
+// bins, its output rows allocated.
+void join_nodes(kg_ctx* c, kg_ctx::ServeWorker& w, const std::shared_ptr<Request>& rq, std::vector<NodeRequest>& live) {
+    NodeRequest q;
+    q.r = rq;
+    q.pairs = rq->n_query * c->panel.n_samples;
+    {
+        std::lock_guard<std::mutex> lk(c->mu);
+        if (!w.idle.empty()) {
+            q.b = std::move(w.idle.front());   // in order: a repeated request finds its sizes
+            w.idle.erase(w.idle.begin());
+        }
+    }
+    if (!q.b) q.b = std::make_unique<kg_ctx::ServeBuffers>();
+    std::string err;
+    int r = kg::prepare_query_nodes(c->panel, q.b->query, rq->codes.data(), rq->n_query, c->panel.n_sites,
+                                    rq->mask.empty() ? nullptr : rq->mask.data(), w.stream, err);
+    if (r == KG_OK && q.b->rows.reserve(sizeof(kg_output) * q.pairs) != cudaSuccess) {
+        r = KG_ENOMEM;
+        err = "request rows do not fit";
+    }
+    if (r == KG_OK) {
+        live.push_back(std::move(q));
+        return;
+    }
+    cudaStreamSynchronize(w.stream);
+    end_request(c, w, q, r, err);
+}
+
+// One serving worker: continuous batching.  On frequency nodes, queued requests
+// whose inputs and rows fit the memory budget join between two runs over a
+// bounded number of pairs (serve_run).  On site lists (FP64, and panels that nodes
+// do not take) the wave engine runs while requests are in flight, and requests
+// join its job table between waves, their pairs taking slots as slots free.
+// A request is answered as soon as its own pairs are done.  A pair's result does
+// not depend on which requests share its waves.
 void serve_loop(kg_ctx* c, int wid) {
     cudaSetDevice(c->device);
     const cudaStream_t st = c->workers[wid].stream;
@@ -284,6 +337,8 @@ void serve_loop(kg_ctx* c, int wid) {
     std::map<int, LiveRequest> live;     // by job index
     int next_job = 0;
     bool on_nodes = false;
+    kg_ctx::ServeWorker& w = c->workers[wid];
+    std::vector<NodeRequest> nodes;      // in arrival order
     std::string err;
     auto fail_all = [&](int status, const std::string& why) {
         std::lock_guard<std::mutex> lk(c->mu);
@@ -302,7 +357,8 @@ void serve_loop(kg_ctx* c, int wid) {
         std::vector<std::shared_ptr<Request>> admit;
         {
             std::unique_lock<std::mutex> lk(c->mu);
-            c->cv.wait(lk, [&] { return c->stop || !live.empty() || !c->pending.empty(); });
+            w.busy = !live.empty() || !nodes.empty();
+            c->cv.wait(lk, [&] { return c->stop || w.busy || !c->pending.empty(); });
             if (c->stop) {
                 for (int64_t id : c->pending) {
                     auto it = c->requests.find(id);
@@ -315,13 +371,18 @@ void serve_loop(kg_ctx* c, int wid) {
                 c->cv.notify_all();
                 lk.unlock();
                 fail_all(KG_ECANCELED, "context destroyed");
+                for (auto& q : nodes) end_request(c, w, q, KG_ECANCELED, "context destroyed");
                 break;
             }
-            // the queued requests that fit, in arrival order
+            // the queued requests that fit, in arrival order; on nodes, where a
+            // run is shared, a worker also takes them while the others are busy
+            const bool others = std::all_of(c->workers.begin(), c->workers.end(),
+                                            [&](const kg_ctx::ServeWorker& o) { return &o == &w || o.busy; });
             size_t bytes = 0;
             int64_t take = my_backlog;
             while (!c->pending.empty() && next_job + (int)admit.size() < kMaxServeJobs &&
-                   (admit.empty() && live.empty() ? true : take < kWorkerBacklog)) {
+                   (!on_nodes || nodes.size() + admit.size() < kServeRunRequests) &&
+                   (admit.empty() && !w.busy ? true : take < kWorkerBacklog || (on_nodes && others))) {
                 const int64_t id = c->pending.front();
                 auto it = c->requests.find(id);
                 if (it == c->requests.end() || it->second->cancelled) {
@@ -331,31 +392,43 @@ void serve_loop(kg_ctx* c, int wid) {
                 auto& r = it->second;
                 const size_t nb = (size_t)(r->n_query * c->panel.n_samples) * sizeof(kg_output) +
                                   (size_t)r->n_query * (size_t)(c->panel.n_sites + c->panel.plane_stride * 8);
-                if ((!admit.empty() || !live.empty()) && !budget_ok(c, bytes + nb)) break;
+                if ((!admit.empty() || w.busy) && !budget_ok(c, bytes + nb)) {
+                    w.idle.clear();
+                    if (!budget_ok(c, bytes + nb)) break;
+                }
                 admit.push_back(r);
                 bytes += nb;
                 take += r->n_query * c->panel.n_samples;
                 c->pending.pop_front();
             }
             c->in_flight += (int64_t)admit.size();
+            w.busy = w.busy || !admit.empty();
         }
-        if (eng_gen != c->panel_gen && live.empty())
+        if (eng_gen != c->panel_gen && live.empty() && nodes.empty())
             on_nodes = c->panel.nd_n > 0 && c->precision == KG_PREC_FP32C;
         if (on_nodes && live.empty()) {
             eng_gen = c->panel_gen;
+            size_t joined = 0;
             try {
-                serve_nodes(c, c->workers[wid], admit);
+                for (; joined < admit.size(); joined++) join_nodes(c, w, admit[joined], nodes);
+                if (!nodes.empty()) serve_run(c, w, nodes, err);
             } catch (const std::exception& ex) {
+                cudaStreamSynchronize(st);
+                for (auto& q : nodes)
+                    if (q.r) end_request(c, w, q, KG_ENOMEM, ex.what());
+                nodes.clear();
                 std::lock_guard<std::mutex> lk(c->mu);
-                for (auto& rq : admit) {
-                    if (rq->done) continue;
-                    rq->status = KG_ENOMEM;
-                    rq->err = ex.what();
-                    rq->done = true;
+                for (; joined < admit.size(); joined++) {
+                    if (admit[joined]->done) continue;
+                    admit[joined]->status = KG_ENOMEM;
+                    admit[joined]->err = ex.what();
+                    admit[joined]->done = true;
                     c->in_flight--;
                 }
                 c->cv.notify_all();
             }
+            my_backlog = 0;
+            for (const auto& q : nodes) my_backlog += q.pairs - q.next;
             continue;
         }
         if (!eng || (eng_gen != c->panel_gen && live.empty())) {

@@ -183,6 +183,7 @@ struct QueryPlanes {
     DevBuf raw;
     DevBuf mask;
     DevBuf planes;
+    size_t device_bytes() const { return raw.bytes + mask.bytes + planes.bytes; }
 };
 int prepare_query(const Cohort& panel, QueryPlanes& q, const uint8_t* codes, int64_t n_rows,
                   int64_t row_stride, const uint8_t* site_mask, cudaStream_t st, std::string& err);
@@ -197,6 +198,8 @@ struct PairJob {
     kg_output* d_out = nullptr;         // device rows
     uint64_t iterations = 0;            // SQP iteration limit (0 = the run's); CLS: QP iterations
     int method = 0;                     // ESTIMATOR_ML or ESTIMATOR_CLS (panel prepared with cls)
+    // on frequency nodes: only pairs first .. first + count - 1 of them (rect: x n_y + y), -1: all
+    int64_t first = 0, count = -1;
     int64_t n_pairs() const { return kind == 0 ? n_x * (n_x + 1) / 2 : n_x * n_y; }
 };
 

@@ -1133,7 +1133,7 @@ int run_nodes(const std::vector<PairJob>& jobs, const RunConfig& cfg, Workspace&
     for (int i = 0; i < n_jobs; i++) {
         table[i] = make_cohort_dev(jobs[i], cfg.iterations);
         table[i].pair_begin = total;
-        total += table[i].n_pairs;
+        total += jobs[i].count < 0 ? table[i].n_pairs : jobs[i].count;
         nk_max = std::max(nk_max, jobs[i].panel->nd_n * J);
         max_iter = std::max<uint64_t>(max_iter, table[i].max_iter);
     }
@@ -1238,7 +1238,7 @@ int run_nodes(const std::vector<PairJob>& jobs, const RunConfig& cfg, Workspace&
     RunCounters* d_run = reinterpret_cast<RunCounters*>(counts + off_run);
     const WaveClock* d_clk = reinterpret_cast<const WaveClock*>(counts + off_clk);
     int job = 0;
-    int64_t at = 0;   // the job's next pair, y-major
+    int64_t at = jobs[0].first;   // the job's next pair, y-major
     bool limit_hit = false;
     double build_ms = 0.0;
     uint64_t waves = 0, launches = 0;
@@ -1247,9 +1247,11 @@ int run_nodes(const std::vector<PairJob>& jobs, const RunConfig& cfg, Workspace&
         int n_seg = 0;
         int64_t n = 0;
         while (job < n_jobs && n < cap) {
-            const int64_t np = table[job].n_pairs, take = std::min<int64_t>(np - at, cap - n);
+            const PairJob& jb = jobs[job];
+            const int64_t end = jb.count < 0 ? table[job].n_pairs : jb.first + jb.count;
+            const int64_t take = std::min<int64_t>(end - at, cap - n);
             if (take > 0) {
-                const Cohort& c = *jobs[job].panel;
+                const Cohort& c = *jb.panel;
                 h_seg[n_seg] = PairSeg{at, (int32_t)n, (int32_t)take, job, 0};
                 NodeDev& nd = h_nodes[job];
                 nd.w = ws.scratch.as<double>();
@@ -1261,9 +1263,9 @@ int run_nodes(const std::vector<PairJob>& jobs, const RunConfig& cfg, Workspace&
                 n += take;
                 at += take;
             }
-            if (at == np) {
+            if (at >= end) {
                 job++;
-                at = 0;
+                at = job < n_jobs ? jobs[job].first : 0;
             }
         }
         KG_NODE_TRY(cudaMemcpyAsync(dtab, htab, blob, cudaMemcpyHostToDevice, st));
