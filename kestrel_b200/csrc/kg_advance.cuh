@@ -419,6 +419,13 @@ __device__ __forceinline__ void advance_wave(const SlotArgs& A, const Sums& src,
     }
 }
 
+// Waves that no pair needs more of, which only bound a loop that would not end: at
+// most (1 + backtracks) passes per iteration, in each of its forms (FP32 and FP64).
+inline unsigned long long wave_bound(uint64_t iterations, int forms) {
+    const uint64_t most = 1ull << 50;   // whatever the caller asks for, the product does not wrap
+    return (unsigned long long)forms * ((iterations < most ? iterations : most) + 2) * 32ull + 64ull;
+}
+
 // The waves as one graph launch: a WHILE node over an even and an odd wave.
 // wave(par, in_loop, handle) launches one on st, which captures.  Returns a
 // CUDA error.

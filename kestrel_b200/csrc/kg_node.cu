@@ -1191,9 +1191,7 @@ int run_nodes(const std::vector<PairJob>& jobs, const RunConfig& cfg, Workspace&
     char* htab = ws.host.as<char>();
     WaveClock* h_clk = reinterpret_cast<WaveClock*>(htab + blob);
     RunCounters* h_run = reinterpret_cast<RunCounters*>(h_clk + 1);
-    // without a caller's wave limit, one that only bounds a loop that would not
-    // end: a pair takes at most (1 + backtracks) passes per iteration
-    const unsigned long long bound = 2ull * (max_iter + 2) * 16ull + 64ull;
+    const unsigned long long bound = wave_bound(max_iter, 1);   // without a caller's wave limit
     const char* hw = std::getenv("KESTREL_HOST_WAVES");
     const bool host_waves = hw && hw[0] == '1';
     const std::vector<void*> key{ws.slots.p, ws.node_counts.p, ws.node_table.p};

@@ -1113,7 +1113,7 @@ static int run_soft_waves(SoftWork& w, const SoftCall& call, int64_t ns, uint64_
     const char* hw = std::getenv("KESTREL_HOST_WAVES");
     const bool host_waves = hw && hw[0] == '1';   // for kernel profilers, as in run_nodes
     uint64_t launches = 0;
-    const unsigned long long bound = 4ull * (iterations + 2) * 16ull + 64ull;   // FP32, then once more in FP64
+    const unsigned long long bound = wave_bound(iterations, 2);
     for (int64_t at = 0; at < total; at += E.cap) {
         const int n = (int)std::min<int64_t>(E.cap, total - at);
         H->seg = PairSeg{at, 0, n, 0, 0};

@@ -127,5 +127,16 @@ int main(int argc, char** argv) {
         worst = e > worst ? e : worst;
     }
     std::printf("step %.4Lf\n", worst);
+    // the bound of a call's waves grows with its iteration limit, up to the largest
+    unsigned long long last = 0;
+    double wrapped = 0.0;
+    for (int b = 0; b < 64; b++)
+        for (uint64_t it : {((uint64_t)1 << b) - 2 * (b > 0), ((uint64_t)1 << b) - 1, (uint64_t)1 << b, ~(uint64_t)0 >> (63 - b)}) {
+            const unsigned long long w = kg::wave_bound(it, 2);
+            const uint64_t least = it < 1ull << 40 ? it : 1ull << 40;
+            if (w / 11 < least || w / 22 < least || w + 4096 < last) wrapped = 2.0;
+            last = w;
+        }
+    std::printf("wave_bound %.4f\n", wrapped);
     return 0;
 }

@@ -10,7 +10,9 @@ Bounds, from the functions' terms (U = 2^-53):
   neg_log1m  |z| <= 1/64: 1e-15 relative (the first term left out is 3.9e-16); else the
              logarithm's bound and 1 - z rounded, for ratios from 5e-9 to 1.9e8;
   step       what is left of the difference step along the iterate: the roundings of
-             its nine terms.
+             its nine terms;
+  wave_bound the waves that a call may run: at least 11 passes of both forms for every
+             iteration up to 2^40, whatever the limit (2 where it wraps).
 Errors are printed as fractions of these bounds."""
 import os
 import shutil
@@ -37,12 +39,12 @@ def fractions(tmp_path, *args):
 
 def test_on_the_host(tmp_path):
     got = fractions(tmp_path)
-    assert set(got) == {"recip", "log", "neg_log1m", "step"}
+    assert set(got) == {"recip", "log", "neg_log1m", "step", "wave_bound"}
     assert all(v <= 1.0 for v in got.values()), got
 
 
 @pytest.mark.gpu
 def test_on_the_device(tmp_path):
     got = fractions(tmp_path, "device")
-    assert set(got) == {"recip", "log", "neg_log1m", "step"}
+    assert set(got) == {"recip", "log", "neg_log1m", "step", "wave_bound"}
     assert all(v <= 1.0 for v in got.values()), got
