@@ -612,7 +612,7 @@ int prepare_cohort(Cohort& c, const uint8_t* codes, int64_t n_samples, int64_t n
         }
         const int bins = node_bins(cls, c.n_kept, n_samples, t_min);
         if (bins > 0) {
-            const int r = prepare_nodes(c, draw, stride, bins, t_min, st, err);
+            const int r = prepare_nodes(c, draw, stride, bins, st, err);
             if (r || !both) return r;
         }
     }

@@ -259,15 +259,13 @@ static void pack_placed(const uint8_t* codes, int64_t rows, int64_t stride, cons
                                                                   planes.as<uint2>());
 }
 
-int prepare_nodes(Cohort& c, const uint8_t* codes, int64_t stride, int bins, double t_min, cudaStream_t st,
-                  std::string& err) {
+int prepare_nodes(Cohort& c, const uint8_t* codes, int64_t stride, int bins, cudaStream_t st, std::string& err) {
     const int64_t mp = ((c.n_kept + NODE_STAGE - 1) / NODE_STAGE + bins) * NODE_STAGE;
     NodeGrid G;
     G.bins = bins;
     G.by_index = c.cls ? 1 : 0;
-    // the bins end at the smallest frequency (a hair below, so that it lies inside)
-    G.q = c.cls ? 1.0
-                : std::min(1.0 / NODE_RATIO, std::pow(std::min(1.0, 2.0 * t_min) * (1.0 - 1e-12), 1.0 / bins));
+    // the last bin holds the smallest frequency and reaches below it, by less than a bin
+    G.q = c.cls ? 1.0 : 1.0 / NODE_RATIO;
     G.inv_log_q = c.cls ? 0.0 : 1.0 / std::log(G.q);
     G.n_kept = c.n_kept;
     const size_t head = sizeof(int) * NODE_MAX_BINS + sizeof(NodeBin) * NODE_MAX_BINS;

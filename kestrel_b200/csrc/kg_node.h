@@ -63,15 +63,18 @@ static_assert((int64_t)NODE_SEG_STAGES * NODE_STAGE * 128 < ((int64_t)1 << 31), 
 // Whether a prepared cohort's pairs run on nodes, given its kept sites and
 // their smallest min(p, 1 - p), and the bins that takes (0: it does not: a
 // frequency outside 0..1, or below 1/2 x 2^(-64/3) = 1.9e-7, the end of 64 bins).
-// Nodes win at any size: whole calls of 2 samples x 300 sites took 0.50 ms
-// against 1.35 ms on lists, 64 x 1,200 0.95 against 1.93, 600 x 300 9.0 against
-// 30.4, 600 x 10,000 11.3 against 43.2 ms.
+// Nodes win at any size and range measured.  Whole calls of 2 samples x 300 sites took
+// 0.50 ms against 1.35 ms on lists, 64 x 1,200 0.95 against 1.93, 600 x 300 9.0
+// against 30.4, 600 x 10,000 11.3 against 43.2 ms, with frequencies from 0.05 up (10
+// bins).  A pass costs the bins, not the sites, so wide ranges at few sites are
+// nearest to the lists: from 4e-7 up (61 bins) 1,024 x 10 took 37 against 46 ms on
+// the device, 1,024 x 100 62 against 170, 1,024 x 300 68 against 88, 64 x 40 0.90
+// against 3.0, 1,024 x 30,000 80 against 198.
 int node_bins(bool cls, int64_t n_kept, int64_t n_samples, double t_min);
 
 // After the kept sites are compacted: bins, node points, digits and the
 // samples' planes in bin order (c.nd_*).  codes: device byte codes.
-int prepare_nodes(Cohort& c, const uint8_t* codes, int64_t stride, int bins, double t_min, cudaStream_t st,
-                  std::string& err);
+int prepare_nodes(Cohort& c, const uint8_t* codes, int64_t stride, int bins, cudaStream_t st, std::string& err);
 
 // A query's rows against a node-prepared panel (prepare_query for site lists).
 int prepare_query_nodes(const Cohort& panel, QueryPlanes& q, const uint8_t* codes, int64_t n_rows, int64_t row_stride,

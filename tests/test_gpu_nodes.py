@@ -160,3 +160,46 @@ def test_calls_of_other_sizes_on_one_context():
             got = batch(est, step) if isinstance(step, int) else calls(est, step)
             for g, w in zip(got, want[step]):
                 assert np.array_equal(g.view(np.uint8), w.view(np.uint8)), step
+
+
+def test_frequencies_down_to_the_last_bin(oracle):
+    """Frequencies from 2e-7 (the 64th bin) to 1/2, given by the caller, and one cohort
+    just below, which stays on site lists."""
+    n, m = 12, 9000
+    rng = np.random.default_rng(15)
+    p = np.exp(rng.uniform(np.log(2e-7), np.log(0.5), m))
+    p[0] = 2e-7
+    p = np.where(rng.random(m) < 0.5, p, 1.0 - p)
+    codes = synth.apply_missing(rng, synth.hwe_genotypes(rng, p, n), 0.02)
+    codes[:3, 0], codes[3, 0] = 0, 1     # the rarest allele is seen
+    af = np.stack([p, 1.0 - p], 1)
+    with kb.Estimator() as est:
+        check(est, codes, oracle.relatedness(codes, af=af, maf=0.0), af=af, maf=0.0)
+        af[0] = (1.8e-7, 1.0 - 1.8e-7)
+        est.load(codes, af)
+        est.relatedness(maf=0.0)
+        assert est.run_stats()["fp64_passes"] < est.run_stats()["gh_passes"]
+
+
+def test_rare_sites_at_the_default_cut(oracle):
+    """300 samples, frequencies from the cut of 1/600 up, fitted on the device."""
+    n, m = 300, 16_000
+    rng = np.random.default_rng(16)
+    p = np.exp(rng.uniform(np.log(1.0 / 600), np.log(0.5), m))
+    p = np.where(rng.random(m) < 0.5, p, 1.0 - p)
+    codes = synth.apply_missing(rng, synth.hwe_genotypes(rng, p, n), 0.05)
+    with kb.Estimator() as est:
+        check(est, codes, oracle.relatedness(codes, num_samples=50), num_samples=50)
+
+
+def test_a_query_against_a_panel_in_chunks():
+    """Chunks that end inside a query's row of pairs."""
+    panel, query = cohort(150, 3000, 17), cohort(9, 3000, 18)
+    rows = {}
+    for slots in (0, 1000, 37):
+        with kb.Estimator() as est:
+            est.set_launch(slots)
+            est.panel_load(panel)
+            rows[slots] = est.wait(est.submit(query))
+    assert np.array_equal(rows[0].view(np.uint8), rows[1000].view(np.uint8))
+    assert np.array_equal(rows[0].view(np.uint8), rows[37].view(np.uint8))
