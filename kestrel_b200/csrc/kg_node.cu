@@ -1095,7 +1095,7 @@ extern "C" __global__ void __launch_bounds__(NA_THREADS) node_cls_kernel(NodeArg
 
 // The waves of a chunk as one graph launch (a WHILE node over two waves), kept
 // between calls: it depends on the workspace's buffers and on what they are laid
-// out for (slots and jobs, grown in powers of two), not on the cohort.  Capturing
+// out for (the most slots and jobs so far), not on the cohort.  Capturing
 // and instantiating it takes 0.25 ms: with the layout of the call itself, 64 x
 // 10,000 sites took 1.01 ms again and again, and 1.26 ms among other sizes.
 struct NodeEngine {
@@ -1163,18 +1163,13 @@ int run_nodes(const std::vector<PairJob>& jobs, const RunConfig& cfg, Workspace&
         cap = std::max<int64_t>(1, std::min<int64_t>(cap, (int64_t)((fr + held) / 2 / per_slot)));
     }
     const int64_t group = (int64_t)NODE_UNITS * nk_max * 8;
-    KG_NODE_TRY((cudaError_t)ws.scratch.reserve(sizeof(double) * (size_t)group * ((cap + 7) / 8)));
-    int64_t stride = 4096;
-    while (stride < cap) stride *= 2;
+    KG_NODE_TRY((cudaError_t)ws.scratch.reserve(sizeof(double) * (size_t)group * ((cap + 31) / 32 * 4)));
+    // the layout of the largest call so far, not rounded up
+    int64_t stride = (cap + 31) / 32 * 32;
     if (stride < E.stride && slot_bytes * (size_t)E.stride <= ws.slots.bytes) stride = E.stride;
-    if (ws.slots.reserve(slot_bytes * (size_t)stride) != cudaSuccess) {
-        cudaGetLastError();
-        stride = (cap + 31) / 32 * 32;
-        KG_NODE_TRY((cudaError_t)ws.slots.reserve(slot_bytes * (size_t)stride));
-    }
+    KG_NODE_TRY((cudaError_t)ws.slots.reserve(slot_bytes * (size_t)stride));
     // (the tables are copied whole: no more than 64 jobs are kept for fewer)
-    int job_cap = 16;
-    while (job_cap < n_jobs) job_cap *= 2;
+    int job_cap = n_jobs;
     if (job_cap < E.jobs && E.jobs <= 64) job_cap = E.jobs;
     // control words, one buffer: {control, clock, run counters}
     const size_t off_clk = sizeof(SlotCtl), off_run = off_clk + sizeof(WaveClock);
