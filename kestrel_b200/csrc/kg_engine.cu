@@ -507,6 +507,13 @@ static inline int64_t ceil_div(int64_t a, int64_t b) { return (a + b - 1) / b; }
 
 static int grid_for(int64_t n, int threads) { return (int)std::max<int64_t>(1, ceil_div(n, threads)); }
 
+// Gives a cohort's node layout back, where the memory does not take it.
+static void drop_nodes(Cohort& c) {
+    cudaGetLastError();
+    for (DevBuf* b : {&c.nd_bins, &c.nd_t, &c.nd_place, &c.nd_dig, &c.nd_planes}) b->release();
+    c.nd_n = 0;
+}
+
 int prepare_cohort(Cohort& c, const uint8_t* codes, int64_t n_samples, int64_t n_sites,
                    int64_t row_stride, bool codes_on_device, const double* af, double maf,
                    cudaStream_t st, std::string& err, bool cls, uint64_t iterations, bool nodes, bool both) {
@@ -613,10 +620,14 @@ int prepare_cohort(Cohort& c, const uint8_t* codes, int64_t n_samples, int64_t n
         const int bins = node_bins(cls, c.n_kept, n_samples, t_min);
         if (bins > 0) {
             const int r = prepare_nodes(c, draw, stride, bins, st, err);
-            if (r || !both) return r;
+            if (r != KG_ENOMEM && (r || !both)) return r;
+            if (r == KG_ENOMEM) drop_nodes(c);   // the lists' layout takes 36 bytes a site less
         }
     }
-    KG_CUDA_TRY((cudaError_t)c.planes.reserve(sizeof(uint2) * n_samples * c.plane_stride));
+    if (c.planes.reserve(sizeof(uint2) * n_samples * c.plane_stride) != cudaSuccess) {
+        drop_nodes(c);
+        KG_CUDA_TRY((cudaError_t)c.planes.reserve(sizeof(uint2) * n_samples * c.plane_stride));
+    }
     const int64_t work = n_samples * c.plane_stride;
     const int blocks = (int)std::min<int64_t>(ceil_div(work, 8), 148 * 32);
     pack_kernel<<<blocks, 256, 0, st>>>(draw, n_samples, stride, c.site_of.as<int32_t>(), c.nkept.as<int32_t>(),

@@ -203,3 +203,34 @@ def test_a_query_against_a_panel_in_chunks():
             rows[slots] = est.wait(est.submit(query))
     assert np.array_equal(rows[0].view(np.uint8), rows[1000].view(np.uint8))
     assert np.array_equal(rows[0].view(np.uint8), rows[37].view(np.uint8))
+
+
+def test_lists_where_the_node_layout_does_not_fit():
+    """A cohort of few samples and many sites, with memory left for the lists' layout (57
+    bytes a site, and 4 a listed site) but not for the nodes' (36 more): it is
+    estimated on lists, as without them."""
+    import torch
+    n, m = 2, 40_000_000
+    rng = np.random.default_rng(19)
+    half = rng.integers(0, 3, (n, m // 8), dtype=np.uint8)
+    codes = np.tile(half, (1, 8))
+    small = cohort(n, 2000, 20)
+    with kb.Estimator() as est:
+        est.load(codes)
+        want = est.relatedness(maf=0.0)
+        assert est.run_stats()["fp64_passes"] == est.run_stats()["gh_passes"] > 0
+    torch.cuda.empty_cache()
+    with kb.Estimator() as est:
+        est.load(small)
+        est.relatedness(allow_nosites=True)
+        est.set_precision("fp64")
+        est.relatedness(allow_nosites=True)      # both engines' fixed parts are there
+        est.set_precision("fp32c")
+        free = torch.cuda.mem_get_info()[0]
+        held = torch.empty(free - 57 * m - n * m - 18 * m, dtype=torch.uint8, device="cuda")
+        est.load(codes)
+        rows = est.relatedness(maf=0.0)
+        assert est.run_stats()["fp64_passes"] < est.run_stats()["gh_passes"]
+        del held
+        torch.cuda.empty_cache()
+    compare(rows, want)
