@@ -581,21 +581,7 @@ def run_gt_cls(args, local):
         est.relatedness_gt(out=out_pin)
         e2e_ms.append((time.perf_counter() - t0) * 1e3)
     te = float(np.mean(e2e_ms))
-    pair_sites = float(st["pair_sites"])
-    admit_ms, pass_ms = st["admit_ms"], st["pass_ms"]
-    if args.precision == "fp32c" and mg is None:
-        roof = node_weights_roof(admit_ms, pair_sites)
-    else:
-        # on site lists: HBM-bound, 4 bytes written per listed pair-site by the
-        # admit kernel, which the moment pass reads once
-        top_ms = max(admit_ms, pass_ms)
-        achieved = 4.0 * pair_sites / (top_ms * 1e-3) / 1e9
-        peak = measured_hbm_peak()
-        roof = {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
-                "frac": achieved / peak if peak else None, "traffic": None,
-                "kernel": "wave_admit_kernel" if admit_ms >= pass_ms else "wave_pass_kernel",
-                "algorithmic_bytes": 4.0 * pair_sites / max(1, int(st["waves"])),
-                "note": "4 bytes per listed pair-site (written by the admit kernel, read once by the moment pass)"}
+    roof = cls_roof(args.precision, st)
     cpu = None
     if not args.no_cpu:
         sub = min(n_s, 192)
@@ -620,7 +606,7 @@ def run_gt_cls(args, local):
                     "d2h_bytes_per_step": int(out_pin.nbytes), "ms_per_step": te},
             "roofline": roof, "cpu_baseline": cpu, "clocks": clk,
             "gpu_launches": int(st["launches"]),
-            "phases_ms": {"admit": admit_ms, "pass": pass_ms, "solve": st["solve_ms"]},
+            "phases_ms": {"admit": st["admit_ms"], "pass": st["pass_ms"], "solve": st["solve_ms"]},
             "stats": {k2: st[k2] for k2 in ("gh_passes", "waves", "slots", "nonconverged", "pair_sites")}}
 
 
@@ -791,6 +777,24 @@ def measure_fp64_form(est, fp32c_value, steps=2):
 # FP64 operations of a pass at one frequency node: the nine genotype pairs'
 # site arithmetic (two orientations of four shapes and the double heterozygote).
 NODE_FLOPS = 2 * (50 + 39 + 39 + 55) + 27
+
+
+def cls_roof(precision, st):
+    """The roofline of a CLS run's longest kernel.  FP32C cohorts run on frequency
+    nodes, with tri- and tetra-allelic sites or without; FP64 ones on site lists,
+    HBM-bound: 8 bytes written per listed pair-site by the admit kernel, which
+    the moment pass reads once."""
+    if precision == "fp32c":
+        return node_weights_roof(st["admit_ms"], float(st["pair_sites"]))
+    admit_ms, pass_ms = st["admit_ms"], st["pass_ms"]
+    nbytes = 8.0 * float(st["pair_sites"])
+    achieved = nbytes / (max(admit_ms, pass_ms) * 1e-3) / 1e9
+    peak = measured_hbm_peak()
+    return {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
+            "frac": achieved / peak if peak else None, "traffic": None,
+            "kernel": "wave_admit_kernel" if admit_ms >= pass_ms else "wave_pass_kernel",
+            "algorithmic_bytes": nbytes / max(1, int(st["waves"])),
+            "note": "8 bytes per listed pair-site (written by the admit kernel, read once by the moment pass)"}
 
 
 def node_weights_roof(ms, pair_sites):

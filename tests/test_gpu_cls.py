@@ -170,3 +170,17 @@ def test_python_gt_api_routes_multiallelic_sites(oracle, complete, multi):
     below = np.isfinite(lc) & (lc < 15)
     assert np.abs(co.jacquard[x, y] - ref["jacquard"]).max(1)[below].max() <= 1e-5
     assert co.jacquard.shape == (n, n, 9)
+
+
+def test_cls_with_multiallelic_sites_runs_on_nodes(oracle):
+    """FP32C CLS stays on frequency nodes (no passes over lists) with tri- and
+    tetra-allelic sites, at a sample count past one tile of 128."""
+    codes = synth.make_cohort(131, 3001, 24, missing=0.0).codes
+    g, al = synth.make_multiallelic(131, 90, 25)
+    with kb.Estimator() as e:
+        e.load(codes)
+        e.load_multiallelic(g, al)
+        rows = e.relatedness_gt()
+        st = e.run_stats()
+    assert st["pass_ms"] == 0.0 and st["flops_fp32"] == 0 and st["admit_ms"] > 0.0
+    compare(rows, oracle.cls_relatedness(codes, multi=(g, al, None)))

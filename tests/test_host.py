@@ -99,3 +99,15 @@ def test_bench_reference_arm_prints_one_line():
     assert d["impl"] == "reference" and d["unit"] == "pairs/s" and d["value"] > 0
     assert d["cpu_baseline"]["kind"] == "port" and d["cpu_baseline"]["cores"] >= 1
     assert d["e2e"]["h2d_bytes_per_step"] == 0 and d["e2e"]["d2h_bytes_per_step"] == 0
+
+
+def test_bench_cls_roofline_follows_the_path():
+    """FP32C CLS runs on frequency nodes whatever its sites, FP64 on site lists of doubles."""
+    sys.path.insert(0, ROOT)
+    import bench
+    st = {"admit_ms": 2.0, "pass_ms": 0.0, "pair_sites": 10 ** 9, "waves": 1}
+    roof = bench.cls_roof("fp32c", st)
+    assert roof["kernel"] == "node_weights_kernel" and roof["unit"] == "TOP/s"
+    assert abs(roof["achieved"] - 2.0 * 9 * 32 * 1e9 / 2e-3 / 1e12) < 1e-9
+    roof = bench.cls_roof("fp64", st)
+    assert roof["kernel"] == "wave_admit_kernel" and abs(roof["achieved"] - 8e9 / 2e-3 / 1e9) < 1e-9
