@@ -250,10 +250,12 @@ def run_reference(args, codes, planted):
 
 
 def run_batch(args, local):
-    """Eight cohorts of uneven N, M and missingness in one launch: timed with
-    the default launch shape and with the one kg_autotune picks on a sample of
-    the largest cohort, the two alternating step by step (both reported; the
-    line's value is the default shape's, the tuned shape's beside it)."""
+    """Eight cohorts of uneven N, M and missingness in one launch.  The FP64 form, on
+    site lists, is timed with the default launch shape and with the one
+    kg_autotune picks on a sample of the largest cohort, the two alternating step
+    by step (both reported; the line's value is the default shape's, the tuned
+    shape's beside it).  FP32C cohorts run on frequency nodes, which the tuned
+    parameters do not touch: the default shape only."""
     import kestrel_b200 as kb
     from kestrel_b200 import synth
     cohorts = synth.config2()
@@ -275,13 +277,15 @@ def run_batch(args, local):
     # the default shape first, for the warm-up and the tuner's sample
     for _ in range(max(1, args.warmup)):
         est.relatedness_batch(inputs, out=outs)
-    default_shape = est.launch()
-    big = max(cohorts, key=lambda c: c.codes.shape[0])
-    est.load(big.codes)
-    t0 = time.perf_counter()
-    est.autotune()
-    t_tune = time.perf_counter() - t0
-    shape = est.launch()
+    shapes = {"default": est.launch()}
+    t_tune = None
+    if args.precision == "fp64":
+        big = max(cohorts, key=lambda c: c.codes.shape[0])
+        est.load(big.codes)
+        t0 = time.perf_counter()
+        est.autotune()
+        t_tune = time.perf_counter() - t0
+        shapes["tuned"] = est.launch()
 
     def apply(sh):
         est.set_launch(args.slots, sh["blocks_per_sm"] or args.pass_bps)
@@ -293,10 +297,10 @@ def run_batch(args, local):
     # most in blocks per SM and the work unit); a change of shape rebuilds
     # the engine's buffers and graphs, so each shape's timed call follows an
     # untimed one
-    runs = {"default": ([], []), "tuned": ([], [])}
+    runs = {name: ([], []) for name in shapes}
     st = None
     for _ in range(max(1, args.steps)):
-        for name, sh in (("default", default_shape), ("tuned", shape)):
+        for name, sh in shapes.items():
             apply(sh)
             est.relatedness_batch(inputs, out=outs)
             dt, st = run_once()
@@ -305,7 +309,13 @@ def run_batch(args, local):
     # the median step: one host stall (page faults, another process) does
     # not move it
     t_default, w_default = float(np.median(runs["default"][0])), float(np.median(runs["default"][1]))
-    tw, w_tuned = float(np.median(runs["tuned"][0])), float(np.median(runs["tuned"][1]))
+    tuned = None
+    if t_tune is not None:
+        tw, w_tuned = float(np.median(runs["tuned"][0])), float(np.median(runs["tuned"][1]))
+        tuned = {"shape": shapes["tuned"], "tune_s": t_tune, "default_pairs_per_s": pairs / t_default,
+                 "default_waves_ms": w_default, "tuned_pairs_per_s": pairs / tw, "tuned_waves_ms": w_tuned,
+                 "note": "0 = the default (occupancy limit, 32768-entry units, a fifth of the pairs in "
+                         "flight); tuned on about 131,072 pairs of the 2048 x 100000 cohort"}
     est.close()
     waves_ms = [w_default]
     return {"metric": "all-pairs/s, 8 uneven cohorts in one launch", "value": pairs / t_default,
@@ -317,13 +327,10 @@ def run_batch(args, local):
                                    " x M=" + "/".join(str(c.codes.shape[1]) for c in cohorts) +
                                    ", per-sample missingness U(0, 0.2)", "pairs": pairs},
             "timing": "host wall clock around kg_relatedness_batch (uploads from page-locked memory, "
-                      "preparation, waves, rows back into page-locked buffers), median of the steps; default and "
-                      "tuned shapes alternate",
+                      "preparation, waves, rows back into page-locked buffers), median of the steps"
+                      + ("; default and tuned shapes alternate" if tuned else ""),
             "waves_ms": float(np.mean(waves_ms)), "waves_pairs_per_s": pairs / (np.mean(waves_ms) * 1e-3),
-            "autotune": {"shape": shape, "tune_s": t_tune, "default_pairs_per_s": pairs / t_default,
-                         "default_waves_ms": w_default, "tuned_pairs_per_s": pairs / tw, "tuned_waves_ms": w_tuned,
-                         "note": "0 = the default (occupancy limit, 32768-entry units, a fifth of the pairs in "
-                                 "flight); tuned on about 131,072 pairs of the 2048 x 100000 cohort"},
+            "autotune": tuned,
             "stats": {k: st[k] for k in ("gh_passes", "fp64_pairs", "waves", "slots", "nonconverged")}}
 
 

@@ -110,7 +110,10 @@ int kg_set_work_unit(kg_ctx *ctx, int entries);
  * Any pointer may be NULL. */
 int kg_get_launch(const kg_ctx *ctx, int *slots, int *blocks_per_sm, int *unit_entries, int *slot_divisor);
 
-/* Runs the autotuner on a sample of the loaded cohort (about 131,072 pairs of
+/* Tunes the site-list engine (the FP64 form, and FP32C cohorts with tri- or
+ * tetra-allelic sites; pairs on frequency nodes use none of its parameters but
+ * the pairs in flight, which it leaves automatic) on a sample of the loaded
+ * cohort (about 131,072 pairs of
  * its first samples) and keeps the fastest launch shape, by coordinate descent,
  * a change kept only when it is more than 2% faster: site-pass blocks per SM
  * (occupancy limit, 4, 3) and the work unit (32768, 65536, 16384, 8192

@@ -1096,7 +1096,8 @@ int kg_last_run_stats(kg_ctx* c, kg_run_stats* s) {
     return KG_OK;
 }
 
-// The autotuner: the launch shape that gives the fewest device milliseconds
+// The autotuner of the site-list engine (cohorts on frequency nodes use none of
+// what it sets): the launch shape that gives the fewest device milliseconds
 // per pair on a sample of the loaded cohort (the first samples, about 32,768
 // pairs, every site), by coordinate descent over three parameters in turn,
 // each candidate run twice and timed the second time (the first instantiates
