@@ -19,9 +19,9 @@
 //             bin's nodes.  Within a word of 32 sites
 //             byte 4 q + i is site q + 8 i, the order in which four shifted
 //             bits of a plane word become four bytes with one AND.
-// CLS needs sum t^k, k <= 4, only: one interval [0, 1/2] is exact with five
-// nodes, so its bins are equal runs of sites (to spread a small cohort over the
-// SMs), all on that interval.
+// CLS needs sum t^k, k <= 4, only, for which the same eight nodes are exact on
+// one interval [0, 1/2] (five would be): its bins are equal runs of sites (to
+// spread a small cohort over the SMs), all on that interval.
 #include <cuda_runtime.h>
 #include <math_constants.h>
 

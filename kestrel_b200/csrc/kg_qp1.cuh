@@ -33,8 +33,9 @@ __host__ __device__ __forceinline__ int popc9(unsigned v) {
     return n;
 }
 
-// 1 / d: the correctly rounded quotient, or (FAST) the hardware's approximation
-// and one cubic Newton step, to an ulp, at a third of the latency (a division
+// 1 / d: the correctly rounded quotient, or (FAST) the hardware's approximation r
+// and one step of third order (1 / d = r / (1 - e) with e = 1 - d r, its series to
+// e^2: the rest is e^3 = 2^-60), to an ulp, at a third of the latency (a division
 // is a chain of 127 cycles, and an iteration has a pivot's in each of its nine
 // columns one after the other).
 template <bool FAST>

@@ -8,17 +8,18 @@
 // linear scale; a NaN marks a missing sample) as loaded; the kept sites'
 // likelihoods are also packed as FP32, two sites a record [sample][site pair]
 // {l0a, l0b, l1a, l1b}, {l2a, l2b, 0, 0} (NaN where a sample is missing and
-// past the last site), beside {pa, pb, qa, qb} of the kept frequencies.  Tri- and tetra-allelic sites: double [sample][site][6] and
-// [sample][site][10] in the VCF genotype order.
+// past the last site), beside {pa, pb, qa, qb} of the kept frequencies.  Tri-
+// and tetra-allelic sites: double [sample][site][6] and [sample][site][10] in the
+// VCF genotype order.
 //
-// A warp per pair, lanes over the kept sites; the SQP itself is FP64.  FP32C
-// pairs without tri- and tetra-allelic sites run in waves: the evaluations in
-// soft_pass_kernel, the solver between them in soft_advance_kernel, a thread per
+// Lanes take the kept sites; the SQP itself is FP64.  FP32C pairs without tri-
+// and tetra-allelic sites run in waves: the evaluations in soft_pass_kernel, four
+// warps a pair, the solver between them in soft_advance_kernel, a thread per
 // pair (kg_advance.cuh).  In one kernel the solver's 1,300 straight instructions an
 // iteration pushed the site loop out of the instruction caches (its warps waited
 // for instructions twice as long as they issued) and took 145,000 cycles a QP.
-// The other pairs run in soft_pairs_kernel, from a counter.  The evaluations (f,
-// g and H at a point) of the biallelic sites have one of two forms:
+// The other pairs run in soft_pairs_kernel, a warp per pair from a counter.  The
+// evaluations (f, g and H at a point) of the biallelic sites have one of two forms:
 //   * FP32 (the default, KG_PREC_FP32C): from the FP32 likelihoods, which stay
 //     L2-resident for cohorts of a few hundred samples, each site's row L is
 //     formed from the pair's nine likelihood products in closed form, two sites
@@ -633,10 +634,10 @@ __device__ __forceinline__ void soft_sites32(const float4* __restrict__ g32, con
 
 // The FP32 evaluation (see the file comment) at xt; in a difference pass
 // (DIFF) the objective is f_old - (1/n) sum log(d / d_old) with d_old at xc,
-// step = xt - xc less its part along xc (difference_step).  // hs: the warp's FP64 Hessian sums in shared memory; R, nm: the pair's
-// multi-allelic rows, added in FP64 after the lo correction of the biallelic
-// sums.  Returns n.  Not inlined: the site loop gets the registers the pair's
-// SQP state would hold.
+// step = xt - xc less its part along xc (difference_step).  hs: the warp's FP64
+// Hessian sums in shared memory; R, nm: the pair's multi-allelic rows, added in
+// FP64 after the lo correction of the biallelic sums.  Returns n.  Not inlined:
+// the site loop gets the registers the pair's SQP state would hold.
 template <bool DIFF>
 __device__ __noinline__ int64_t soft_evaluate32(const float4* __restrict__ g32, const float4* __restrict__ pq32,
                                                 int64_t nk, int64_t x, int64_t y,
