@@ -114,9 +114,11 @@ int use_device(kg_ctx* c) {
     return KG_OK;
 }
 
-// What kg_relatedness_batch keeps: allocating and freeing some 20 buffers a
-// cohort took 9 of a four-cohort call's 20.7 ms.
-constexpr size_t kBatchKeep = 16, kBatchKeepBytes = (size_t)256 << 20;
+// What kg_relatedness_batch keeps: allocating and freeing some 25 buffers a
+// cohort took 9 of a four-cohort call's 20.7 ms.  With 16 cohorts kept, 100 of 6 x
+// 1,500 sites took 23 ms (site lists, which have fewer buffers, 20), with all of them
+// 11; 400 of 2 x 500 100 (80) and 44.
+constexpr size_t kBatchKeep = 1024, kBatchKeepBytes = (size_t)256 << 20;
 
 bool budget_ok(kg_ctx* c, size_t extra) {
     size_t fr = 0, tot = 0;
@@ -985,7 +987,9 @@ int kg_relatedness_batch(kg_ctx* c, kg_cohort* cohorts, int n_cohorts, uint64_t 
         auto t0 = std::chrono::steady_clock::now();
         int st = use_device(c);
         if (st) return st;
-        std::vector<std::unique_ptr<kg::Cohort>> prep;
+        std::vector<std::unique_ptr<kg::Cohort>> prep, pool;
+        pool.swap(c->batch);
+        size_t reused = 0;
         std::vector<kg::PairJob> jobs;
         std::vector<int> job_of(n_cohorts, -1);
         std::vector<int64_t> offs(n_cohorts, 0);
@@ -1000,13 +1004,9 @@ int kg_relatedness_batch(kg_ctx* c, kg_cohort* cohorts, int n_cohorts, uint64_t 
                 k.status = KG_EINVAL;
                 continue;
             }
-            std::unique_ptr<kg::Cohort> co;
-            if (c->batch.empty()) {
-                co = std::make_unique<kg::Cohort>();
-            } else {
-                co = std::move(c->batch.front());   // in order: a repeated call finds its sizes
-                c->batch.erase(c->batch.begin());
-            }
+            // in order: a repeated call finds its sizes
+            std::unique_ptr<kg::Cohort> co =
+                reused < pool.size() ? std::move(pool[reused++]) : std::make_unique<kg::Cohort>();
             if (raw.bytes > co->raw.bytes) std::swap(raw, co->raw);
             std::string e1;
             int s1 = kg::prepare_cohort(*co, k.codes, k.n_samples, k.n_sites, k.row_stride, false,
@@ -1063,8 +1063,8 @@ int kg_relatedness_batch(kg_ctx* c, kg_cohort* cohorts, int n_cohorts, uint64_t 
         }
         // nothing is in flight: keep the buffers for the next call, as far as they fit
         if (!prep.empty()) std::swap(prep.back()->raw, raw);
+        for (; reused < pool.size(); reused++) prep.push_back(std::move(pool[reused]));
         size_t kept = 0;
-        for (const auto& b : c->batch) kept += b->device_bytes();
         for (auto& b : prep) {
             const size_t n = b->device_bytes();
             if (c->batch.size() >= kBatchKeep || kept + n > kBatchKeepBytes) continue;
