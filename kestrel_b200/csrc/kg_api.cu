@@ -11,6 +11,7 @@
 #include <condition_variable>
 #include <cstring>
 #include <deque>
+#include <iterator>
 #include <map>
 #include <memory>
 #include <mutex>
@@ -90,7 +91,6 @@ struct kg_ctx {
     struct ServeWorker {
         cudaStream_t stream = nullptr;
         kg::Workspace ws;
-        bool busy = false;                                   // has requests in flight (under mu)
         std::vector<std::unique_ptr<ServeBuffers>> idle;     // kept for the next requests (under mu)
     };
     std::vector<ServeWorker> workers;
@@ -201,9 +201,17 @@ constexpr int64_t kServeSlots = 32768;
 constexpr int64_t kWorkerBacklog = 1 << 16;
 // On frequency nodes, the pairs of a worker's run (10 ms at 100,000 sites: what a
 // request that arrives meanwhile waits; with 64 queries x 1,024 panel samples one
-// run still takes a request whole), and the requests that share it.
+// run still takes a request whole), and the requests in flight on a worker.
 constexpr int64_t kServeRunPairs = 1 << 17;
-constexpr size_t kServeRunRequests = 64;
+constexpr size_t kServeRunRequests = 256;
+// A request with at most this many pairs left ends with the next run, whatever
+// arrived before it (such requests get up to half a run); the others go in arrival
+// order.  (Equal shares: 60 requests of 16 x 512 pairs had a median latency of 44
+// ms, in arrival order 17.)
+constexpr int64_t kServeQuantum = 1 << 14;
+// What a request counts for at most in a worker's backlog there: one large request
+// does not keep small ones from joining.
+constexpr int64_t kServeBacklogShare = kWorkerBacklog / 2;
 
 // A request on frequency nodes: its buffers, and the pairs of it that are done.
 struct NodeRequest {
@@ -231,24 +239,26 @@ void end_request(kg_ctx* c, kg_ctx::ServeWorker& w, NodeRequest& q, int status, 
 }
 
 // One run over a worker's node requests (0.5 ms for 6,000 pairs): up to
-// kServeRunPairs pairs, an equal share for each request and what that leaves for
-// the oldest, so that a small request is not held up by a large one.  Those
-// whose pairs are all done are answered and leave `live`.  Returns the run's
-// status; after an error every request has been answered with it.
+// kServeRunPairs pairs, those that kServeQuantum ends first, then in arrival
+// order.  Requests whose pairs are all done are answered, small ones first, and
+// leave `live`.  Returns the run's status; after an error every request has been
+// answered with it.
 int serve_run(kg_ctx* c, kg_ctx::ServeWorker& w, std::vector<NodeRequest>& live, std::string& err) {
     const cudaStream_t st = w.stream;
-    std::vector<int64_t> take(live.size());
+    std::vector<int64_t> take(live.size(), 0);
     int64_t left = kServeRunPairs;
-    const int64_t share = std::max<int64_t>(1, left / (int64_t)live.size());
-    for (size_t k = 0; k < live.size(); k++) {
-        take[k] = std::min(live[k].pairs - live[k].next, share);
-        left -= take[k];
+    for (size_t k = 1; k < live.size(); k++) {
+        const int64_t rest = live[k].pairs - live[k].next;
+        if (rest > kServeQuantum || rest > left - kServeRunPairs / 2) continue;
+        take[k] = rest;
+        left -= rest;
     }
     std::vector<kg::PairJob> jobs;
     for (size_t k = 0; k < live.size(); k++) {
-        const int64_t more = std::min(live[k].pairs - live[k].next - take[k], std::max<int64_t>(0, left));
+        const int64_t more = std::min(live[k].pairs - live[k].next - take[k], left);
         take[k] += more;
         left -= more;
+        if (take[k] == 0) continue;
         kg::PairJob jb;
         jb.panel = &c->panel;
         jb.query = &live[k].b->query;
@@ -270,15 +280,18 @@ int serve_run(kg_ctx* c, kg_ctx::ServeWorker& w, std::vector<NodeRequest>& live,
         std::lock_guard<std::mutex> lk(c->mu);
         c->served_launches += (int64_t)stats.waves;
     }
+    std::vector<NodeRequest*> ended;
     for (size_t k = 0; k < live.size(); k++) {
-        NodeRequest& q = live[k];
-        q.next += take[k];
-        if (r == KG_OK && q.next < q.pairs) continue;
+        live[k].next += take[k];
+        if (r != KG_OK || live[k].next == live[k].pairs) ended.push_back(&live[k]);
+    }
+    std::stable_sort(ended.begin(), ended.end(), [](const NodeRequest* a, const NodeRequest* b) { return a->pairs < b->pairs; });
+    for (NodeRequest* q : ended) {
         int rk = r;
         std::string why = err;
         if (rk == KG_OK) {
-            q.r->rows.resize((size_t)q.pairs);
-            cudaError_t ce = cudaMemcpyAsync(q.r->rows.data(), q.b->rows.p, sizeof(kg_output) * q.pairs,
+            q->r->rows.resize((size_t)q->pairs);
+            cudaError_t ce = cudaMemcpyAsync(q->r->rows.data(), q->b->rows.p, sizeof(kg_output) * q->pairs,
                                              cudaMemcpyDeviceToHost, st);
             if (ce == cudaSuccess) ce = cudaStreamSynchronize(st);
             if (ce != cudaSuccess) {
@@ -286,27 +299,23 @@ int serve_run(kg_ctx* c, kg_ctx::ServeWorker& w, std::vector<NodeRequest>& live,
                 why = cudaGetErrorString(ce);
             }
         }
-        end_request(c, w, q, rk, why);
-        q.r.reset();
+        end_request(c, w, *q, rk, why);
+        q->r.reset();
     }
     live.erase(std::remove_if(live.begin(), live.end(), [](const NodeRequest& q) { return !q.r; }), live.end());
     return r;
 }
 
 // A request that joins a worker's node requests: its rows packed on the panel's
-// bins, its output rows allocated.
-void join_nodes(kg_ctx* c, kg_ctx::ServeWorker& w, const std::shared_ptr<Request>& rq, std::vector<NodeRequest>& live) {
+// bins, its output rows allocated.  (The buffers were taken from the worker's while
+// the mutex was held: a lock for each request here waited for kg_submit's checks,
+// 42 ms instead of 28 for a burst of 60 requests.)
+void join_nodes(kg_ctx* c, kg_ctx::ServeWorker& w, const std::shared_ptr<Request>& rq,
+                std::unique_ptr<kg_ctx::ServeBuffers> buffers, std::vector<NodeRequest>& live) {
     NodeRequest q;
     q.r = rq;
     q.pairs = rq->n_query * c->panel.n_samples;
-    {
-        std::lock_guard<std::mutex> lk(c->mu);
-        if (!w.idle.empty()) {
-            q.b = std::move(w.idle.front());   // in order: a repeated request finds its sizes
-            w.idle.erase(w.idle.begin());
-        }
-    }
-    if (!q.b) q.b = std::make_unique<kg_ctx::ServeBuffers>();
+    q.b = buffers ? std::move(buffers) : std::make_unique<kg_ctx::ServeBuffers>();
     std::string err;
     int r = kg::prepare_query_nodes(c->panel, q.b->query, rq->codes.data(), rq->n_query, c->panel.n_sites,
                                     rq->mask.empty() ? nullptr : rq->mask.data(), w.stream, err);
@@ -357,10 +366,11 @@ void serve_loop(kg_ctx* c, int wid) {
     };
     for (;;) {
         std::vector<std::shared_ptr<Request>> admit;
+        std::vector<std::unique_ptr<kg_ctx::ServeBuffers>> buffers;   // kept ones for them
         {
             std::unique_lock<std::mutex> lk(c->mu);
-            w.busy = !live.empty() || !nodes.empty();
-            c->cv.wait(lk, [&] { return c->stop || w.busy || !c->pending.empty(); });
+            const bool busy = !live.empty() || !nodes.empty();
+            c->cv.wait(lk, [&] { return c->stop || busy || !c->pending.empty(); });
             if (c->stop) {
                 for (int64_t id : c->pending) {
                     auto it = c->requests.find(id);
@@ -376,15 +386,12 @@ void serve_loop(kg_ctx* c, int wid) {
                 for (auto& q : nodes) end_request(c, w, q, KG_ECANCELED, "context destroyed");
                 break;
             }
-            // the queued requests that fit, in arrival order; on nodes, where a
-            // run is shared, a worker also takes them while the others are busy
-            const bool others = std::all_of(c->workers.begin(), c->workers.end(),
-                                            [&](const kg_ctx::ServeWorker& o) { return &o == &w || o.busy; });
+            // the queued requests that fit, in arrival order
             size_t bytes = 0;
             int64_t take = my_backlog;
             while (!c->pending.empty() && next_job + (int)admit.size() < kMaxServeJobs &&
                    (!on_nodes || nodes.size() + admit.size() < kServeRunRequests) &&
-                   (admit.empty() && !w.busy ? true : take < kWorkerBacklog || (on_nodes && others))) {
+                   (admit.empty() && !busy ? true : take < kWorkerBacklog)) {
                 const int64_t id = c->pending.front();
                 auto it = c->requests.find(id);
                 if (it == c->requests.end() || it->second->cancelled) {
@@ -394,17 +401,22 @@ void serve_loop(kg_ctx* c, int wid) {
                 auto& r = it->second;
                 const size_t nb = (size_t)(r->n_query * c->panel.n_samples) * sizeof(kg_output) +
                                   (size_t)r->n_query * (size_t)(c->panel.n_sites + c->panel.plane_stride * 8);
-                if ((!admit.empty() || w.busy) && !budget_ok(c, bytes + nb)) {
+                if ((!admit.empty() || busy) && !budget_ok(c, bytes + nb)) {
                     w.idle.clear();
                     if (!budget_ok(c, bytes + nb)) break;
                 }
                 admit.push_back(r);
                 bytes += nb;
-                take += r->n_query * c->panel.n_samples;
+                const int64_t np = r->n_query * c->panel.n_samples;
+                take += on_nodes ? std::min(np, kServeBacklogShare) : np;
                 c->pending.pop_front();
             }
             c->in_flight += (int64_t)admit.size();
-            w.busy = w.busy || !admit.empty();
+            // in order: a repeated request finds its sizes
+            const size_t n = std::min(admit.size(), w.idle.size());
+            std::move(w.idle.begin(), w.idle.begin() + n, std::back_inserter(buffers));
+            w.idle.erase(w.idle.begin(), w.idle.begin() + n);
+            buffers.resize(admit.size());
         }
         if (eng_gen != c->panel_gen && live.empty() && nodes.empty())
             on_nodes = c->panel.nd_n > 0 && c->precision == KG_PREC_FP32C;
@@ -412,7 +424,8 @@ void serve_loop(kg_ctx* c, int wid) {
             eng_gen = c->panel_gen;
             size_t joined = 0;
             try {
-                for (; joined < admit.size(); joined++) join_nodes(c, w, admit[joined], nodes);
+                for (; joined < admit.size(); joined++) 
+                    join_nodes(c, w, admit[joined], std::move(buffers[joined]), nodes);
                 if (!nodes.empty()) serve_run(c, w, nodes, err);
             } catch (const std::exception& ex) {
                 cudaStreamSynchronize(st);
@@ -430,7 +443,7 @@ void serve_loop(kg_ctx* c, int wid) {
                 c->cv.notify_all();
             }
             my_backlog = 0;
-            for (const auto& q : nodes) my_backlog += q.pairs - q.next;
+            for (const auto& q : nodes) my_backlog += std::min(q.pairs - q.next, kServeBacklogShare);
             continue;
         }
         if (!eng || (eng_gen != c->panel_gen && live.empty())) {

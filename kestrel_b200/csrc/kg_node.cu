@@ -1168,9 +1168,9 @@ int run_nodes(const std::vector<PairJob>& jobs, const RunConfig& cfg, Workspace&
     int64_t stride = (cap + 31) / 32 * 32;
     if (stride < E.stride && slot_bytes * (size_t)E.stride <= ws.slots.bytes) stride = E.stride;
     KG_NODE_TRY((cudaError_t)ws.slots.reserve(slot_bytes * (size_t)stride));
-    // (the tables are copied whole: no more than 64 jobs are kept for fewer)
+    // (the tables are copied whole: no more than 256 jobs are kept for fewer)
     int job_cap = n_jobs;
-    if (job_cap < E.jobs && E.jobs <= 64) job_cap = E.jobs;
+    if (job_cap < E.jobs && E.jobs <= 256) job_cap = E.jobs;
     // control words, one buffer: {control, clock, run counters}
     const size_t off_clk = sizeof(SlotCtl), off_run = off_clk + sizeof(WaveClock);
     const size_t ctl_bytes = off_run + sizeof(RunCounters);
