@@ -401,7 +401,7 @@ __device__ __forceinline__ NodeUnit node_unit(const NodeProduct& P, const int* s
     NodeUnit U;
     U.k = (int)(un / P.n_yx);
     decode_yx(P, P.first_unit + (un - U.k * P.n_yx), U.y, U.xb);
-    int first = 0;
+    int seg = 0, parts = 1;
     if (SEGS) {
         const int q = U.k;
         int lo = 0, hi = P.bins - 1;
@@ -411,10 +411,13 @@ __device__ __forceinline__ NodeUnit node_unit(const NodeProduct& P, const int* s
             else hi = mid - 1;
         }
         U.k = lo;
-        first = (q - seg0[lo]) * P.seg;
+        seg = q - seg0[lo];
+        parts = seg0[lo + 1] - seg0[lo];
     }
+    // (a bin's segments are equal to a stage, and none is empty)
     const NodeBin bn = P.bin[U.k];
-    U.stages = SEGS ? min(P.seg, bn.stages - first) : bn.stages;
+    const int first = SEGS ? (int)((int64_t)bn.stages * seg / parts) : 0;
+    U.stages = SEGS ? (int)((int64_t)bn.stages * (seg + 1) / parts) - first : bn.stages;
     U.start = bn.start + first * NODE_STAGE;
     return U;
 }

@@ -48,13 +48,15 @@ constexpr int NODE_STAGE = 128;      // sites per tile of the product; a bin's s
 constexpr int NODE_SEG_STAGES = 1 << 16;
 // The stages of a segment for a cohort of `stages` stages and `units` (y, x block)
 // pairs.  With few pairs the fullest bin is one SM's work from end to end: 2
-// samples x 3,000,000 sites took 3.9 ms of weights, in segments for two units an SM
-// 0.29 ms.  Below 2,048 stages, or with more pairs than half the SMs, the
-// segments' two further passes over the weights cost what they save.
+// samples x 3,000,000 sites took 3.9 ms of weights, in segments 0.23; eight units an SM
+// even the blocks out (two, four, eight, sixteen: 3.67, 2.72, 2.73, 2.67 ms for 32 x
+// 3,000,000, CLS 3.58, 3.01, 2.73, 2.76; whole bins 6.17 and 3.57).  Below 2,048
+// stages, or with more pairs than half the SMs, the segments' two further passes over
+// the weights cost what they save.
 inline int64_t node_seg_stages(int64_t stages, int64_t units, int sms) {
     if (stages < 2048 || 2 * units > sms) return NODE_SEG_STAGES;
-    const int64_t fair = (stages * units + 2 * sms - 1) / (2 * sms);
-    return fair < 256 ? 256 : fair > NODE_SEG_STAGES ? NODE_SEG_STAGES : fair;
+    const int64_t fair = (stages * units + 8 * sms - 1) / (8 * sms);
+    return fair < 128 ? 128 : fair > NODE_SEG_STAGES ? NODE_SEG_STAGES : fair;
 }
 // The segments that a bin of up to `stages` stages takes at `seg` a segment.
 inline int node_segments(int64_t stages, int64_t seg) { return (int)((stages + seg - 1) / seg); }

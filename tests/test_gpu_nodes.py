@@ -129,7 +129,12 @@ def test_split_bins_leave_the_rows_unchanged():
         assert est.run_stats()["fp64_passes"] == est.run_stats()["gh_passes"] > 0
         est.set_launch(1000)
         parts = est.relatedness()
+        est.load(np.where(codes == 3, 0, codes))
+        cls_parts = est.relatedness_gt()
+        est.set_launch(0)
+        cls_whole = est.relatedness_gt()
     assert np.array_equal(whole.view(np.uint8), parts.view(np.uint8))
+    assert np.array_equal(cls_whole.view(np.uint8), cls_parts.view(np.uint8))
 
 
 def test_calls_of_other_sizes_on_one_context():
