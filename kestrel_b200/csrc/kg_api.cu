@@ -192,8 +192,9 @@ struct LiveRequest {
 // Serving workers, each with its own stream and engine; their kernels overlap
 // on the device.
 constexpr int kServeWorkers = 2;
-// Requests' buffers that a worker keeps for its next ones, and their bytes in all.
-constexpr size_t kServeKeep = 16, kServeKeepBytes = (size_t)64 << 20;
+// Requests' buffers that a worker keeps for its next ones, and their bytes in all (37
+// MB a request of 64 x 4,096 pairs at 100,000 sites).
+constexpr size_t kServeKeep = 16, kServeKeepBytes = (size_t)512 << 20;
 // Pairs in flight per worker (as memory allows).
 constexpr int64_t kServeSlots = 32768;
 // A worker takes more requests only while fewer than this many of its pairs
@@ -209,9 +210,6 @@ constexpr size_t kServeRunRequests = 256;
 // order.  (Equal shares: 60 requests of 16 x 512 pairs had a median latency of 44
 // ms, in arrival order 17.)
 constexpr int64_t kServeQuantum = 1 << 14;
-// What a request counts for at most in a worker's backlog there: one large request
-// does not keep small ones from joining.
-constexpr int64_t kServeBacklogShare = kWorkerBacklog / 2;
 
 // A request on frequency nodes: its buffers, and the pairs of it that are done.
 struct NodeRequest {
@@ -342,7 +340,8 @@ void serve_loop(kg_ctx* c, int wid) {
     cudaSetDevice(c->device);
     const cudaStream_t st = c->workers[wid].stream;
     kg::Workspace& wws = c->workers[wid].ws;
-    int64_t my_backlog = 0;   // pairs of this worker's requests not yet in a slot
+    int64_t my_backlog = 0;   // pairs of this worker's requests not yet in a slot (on nodes: not yet done)
+    int64_t my_small = 0;     // on nodes: those of requests that kServeQuantum ends
     std::unique_ptr<kg::WaveEngine> eng;   // (re)opened for each panel
     int64_t eng_gen = -1;
     std::map<int, LiveRequest> live;     // by job index
@@ -386,20 +385,26 @@ void serve_loop(kg_ctx* c, int wid) {
                 for (auto& q : nodes) end_request(c, w, q, KG_ECANCELED, "context destroyed");
                 break;
             }
-            // the queued requests that fit, in arrival order
-            size_t bytes = 0;
-            int64_t take = my_backlog;
-            while (!c->pending.empty() && next_job + (int)admit.size() < kMaxServeJobs &&
-                   (!on_nodes || nodes.size() + admit.size() < kServeRunRequests) &&
-                   (admit.empty() && !busy ? true : take < kWorkerBacklog)) {
-                const int64_t id = c->pending.front();
-                auto it = c->requests.find(id);
+            // the queued requests that fit, in arrival order; on nodes small ones
+            // also join while the backlog is large ones'
+            size_t bytes = 0, seen = 0;
+            int64_t take = my_backlog, small = my_small;
+            for (auto p = c->pending.begin(); p != c->pending.end() && next_job + (int)admit.size() < kMaxServeJobs;) {
+                auto it = c->requests.find(*p);
                 if (it == c->requests.end() || it->second->cancelled) {
-                    c->pending.pop_front();
+                    p = c->pending.erase(p);
                     continue;
                 }
+                if (on_nodes && (seen++ >= kServeRunRequests || nodes.size() + admit.size() >= kServeRunRequests)) break;
                 auto& r = it->second;
-                const size_t nb = (size_t)(r->n_query * c->panel.n_samples) * sizeof(kg_output) +
+                const int64_t np = r->n_query * c->panel.n_samples;
+                const bool little = on_nodes && np <= kServeQuantum;
+                if (!(admit.empty() && !busy) && take >= kWorkerBacklog && !(little && small < kServeRunPairs / 2)) {
+                    if (!on_nodes) break;
+                    ++p;
+                    continue;
+                }
+                const size_t nb = (size_t)np * sizeof(kg_output) +
                                   (size_t)r->n_query * (size_t)(c->panel.n_sites + c->panel.plane_stride * 8);
                 if ((!admit.empty() || busy) && !budget_ok(c, bytes + nb)) {
                     w.idle.clear();
@@ -407,16 +412,23 @@ void serve_loop(kg_ctx* c, int wid) {
                 }
                 admit.push_back(r);
                 bytes += nb;
-                const int64_t np = r->n_query * c->panel.n_samples;
-                take += on_nodes ? std::min(np, kServeBacklogShare) : np;
-                c->pending.pop_front();
+                take += np;
+                small += little ? np : 0;
+                p = c->pending.erase(p);
+                // the smallest kept buffers whose rows hold it, else the largest
+                const size_t need = (size_t)np * sizeof(kg_output);
+                size_t best = 0;
+                for (size_t k = 1; k < w.idle.size(); k++) {
+                    const size_t a = w.idle[best]->rows.bytes, b = w.idle[k]->rows.bytes;
+                    if (b >= need ? a < need || b < a : a < b) best = k;
+                }
+                buffers.emplace_back();
+                if (best < w.idle.size()) {
+                    buffers.back() = std::move(w.idle[best]);
+                    w.idle.erase(w.idle.begin() + best);
+                }
             }
             c->in_flight += (int64_t)admit.size();
-            // in order: a repeated request finds its sizes
-            const size_t n = std::min(admit.size(), w.idle.size());
-            std::move(w.idle.begin(), w.idle.begin() + n, std::back_inserter(buffers));
-            w.idle.erase(w.idle.begin(), w.idle.begin() + n);
-            buffers.resize(admit.size());
         }
         if (eng_gen != c->panel_gen && live.empty() && nodes.empty())
             on_nodes = c->panel.nd_n > 0 && c->precision == KG_PREC_FP32C;
@@ -424,7 +436,7 @@ void serve_loop(kg_ctx* c, int wid) {
             eng_gen = c->panel_gen;
             size_t joined = 0;
             try {
-                for (; joined < admit.size(); joined++) 
+                for (; joined < admit.size(); joined++)
                     join_nodes(c, w, admit[joined], std::move(buffers[joined]), nodes);
                 if (!nodes.empty()) serve_run(c, w, nodes, err);
             } catch (const std::exception& ex) {
@@ -442,8 +454,11 @@ void serve_loop(kg_ctx* c, int wid) {
                 }
                 c->cv.notify_all();
             }
-            my_backlog = 0;
-            for (const auto& q : nodes) my_backlog += std::min(q.pairs - q.next, kServeBacklogShare);
+            my_backlog = my_small = 0;
+            for (const auto& q : nodes) {
+                my_backlog += q.pairs - q.next;
+                my_small += q.pairs <= kServeQuantum ? q.pairs - q.next : 0;
+            }
             continue;
         }
         if (!eng || (eng_gen != c->panel_gen && live.empty())) {
