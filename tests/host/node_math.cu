@@ -10,6 +10,7 @@
 
 #include "kg_advance.cuh"
 #include "kg_log.cuh"
+#include "kg_node.h"
 #include "kg_qp1.cuh"
 
 enum { RECIP, LOG, LOG1M, STEP, N_FN };
@@ -138,5 +139,23 @@ int main(int argc, char** argv) {
             last = w;
         }
     std::printf("wave_bound %.4f\n", wrapped);
+    // no segment of a bin, cut into equal parts as the kernel cuts it, has more digits of
+    // -128 than 32 bits hold, up to the most sites that places allow
+    double sums = 0.0;
+    for (int64_t stages : {1ll, 127ll, 2047ll, 2048ll, 2049ll, 65535ll, 65536ll, 65537ll, 131071ll, 131072ll, 131073ll, 156251ll, 16777215ll})
+        for (int64_t units : {1ll, 2ll, 73ll, 74ll, 75ll, 4608ll, 1ll << 40}) {
+            const int64_t seg = kg::node_seg_stages(stages, units, 148);
+            const int64_t parts = kg::node_segments(stages, seg);
+            int64_t last = 0;
+            for (int64_t k = 0; k < parts; k++) {
+                const int64_t end = stages * (k + 1) / parts, n = end - last;
+                const double sum = (double)n * kg::NODE_STAGE * 128.0 / 2147483648.0;
+                if (n < 1) sums = 2.0;
+                if (sum > sums) sums = sum;
+                last = end;
+            }
+            if (last != stages) sums = 2.0;
+        }
+    std::printf("segments %.4f\n", sums);
     return 0;
 }

@@ -12,7 +12,9 @@ Bounds, from the functions' terms (U = 2^-53):
   step       what is left of the difference step along the iterate: the roundings of
              its nine terms;
   wave_bound the waves that a call may run: at least 11 passes of both forms for every
-             iteration up to 2^40, whatever the limit (2 where it wraps).
+             iteration up to 2^40, whatever the limit (2 where it wraps);
+  segments   the largest sum of signed digits in a 32-bit accumulator, of 2^31 (2 where a
+             bin's segments are empty or leave stages out).
 Errors are printed as fractions of these bounds."""
 import os
 import shutil
@@ -39,12 +41,12 @@ def fractions(tmp_path, *args):
 
 def test_on_the_host(tmp_path):
     got = fractions(tmp_path)
-    assert set(got) == {"recip", "log", "neg_log1m", "step", "wave_bound"}
+    assert set(got) == {"recip", "log", "neg_log1m", "step", "wave_bound", "segments"}
     assert all(v <= 1.0 for v in got.values()), got
 
 
 @pytest.mark.gpu
 def test_on_the_device(tmp_path):
     got = fractions(tmp_path, "device")
-    assert set(got) == {"recip", "log", "neg_log1m", "step", "wave_bound"}
+    assert set(got) == {"recip", "log", "neg_log1m", "step", "wave_bound", "segments"}
     assert all(v <= 1.0 for v in got.values()), got
